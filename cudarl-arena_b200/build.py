@@ -1,6 +1,6 @@
 """Build recipe for the native pieces: explicit nvcc / g++ command lines, outputs in-tree.
 
-  libcudarl.so          cudarl-arena_b200/csrc/{kernels.cu,context.cu,update_static.cu,facade.cpp}  (sm_100a only)
+  libcudarl.so          cudarl-arena_b200/csrc/*.cu, facade.cpp  (sm_100a only)
   cudarl_core*.so       pybind11 module with the reference's `cudarl_core` surface
   oracle/liboracle.so   the CPU oracle (test infrastructure)
   oracle/_ref/libref.so the reference's own kernels, compiled from the reference checkout when it
@@ -58,13 +58,13 @@ def _run(cmd, log=None):
 
 
 def build_lib(force=False):
-    srcs = [os.path.join(CSRC, f) for f in ("kernels.cu", "tile_engine.cu", "context.cu", "update_static.cu", "facade.cpp")]
-    deps = srcs + [os.path.join(CSRC, "kernels.cuh"), os.path.join(CSRC, "rules.cuh"), os.path.join(CSRC, "facade.h"), os.path.join(ROOT, "include", "cudarl.h")]
+    srcs = [os.path.join(CSRC, f) for f in ("kernels.cu", "tile_engine.cu", "context.cu", "update_static.cu", "hostio.cpp", "facade.cpp")]
+    deps = srcs + [os.path.join(CSRC, "kernels.cuh"), os.path.join(CSRC, "rules.cuh"), os.path.join(CSRC, "hostio.h"), os.path.join(CSRC, "internal.h"), os.path.join(CSRC, "facade.h"), os.path.join(ROOT, "include", "cudarl.h")]
     deps = [d for d in deps if os.path.exists(d)]
     srcs = [s for s in srcs if os.path.exists(s)]
     if not force and _newer(LIB, deps):
         return LIB
-    cmd = [_nvcc()] + NVCC_FLAGS + ["-shared", "-o", LIB] + srcs + ["-I" + os.path.join(ROOT, "include"), "-ldl"]
+    cmd = [_nvcc()] + NVCC_FLAGS + ["-shared", "-o", LIB] + srcs + ["-I" + os.path.join(ROOT, "include"), "-ldl", "-lpthread"]
     _run(cmd, log=os.path.join(HERE, "build_libcudarl.log"))
     return LIB
 

@@ -5,8 +5,11 @@
 // returns an error code.
 #include "../../include/cudarl.h"
 #include "kernels.cuh"
+#include "hostio.h"
+#include "internal.h"
 #include <nccl.h>
 #include <dlfcn.h>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -70,10 +73,10 @@ struct NcclApi {
 };
 NcclApi g_nccl;
 
+__global__ void k_ctl_eval_clear(Ctl* c) { c->eval_reached = 0; c->eval_steps = 0; }
 __global__ void k_ctl_eps(Ctl* c, unsigned mode, unsigned len, unsigned long long base_k) {
     c->eps_idx = 0; c->eps_mode = mode; c->eps_len = len; c->eps_base_k = base_k;
 }
-__global__ void k_ctl_eval_clear(Ctl* c) { c->eval_reached = 0; c->eval_steps = 0; }
 
 }  // namespace
 
@@ -87,6 +90,8 @@ struct cudarl_ctx {
     void* dtraps = nullptr; size_t traps_cap = 0;
     void* dtq = nullptr;                    // ticket counters of the step kernel's tile queues
     void* dpolicy = nullptr;                // greedy policy map of the evaluation rollout (one byte per cell), allocated on first use
+    Stage stage; bool retained = false;     // pinned, mapped block: the box for small results at its head, small arrays behind it
+    HostBox* box = nullptr; unsigned ticket = 0;                                    // the box, and the last call's ticket
     // device buffers
     void *dci = nullptr, *dreward = nullptr, *ddone = nullptr;
     void *dstate[2] = {nullptr, nullptr};   // int4 {x,y,t,id} per environment, and a scratch copy of the same size
@@ -103,7 +108,7 @@ struct cudarl_ctx {
     void *dtra = nullptr, *dtrr = nullptr, *dtrd = nullptr, *dsckey = nullptr, *dscval = nullptr;
     void *dgather = nullptr;              // replica averaging: the other ranks' rows of this rank's slice
     void* dub[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr}; size_t ub_cap = 0;   // update_batch staging
-    void* dact = nullptr;                 // actions staging for the host form of step_actions
+    void* dact = nullptr;                 // actions of the host form of step_actions, where the stage is too small for them
     size_t ent_cap = 0, eps_cap = 0;
     float* h_eps = nullptr; size_t h_eps_cap = 0; cudaEvent_t ev_eps = nullptr; bool eps_inflight = false;
     float eps_fixed_cached = -1.0f; bool eps_fixed_valid = false;
@@ -246,11 +251,10 @@ int alloc_hot(cudarl_ctx* c) {
 int ensure_step_buffers(cudarl_ctx* c) {
     if (c->dreward) return 0;
     size_t N = c->p.N ? c->p.N : 1;
-    CK(cudaMalloc(&c->dreward, N * sizeof(float)));
-    CK(cudaMalloc(&c->ddone, N));
-    CK(cudaMalloc(&c->dact, N * sizeof(int)));
-    CK(cudaMemsetAsync(c->dreward, 0, N * sizeof(float), c->st));
-    CK(cudaMemsetAsync(c->ddone, 0, N, c->st));
+    CK(cudaMalloc(&c->dreward, N * sizeof(float) + 16));     // + 16: small results are copied out in 16-byte pieces
+    CK(cudaMalloc(&c->ddone, N + 16));
+    CK(cudaMemsetAsync(c->dreward, 0, N * sizeof(float) + 16, c->st));
+    CK(cudaMemsetAsync(c->ddone, 0, N + 16, c->st));
     c->p.reward = (float*)c->dreward; c->p.done = (unsigned char*)c->ddone;
     return 0;
 }
@@ -300,14 +304,39 @@ int drain_kernel_events(cudarl_ctx* c) {
     return 0;
 }
 
-// After a synchronisation: has any kernel recorded an internal failure (a copy that never landed, a full
+// Wait until the kernel launched with the current ticket has written words 0 .. last of the box.  A kernel that fails never does:
+// the stream is asked every few thousand looks whether it has stopped.
+int wait_box(cudarl_ctx* c, unsigned last = 0) {
+    for (unsigned k = 0, looks = 1u; k <= last; ++looks) {
+        const unsigned long long w = *reinterpret_cast<const volatile unsigned long long*>(&c->box->w[k]);
+        if ((unsigned)(w >> 32) == c->ticket) { ++k; continue; }
+        if ((looks & 4095u) == 0u) {
+            const cudaError_t e = cudaStreamQuery(c->st);
+            if (e == cudaErrorNotReady) continue;
+            CK(e);
+            CK(cudaStreamSynchronize(c->st));
+            const unsigned long long v = *reinterpret_cast<const volatile unsigned long long*>(&c->box->w[k]);
+            if ((unsigned)(v >> 32) != c->ticket) return fail(c, -6, "a kernel ended without handing over its results");
+        }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return 0;
+}
+inline uint32_t box32(const cudarl_ctx* c, unsigned k) { return (uint32_t)c->box->w[k]; }
+inline uint64_t box64(const cudarl_ctx* c, unsigned k) { return (uint64_t)box32(c, k) | ((uint64_t)box32(c, k + 1) << 32); }
+inline float boxf(const cudarl_ctx* c, unsigned k) { const uint32_t b = box32(c, k); float f; std::memcpy(&f, &b, 4); return f; }
+// The next kernel's hand-over: where it puts small results, and under which number it reports them.
+Handover handover(cudarl_ctx* c) { return Handover{(HostBox*)c->stage.dev, ++c->ticket}; }
+// Arrays in the stage, behind the box.
+constexpr size_t STAGE_DATA = 256, STAGE_ROOM = STAGE_BYTES - STAGE_DATA;
+inline size_t up16(size_t b) { return (b + 15) / 16 * 16; }
+
+// After the box has been posted: has any kernel recorded an internal failure (a copy that never landed, a full
 // scratch area, a record outside its tile)?  The word is sticky; the results of the context are not to be trusted.
-int check_device_error(cudarl_ctx* c) {
-    unsigned err = 0;
-    CK(cudaMemcpyAsync(&err, (const char*)c->dctl + offsetof(Ctl, error), sizeof(err), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
+int check_posted_error(cudarl_ctx* c) {
+    const unsigned err = box32(c, 0);
     if (err) return fail(c, CUDARL_ERR_DEVICE + (int)err, "device error bits " + std::to_string(err) +
-                         ((err & ERR_COPY_TIMEOUT) ? " (a tile copy did not land within its wait bound)" : "") +
+                         ((err & ERR_COPY_TIMEOUT) ? " (a wait of a kernel ran out)" : "") +
                          ((err & ERR_SCRATCH_OVERFLOW) ? " (scratch area full)" : "") + ((err & ERR_BAD_STATE) ? " (a record outside its tile or the grid)" : "") +
                          ((err & ERR_CHAIN_CYCLE) ? " (update_batch chain longer than the batch)" : ""));
     if (c->comm && g_nccl.CommGetAsyncError) {               // a collective that failed after it was enqueued (a peer that went away)
@@ -317,6 +346,33 @@ int check_device_error(cudarl_ctx* c) {
             return fail(c, 2000 + (int)ar, std::string("replica averaging failed asynchronously: ") + (g_nccl.GetErrorString ? g_nccl.GetErrorString(ar) : "nccl error"));
     }
     return 0;
+}
+// Everything enqueued so far is done, the counters are in the box, and no kernel has recorded a failure.
+int wait_counters(cudarl_ctx* c) {
+    launch_post(c->p, handover(c), c->st);
+    CK(cudaGetLastError());
+    return wait_box(c, 13);
+}
+// Device arrays into the caller's: through the stage when they are small (one kernel, no copies), else through the pinned ring.
+int hand_out(cudarl_ctx* c, const Segment* segs, int n) {
+    size_t room = 0;
+    for (int k = 0; k < n; ++k) room += up16(segs[k].bytes);
+    if (room <= STAGE_ROOM && n <= 2) {
+        CopySpan spans[2]; size_t off = STAGE_DATA;
+        for (int k = 0; k < n; ++k) { spans[k] = CopySpan{segs[k].dev, c->stage.dev + off, (unsigned)segs[k].bytes}; off += up16(segs[k].bytes); }
+        launch_copy_out(c->p, spans, n, handover(c), c->st);
+        CK(cudaGetLastError());
+        { int rw = wait_box(c); if (rw) return rw; }
+        off = STAGE_DATA;
+        Segment parts[2];
+        for (int k = 0; k < n; ++k) { parts[k] = Segment{segs[k].host, c->stage.host + off, segs[k].bytes}; off += up16(segs[k].bytes); }
+        copy_host(parts, n, false);
+        return 0;
+    }
+    launch_post(c->p, handover(c), c->st);
+    CK(cudaGetLastError());
+    CK(copy_out(segs, n, c->cfg.device, c->st));
+    return wait_box(c);
 }
 
 // ---- tile engine: buffers, entering and leaving the tile layout ------------------------------------
@@ -413,6 +469,15 @@ int leave_tiles(cudarl_ctx* c) {
     launch_tile_export(c->p, c->st);
     CK(cudaGetLastError());
     c->tile_mode = false;
+    return 0;
+}
+// the records in environment order for reading; the tile regions stay as they are
+int records_in_order(cudarl_ctx* c) {
+    if (!c->tile_mode) return 0;
+    { int rc = close_kernel_segment(c); if (rc) return rc; }
+    c->p.step = (unsigned long long)c->h_step;
+    launch_tile_export(c->p, c->st);
+    CK(cudaGetLastError());
     return 0;
 }
 // re-size the tile regions from the current populations
@@ -548,6 +613,8 @@ void free_all(cudarl_ctx* c) {
                     c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dpolicy, c->dtq, c->dpeer_ptrs, c->dbarrier_word};
     for (void* b : bufs) if (b) cudaFree(b);
     if (c->h_eps) cudaFreeHost(c->h_eps);
+    stage_give(&c->stage);
+    if (c->retained) hostio_release();
     for (auto e : c->kev) cudaEventDestroy(e);
     if (c->ev_eps) cudaEventDestroy(c->ev_eps);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -611,6 +678,9 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
             CK(cudaMemsetAsync(c->dctl, 0, sizeof(Ctl), c->st));
             p.st = (int4*)c->dstate[0]; p.st2 = (int4*)c->dstate[1];
             p.ctl = (Ctl*)c->dctl;
+            hostio_retain(); c->retained = true;
+            CK(stage_take(&c->stage));
+            c->box = (HostBox*)c->stage.host;
             int r2 = ensure_entry_capacity(c, N); if (r2) return r2;
             r2 = alloc_tiles(c); if (r2) return r2;
             r2 = upload_cells(c); if (r2) return r2;
@@ -644,8 +714,8 @@ int cudarl_get_config(const cudarl_ctx* c, cudarl_config* out) { if (!c || !out)
 int cudarl_synchronize(cudarl_ctx* c) {
     if (!c) return -1;
     CK(cudaSetDevice(c->cfg.device));
-    CK(cudaStreamSynchronize(c->st));
-    return check_device_error(c);
+    { int rw = wait_counters(c); if (rw) return rw; }
+    return check_posted_error(c);
 }
 int cudarl_debug_set_copy_wait_polls(cudarl_ctx* c, int32_t polls) {
     if (!c || polls < 0) return fail(c, -1, "bad argument");
@@ -669,7 +739,7 @@ int cudarl_step_actions_device(cudarl_ctx* c, const int32_t* d_actions, float* d
     CK(cudaSetDevice(c->cfg.device));
     { int rl = leave_tiles(c); if (rl) return rl; }
     int rc = ensure_step_buffers(c); if (rc) return rc;
-    launch_step_actions(c->p, d_actions, d_rewards, d_dones, c->st);
+    launch_step_actions(c->p, d_actions, d_rewards, d_dones, Handover{}, c->st);
     CK(cudaGetLastError());
     return 0;
 }
@@ -680,24 +750,59 @@ int cudarl_step_actions(cudarl_ctx* c, const int32_t* actions, float* rewards, u
     { int rl = leave_tiles(c); if (rl) return rl; }
     int rc = ensure_step_buffers(c); if (rc) return rc;
     const size_t N = c->p.N;
-    CK(cudaMemcpyAsync(c->dact, actions, N * sizeof(int), cudaMemcpyHostToDevice, c->st));
-    launch_step_actions(c->p, (const int*)c->dact, nullptr, nullptr, c->st);
+    if (N == 0) return 0;
+    const size_t off_r = STAGE_DATA + up16(N * 4), off_d = off_r + up16(N * 4);
+    if (off_d + N <= STAGE_BYTES) {
+        // actions read, rewards and flags written by the kernel itself across the link: one launch and one wait instead of three copies
+        const Segment in{c->stage.host + STAGE_DATA, const_cast<int32_t*>(actions), N * 4};
+        copy_host(&in, 1, true);
+        launch_step_actions(c->p, (const int*)(c->stage.dev + STAGE_DATA), (float*)(c->stage.dev + off_r), c->stage.dev + off_d, handover(c), c->st);
+        CK(cudaGetLastError());
+        { int rw = wait_box(c); if (rw) return rw; }
+        Segment out[2]; int n = 0;
+        if (rewards) out[n++] = Segment{rewards, c->stage.host + off_r, N * 4};
+        if (dones) out[n++] = Segment{dones, c->stage.host + off_d, N};
+        copy_host(out, n, false);
+        return 0;
+    }
+    if (!c->dact) CK(cudaMalloc(&c->dact, N * sizeof(int)));
+    const Segment in{const_cast<int32_t*>(actions), c->dact, N * 4};
+    CK(copy_in(&in, 1, c->cfg.device, c->st));
+    launch_step_actions(c->p, (const int*)c->dact, nullptr, nullptr, Handover{}, c->st);
     CK(cudaGetLastError());
-    if (rewards) CK(cudaMemcpyAsync(rewards, c->dreward, N * sizeof(float), cudaMemcpyDeviceToHost, c->st));
-    if (dones) CK(cudaMemcpyAsync(dones, c->ddone, N, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    return 0;
+    return cudarl_get_reward_done(c, rewards, dones);
 }
 
 int cudarl_get_reward_done(cudarl_ctx* c, float* rewards, uint8_t* dones) {
     if (!c) return -1;
     CK(cudaSetDevice(c->cfg.device));
     int rc = ensure_step_buffers(c); if (rc) return rc;
-    if (rewards) CK(cudaMemcpyAsync(rewards, c->dreward, (size_t)c->p.N * sizeof(float), cudaMemcpyDeviceToHost, c->st));
-    if (dones) CK(cudaMemcpyAsync(dones, c->ddone, (size_t)c->p.N, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    return 0;
+    Segment out[2]; int n = 0;
+    if (rewards) out[n++] = Segment{rewards, c->dreward, (size_t)c->p.N * 4};
+    if (dones) out[n++] = Segment{dones, c->ddone, (size_t)c->p.N};
+    return hand_out(c, out, n);
 }
+
+}  // extern "C"
+
+namespace cudarl {
+// One environment, everything a caller of the facade asks for from one launch.
+int step_single(cudarl_ctx* c, bool reset, int32_t action, SingleStep* out) {
+    if (!c || !out || c->p.N != 1) return fail(c, -1, "bad argument");
+    CK(cudaSetDevice(c->cfg.device));
+    { int rl = leave_tiles(c); if (rl) return rl; }
+    int rc = ensure_step_buffers(c); if (rc) return rc;
+    c->p.step = (unsigned long long)c->h_step;
+    launch_step_one(c->p, action, reset, handover(c), c->st);
+    CK(cudaGetLastError());
+    { int rw = wait_box(c, 4); if (rw) return rw; }
+    if (reset) c->epoch_step = c->h_step;
+    out->x = (int32_t)box32(c, 1); out->y = (int32_t)box32(c, 2); out->reward = boxf(c, 3); out->done = box32(c, 4) != 0;
+    return check_posted_error(c);
+}
+}  // namespace cudarl
+
+extern "C" {
 
 int cudarl_train_steps(cudarl_ctx* c, int64_t n) {
     if (!c || n < 0) return fail(c, -1, "bad argument");
@@ -726,9 +831,8 @@ int cudarl_train_steps(cudarl_ctx* c, int64_t n) {
         k_ctl_eps<<<1, 1, 0, c->st>>>(c->p.ctl, 1u, (unsigned)n, 0ull);
         c->eps_mode = 1;
     } else {  // per episode: index = episodes finished / environments, resolved on the device every step
-        Ctl h; CK(cudaMemcpyAsync(&h, c->dctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->st));
-        CK(cudaStreamSynchronize(c->st));
-        unsigned long long k0 = h.episodes / (unsigned long long)c->p.N;
+        { int rw = wait_counters(c); if (rw) return rw; }
+        unsigned long long k0 = box64(c, 1) / (unsigned long long)c->p.N;
         std::vector<float> tab((size_t)n + 1);
         double e = (double)f.eps0;
         for (unsigned long long j = 0; j < k0; ++j) e *= (double)f.eps_decay;
@@ -755,7 +859,7 @@ int cudarl_set_trace(cudarl_ctx* c, int on) {
     CK(cudaSetDevice(c->cfg.device));
     if (on && !c->dtra) {
         size_t N = c->p.N ? c->p.N : 1;
-        CK(cudaMalloc(&c->dtra, N * 4)); CK(cudaMalloc(&c->dtrr, N * 4)); CK(cudaMalloc(&c->dtrd, N));
+        CK(cudaMalloc(&c->dtra, N * 4 + 16)); CK(cudaMalloc(&c->dtrr, N * 4 + 16)); CK(cudaMalloc(&c->dtrd, N + 16));
         c->p.tr_a = (int*)c->dtra; c->p.tr_r = (float*)c->dtrr; c->p.tr_d = (unsigned char*)c->dtrd;
     }
     c->trace = on != 0;
@@ -765,11 +869,11 @@ int cudarl_get_trace(cudarl_ctx* c, int32_t* a, float* r, uint8_t* d) {
     if (!c || !c->dtra) return fail(c, -2, "trace is off");
     CK(cudaSetDevice(c->cfg.device));
     const size_t N = c->p.N;
-    if (a) CK(cudaMemcpyAsync(a, c->dtra, N * 4, cudaMemcpyDeviceToHost, c->st));
-    if (r) CK(cudaMemcpyAsync(r, c->dtrr, N * 4, cudaMemcpyDeviceToHost, c->st));
-    if (d) CK(cudaMemcpyAsync(d, c->dtrd, N, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    return 0;
+    Segment out[3]; int n = 0;
+    if (a) out[n++] = Segment{a, c->dtra, N * 4};
+    if (r) out[n++] = Segment{r, c->dtrr, N * 4};
+    if (d) out[n++] = Segment{d, c->dtrd, N};
+    return hand_out(c, out, n);
 }
 
 int cudarl_eval_rollout(cudarl_ctx* c, int32_t max_steps, cudarl_eval_stats* out) {
@@ -823,16 +927,21 @@ int cudarl_update_batch(cudarl_ctx* c, int64_t n, const int32_t* sx, const int32
 int cudarl_get_state(cudarl_ctx* c, int32_t* x, int32_t* y, int32_t* t) {
     if (!c) return -1;
     CK(cudaSetDevice(c->cfg.device));
-    { int rl = leave_tiles(c); if (rl) return rl; }
-    const size_t b = (size_t)c->p.N * 4;
-    // state lives in slot order as int4 records; the export kernel writes x[N] | y[N] | t[N] in
-    // environment order into the spare copy
-    launch_export_state(c->p, c->st); CK(cudaGetLastError());
-    const char* base = (const char*)c->p.st2;
-    if (x) CK(cudaMemcpyAsync(x, base, b, cudaMemcpyDeviceToHost, c->st));
-    if (y) CK(cudaMemcpyAsync(y, base + b, b, cudaMemcpyDeviceToHost, c->st));
-    if (t) CK(cudaMemcpyAsync(t, base + 2 * b, b, cudaMemcpyDeviceToHost, c->st));
-    return check_device_error(c);
+    { int rl = records_in_order(c); if (rl) return rl; }
+    const size_t N = c->p.N, b = N * 4;
+    // the export kernel writes x[N] | y[N] | t[N] in environment order: into the stage when there is room, else into the spare copy
+    const bool small = 3 * b <= STAGE_ROOM;
+    launch_export_state(c->p, small ? (int*)(c->stage.dev + STAGE_DATA) : (int*)c->p.st2, handover(c), c->st);
+    CK(cudaGetLastError());
+    unsigned char* const base = small ? c->stage.host + STAGE_DATA : (unsigned char*)c->p.st2;
+    Segment out[3]; int n = 0;
+    if (x) out[n++] = Segment{x, base, b};
+    if (y) out[n++] = Segment{y, base + b, b};
+    if (t) out[n++] = Segment{t, base + 2 * b, b};
+    if (!small) CK(copy_out(out, n, c->cfg.device, c->st));
+    { int rw = wait_box(c); if (rw) return rw; }
+    if (small) copy_host(out, n, false);
+    return check_posted_error(c);
 }
 
 int cudarl_set_state(cudarl_ctx* c, const int32_t* x, const int32_t* y, const int32_t* t) {
@@ -845,9 +954,11 @@ int cudarl_set_state(cudarl_ctx* c, const int32_t* x, const int32_t* y, const in
     { int rl = leave_tiles(c); if (rl) return rl; }
     if (!c->dimport) CK(cudaMalloc(&c->dimport, (N ? N : 1) * 12));
     int* dx = (int*)c->dimport; int* dy = dx + N; int* dt = dy + N;
-    if (x) CK(cudaMemcpyAsync(dx, x, N * 4, cudaMemcpyHostToDevice, c->st));
-    if (y) CK(cudaMemcpyAsync(dy, y, N * 4, cudaMemcpyHostToDevice, c->st));
-    if (t) CK(cudaMemcpyAsync(dt, t, N * 4, cudaMemcpyHostToDevice, c->st));
+    Segment in[3]; int n = 0;
+    if (x) in[n++] = Segment{const_cast<int32_t*>(x), dx, N * 4};
+    if (y) in[n++] = Segment{const_cast<int32_t*>(y), dy, N * 4};
+    if (t) in[n++] = Segment{const_cast<int32_t*>(t), dt, N * 4};
+    CK(copy_in(in, n, c->cfg.device, c->st));
     launch_import_state(c->p, x ? dx : nullptr, y ? dy : nullptr, t ? dt : nullptr, c->st);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->st));
@@ -857,16 +968,17 @@ int cudarl_set_state(cudarl_ctx* c, const int32_t* x, const int32_t* y, const in
 int cudarl_get_q(cudarl_ctx* c, float* q) {
     if (!c || !q) return fail(c, -1, "null argument");
     CK(cudaSetDevice(c->cfg.device));
-    { int rl = leave_tiles(c); if (rl) return rl; }
-    CK(cudaMemcpyAsync(q, c->p.Q, (size_t)c->p.S * sizeof(float4), cudaMemcpyDeviceToHost, c->st));   // the table already is in the caller's layout
-    return check_device_error(c);
+    { int rc = close_kernel_segment(c); if (rc) return rc; }
+    const Segment out{q, c->p.Q, (size_t)c->p.S * sizeof(float4)};          // the table already is in the caller's layout
+    { int ro = hand_out(c, &out, 1); if (ro) return ro; }
+    return check_posted_error(c);
 }
 int cudarl_set_q(cudarl_ctx* c, const float* q) {
     if (!c || !q) return fail(c, -1, "null argument");
     CK(cudaSetDevice(c->cfg.device));
     { int rl = leave_tiles(c); if (rl) return rl; }
-    CK(cudaMemcpyAsync(c->p.Q, q, (size_t)c->p.S * sizeof(float4), cudaMemcpyHostToDevice, c->st));
-    CK(cudaStreamSynchronize(c->st));
+    const Segment in{const_cast<float*>(q), c->p.Q, (size_t)c->p.S * sizeof(float4)};
+    CK(copy_in(&in, 1, c->cfg.device, c->st));
     return 0;
 }
 
@@ -938,15 +1050,15 @@ int cudarl_set_legacy_clamp(cudarl_ctx* c, int on) {
 int cudarl_get_stats(cudarl_ctx* c, cudarl_stats* out) {
     if (!c || !out) return -1;
     CK(cudaSetDevice(c->cfg.device));
-    Ctl h; CK(cudaMemcpyAsync(&h, c->dctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
+    { int rw = wait_counters(c); if (rw) return rw; }
     std::memset(out, 0, sizeof(*out));
     out->steps = c->h_step; out->env_steps = c->h_step * (int64_t)c->p.N;
-    out->episodes = (int64_t)h.episodes; out->goals = (int64_t)h.goals; out->timeouts = (int64_t)h.timeouts;
-    out->conflicts = (int64_t)h.conflicts; out->long_chains = (int64_t)h.long_chains; out->chained = (int64_t)h.general;
+    out->episodes = (int64_t)box64(c, 1); out->goals = (int64_t)box64(c, 3); out->timeouts = (int64_t)box64(c, 5);
+    out->conflicts = (int64_t)box64(c, 7); out->long_chains = (int64_t)box64(c, 9); out->chained = (int64_t)box64(c, 11);
     out->reward_sum = (double)out->goals * 1.0 - 0.01 * (double)(out->env_steps - out->goals);
-    out->epsilon = c->eps_mode == 2 ? h.eps_used : c->eps_used; out->device_error = (int32_t)h.error;
-    if (h.error) return fail(c, CUDARL_ERR_DEVICE + (int)h.error, "device error bits " + std::to_string(h.error) + " (statistics filled in; the results of this context are not to be trusted)");
+    const unsigned err = box32(c, 0);
+    out->epsilon = c->eps_mode == 2 ? boxf(c, 13) : c->eps_used; out->device_error = (int32_t)err;
+    if (err) return fail(c, CUDARL_ERR_DEVICE + (int)err, "device error bits " + std::to_string(err) + " (statistics filled in; the results of this context are not to be trusted)");
     return 0;
 }
 

@@ -1,6 +1,7 @@
 // facade.cpp -- Environment / EnvironmentBridge / CudaQLearning of the reference over the C ABI.
 #include "facade.h"
 #include "../../include/cudarl.h"
+#include "internal.h"
 #include <sstream>
 #include <stdexcept>
 
@@ -46,17 +47,15 @@ void Environment::refresh_grid() {
 }
 
 void Environment::reset() {
-    check(cudarl_reset_all(ctx_), ctx_, "reset");
-    int32_t x, y;
-    check(cudarl_get_state(ctx_, &x, &y, nullptr), ctx_, "get_state");
-    x_ = x; y_ = y; reward_ = 0.0f; done_ = false;
+    cudarl::SingleStep s;
+    check(cudarl::step_single(ctx_, true, 0, &s), ctx_, "reset");
+    x_ = s.x; y_ = s.y; reward_ = 0.0f; done_ = false;
 }
 
 void Environment::step(int action) {
-    int32_t a = action, x, y; float r; uint8_t d;
-    check(cudarl_step_actions(ctx_, &a, &r, &d), ctx_, "step");       // obstacles, goals and traps are looked up on the device
-    check(cudarl_get_state(ctx_, &x, &y, nullptr), ctx_, "get_state");
-    x_ = x; y_ = y; reward_ = r; done_ = d != 0;
+    cudarl::SingleStep s;
+    check(cudarl::step_single(ctx_, false, action, &s), ctx_, "step");       // obstacles, goals and traps are looked up on the device
+    x_ = s.x; y_ = s.y; reward_ = s.reward; done_ = s.done;
 }
 
 float Environment::getCellValue(int x, int y) const {

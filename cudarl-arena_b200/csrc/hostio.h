@@ -1,0 +1,34 @@
+// hostio.h -- moving caller memory to and from the device.
+//
+// Caller buffers are pageable, and a copy the driver makes from or to pageable memory runs at the speed of ONE core copying (and, into
+// a freshly allocated array, faulting its pages in): 268 MB came back at 4.8 GB/s, with the link at 56 GB/s.  Here large copies go
+// through a ring of pinned slots: the copy engine fills a slot while several cores empty others.
+//
+// The ring, its worker threads and the pinned blocks below belong to the process, are shared by its contexts, bounded in size, and
+// given back when the last context goes.  Every function may be called from several threads at once.
+#pragma once
+#include <cuda_runtime.h>
+#include <cstddef>
+
+namespace cudarl {
+
+struct Segment { void* host; void* dev; size_t bytes; };
+
+// One pinned block mapped into the device, for the small results and inputs of a context.
+constexpr size_t STAGE_BYTES = (size_t)1 << 20;
+struct Stage { unsigned char* host = nullptr; unsigned char* dev = nullptr; };
+
+void hostio_retain();                         // one per context: keeps the process-wide parts alive
+void hostio_release();
+cudaError_t stage_take(Stage* s);             // zeroed first 256 bytes
+void stage_give(Stage* s);
+
+// Device -> host: everything enqueued on `st` before has been waited for and the data is in the caller's arrays on return.
+cudaError_t copy_out(const Segment* segs, int n, int device, cudaStream_t st);
+// Host -> device, ordered on `st`: the caller's arrays may be reused on return.
+cudaError_t copy_in(const Segment* segs, int n, int device, cudaStream_t st);
+
+// Between a stage and the caller: `dev` is the source, `host` the destination, both host memory; into_stage: the device reads it next.
+void copy_host(const Segment* segs, int n, bool into_stage);
+
+}  // namespace cudarl

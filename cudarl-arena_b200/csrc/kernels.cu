@@ -1,5 +1,5 @@
 // kernels.cu -- sm_100a kernels of the batched grid-world + tabular Q-learning path other than the fused
-// train step (tile_engine.cu): environment reset and caller-driven stepping, the greedy rollout, the
+// train step (tile_engine.cu) and the greedy rollout (rollout.cu): environment reset and caller-driven stepping, the
 // ordered TD update of caller-supplied transitions (update_batch) and table initialisation.
 //
 // Data layout in HBM (per context = per GPU):
@@ -13,7 +13,6 @@
 //   step        src/environment.cu:17-48, obstacle test src/kernels.cu:29-44, goal src/kernels.cu:56-59
 //   reset       src/environment.cu:6-14
 //   TD update   src/kernels.cu:96-114 (true max as in src/gpu/kernels.cu:36-45, src/train.py:134)
-//   first-max argmax src/q_learning.cu:196-206; greedy rollout src/train.py:262-311
 #include "kernels.cuh"
 #include "rules.cuh"
 #include <cstdio>
@@ -60,12 +59,29 @@ __global__ void k_import_state(Params p, const int* x, const int* y, const int* 
     r.w = (int)i;
     p.st[i] = r;
 }
-__global__ void k_export_state(Params p) {
+// x[N] | y[N] | t[N] in environment order, into the spare copy or straight into the mapped stage
+__global__ void k_export_state(Params p, int* __restrict__ out, Handover h) {
     unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.N) return;
-    const int4 r = p.st[i];
-    int* out = reinterpret_cast<int*>(p.st2);          // the spare copy, viewed as x[N] | y[N] | t[N]
-    out[r.w] = r.x; out[p.N + r.w] = r.y; out[2u * p.N + r.w] = r.z;
+    if (i < p.N) {
+        const int4 r = p.st[i];
+        out[r.w] = r.x; out[p.N + r.w] = r.y; out[2u * p.N + r.w] = r.z;
+    }
+    if (last_to_finish<true>(p)) box_put_error(p, h);
+}
+// Small results: device memory into mapped host memory, 16 bytes per thread and turn (both ends are 16-byte aligned, the tail is
+// copied to the next multiple of 16: every buffer of the context and the stage have that room).
+__global__ void k_copy_out(Params p, CopySpan a, CopySpan b, Handover h) {
+    const unsigned n = gridDim.x * blockDim.x, i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    for (unsigned i = i0; i * 16u < a.bytes; i += n) reinterpret_cast<uint4*>(a.dst)[i] = reinterpret_cast<const uint4*>(a.src)[i];
+    for (unsigned i = i0; i * 16u < b.bytes; i += n) reinterpret_cast<uint4*>(b.dst)[i] = reinterpret_cast<const uint4*>(b.src)[i];
+    if (last_to_finish<true>(p)) box_put_error(p, h);
+}
+__global__ void k_post(Params p, Handover h) {
+    const unsigned long long* const c[6] = {&p.ctl->episodes, &p.ctl->goals, &p.ctl->timeouts, &p.ctl->conflicts, &p.ctl->long_chains, &p.ctl->general};
+#pragma unroll
+    for (unsigned k = 0; k < 6u; ++k) if (threadIdx.x == k) box_put64(h, 1u + 2u * k, *c[k]);       // one counter per lane
+    if (threadIdx.x == 6u) box_put(h, 13u, __float_as_uint(p.ctl->eps_used));
+    if (threadIdx.x == 7u) box_put_error(p, h);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -358,24 +374,41 @@ __global__ void __launch_bounds__(BLOCK) k_fix_long2(Params p) {
 // ------------------------------------------------------------------------------------------------
 // Caller-driven step (no learning, sticky done, no auto-reset): Environment::step for all envs.
 // actions / rewards / dones are indexed by environment id.
-__global__ void k_step_actions(Params p, const int* actions, float* rewards, unsigned char* dones) {
-    unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.N) return;
-    const int4 rec = p.st[i];
-    unsigned e = (unsigned)rec.w;
-    int x = rec.x, y = rec.y;
-    unsigned s = (unsigned)y * (unsigned)p.W + (unsigned)x;
+// The record of one environment after `a`; reward and sticky done flag in `r` and `dn`.
+__device__ __forceinline__ int4 stepped(const Params& p, const int4 rec, int a, float& r, unsigned char& dn) {
+    const int x = rec.x, y = rec.y;
+    const unsigned s = (unsigned)y * (unsigned)p.W + (unsigned)x;
     unsigned cs = cw_load(p.cw, s), c2;
-    int a = actions[e];
     if (a < 0 || a > 3) a = -1;                         // any other value: no movement (src/gpu/environment.cu:31)
-    unsigned s2 = move_cell(p, x, y, s, cs, a, c2);
-    float r = (s2 == s && a >= 0) ? blocked_step_reward(p, x, y, a) : -0.01f;    // a trap charges its penalty (src/kernels.cu:61-63)
-    unsigned char dn = p.done[e];
+    const unsigned s2 = move_cell(p, x, y, s, cs, a, c2);
+    r = (s2 == s && a >= 0) ? blocked_step_reward(p, x, y, a) : -0.01f;    // a trap charges its penalty (src/kernels.cu:61-63)
     if (c2 & CW_GOAL) { r = 1.0f; dn = 1; }
-    p.st[i] = make_int4((int)(s2 % (unsigned)p.W), (int)(s2 / (unsigned)p.W), rec.z + 1, rec.w);
-    p.reward[e] = r; p.done[e] = dn;
-    if (rewards) rewards[e] = r;
-    if (dones) dones[e] = dn;
+    return make_int4((int)(s2 % (unsigned)p.W), (int)(s2 / (unsigned)p.W), rec.z + 1, rec.w);
+}
+__global__ void k_step_actions(Params p, const int* __restrict__ actions, float* __restrict__ rewards, unsigned char* __restrict__ dones, Handover h) {
+    unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < p.N) {
+        const int4 rec = p.st[i];
+        const unsigned e = (unsigned)rec.w;
+        float r; unsigned char dn = p.done[e];
+        p.st[i] = stepped(p, rec, actions[e], r, dn);
+        p.reward[e] = r; p.done[e] = dn;
+        if (rewards) rewards[e] = r;
+        if (dones) dones[e] = dn;
+    }
+    if (h.box && last_to_finish<true>(p)) box_put_error(p, h);
+}
+// A context with one environment: the action comes with the launch, everything a caller asks for goes back in the box.
+__global__ void k_step_one(Params p, int action, bool reset, Handover h) {
+    int4 rec = p.st[0];
+    float r = 0.0f; unsigned char dn = 0;
+    if (reset) {
+        const unsigned c = sample_start(p, p.env_offset + (unsigned)rec.w, p.step, TAG_START);
+        rec = make_int4((int)(c % (unsigned)p.W), (int)(c / (unsigned)p.W), 0, rec.w);
+    } else { dn = p.done[0]; rec = stepped(p, rec, action, r, dn); }
+    p.st[0] = rec; p.reward[0] = r; p.done[0] = dn;
+    box_put(h, 1u, (unsigned)rec.x); box_put(h, 2u, (unsigned)rec.y); box_put(h, 3u, __float_as_uint(r)); box_put(h, 4u, dn);
+    box_put_error(p, h);
 }
 
 // Greedy rollout of every environment from a fresh start cell.  The table does not change during a rollout, so the greedy
@@ -498,14 +531,21 @@ static inline unsigned fix_blocks(const Params& p) { unsigned b = p.mb_slots / B
 static inline unsigned sweep_blocks(unsigned S) { unsigned b = nblk((2u * S + 15u) / 16u); return b < 1u ? 1u : (b > 1184u ? 1184u : b); }
 
 void launch_identity_ids(const Params& p, cudaStream_t st) { if (p.N) k_ids_identity<<<nblk(p.N), BLOCK, 0, st>>>(p); }
-void launch_export_state(const Params& p, cudaStream_t st) { if (p.N) k_export_state<<<nblk(p.N), BLOCK, 0, st>>>(p); }
+void launch_export_state(const Params& p, int* out, Handover h, cudaStream_t st) { k_export_state<<<p.N ? nblk(p.N) : 1u, BLOCK, 0, st>>>(p, out, h); }
+void launch_copy_out(const Params& p, const CopySpan* spans, int n, Handover h, cudaStream_t st) {
+    const CopySpan none{nullptr, nullptr, 0u}, a = n > 0 ? spans[0] : none, b = n > 1 ? spans[1] : none;
+    const unsigned blocks = nblk(((a.bytes > b.bytes ? a.bytes : b.bytes) + 15u) / 16u);
+    k_copy_out<<<blocks < 1u ? 1u : (blocks > 64u ? 64u : blocks), BLOCK, 0, st>>>(p, a, b, h);
+}
+void launch_post(const Params& p, Handover h, cudaStream_t st) { k_post<<<1, 32, 0, st>>>(p, h); }
 void launch_import_state(const Params& p, const int* x, const int* y, const int* t, cudaStream_t st) { if (p.N) k_import_state<<<nblk(p.N), BLOCK, 0, st>>>(p, x, y, t); }
 void launch_reset_all(const Params& p, cudaStream_t st) {
     if (p.N) k_reset_all<<<nblk(p.N), BLOCK, 0, st>>>(p);
 }
-void launch_step_actions(const Params& p, const int* a, float* r, unsigned char* d, cudaStream_t st) {
-    if (p.N) k_step_actions<<<nblk(p.N), BLOCK, 0, st>>>(p, a, r, d);
+void launch_step_actions(const Params& p, const int* a, float* r, unsigned char* d, Handover h, cudaStream_t st) {
+    if (p.N) k_step_actions<<<nblk(p.N), BLOCK, 0, st>>>(p, a, r, d, h);
 }
+void launch_step_one(const Params& p, int action, bool reset, Handover h, cudaStream_t st) { k_step_one<<<1, 1, 0, st>>>(p, action, reset, h); }
 void launch_eval(const Params& p, unsigned char* policy, int max_steps, unsigned long long nonce, cudaStream_t st) {
     if (!p.N) return;
     k_eval_policy<<<nblk(p.S) < 4736u ? nblk(p.S) : 4736u, BLOCK, 0, st>>>(p, policy);

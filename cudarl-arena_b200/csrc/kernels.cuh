@@ -22,7 +22,8 @@ constexpr unsigned LINK_POS_MASK = (1u << LINK_POS_BITS) - 1u;
 // ---- control block in device memory ------------------------------------------------------------
 struct Ctl {
     unsigned long long episodes, goals, timeouts, conflicts, long_chains;
-    unsigned long long eval_reached, eval_steps;
+    unsigned long long eval_reached, eval_steps;   // sums of a running rollout; zero between rollouts
+    unsigned int done_blocks;       // blocks of a kernel that hands results to the host: those that have written theirs; zero between kernels
     unsigned long long general;     // environment-steps that went through the entry/chain path
     unsigned int eps_idx;           // index of the current step's epsilon in the table
     unsigned int eps_mode;          // 0 fixed index, 1 advance by one per step, 2 per-episode index
@@ -37,6 +38,14 @@ struct Ctl {
 };
 
 enum : unsigned { ERR_SCRATCH_OVERFLOW = 1u, ERR_BAD_STATE = 2u, ERR_CHAIN_CYCLE = 8u, ERR_COPY_TIMEOUT = 32u };   // = CUDARL_DEVERR_* of cudarl.h
+
+// ---- results handed to the host without a copy ---------------------------------------------------
+// One per context, at the head of its pinned, mapped stage block.  A word carries 32 bits of a result and, above them, the number of
+// the call it belongs to: the host waits for each word it needs by its number, so the words need no order among themselves and no
+// fence (launch to seen result 7.3 us on the B200 box, 9.3 with values, fence and flag, 9 - 10 for a copy or a synchronisation of
+// the stream).  Word 0 carries Ctl::error and is also the flag behind arrays in the stage, which do take a fence.
+struct HostBox { unsigned long long w[32]; };
+struct Handover { HostBox* box; unsigned ticket; };              // box == nullptr: nothing to hand over
 
 // ---- tile engine (tile_engine.cu): the layout the train step runs on ---------------------------
 // The grid is cut into T x T tiles (T = 16 or 8); one WARP steps one tile at a time.  The table is a single
@@ -114,14 +123,18 @@ constexpr int BLOCK = 256;
 
 // launch wrappers (kernels.cu); all asynchronous on `st`
 void launch_identity_ids(const Params& p, cudaStream_t st);
-void launch_export_state(const Params& p, cudaStream_t st);       // st2 viewed as x[N]|y[N]|t[N] in environment order
+void launch_export_state(const Params& p, int* out, Handover h, cudaStream_t st);                 // out = x[N]|y[N]|t[N] in environment order
+struct CopySpan { const void* src; void* dst; unsigned bytes; };
+void launch_copy_out(const Params& p, const CopySpan* spans, int n, Handover h, cudaStream_t st); // up to two spans of device memory into mapped host memory
+void launch_post(const Params& p, Handover h, cudaStream_t st);                                   // words 1.. = the counters of the control block, in the order of cudarl_stats, low half first; then epsilon
 void launch_import_state(const Params& p, const int* x, const int* y, const int* t, cudaStream_t st);
 void launch_reset_all(const Params& p, cudaStream_t st);
-void launch_step_actions(const Params& p, const int* d_actions, float* d_rewards, unsigned char* d_dones, cudaStream_t st);
-void launch_eval(const Params& p, unsigned char* policy, int max_steps, unsigned long long nonce, cudaStream_t st);   // policy: one byte per cell, scratch
+void launch_step_actions(const Params& p, const int* d_actions, float* d_rewards, unsigned char* d_dones, Handover h, cudaStream_t st);
+void launch_step_one(const Params& p, int action, bool reset, Handover h, cudaStream_t st);        // one environment: words 1-4 = x, y, reward bits, done
 void launch_update_batch(const Params& p, unsigned n, const int* sx, const int* sy, const int* a, const float* r,
                          const int* nx, const int* ny, const unsigned char* dn, cudaStream_t st);
 void launch_q_init(const Params& p, int kind, float scale, cudaStream_t st);
+void launch_eval(const Params& p, unsigned char* policy, int max_steps, unsigned long long nonce, cudaStream_t st);   // policy: one byte per cell, scratch
 // tile engine (tile_engine.cu)
 size_t tile_step_smem(const Params& p);
 int  tile_engine_configure(Params& p, int device);                  // opt in to the dynamic shared memory the step needs; sets tp.grid

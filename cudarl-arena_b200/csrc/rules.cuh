@@ -37,6 +37,32 @@ __device__ __forceinline__ float u01(unsigned w) { return (float)(w >> 8) * 5.96
 
 __device__ __forceinline__ unsigned cw_load(const unsigned short* cw, unsigned cell) { return cw[cell]; }
 
+// The move byte of a cell (written by k_te_cls, tile by tile): bit a = a move in direction a is blocked, bit 4+a = the cell an
+// environment stands on after choosing a is a goal.
+__device__ __forceinline__ unsigned move_byte(const TileP& tp, int x, int y) {
+    const unsigned m = tp.T - 1u, tile = ((unsigned)y >> tp.tshift) * tp.tiles_x + ((unsigned)x >> tp.tshift);
+    return __ldg(tp.tcls + (size_t)tile * tp.cls_stride + ((((unsigned)y & m) << tp.tshift) | ((unsigned)x & m)));
+}
+
+__device__ __forceinline__ void box_put(const Handover& h, unsigned k, unsigned v) {
+    *reinterpret_cast<volatile unsigned long long*>(&h.box->w[k]) = ((unsigned long long)h.ticket << 32) | v;
+}
+__device__ __forceinline__ void box_put64(const Handover& h, unsigned k, unsigned long long v) { box_put(h, k, (unsigned)v); box_put(h, k + 1u, (unsigned)(v >> 32)); }
+__device__ __forceinline__ void box_put_error(const Params& p, const Handover& h) { box_put(h, 0u, *reinterpret_cast<volatile unsigned*>(&p.ctl->error)); }
+// To be called by all threads of every block, after their writes: true in one thread of the last block to get here, which sees what
+// the other blocks have written -- and, when HOST, after which the host sees it too (arrays in the stage).
+template <bool HOST>
+__device__ __forceinline__ bool last_to_finish(const Params& p) {
+    __syncthreads();
+    if (threadIdx.x != 0u) return false;
+    if (HOST) __threadfence_system(); else __threadfence();
+    if (gridDim.x == 1u) return true;
+    if (atomicAdd(&p.ctl->done_blocks, 1u) + 1u != gridDim.x) return false;
+    if (HOST) __threadfence_system(); else __threadfence();
+    p.ctl->done_blocks = 0u;
+    return true;
+}
+
 // Start cell of an episode.  CENTRE/FIXED: the configured cell (reference: src/environment.cu:9-10).
 // RANDOM: first free non-goal cell among 64 seeded candidates, else the precomputed fallback cell.
 __device__ __forceinline__ unsigned sample_start(const Params& p, unsigned gi, unsigned long long nonce, unsigned tag) {
