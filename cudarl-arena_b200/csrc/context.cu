@@ -73,7 +73,6 @@ struct NcclApi {
 };
 NcclApi g_nccl;
 
-__global__ void k_ctl_eval_clear(Ctl* c) { c->eval_reached = 0; c->eval_steps = 0; }
 __global__ void k_ctl_eps(Ctl* c, unsigned mode, unsigned len, unsigned long long base_k) {
     c->eps_idx = 0; c->eps_mode = mode; c->eps_len = len; c->eps_base_k = base_k;
 }
@@ -89,7 +88,7 @@ struct cudarl_ctx {
     std::map<uint32_t, float> traps;      // cell -> penalty; mirrored on the device as a table sorted by cell
     void* dtraps = nullptr; size_t traps_cap = 0;
     void* dtq = nullptr;                    // ticket counters of the step kernel's tile queues
-    void* dpolicy = nullptr;                // greedy policy map of the evaluation rollout (one byte per cell), allocated on first use
+    void* dhop = nullptr;                   // folded greedy policy of the evaluation rollout (one word per cell), allocated on first use
     Stage stage; bool retained = false;     // pinned, mapped block: the box for small results at its head, small arrays behind it
     HostBox* box = nullptr; unsigned ticket = 0;                                    // the box, and the last call's ticket
     // device buffers
@@ -610,7 +609,7 @@ void free_all(cudarl_ctx* c) {
                     c->dtra, c->dtrr, c->dtrd, c->dsckey, c->dscval, c->dgather, c->dact,
                     c->dub[0], c->dub[1], c->dub[2], c->dub[3], c->dub[4], c->dub[5], c->dub[6],
                     c->dQ, c->drec[0], c->drec[1], c->darr[0], c->darr[1], c->dovf[0], c->dovf[1], c->dbmax[0], c->dbmax[1],
-                    c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dpolicy, c->dtq, c->dpeer_ptrs, c->dbarrier_word};
+                    c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dhop, c->dtq, c->dpeer_ptrs, c->dbarrier_word};
     for (void* b : bufs) if (b) cudaFree(b);
     if (c->h_eps) cudaFreeHost(c->h_eps);
     stage_give(&c->stage);
@@ -879,16 +878,16 @@ int cudarl_get_trace(cudarl_ctx* c, int32_t* a, float* r, uint8_t* d) {
 int cudarl_eval_rollout(cudarl_ctx* c, int32_t max_steps, cudarl_eval_stats* out) {
     if (!c || !out || max_steps < 0) return fail(c, -1, "bad argument");
     CK(cudaSetDevice(c->cfg.device));
-    { int rl = leave_tiles(c); if (rl) return rl; }
-    if (c->cls_dirty) { launch_tile_classes(c->p, c->st); c->cls_dirty = false; }       // the rollout reads the per-tile move bytes
-    k_ctl_eval_clear<<<1, 1, 0, c->st>>>(c->p.ctl);
-    if (!c->dpolicy) CK(cudaMalloc(&c->dpolicy, c->p.S));                                // one byte per cell, kept until the context goes
-    launch_eval(c->p, (unsigned char*)c->dpolicy, max_steps, (unsigned long long)c->eval_calls, c->st);
-    CK(cudaGetLastError());
-    Ctl h; CK(cudaMemcpyAsync(&h, c->dctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
+    out->envs = c->p.N; out->reached = 0; out->total_steps = 0;
+    if (c->p.N) {                                        // the records stay where they are: a rollout reads the table and the grid only
+        if (c->cls_dirty) { launch_tile_classes(c->p, c->st); c->cls_dirty = false; }       // it reads the per-tile move bytes
+        if (!c->dhop) CK(cudaMalloc(&c->dhop, (size_t)c->p.S * sizeof(unsigned)));           // kept until the context goes
+        launch_rollout(c->p, (unsigned*)c->dhop, (unsigned)max_steps, (unsigned long long)c->eval_calls, handover(c), c->st);
+        CK(cudaGetLastError());
+        { int rw = wait_box(c, 4); if (rw) return rw; }
+        out->reached = (int64_t)box64(c, 1); out->total_steps = (int64_t)box64(c, 3);
+    }
     c->eval_calls += 1;
-    out->envs = c->p.N; out->reached = (int64_t)h.eval_reached; out->total_steps = (int64_t)h.eval_steps;
     out->reward_sum = (double)out->reached * 1.0 - 0.01 * (double)(out->total_steps - out->reached);
     return 0;
 }

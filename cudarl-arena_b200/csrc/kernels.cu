@@ -411,61 +411,6 @@ __global__ void k_step_one(Params p, int action, bool reset, Handover h) {
     box_put_error(p, h);
 }
 
-// Greedy rollout of every environment from a fresh start cell.  The table does not change during a rollout, so the greedy
-// policy is folded into one byte per cell first (k_eval_policy: bits 0-1 the first-max action, bit 2 "that move is blocked",
-// bit 3 "it ends on a goal") -- one pass over the table -- and the rollout itself walks that map: one byte per step instead
-// of a 16-byte row and a move byte, and the map (one byte per cell) stays in L2.  Positions stay in registers, so the whole
-// rollout is one launch; every thread walks four environments, so that four dependent chains of loads overlap.
-__global__ void __launch_bounds__(BLOCK) k_eval_policy(Params p, unsigned char* __restrict__ pol) {
-    const TileP& tp = p.tp;
-    for (unsigned s = blockIdx.x * BLOCK + threadIdx.x; s < p.S; s += gridDim.x * BLOCK) {
-        const unsigned y = s / (unsigned)p.W, x = s - y * (unsigned)p.W;
-        const unsigned tile = (y >> tp.tshift) * tp.tiles_x + (x >> tp.tshift);
-        const float4 row = __ldcs(p.Q + s);
-        const unsigned mvb = __ldg(tp.tcls + (size_t)tile * tp.cls_stride + (((y & (tp.T - 1u)) << tp.tshift) | (x & (tp.T - 1u))));
-        const int a = argmax4(row);
-        pol[s] = (unsigned char)((unsigned)a | (((mvb >> a) & 1u) << 2) | (((mvb >> (4 + a)) & 1u) << 3));
-    }
-}
-constexpr int EVAL_EPT = 4;     // environments per thread
-__global__ void __launch_bounds__(BLOCK) k_eval(Params p, const unsigned char* __restrict__ pol, int max_steps, unsigned long long nonce) {
-    __shared__ unsigned s_reached; __shared__ unsigned long long s_steps;
-    if (threadIdx.x == 0) { s_reached = 0; s_steps = 0; }
-    __syncthreads();
-    const unsigned part = (p.N + (unsigned)EVAL_EPT - 1u) / (unsigned)EVAL_EPT;
-    const unsigned i0 = blockIdx.x * BLOCK + threadIdx.x;
-    if (i0 < part) {
-        unsigned pos[EVAL_EPT]; unsigned live = 0u, reached = 0u, steps = 0u;
-#pragma unroll
-        for (int k = 0; k < EVAL_EPT; ++k) {
-            const unsigned i = i0 + (unsigned)k * part;
-            if (i < p.N) live |= 1u << k;
-            pos[k] = i < p.N ? sample_start(p, p.env_offset + i, nonce, TAG_EVAL) : 0u;
-        }
-        for (int it = 0; it < max_steps && live; ++it) {
-            unsigned b[EVAL_EPT];
-#pragma unroll
-            for (int k = 0; k < EVAL_EPT; ++k) b[k] = __ldg(pol + pos[k]);
-#pragma unroll
-            for (int k = 0; k < EVAL_EPT; ++k) {
-                if (!((live >> k) & 1u)) continue;
-                const unsigned a = b[k] & 3u;
-                // per action the step in cells: up -W, right +1, down +W, left -1; none when the move is blocked
-                if (!(b[k] & 4u)) pos[k] += a == 0u ? 0u - (unsigned)p.W : a == 1u ? 1u : a == 2u ? (unsigned)p.W : 0u - 1u;
-                ++steps;
-                if (b[k] & 8u) { ++reached; live &= ~(1u << k); }
-            }
-        }
-        if (reached) atomicAdd(&s_reached, reached);
-        atomicAdd(&s_steps, (unsigned long long)steps);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (s_reached) atomicAdd(&p.ctl->eval_reached, (unsigned long long)s_reached);
-        if (s_steps) atomicAdd(&p.ctl->eval_steps, s_steps);
-    }
-}
-
 __global__ void k_active_reset(Params p) { p.ctl->active_count[p.step & 1ull] = 0; p.ctl->long_count[p.step & 1ull] = 0; p.ctl->long2_count[p.step & 1ull] = 0; }
 
 // update_batch, phase 1: TD target of every transition from the table as it is now; every
@@ -546,11 +491,6 @@ void launch_step_actions(const Params& p, const int* a, float* r, unsigned char*
     if (p.N) k_step_actions<<<nblk(p.N), BLOCK, 0, st>>>(p, a, r, d, h);
 }
 void launch_step_one(const Params& p, int action, bool reset, Handover h, cudaStream_t st) { k_step_one<<<1, 1, 0, st>>>(p, action, reset, h); }
-void launch_eval(const Params& p, unsigned char* policy, int max_steps, unsigned long long nonce, cudaStream_t st) {
-    if (!p.N) return;
-    k_eval_policy<<<nblk(p.S) < 4736u ? nblk(p.S) : 4736u, BLOCK, 0, st>>>(p, policy);
-    k_eval<<<nblk((p.N + (unsigned)EVAL_EPT - 1u) / (unsigned)EVAL_EPT), BLOCK, 0, st>>>(p, policy, max_steps, nonce);
-}
 void launch_update_batch(const Params& p, unsigned n, const int* sx, const int* sy, const int* a, const float* r,
                          const int* nx, const int* ny, const unsigned char* dn, cudaStream_t st) {
     if (!n) return;

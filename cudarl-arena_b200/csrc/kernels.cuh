@@ -134,7 +134,8 @@ void launch_step_one(const Params& p, int action, bool reset, Handover h, cudaSt
 void launch_update_batch(const Params& p, unsigned n, const int* sx, const int* sy, const int* a, const float* r,
                          const int* nx, const int* ny, const unsigned char* dn, cudaStream_t st);
 void launch_q_init(const Params& p, int kind, float scale, cudaStream_t st);
-void launch_eval(const Params& p, unsigned char* policy, int max_steps, unsigned long long nonce, cudaStream_t st);   // policy: one byte per cell, scratch
+// greedy rollout (rollout.cu); hop: one word per cell, scratch; words 1-4 = environments that reached a goal, steps taken, low halves first
+void launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st);
 // tile engine (tile_engine.cu)
 size_t tile_step_smem(const Params& p);
 int  tile_engine_configure(Params& p, int device);                  // opt in to the dynamic shared memory the step needs; sets tp.grid
