@@ -9,6 +9,7 @@
 #include "internal.h"
 #include <nccl.h>
 #include <dlfcn.h>
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -100,6 +101,10 @@ struct cudarl_ctx {
     void *dQ = nullptr;                    // the table (padded so that it splits into equal slices for any number of ranks)
     void *drec[2] = {nullptr, nullptr}, *darr[2] = {nullptr, nullptr}, *dovf[2] = {nullptr, nullptr}, *dbmax[2] = {nullptr, nullptr};
     void *dtmeta = nullptr, *dtscratch = nullptr, *dtcls = nullptr;   // per-tile regions / counters; 32-bit counters of crowded tiles
+    // gather engine
+    bool gather = false;                   // the engine of this context's train steps: gather, or the tiles
+    void *dgbar = nullptr, *dgcnt = nullptr, *dgmv = nullptr, *dgown = nullptr, *dgdv = nullptr;
+    uint32_t barrier_base = 0;             // arrivals at the grid barrier by all launches so far
     bool tile_mode = false;               // true: the records live in tile regions (train steps), false: in environment order
     bool cls_dirty = true;                // the per-tile class bytes must be rebuilt from the cell words
     int64_t bucket_every = 256, since_bucket = 0;
@@ -404,9 +409,6 @@ int make_table_map(cudarl_ctx* c) {
 int alloc_tiles(cudarl_ctx* c) {
     Params& p = c->p; TileP& tp = p.tp;
     const size_t S = p.S, N = p.N ? p.N : 1;
-    CK(cudaMalloc(&c->dQ, (S + 64) * sizeof(float4)));
-    CK(cudaMemsetAsync(c->dQ, 0, (S + 64) * sizeof(float4), c->st));
-    p.Q = (float4*)c->dQ;
     const size_t nt16 = (((size_t)p.W + 15) >> 4) * (((size_t)p.H + 15) >> 4);
     unsigned tsh = (N / nt16 <= 104) ? 4u : 3u;
     if (c->cfg.tile_edge == 8) tsh = 3u; else if (c->cfg.tile_edge == 16) tsh = 4u;
@@ -449,11 +451,48 @@ int alloc_tiles(cudarl_ctx* c) {
     return 0;
 }
 
+int alloc_table(cudarl_ctx* c) {
+    const size_t S = c->p.S;
+    CK(cudaMalloc(&c->dQ, (S + 64) * sizeof(float4)));
+    CK(cudaMemsetAsync(c->dQ, 0, (S + 64) * sizeof(float4), c->st));
+    c->p.Q = (float4*)c->dQ;
+    return 0;
+}
+// The gather engine where its scattered accesses stay in L2 (a table of up to 32 MB), or are few whatever the size of the grid: up
+// to 262,144 environments; the tile engine streams the table, 16 bytes per cell, however few there are.  An explicit tile edge asks for tiles.
+bool use_gather(const cudarl_ctx* c) {
+    const cudarl_config& f = c->cfg;
+    if (f.tile_edge != 0) return false;
+    return c->p.S <= (1u << 21) || c->p.N <= (1u << 18);
+}
+int alloc_gather(cudarl_ctx* c) {
+    Params& p = c->p; GatherP& gp = p.gp;
+    const size_t S = p.S, N = p.N ? p.N : 1;
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
+    CK(cudaMalloc(&c->dgbar, 256)); CK(cudaMemsetAsync(c->dgbar, 0, 256, c->st));
+    CK(cudaMalloc(&c->dgcnt, 8 * S * sizeof(unsigned))); CK(cudaMemsetAsync(c->dgcnt, 0, 8 * S * sizeof(unsigned), c->st));
+    CK(cudaMalloc(&c->dgmv, S));
+    gather_plan(p, sms);
+    gp.barrier = (unsigned*)c->dgbar;
+    gp.cnt[0] = (unsigned*)c->dgcnt; gp.cnt[1] = gp.cnt[0] + 4 * S;
+    gp.mv = (unsigned char*)c->dgmv;
+    if (gp.stream) { CK(cudaMalloc(&c->dgown, N * sizeof(unsigned))); CK(cudaMalloc(&c->dgdv, N * sizeof(float2))); gp.own = (unsigned*)c->dgown; gp.dv = (float2*)c->dgdv; }
+    return 0;
+}
+
+// the move bytes of the engine in use, after a change of the grid
+void refresh_moves(cudarl_ctx* c) {
+    if (!c->cls_dirty) return;
+    if (c->gather) launch_gather_moves(c->p, c->st); else launch_tile_classes(c->p, c->st);
+    c->cls_dirty = false;
+}
+
 // records in environment order -> tile regions; border values from the table as it is now
 int enter_tiles(cudarl_ctx* c) {
     if (c->tile_mode) return 0;
     c->p.step = (unsigned long long)c->h_step;
-    if (c->cls_dirty) { launch_tile_classes(c->p, c->st); c->cls_dirty = false; }
+    refresh_moves(c);
     launch_tile_bucket(c->p, c->st);
     launch_tile_border(c->p, c->st);
     CK(cudaGetLastError());
@@ -574,7 +613,39 @@ int average_now(cudarl_ctx* c) {
     return 0;
 }
 
+// Start counting an uninterrupted run of step kernels, when they are timed.
+int open_kernel_segment(cudarl_ctx* c) {
+    if (!c->ktiming || c->kseg_open) return 0;
+    if (c->kev_used + 2 > c->kev.size()) { int rc = drain_kernel_events(c); if (rc) return rc; }
+    CK(cudaEventRecord(c->kev[c->kev_used], c->st));
+    c->kseg_open = true; c->kseg_count = 0;
+    return 0;
+}
+
+// n steps in launches of many: up to the next averaging of the replicas, and not so many that a launch keeps the GPU for long or
+// that a block's 32-bit sums could overflow.
+int run_gather(cudarl_ctx* c, int64_t n) {
+    refresh_moves(c);
+    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(4096, (int64_t)(0x7FFFFFFFu / (c->p.N ? c->p.N : 1u))));
+    for (int64_t k = 0; k < n;) {
+        int64_t m = std::min(n - k, most);
+        if (c->cfg.sync_every > 0 && c->comm) m = std::min<int64_t>(m, c->cfg.sync_every - c->h_step % c->cfg.sync_every);
+        { int rc = open_kernel_segment(c); if (rc) return rc; }
+        c->p.step = (unsigned long long)c->h_step;
+        c->p.eps_idx = c->eps_mode == 1 ? (unsigned)k : 0u;
+        GatherLaunch l{};
+        l.steps = (unsigned)m; l.chunk = c->p.gp.chunk; l.barrier_base = c->barrier_base; l.eps_mode = c->eps_mode; l.trace = c->trace ? 1 : 0;
+        CK(launch_gather_steps(c->p, l, c->st));
+        c->barrier_base += c->p.gp.grid * gather_barriers(l.steps);
+        c->h_step += m; c->kseg_count += m; k += m;
+        if (c->eps_mode != 2 && c->h_eps) c->eps_used = c->h_eps[c->eps_mode == 1 ? k - 1 : 0];
+        if (c->cfg.sync_every > 0 && c->comm && (c->h_step % c->cfg.sync_every) == 0) { int rc = average_now(c); if (rc) return rc; }
+    }
+    return close_kernel_segment(c);
+}
+
 int run_steps(cudarl_ctx* c, int64_t n) {
+    if (c->gather) return run_gather(c, n);
     { int re = enter_tiles(c); if (re) return re; }
     for (int64_t k = 0; k < n; ++k) {
         if (c->bucket_every > 0 && c->since_bucket >= c->bucket_every) { int rs = rebucket_tiles(c); if (rs) return rs; }
@@ -583,11 +654,7 @@ int run_steps(cudarl_ctx* c, int64_t n) {
         // list that every tile would have to filter.  Re-bucketing now puts them into regions instead (same results either way).
         if (c->bucket_every > 0 && c->cfg.max_steps > 0 && c->since_bucket > 0 && c->h_step > c->epoch_step &&
             (c->h_step - c->epoch_step) % c->cfg.max_steps == 0) { int rs = rebucket_tiles(c); if (rs) return rs; }
-        if (c->ktiming && !c->kseg_open) {
-            if (c->kev_used + 2 > c->kev.size()) { int rc = drain_kernel_events(c); if (rc) return rc; }
-            CK(cudaEventRecord(c->kev[c->kev_used], c->st));
-            c->kseg_open = true; c->kseg_count = 0;
-        }
+        { int rc = open_kernel_segment(c); if (rc) return rc; }
         c->p.step = (unsigned long long)c->h_step;
         c->p.eps_idx = c->eps_mode == 1 ? (unsigned)k : 0u;
         c->p.eps_from_ctl = c->eps_mode == 2 ? 1 : 0;
@@ -609,7 +676,7 @@ void free_all(cudarl_ctx* c) {
                     c->dtra, c->dtrr, c->dtrd, c->dsckey, c->dscval, c->dgather, c->dact,
                     c->dub[0], c->dub[1], c->dub[2], c->dub[3], c->dub[4], c->dub[5], c->dub[6],
                     c->dQ, c->drec[0], c->drec[1], c->darr[0], c->darr[1], c->dovf[0], c->dovf[1], c->dbmax[0], c->dbmax[1],
-                    c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dhop, c->dtq, c->dpeer_ptrs, c->dbarrier_word};
+                    c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dhop, c->dtq, c->dpeer_ptrs, c->dbarrier_word, c->dgbar, c->dgcnt, c->dgmv, c->dgown, c->dgdv};
     for (void* b : bufs) if (b) cudaFree(b);
     if (c->h_eps) cudaFreeHost(c->h_eps);
     stage_give(&c->stage);
@@ -681,7 +748,9 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
             CK(stage_take(&c->stage));
             c->box = (HostBox*)c->stage.host;
             int r2 = ensure_entry_capacity(c, N); if (r2) return r2;
-            r2 = alloc_tiles(c); if (r2) return r2;
+            r2 = alloc_table(c); if (r2) return r2;
+            c->gather = use_gather(c);
+            r2 = c->gather ? alloc_gather(c) : alloc_tiles(c); if (r2) return r2;
             r2 = upload_cells(c); if (r2) return r2;
             launch_q_init(p, f->q_init_kind, f->q_init_scale, c->st);
             float e0 = (float)f->eps0; r2 = upload_eps(c, &e0, 1); if (r2) return r2;
@@ -880,7 +949,7 @@ int cudarl_eval_rollout(cudarl_ctx* c, int32_t max_steps, cudarl_eval_stats* out
     CK(cudaSetDevice(c->cfg.device));
     out->envs = c->p.N; out->reached = 0; out->total_steps = 0;
     if (c->p.N) {                                        // the records stay where they are: a rollout reads the table and the grid only
-        if (c->cls_dirty) { launch_tile_classes(c->p, c->st); c->cls_dirty = false; }       // it reads the per-tile move bytes
+        refresh_moves(c);                                // it reads the move bytes
         if (!c->dhop) CK(cudaMalloc(&c->dhop, (size_t)c->p.S * sizeof(unsigned)));           // kept until the context goes
         launch_rollout(c->p, (unsigned*)c->dhop, (unsigned)max_steps, (unsigned long long)c->eval_calls, handover(c), c->st);
         CK(cudaGetLastError());

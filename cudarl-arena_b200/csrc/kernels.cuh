@@ -79,6 +79,17 @@ struct TileP {
     CUtensorMap tmq;           // the table as a 2-D tensor of floats (4W x H), box 4T x T: one copy instruction per tile
 };
 
+// ---- gather engine (gather_engine.cu): many train steps per launch, for tables that stay in L2 -----
+struct GatherP {
+    unsigned* barrier;         // arrivals of all blocks of all launches so far (wraps)
+    unsigned* cnt[2];          // 4 S counters: environments on a (cell, action) in this step, by step parity; zero between launches
+    unsigned char* mv;         // S move bytes
+    unsigned* own;             // N: streamed populations: the (cell, action) an environment owns in this step,
+    float2* dv;                // N: and its TD target and value
+    unsigned ept, chunk, grid, stream;      // environments per thread and turn, per block; blocks; whether the population is streamed
+};
+struct GatherLaunch { unsigned steps, chunk, barrier_base; int eps_mode, trace; };
+
 // ---- everything a kernel needs, passed by value ------------------------------------------------
 struct Params {
     int W, H;
@@ -117,6 +128,7 @@ struct Params {
     unsigned eps_idx;          // index of this step's epsilon in eps_tab
     int eps_from_ctl;          // 1: take the index from ctl (per-episode schedule)
     TileP tp;
+    GatherP gp;
 };
 
 constexpr int BLOCK = 256;
@@ -145,6 +157,11 @@ void launch_tile_export(const Params& p, cudaStream_t st);         // tile regio
 void launch_tile_step(const Params& p, bool trace, cudaStream_t st);
 unsigned tile_cls_stride(unsigned tshift);                         // bytes of one tile's class block
 void launch_tile_border(const Params& p, cudaStream_t st);         // border array of parity p.step & 1 from the table (after any change of the table outside train steps)
+// gather engine (gather_engine.cu)
+void gather_plan(Params& p, int sms);
+unsigned gather_barriers(unsigned steps);                           // arrivals per block of a launch of so many steps
+void launch_gather_moves(const Params& p, cudaStream_t st);         // cell words -> move bytes
+cudaError_t launch_gather_steps(const Params& p, const GatherLaunch& l, cudaStream_t st);
 // Replica averaging, the slice this rank owns: table[cell0 + i] = (sum over ranks 0..R-1 in that order) / R, where rank `self`'s
 // rows are the table's own and the other ranks' rows lie in `others` (R - 1 slices of n rows, ascending rank).
 void launch_q_average_peers(float4* const* tables, unsigned R, unsigned self, size_t cell0, size_t n, float scale, cudaStream_t st);

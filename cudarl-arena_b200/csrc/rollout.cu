@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(RT_THREADS) k_rollout_tiles(const __grid_const
         unsigned w = KIND_LIVE | ic;
         if (x < p.W && y < p.H) {
             const float4 row = __ldcs(p.Q + (size_t)y * (size_t)p.W + (size_t)x);
-            const unsigned mvb = move_byte(p.tp, x, y);
+            const unsigned mvb = move_byte(p, x, y);
             const unsigned a = (unsigned)argmax4(row);
             if ((mvb >> (4u + a)) & 1u) w = KIND_GOAL | 1u;
             else if (!((mvb >> a) & 1u)) {

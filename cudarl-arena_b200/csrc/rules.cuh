@@ -12,6 +12,8 @@
 namespace cudarl {
 
 constexpr unsigned FULL = 0xFFFFFFFFu;
+constexpr unsigned CROWDED_CELL = 24;       // a cell with more environments than this counts as "crowded" in the run statistics
+constexpr unsigned STEP_SAT = 0xFFFFFEu;    // an episode's step counter saturates here (the tile records keep 24 bits of it)
 
 // ------------------------------------------------------------------------------------------------
 // Philox4x32-10, counter-based: no generator state is stored anywhere.
@@ -37,9 +39,11 @@ __device__ __forceinline__ float u01(unsigned w) { return (float)(w >> 8) * 5.96
 
 __device__ __forceinline__ unsigned cw_load(const unsigned short* cw, unsigned cell) { return cw[cell]; }
 
-// The move byte of a cell (written by k_te_cls, tile by tile): bit a = a move in direction a is blocked, bit 4+a = the cell an
+// The move byte of a cell (written tile by tile by k_te_cls, row by row by k_gather_moves, for the engine in use): bit a = a move in direction a is blocked, bit 4+a = the cell an
 // environment stands on after choosing a is a goal.
-__device__ __forceinline__ unsigned move_byte(const TileP& tp, int x, int y) {
+__device__ __forceinline__ unsigned move_byte(const Params& p, int x, int y) {
+    if (p.gp.mv) return __ldg(p.gp.mv + (size_t)y * (size_t)p.W + (size_t)x);
+    const TileP& tp = p.tp;
     const unsigned m = tp.T - 1u, tile = ((unsigned)y >> tp.tshift) * tp.tiles_x + ((unsigned)x >> tp.tshift);
     return __ldg(tp.tcls + (size_t)tile * tp.cls_stride + ((((unsigned)y & m) << tp.tshift) | ((unsigned)x & m)));
 }

@@ -45,7 +45,6 @@
 
 namespace cudarl {
 
-constexpr unsigned CROWDED_CELL = 24;   // a cell with more environments than this counts as "crowded" in the run statistics
 constexpr unsigned NMAX16 = 65535u;     // records of a tile the 16-bit counters can hold
 constexpr unsigned WPB = 4;             // warps per block; every warp works on its own
 constexpr unsigned FAST_MAX = 128;      // records of a tile the fast path stages in shared memory (a multiple of 32, below 256)
@@ -55,7 +54,7 @@ __device__ __forceinline__ unsigned tile_of(const TileP& tp, int x, int y) {
 }
 // A record inside a tile's region or arrival buffer, 8 bytes: .x = environment, .y = steps of the episode << 8 | row inside the
 // tile << 4 | column inside the tile (the tile is known from where the record lies).  The step counter saturates at 2^24 - 2 (step caps beyond that are refused).
-constexpr unsigned T_SAT = 0xFFFFFEu;     // (T_SAT << 8 | 0xFF) stays clear of the all-ones word that marks a restart inside the step kernel
+constexpr unsigned T_SAT = STEP_SAT;      // (T_SAT << 8 | 0xFF) stays clear of the all-ones word that marks a restart inside the step kernel
 __device__ __forceinline__ uint2 pack_rec(const TileP& tp, const int4 r) {
     const unsigned m = tp.T - 1u, t = (unsigned)r.z < T_SAT ? (unsigned)r.z : T_SAT;
     return make_uint2((unsigned)r.w, (t << 8) | (((unsigned)r.y & m) << 4) | ((unsigned)r.x & m));

@@ -1,0 +1,62 @@
+"""The engines of the train step at the sizes where their dispatch changes, against the oracle: populations on both sides of every
+number of environments per thread of the gather engine, and the tile engine (forced by `tile_edge`) on the worlds whose default is
+another engine by now."""
+import os
+
+import numpy as np
+import pytest
+
+from test_gpu_parity import assert_same, lockstep, pair
+
+pytestmark = pytest.mark.gpu
+SMS = 148
+THREADS = min(8, os.cpu_count() or 1)
+
+
+def world(pkg, w, h, n, **kw):
+    base = dict(start_mode=pkg.START_RANDOM, goal_mode=pkg.GOAL_SEEDED, num_goals=3, obstacle_kind=pkg.OBST_BERNOULLI, obstacle_p=0.15,
+                eps_kind=pkg.EPS_FIXED, eps0=0.3, max_steps=11, lr=0.2)
+    base.update(kw)
+    return pkg.make_config(w, h, n, **base)
+
+
+@pytest.mark.parametrize("n", [511, 513, SMS * 512, SMS * 512 + 1, SMS * 1024, SMS * 1024 + 1, SMS * 2048, SMS * 2048 + 1, 4 * SMS * 1024 + 77])
+def test_gather_engine_population_limits(pkg, orc, n):
+    """512 environments per SM and environment-per-thread: the last population of one kind and the first of the next."""
+    cfg = world(pkg, 120, 97, n, env_offset=5)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    lockstep(gpu, cpu, 3, what="n=%d" % n)
+    gpu.train_steps(14); cpu.train_steps(14)             # one launch across a step cap that everybody reaches together
+    assert_same(gpu, cpu, "n=%d, many steps per launch" % n)
+    sa, sb = gpu.get_stats(), cpu.get_stats()
+    assert (sa.conflicts, sa.goals, sa.timeouts, sa.device_error) == (sb.conflicts, sb.goals, sb.timeouts, 0)
+
+
+@pytest.mark.parametrize("n,kw", [(700, {}), (90000, {"legacy_clamp": 1}), (400000, {"start_mode": 0}), (2000, {"start_mode": 0, "max_steps": 0})])
+def test_gather_engine_common_start_traps_and_episode_epsilon(pkg, orc, n, kw):
+    """Everybody on one start cell (whole warps count once), traps, the clamp, and the epsilon that follows the finished episodes."""
+    cfg = world(pkg, 91, 93, n, eps_kind=pkg.EPS_MULT_PER_EPISODE, eps0=1.0, eps_decay=0.9, **kw)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    cells = gpu.get_cells()
+    for k in np.flatnonzero(cells == 1)[:40]:
+        gpu.add_trap(int(k % 91), int(k // 91), -0.3); cpu.add_trap(int(k % 91), int(k // 91), -0.3)
+    for k in (1, 2, 40):
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert gpu.get_stats().epsilon == cpu.get_stats().epsilon
+        assert_same(gpu, cpu, "n=%d after +%d" % (n, k))
+
+
+@pytest.mark.parametrize("edge", [8, 16])
+@pytest.mark.parametrize("w,h,n,kw", [(96, 96, 20000, {}), (3, 2, 70000, {}), (500, 490, 60000, {"max_steps": 20}), (24, 17, 3000, {"eps_kind": 2, "eps_decay": 0.97})])
+def test_tile_engine_forced(pkg, orc, edge, w, h, n, kw):
+    """What the tile engine alone has: region re-sizing, 32-bit counters, mass restarts through the spill list, its epsilon kernel."""
+    cfg = world(pkg, w, h, n, num_goals=1, obstacle_p=0.0 if w < 10 else 0.15, tile_edge=edge, rebucket_every=3, **kw)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    for k in (1, 19, 1, 1, 9):
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert_same(gpu, cpu, "edge %d after +%d" % (edge, k))
+    a, b = gpu.eval_rollout(60), cpu.eval_rollout(60)    # reads the tiles' move bytes, leaves the regions alone
+    assert (a.reached, a.total_steps) == (b.reached, b.total_steps)
+    gpu.train_steps(5); cpu.train_steps(5)
+    assert_same(gpu, cpu, "edge %d after the rollout" % edge)
+    assert gpu.get_stats().device_error == 0
