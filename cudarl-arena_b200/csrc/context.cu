@@ -103,7 +103,9 @@ struct cudarl_ctx {
     void *dtmeta = nullptr, *dtscratch = nullptr, *dtcls = nullptr;   // per-tile regions / counters; 32-bit counters of crowded tiles
     // gather engine
     bool gather = false;                   // the engine of this context's train steps: gather, or the tiles
-    void *dgbar = nullptr, *dgcnt = nullptr, *dgmv = nullptr, *dgown = nullptr, *dgdv = nullptr;
+    void *dgbar = nullptr, *dgcnt = nullptr, *dgmv = nullptr, *dgstate = nullptr, *dgbins = nullptr;
+    int dealt = -1;                        // the work buffer the records are in, dealt by cell; -1: in environment order
+    void* dwork[2] = {nullptr, nullptr};
     uint32_t barrier_base = 0;             // arrivals at the grid barrier by all launches so far
     bool tile_mode = false;               // true: the records live in tile regions (train steps), false: in environment order
     bool cls_dirty = true;                // the per-tile class bytes must be rebuilt from the cell words
@@ -408,7 +410,7 @@ int make_table_map(cudarl_ctx* c) {
 // 64 per tile 124 / 250, 96 per tile 182 / 271, 128 per tile 731 / 323 -- the crossover lies near 110.
 int alloc_tiles(cudarl_ctx* c) {
     Params& p = c->p; TileP& tp = p.tp;
-    const size_t S = p.S, N = p.N ? p.N : 1;
+    const size_t N = p.N ? p.N : 1;
     const size_t nt16 = (((size_t)p.W + 15) >> 4) * (((size_t)p.H + 15) >> 4);
     unsigned tsh = (N / nt16 <= 104) ? 4u : 3u;
     if (c->cfg.tile_edge == 8) tsh = 3u; else if (c->cfg.tile_edge == 16) tsh = 4u;
@@ -458,8 +460,11 @@ int alloc_table(cudarl_ctx* c) {
     c->p.Q = (float4*)c->dQ;
     return 0;
 }
-// The gather engine where its scattered accesses stay in L2 (a table of up to 32 MB), or are few whatever the size of the grid: up
-// to 262,144 environments; the tile engine streams the table, 16 bytes per cell, however few there are.  An explicit tile edge asks for tiles.
+// The gather engine (and, within it, the arena) where its scattered accesses stay in L2 -- a table of up to 32 MB -- or are few whatever
+// the size of the grid; else the tile engine, which streams the table.  Measured on B200, us per step with gather / tiles of 16 / of 8,
+// before the population bunches up: 1448 x 1448 cells, 262,144 environments 13 / 16 / 34, 1,048,576 32 / 80 / 42; 2048 x 2048 21 / 21 / 60
+// and 80 / 32 / 65; 4096 x 4096 with 131,072 13 / 64 / 162, with 262,144 37 / 66 / 185, with 524,288 93 / 68 / 209.  An explicit tile edge
+// asks for tiles.
 bool use_gather(const cudarl_ctx* c) {
     const cudarl_config& f = c->cfg;
     if (f.tile_edge != 0) return false;
@@ -473,11 +478,17 @@ int alloc_gather(cudarl_ctx* c) {
     CK(cudaMalloc(&c->dgbar, 256)); CK(cudaMemsetAsync(c->dgbar, 0, 256, c->st));
     CK(cudaMalloc(&c->dgcnt, 8 * S * sizeof(unsigned))); CK(cudaMemsetAsync(c->dgcnt, 0, 8 * S * sizeof(unsigned), c->st));
     CK(cudaMalloc(&c->dgmv, S));
-    gather_plan(p, sms);
+    if (!arena_plan(p)) { gp = GatherP{}; gather_plan(p, sms); }
     gp.barrier = (unsigned*)c->dgbar;
     gp.cnt[0] = (unsigned*)c->dgcnt; gp.cnt[1] = gp.cnt[0] + 4 * S;
     gp.mv = (unsigned char*)c->dgmv;
-    if (gp.stream) { CK(cudaMalloc(&c->dgown, N * sizeof(unsigned))); CK(cudaMalloc(&c->dgdv, N * sizeof(float2))); gp.own = (unsigned*)c->dgown; gp.dv = (float2*)c->dgdv; }
+    if (gp.home == 2u) { CK(cudaMalloc(&c->dgstate, N * 24u)); gp.state = (unsigned char*)c->dgstate; }
+    if (gp.deal_every) {
+        const size_t words = (size_t)gp.nbins + gp.grid + N;
+        CK(cudaMalloc(&c->dgbins, words * sizeof(unsigned))); CK(cudaMemsetAsync(c->dgbins, 0, (size_t)gp.nbins * sizeof(unsigned), c->st));
+        gp.bins = (unsigned*)c->dgbins; gp.part = gp.bins + gp.nbins; gp.rank = gp.part + gp.grid;
+        for (auto& wk : c->dwork) CK(cudaMalloc(&wk, N * sizeof(int4)));
+    }
     return 0;
 }
 
@@ -501,6 +512,7 @@ int enter_tiles(cudarl_ctx* c) {
 }
 // tile regions -> records back in environment order
 int leave_tiles(cudarl_ctx* c) {
+    if (c->dealt >= 0) { launch_gather_export(c->p, (const int4*)c->dwork[c->dealt], c->st); CK(cudaGetLastError()); c->dealt = -1; return 0; }
     if (!c->tile_mode) return 0;
     { int rc = close_kernel_segment(c); if (rc) return rc; }
     c->p.step = (unsigned long long)c->h_step;
@@ -511,6 +523,7 @@ int leave_tiles(cudarl_ctx* c) {
 }
 // the records in environment order for reading; the tile regions stay as they are
 int records_in_order(cudarl_ctx* c) {
+    if (c->dealt >= 0) { launch_gather_export(c->p, (const int4*)c->dwork[c->dealt], c->st); CK(cudaGetLastError()); return 0; }
     if (!c->tile_mode) return 0;
     { int rc = close_kernel_segment(c); if (rc) return rc; }
     c->p.step = (unsigned long long)c->h_step;
@@ -630,13 +643,17 @@ int run_gather(cudarl_ctx* c, int64_t n) {
     for (int64_t k = 0; k < n;) {
         int64_t m = std::min(n - k, most);
         if (c->cfg.sync_every > 0 && c->comm) m = std::min<int64_t>(m, c->cfg.sync_every - c->h_step % c->cfg.sync_every);
+        const unsigned deal = c->p.gp.deal_every;
+        if (deal) m = std::min<int64_t>(m, deal);
         { int rc = open_kernel_segment(c); if (rc) return rc; }
         c->p.step = (unsigned long long)c->h_step;
         c->p.eps_idx = c->eps_mode == 1 ? (unsigned)k : 0u;
-        GatherLaunch l{};
+        StepLaunch l{};
         l.steps = (unsigned)m; l.chunk = c->p.gp.chunk; l.barrier_base = c->barrier_base; l.eps_mode = c->eps_mode; l.trace = c->trace ? 1 : 0;
-        CK(launch_gather_steps(c->p, l, c->st));
-        c->barrier_base += c->p.gp.grid * gather_barriers(l.steps);
+        l.in = c->dealt >= 0 ? (const int4*)c->dwork[c->dealt] : c->p.st; l.out = deal ? (int4*)c->dwork[c->dealt == 0 ? 1 : 0] : c->p.st;
+        CK(c->p.gp.arena ? launch_arena_steps(c->p, l, c->st) : launch_gather_steps(c->p, l, c->st));
+        c->barrier_base += c->p.gp.grid * gather_barriers(l);
+        if (deal) c->dealt = c->dealt == 0 ? 1 : 0;
         c->h_step += m; c->kseg_count += m; k += m;
         if (c->eps_mode != 2 && c->h_eps) c->eps_used = c->h_eps[c->eps_mode == 1 ? k - 1 : 0];
         if (c->cfg.sync_every > 0 && c->comm && (c->h_step % c->cfg.sync_every) == 0) { int rc = average_now(c); if (rc) return rc; }
@@ -676,7 +693,7 @@ void free_all(cudarl_ctx* c) {
                     c->dtra, c->dtrr, c->dtrd, c->dsckey, c->dscval, c->dgather, c->dact,
                     c->dub[0], c->dub[1], c->dub[2], c->dub[3], c->dub[4], c->dub[5], c->dub[6],
                     c->dQ, c->drec[0], c->drec[1], c->darr[0], c->darr[1], c->dovf[0], c->dovf[1], c->dbmax[0], c->dbmax[1],
-                    c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dhop, c->dtq, c->dpeer_ptrs, c->dbarrier_word, c->dgbar, c->dgcnt, c->dgmv, c->dgown, c->dgdv};
+                    c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dhop, c->dtq, c->dpeer_ptrs, c->dbarrier_word, c->dgbar, c->dgcnt, c->dgmv, c->dgstate, c->dgbins, c->dwork[0], c->dwork[1]};
     for (void* b : bufs) if (b) cudaFree(b);
     if (c->h_eps) cudaFreeHost(c->h_eps);
     stage_give(&c->stage);
@@ -729,6 +746,9 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
         Params& p = c->p;
         p.W = f->width; p.H = f->height; p.S = (unsigned)(f->width * f->height); p.N = (unsigned)f->num_envs;
         p.env_offset = (unsigned)f->env_offset; p.k0 = (uint32_t)f->seed; p.k1 = (uint32_t)(f->seed >> 32);
+        for (unsigned r = 0; r < 10; ++r) {                  // k1 of the policy stream carries its tag (TAG_POLICY of rules.cuh)
+            p.policy_keys[2 * r] = p.k0 + r * 0x9E3779B9u; p.policy_keys[2 * r + 1] = (p.k1 ^ 0x504F4C49u) + r * 0xBB67AE85u;
+        }
         p.max_steps = f->max_steps; p.start_mode = f->start_mode; p.lr = f->lr; p.gamma = f->gamma; p.legacy_clamp = f->legacy_clamp;
         uint32_t sc = 0, fb = 0;
         rc = build_cells(c, c->cells, sc, fb); if (rc) break;

@@ -34,6 +34,7 @@ struct Ctl {
     unsigned int long2_count[2];    // chains too long for a warp, queued for the block-per-chain kernel
     unsigned int scratch_cursor;    // bump allocator of the long-chain scratch, reset every step
     unsigned int error;             // sticky internal error bits
+    unsigned int never;             // zero for good: what a wait that a test makes run out looks at
     float eps_used;                 // epsilon of the most recent step (for the stats call)
 };
 
@@ -84,11 +85,15 @@ struct GatherP {
     unsigned* barrier;         // arrivals of all blocks of all launches so far (wraps)
     unsigned* cnt[2];          // 4 S counters: environments on a (cell, action) in this step, by step parity; zero between launches
     unsigned char* mv;         // S move bytes
-    unsigned* own;             // N: streamed populations: the (cell, action) an environment owns in this step,
-    float2* dv;                // N: and its TD target and value
-    unsigned ept, chunk, grid, stream;      // environments per thread and turn, per block; blocks; whether the population is streamed
+    unsigned char* state;      // N x 24 bytes: the environments during a launch, where shared memory has no room for them
+    unsigned *bins, *part, *rank;           // dealing by cell: 8 counters per 8 x 8 cells (zero between launches), one word per block, N ranks
+    unsigned bins_x, nbins;
+    unsigned chunk, grid, threads;          // environments per block; blocks; threads per block
+    unsigned home;                          // where the environments are during a launch: 0 registers, 1 shared memory, 2 global memory
+    unsigned deal_every;                    // steps between two dealings by cell; 0 = the environments stay in their order
+    unsigned cluster, arena;                // all blocks in one cluster; the world in the shared memory of one block
 };
-struct GatherLaunch { unsigned steps, chunk, barrier_base; int eps_mode, trace; };
+struct StepLaunch { unsigned steps, chunk, barrier_base; int eps_mode, trace; const int4* in; int4* out; };    // in != out: deal by cell first
 
 // ---- everything a kernel needs, passed by value ------------------------------------------------
 struct Params {
@@ -97,6 +102,7 @@ struct Params {
     unsigned N;            // local environments
     unsigned env_offset;   // global index of local env 0
     unsigned k0, k1;       // Philox key base = seed (k1 is xor-ed with the stream tag)
+    unsigned policy_keys[20];   // the ten round keys of the policy stream, two words each: operands straight from the constant bank
     int max_steps;
     int start_mode;
     unsigned start_cell;   // CENTRE / FIXED start
@@ -159,9 +165,13 @@ unsigned tile_cls_stride(unsigned tshift);                         // bytes of o
 void launch_tile_border(const Params& p, cudaStream_t st);         // border array of parity p.step & 1 from the table (after any change of the table outside train steps)
 // gather engine (gather_engine.cu)
 void gather_plan(Params& p, int sms);
-unsigned gather_barriers(unsigned steps);                           // arrivals per block of a launch of so many steps
+unsigned gather_barriers(const StepLaunch& l);                      // arrivals per block of a launch
+void launch_gather_export(const Params& p, const int4* work, cudaStream_t st);      // records in any order -> p.st
 void launch_gather_moves(const Params& p, cudaStream_t st);         // cell words -> move bytes
-cudaError_t launch_gather_steps(const Params& p, const GatherLaunch& l, cudaStream_t st);
+cudaError_t launch_gather_steps(const Params& p, const StepLaunch& l, cudaStream_t st);
+// arena engine (arena_engine.cu)
+bool arena_plan(Params& p);                                         // false: the world does not fit
+cudaError_t launch_arena_steps(const Params& p, const StepLaunch& l, cudaStream_t st);
 // Replica averaging, the slice this rank owns: table[cell0 + i] = (sum over ranks 0..R-1 in that order) / R, where rank `self`'s
 // rows are the table's own and the other ranks' rows lie in `others` (R - 1 slices of n rows, ascending rank).
 void launch_q_average_peers(float4* const* tables, unsigned R, unsigned self, size_t cell0, size_t n, float scale, cudaStream_t st);

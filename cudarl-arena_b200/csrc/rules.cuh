@@ -23,11 +23,22 @@ __device__ __forceinline__ U4 philox4x32_10(unsigned c0, unsigned c1, unsigned c
                                             unsigned k0, unsigned k1) {
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
-        unsigned hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-        unsigned hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
+        const unsigned long long m0 = (unsigned long long)0xD2511F53u * c0, m1 = (unsigned long long)0xCD9E8D57u * c2;     // one wide multiply each
+        const unsigned hi0 = (unsigned)(m0 >> 32), lo0 = (unsigned)m0, hi1 = (unsigned)(m1 >> 32), lo1 = (unsigned)m1;
         unsigned n0 = hi1 ^ c1 ^ k0, n2 = hi0 ^ c3 ^ k1;
         c0 = n0; c1 = lo1; c2 = n2; c3 = lo0;
         k0 += 0x9E3779B9u; k1 += 0xBB67AE85u;
+    }
+    return U4{c0, c1, c2, c3};
+}
+
+// The same with the round keys given (pairs).
+__device__ __forceinline__ U4 philox4x32_10(unsigned c0, unsigned c1, unsigned c2, unsigned c3, const unsigned (&rk)[20]) {
+#pragma unroll
+    for (int r = 0; r < 10; ++r) {
+        const unsigned long long m0 = (unsigned long long)0xD2511F53u * c0, m1 = (unsigned long long)0xCD9E8D57u * c2;
+        const unsigned n0 = (unsigned)(m1 >> 32) ^ c1 ^ rk[2 * r], n2 = (unsigned)(m0 >> 32) ^ c3 ^ rk[2 * r + 1];
+        c0 = n0; c1 = (unsigned)m1; c2 = n2; c3 = (unsigned)m0;
     }
     return U4{c0, c1, c2, c3};
 }
@@ -122,6 +133,26 @@ __device__ __forceinline__ void fold(float4& r, int a, float lr, float target) {
     const float q = pick(r, a);
     const float v = __fmaf_rn(lr, __fsub_rn(target, q), q);
     r.x = a == 0 ? v : r.x; r.y = a == 1 ? v : r.y; r.z = a == 2 ? v : r.z; r.w = a == 3 ? v : r.w;
+}
+
+// Exclusive prefix of v over the block (any block size up to 1024); *total receives the block sum.
+__device__ __forceinline__ unsigned block_scan_excl(unsigned v, unsigned* s_warp, unsigned* total) {
+    const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    unsigned inc = v;
+    for (int o = 1; o < 32; o <<= 1) { const unsigned t = __shfl_up_sync(FULL, inc, o); if (lane >= (unsigned)o) inc += t; }
+    if (lane == 31u) s_warp[wid] = inc;
+    __syncthreads();
+    if (wid == 0) {
+        const unsigned w = lane < nw ? s_warp[lane] : 0u; unsigned winc = w;
+        for (int o = 1; o < 32; o <<= 1) { const unsigned t = __shfl_up_sync(FULL, winc, o); if (lane >= (unsigned)o) winc += t; }
+        if (lane < nw) s_warp[lane] = winc - w;
+        if (lane == 31u) s_warp[32] = winc;
+    }
+    __syncthreads();
+    const unsigned r = s_warp[wid] + inc - v;
+    *total = s_warp[32];
+    __syncthreads();
+    return r;
 }
 
 }  // namespace cudarl

@@ -1,0 +1,226 @@
+// step_loop.cuh -- the fused train step with one thread per environment, many steps per launch; shared by the engines that differ in
+// where the table and the counters live and in how the threads of a launch wait for one another (gather_engine.cu: L2 and a barrier
+// of the grid or of one cluster; arena_engine.cu: shared memory and the block's barrier).
+//
+//   count   every environment reads the row of its cell, chooses its action, counts itself in the (cell, action) counter with an
+//           atomic, moves on, and takes the TD target of its (cell, action) from Q_t;
+//   -- barrier --
+//   apply   the update of a (cell, action) is applied as many times as were counted, and the one table entry is stored;
+//   -- barrier --
+//
+// All updates of one (cell, action) within a step are the same map, so only their number matters (see tile_engine.cu).  Who applies
+// it: with OWNERS the first to count there, which needs the counter's old value -- right where latency counts and crowds are common;
+// without, everybody who counted (all compute and store the same bits), so that the atomics need no answer -- right where their rate
+// counts (1024 x 1024 cells, 1,048,576 environments: 25.0 -> 24.0 us a step; 1001 x 613, 150,001: 7.6 -> 6.8; but 64 x 64 with 4,096
+// crowded ones 4.7 -> 5.5).  Counters alternate by step parity; who counted clears its counter in the next step's count phase, when
+// everybody has read it and nobody uses that parity.
+//
+// A Space gives: row(s), moves(s), add(par, idx, n) -> old count, count(par, idx, n), note(par, idx) -> marked before, clear(par, idx),
+// counts(par, s) -> uint4, store(idx, v), arrive(), wait() -> false when the launch has to be given up.
+#pragma once
+#include "kernels.cuh"
+#include "rules.cuh"
+
+namespace cudarl {
+
+constexpr unsigned NOBODY = 0xFFFFFFFFu;
+constexpr unsigned NOTED = 0x80000000u;     // a counter's mark: the crowded cell is in the statistics already
+
+// What one environment needs between the two phases of a step, and what the launch sums up.
+struct Tally { unsigned goals, timeouts, conf, crowded, on_crowded; };
+
+// The update of (cell, action) `own` from the counted number of environments on it: the map q <- fma(lr, d - q, q) as often as counted.
+// It is a contraction, so a long run ends at its fixed point: once the value stops changing it never changes again.
+__device__ __forceinline__ float apply_counted(float v, float d, float lr, unsigned n) {
+    for (unsigned i = 0; i < n; ++i) {
+        const float w = __fmaf_rn(lr, __fsub_rn(d, v), v);
+        if (__float_as_uint(w) == __float_as_uint(v)) break;
+        v = w;
+    }
+    return v;
+}
+
+// Whether a launch may start.  A context in which a wait has run out does nothing any more (its barrier counter is off); with a poll
+// bound set (tests only) a wait that nothing can end runs out here.
+__device__ __forceinline__ bool may_start(const Params& p, unsigned* s_flag) {
+    if (threadIdx.x == 0u) {
+        unsigned ok = (*reinterpret_cast<volatile unsigned*>(&p.ctl->error) & ERR_COPY_TIMEOUT) ? 0u : 1u;
+        unsigned left = p.tp.wait_polls;
+        while (left && *reinterpret_cast<volatile unsigned*>(&p.ctl->never) == 0u) --left;
+        if (p.tp.wait_polls && left == 0u) { atomicOr(&p.ctl->error, ERR_COPY_TIMEOUT); ok = 0u; }
+        *s_flag = ok;
+    }
+    __syncthreads();
+    return *s_flag != 0u;
+}
+
+// Where the state of the environments of a block lives during a launch.
+enum class Home { Registers, Shared, Global };
+// One environment of a block: cell, steps of the episode, number; the (cell, action) owned in this step, its TD target and value.
+constexpr unsigned STATE_BYTES = 24u;
+
+// The steps of one launch, GB threads per block.  A block owns `count` slots of the records in `work` from `first` on: one per thread,
+// in registers, or streamed turn by turn from shared (`arrays`: chunk x STATE_BYTES) or global memory (gp.state: N x STATE_BYTES).
+// PLAIN: no traps, no clamp, no trace, epsilon by step -- the options are left out of the code, not skipped in it.
+template <Home HOME, unsigned GB, bool PLAIN, bool OWNERS, class Space>
+__device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, Space& space, int4* __restrict__ work, unsigned char* arrays) {
+    __shared__ unsigned s_sum[5], s_ep;
+    constexpr bool STREAM = HOME != Home::Registers;
+    const unsigned tid = threadIdx.x, first = blockIdx.x * l.chunk, count = first < p.N ? min(l.chunk, p.N - first) : 0u;
+    Ctl* const ctl = p.ctl;
+    const unsigned W = (unsigned)p.W;
+    const unsigned tmax = p.max_steps > 0 ? (unsigned)p.max_steps : 0x7FFFFFFFu;
+    if (tid < 5u) s_sum[tid] = 0u;
+    if (tid == 5u) s_ep = 0u;
+    __syncthreads();
+    Tally tally{0u, 0u, 0u, 0u, 0u};
+    unsigned s = 0u, t = 0u, id = 0u, own = NOBODY; float target = 0.f, value = 0.f;
+    uint2 w = make_uint2(0u, 0u);                                  // the policy draw of the step at hand
+    // streamed state, by slot of the block
+    const size_t room = HOME == Home::Shared ? l.chunk : p.N, at0 = HOME == Home::Shared ? 0u : first;
+    unsigned char* const base = HOME == Home::Shared ? arrays : p.gp.state;
+    uint2* const m_pos = reinterpret_cast<uint2*>(base) + at0;
+    float2* const m_tv = reinterpret_cast<float2*>(base + room * 8u) + at0;
+    unsigned* const m_id = reinterpret_cast<unsigned*>(base + room * 16u) + at0;
+    unsigned* const m_own = reinterpret_cast<unsigned*>(base + room * 20u) + at0;
+    const unsigned end = STREAM ? (count + GB - 1u) / GB * GB : GB;      // slots, rounded up: whole warps take every turn
+    auto draw = [&](unsigned i, unsigned long long g) -> uint2 {
+        const U4 r = philox4x32_10(p.env_offset + i, 0u, (unsigned)g, (unsigned)(g >> 32), p.policy_keys);
+        return make_uint2(r.x, r.y);
+    };
+    unsigned long long g = p.step;
+    for (unsigned j = tid; j < end; j += GB) {
+        if (j >= count) continue;
+        const int4 r = work[first + j];
+        s = (unsigned)r.y * W + (unsigned)r.x; t = (unsigned)r.z; id = (unsigned)r.w;
+        if (STREAM) { m_pos[j] = make_uint2(s, t); m_id[j] = id; m_own[j] = NOBODY; } else w = draw(id, g);
+    }
+    unsigned eps_at = !PLAIN && l.eps_mode == 2 ? *reinterpret_cast<volatile unsigned*>(&ctl->eps_idx) : p.eps_idx;
+    float eps = __ldg(p.eps_tab + eps_at);
+
+    for (unsigned step = 0; step < l.steps; ++step, ++g) {
+        const unsigned par = (unsigned)g & 1u;
+        const unsigned thr = !(eps > 0.0f) ? 0u : eps >= 1.0f ? (1u << 24) : (unsigned)ceilf(eps * 16777216.0f);   // explore iff (w0 >> 8) < thr
+
+        // ---- count ----
+        for (unsigned j = tid; j < end; j += GB) {
+            const bool act = j < count;
+            if (STREAM) {
+                unsigned before = NOBODY;
+                if (act) { const uint2 q = m_pos[j]; s = q.x; t = q.y; id = m_id[j]; before = m_own[j]; }
+                w = draw(id, g);
+                if (before != NOBODY) space.clear(par ^ 1u, before);
+            }
+            unsigned mv = 0u; float4 row = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (act) { row = space.row(s); mv = space.moves(s); }
+            if (!STREAM && own != NOBODY) space.clear(par ^ 1u, own);
+            const int a = (w.x >> 8) < thr ? (int)(w.y & 3u) : argmax4(row);
+            own = act ? s * 4u + (unsigned)a : NOBODY;
+            mv >>= a;                                 // bit 0: the move is blocked, bit 4: it ends on a goal
+            // a whole warp on one (cell, action) -- everybody at a common start cell -- counts once
+            const bool common = __all_sync(FULL, own == __shfl_sync(FULL, own, 0));
+            bool applies = act && !OWNERS;
+            if (act && (!common || (tid & 31u) == 0u)) {
+                const unsigned n = common ? 32u : 1u;
+                if (OWNERS) applies = space.add(par, own, n) == 0u; else space.count(par, own, n);
+            }
+            const unsigned there = a == 0 ? s - W : a == 1 ? s + 1u : a == 2 ? s + W : s - 1u;
+            s = (mv & 1u) ? s : there;
+            float4 next = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (act) next = space.row(s);             // side by side with the atomic
+            const bool done = (mv & 16u) != 0u;
+            value = pick(row, a);
+            float m = max4(next);
+            if (!PLAIN && p.legacy_clamp && m < 0.0f) m = 0.0f;
+            float r = -0.01f;
+            if (!PLAIN && p.ntraps && (mv & 1u)) { const unsigned y = s / W; r = blocked_step_reward(p, (int)(s - y * W), (int)y, a); }     // a trap charges its penalty
+            target = done ? 1.0f : __fmaf_rn(p.gamma, m, r);
+            t = min(t + 1u, STEP_SAT);
+            if (OWNERS && !applies) own = NOBODY;
+            if (!act) continue;
+            if (!PLAIN && l.trace && step + 1u == l.steps) { p.tr_a[id] = a; p.tr_r[id] = done ? 1.0f : r; p.tr_d[id] = done ? 1 : 0; }
+            if (done || t >= tmax) {
+                s = sample_start(p, p.env_offset + id, g + 1ull, TAG_START); t = 0u;
+                if (done) ++tally.goals; else ++tally.timeouts;
+                if (!PLAIN && l.eps_mode == 2) atomicAdd(&s_ep, 1u);
+            }
+            if (STREAM) {
+                m_pos[j] = make_uint2(s, t);
+                m_own[j] = own;
+                if (applies) m_tv[j] = make_float2(target, value);
+            }
+        }
+        if (!PLAIN && l.eps_mode == 2) {              // finished episodes of this step, before anybody can pass the barrier
+            __syncthreads();
+            if (tid == 0u && s_ep) { atomicAdd(&ctl->episodes, (unsigned long long)s_ep); s_ep = 0u; }
+        }
+        space.arrive();
+        if (!STREAM) { w = draw(id, g + 1ull); asm volatile("" : "+r"(w.x), "+r"(w.y)); }      // behind the barrier's latency, and kept there
+        if (!space.wait()) return;
+
+        // ---- apply ----
+        for (unsigned j = tid; j < end; j += GB) {
+            if (STREAM) own = j < count ? m_own[j] : NOBODY;
+            if (own == NOBODY) continue;
+            if (STREAM) { const float2 q = m_tv[j]; target = q.x; value = q.y; }
+            uint4 c = space.counts(par, own >> 2);
+            const unsigned a = own & 3u;
+            unsigned n = a == 0u ? c.x : a == 1u ? c.y : a == 2u ? c.z : c.w;
+            const unsigned tot = c.x + c.y + c.z + c.w;
+            if (tot > 1u) tally.conf += OWNERS ? n : 1u;
+            if (tot > CROWDED_CELL) {                 // the lowest chosen action speaks for the cell
+                if (!OWNERS) {                        // the first to get here, that is; its mark on the counter looks like a huge count to the others
+                    c.x &= ~NOTED; c.y &= ~NOTED; c.z &= ~NOTED; c.w &= ~NOTED; n &= ~NOTED;
+                    ++tally.on_crowded;
+                }
+                const unsigned below = a == 0u ? 0u : a == 1u ? c.x : a == 2u ? c.x + c.y : c.x + c.y + c.z;
+                if (below == 0u) {
+                    if (OWNERS) { ++tally.crowded; tally.on_crowded += tot; }
+                    else if (!space.note(par, own)) ++tally.crowded;
+                }
+            }
+            space.store(own, apply_counted(value, target, p.lr, n));
+        }
+        // the index of the next step's epsilon: by step, or by the episodes finished so far (read between the two barriers: nobody
+        // adds to them before everybody has passed the second)
+        if (l.eps_mode == 1) ++eps_at;
+        else if (!PLAIN && l.eps_mode == 2) {
+            const unsigned long long kk = *reinterpret_cast<volatile unsigned long long*>(&ctl->episodes) / (unsigned long long)p.N;
+            const unsigned long long rel = kk > ctl->eps_base_k ? kk - ctl->eps_base_k : 0ull;
+            eps_at = (unsigned)(rel < (unsigned long long)(ctl->eps_len - 1u) ? rel : (unsigned long long)(ctl->eps_len - 1u));
+        }
+        space.arrive();
+        if (l.eps_mode && step + 1u < l.steps) eps = __ldg(p.eps_tab + eps_at);
+        if (!space.wait()) return;
+    }
+
+    // ---- the last step's counters back to zero, the records out, the sums ----
+    for (unsigned j = tid; j < end; j += GB) {
+        if (j >= count) continue;
+        if (STREAM) { const uint2 q = m_pos[j]; s = q.x; t = q.y; id = m_id[j]; own = m_own[j]; }
+        if (own != NOBODY) space.clear(((unsigned)g & 1u) ^ 1u, own);
+        const unsigned y = s / W;
+        work[first + j] = make_int4((int)(s - y * W), (int)y, (int)t, (int)id);
+    }
+    unsigned sums[5] = {tally.goals, tally.timeouts, tally.conf, tally.crowded, tally.on_crowded};
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const unsigned v = __reduce_add_sync(FULL, sums[k]);
+        if ((tid & 31u) == 0u && v) atomicAdd(&s_sum[k], v);
+    }
+    __syncthreads();
+    if (tid == 0u) {
+        if (s_sum[0]) atomicAdd(&ctl->goals, (unsigned long long)s_sum[0]);
+        if (s_sum[1]) atomicAdd(&ctl->timeouts, (unsigned long long)s_sum[1]);
+        if (l.eps_mode != 2 && s_sum[0] + s_sum[1]) atomicAdd(&ctl->episodes, (unsigned long long)(s_sum[0] + s_sum[1]));
+        if (s_sum[2]) atomicAdd(&ctl->conflicts, (unsigned long long)s_sum[2]);
+        if (s_sum[3]) atomicAdd(&ctl->long_chains, (unsigned long long)s_sum[3]);
+        if (s_sum[4]) atomicAdd(&ctl->general, (unsigned long long)s_sum[4]);
+        if (blockIdx.x == 0u && l.eps_mode == 2) { ctl->eps_used = eps; ctl->eps_idx = eps_at; }
+    }
+}
+
+// Whether a launch needs none of the options PLAIN leaves out.
+inline bool plain(const Params& p, const StepLaunch& l) { return !p.ntraps && !p.legacy_clamp && !l.trace && l.eps_mode != 2; }
+
+}  // namespace cudarl

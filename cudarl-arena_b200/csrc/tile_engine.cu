@@ -63,26 +63,6 @@ __device__ __forceinline__ int4 unpack_rec(const uint2 q, int tx0, int ty0) {
     return make_int4(tx0 + (int)(q.y & 15u), ty0 + (int)((q.y >> 4) & 15u), (int)(q.y >> 8), (int)q.x);
 }
 
-// Exclusive prefix of v over the block (any block size up to 1024); *total receives the block sum.
-__device__ __forceinline__ unsigned block_scan_excl(unsigned v, unsigned* s_warp, unsigned* total) {
-    const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    unsigned inc = v;
-    for (int o = 1; o < 32; o <<= 1) { const unsigned t = __shfl_up_sync(FULL, inc, o); if (lane >= (unsigned)o) inc += t; }
-    if (lane == 31u) s_warp[wid] = inc;
-    __syncthreads();
-    if (wid == 0) {
-        const unsigned w = lane < nw ? s_warp[lane] : 0u; unsigned winc = w;
-        for (int o = 1; o < 32; o <<= 1) { const unsigned t = __shfl_up_sync(FULL, winc, o); if (lane >= (unsigned)o) winc += t; }
-        if (lane < nw) s_warp[lane] = winc - w;
-        if (lane == 31u) s_warp[32] = winc;
-    }
-    __syncthreads();
-    const unsigned r = s_warp[wid] + inc - v;
-    *total = s_warp[32];
-    __syncthreads();
-    return r;
-}
-
 // ---- asynchronous copies into shared memory, completion on an mbarrier ----------------------------------
 // Tensor copy: the box starts at float column 4 * tx0 (a multiple of 4 floats = 16 bytes) and row ty0; cells
 // of the box that lie outside the table arrive as zeros.  Plain bulk copies: 16-byte aligned on both sides,
@@ -446,7 +426,7 @@ __global__ void __launch_bounds__(WPB * 32u, MINB) k_tile_step(const __grid_cons
                 if (act && (lx | ly) >= T) { s_acc[5] = 1u; act = false; }             // never seen: the record does not lie in this tile
                 uint2 nrec = make_uint2(id, 0u); bool stays = false; unsigned key = 0u; float dd = 0.0f;
                 if (act) {
-                    const U4 w = philox4x32_10(p.env_offset + id, 0u, (unsigned)g, (unsigned)(g >> 32), p.k0, p.k1 ^ TAG_POLICY);
+                    const U4 w = philox4x32_10(p.env_offset + id, 0u, (unsigned)g, (unsigned)(g >> 32), p.policy_keys);
                     const unsigned ic = (ly << TSH) | lx;
                     const float4 row = lds_f4(sq + ic * 16u);
                     const unsigned mvb = lds_u8(smv + ic);
@@ -591,7 +571,7 @@ __global__ void __launch_bounds__(WPB * 32u, MINB) k_tile_step(const __grid_cons
                 int4 nrec = rec; bool stays = false;
                 if (act) {
                     const unsigned ic = (ly << TSH) | lx, e = (unsigned)rec.w;
-                    const U4 w = philox4x32_10(p.env_offset + e, 0u, (unsigned)g, (unsigned)(g >> 32), p.k0, p.k1 ^ TAG_POLICY);
+                    const U4 w = philox4x32_10(p.env_offset + e, 0u, (unsigned)g, (unsigned)(g >> 32), p.policy_keys);
                     const unsigned mvb = st[L::ST_MV + ic];
                     const int a = ((w.x >> 8) < c.eps_thr) ? (int)(w.y & 3u) : argmax4(s_q[ic]);
                     const bool blocked = (mvb >> a) & 1u, done = (mvb >> (4 + a)) & 1u;

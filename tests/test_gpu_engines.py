@@ -1,5 +1,5 @@
 """The engines of the train step at the sizes where their dispatch changes, against the oracle: populations on both sides of every
-number of environments per thread of the gather engine, and the tile engine (forced by `tile_edge`) on the worlds whose default is
+limit between the ways the arena and gather engines run, and the tile engine (forced by `tile_edge`) on the worlds whose default is
 another engine by now."""
 import os
 
@@ -20,20 +20,52 @@ def world(pkg, w, h, n, **kw):
     return pkg.make_config(w, h, n, **base)
 
 
-@pytest.mark.parametrize("n", [511, 513, SMS * 512, SMS * 512 + 1, SMS * 1024, SMS * 1024 + 1, SMS * 2048, SMS * 2048 + 1, 4 * SMS * 1024 + 77])
-def test_gather_engine_population_limits(pkg, orc, n):
-    """512 environments per SM and environment-per-thread: the last population of one kind and the first of the next."""
-    cfg = world(pkg, 120, 97, n, env_offset=5)
+LIMITS = [1, 32, 33, 256, 257, 1024, 1025, 4096, 4097, 8193, 16384, 16385, SMS * 512, SMS * 512 + 1, SMS * 1024, SMS * 1024 + 1, 4 * SMS * 1024 + 77, 1300000]
+
+
+@pytest.mark.parametrize("n", LIMITS)
+def test_population_limits(pkg, orc, n):
+    """The last population of one way to run the step and the first of the next: one block's shared memory, one cluster, one environment
+    per thread of the whole GPU, streamed from shared and from global memory, dealt by cell or not."""
+    w, h = (67, 70) if n <= 1024 else (120, 97)
+    cfg = world(pkg, w, h, n, env_offset=5)
     gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
     lockstep(gpu, cpu, 3, what="n=%d" % n)
-    gpu.train_steps(14); cpu.train_steps(14)             # one launch across a step cap that everybody reaches together
-    assert_same(gpu, cpu, "n=%d, many steps per launch" % n)
+    for k in (14, 70) if n < 200000 else (14,):          # many steps per launch: a step cap that everybody reaches together, a second dealing
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert_same(gpu, cpu, "n=%d, many steps per launch" % n)
     sa, sb = gpu.get_stats(), cpu.get_stats()
     assert (sa.conflicts, sa.goals, sa.timeouts, sa.device_error) == (sb.conflicts, sb.goals, sb.timeouts, 0)
 
 
-@pytest.mark.parametrize("n,kw", [(700, {}), (90000, {"legacy_clamp": 1}), (400000, {"start_mode": 0}), (2000, {"start_mode": 0, "max_steps": 0})])
-def test_gather_engine_common_start_traps_and_episode_epsilon(pkg, orc, n, kw):
+@pytest.mark.parametrize("n", [33, 5000, 80000])
+def test_crowded_cells_are_counted_alike(pkg, orc, n):
+    """Cells with more than 24 environments, whoever applies their updates: the number of such (cell, step) pairs and of the
+    environment-steps on them, against a count of the states the oracle went through."""
+    cfg = world(pkg, 9, 8, n, num_goals=1, obstacle_p=0.0, max_steps=0)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    cells = chained = 0
+    for _ in range(12):
+        x, y, _t = cpu.get_state()
+        c = np.bincount(y * 9 + x)
+        cells += int((c > 24).sum()); chained += int(c[c > 24].sum())
+        cpu.train_steps(1)
+    gpu.train_steps(12)
+    s = gpu.get_stats()
+    assert (s.long_chains, s.chained) == (cells, chained)
+    assert_same(gpu, cpu, "crowded")
+
+
+@pytest.mark.parametrize("h", [4722, 4723])
+def test_largest_world_of_one_block(pkg, orc, h):
+    cfg = world(pkg, 1, h, 300)
+    gpu, cpu = pair(pkg, orc, cfg)
+    gpu.train_steps(40); cpu.train_steps(40)
+    assert_same(gpu, cpu, "1 x %d" % h)
+
+
+@pytest.mark.parametrize("n,kw", [(700, {}), (3000, {}), (90000, {"legacy_clamp": 1}), (400000, {"start_mode": 0}), (2000, {"start_mode": 0, "max_steps": 0})])
+def test_common_start_traps_and_episode_epsilon(pkg, orc, n, kw):
     """Everybody on one start cell (whole warps count once), traps, the clamp, and the epsilon that follows the finished episodes."""
     cfg = world(pkg, 91, 93, n, eps_kind=pkg.EPS_MULT_PER_EPISODE, eps0=1.0, eps_decay=0.9, **kw)
     gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
