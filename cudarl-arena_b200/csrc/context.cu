@@ -113,7 +113,7 @@ struct cudarl_ctx {
     void *dent = nullptr, *dctl = nullptr, *deps = nullptr;
     void *dtra = nullptr, *dtrr = nullptr, *dtrd = nullptr, *dsckey = nullptr, *dscval = nullptr;
     void *dgather = nullptr;              // replica averaging: the other ranks' rows of this rank's slice
-    void* dub[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr}; size_t ub_cap = 0;   // update_batch staging
+    void* dub = nullptr; size_t ub_cap = 0;                               // the arrays of a large update_batch, and their bytes
     void* dact = nullptr;                 // actions of the host form of step_actions, where the stage is too small for them
     size_t ent_cap = 0, eps_cap = 0;
     float* h_eps = nullptr; size_t h_eps_cap = 0; cudaEvent_t ev_eps = nullptr; bool eps_inflight = false;
@@ -249,8 +249,8 @@ int alloc_hot(cudarl_ctx* c) {
     CK(cudaMemsetAsync(c->dci, 0, total, c->st));
     c->p.cw = (unsigned short*)c->dci;
     c->p.mailbox = (unsigned*)((char*)c->dci + ci_bytes); c->p.mb_slots = (unsigned)slots;
-    CK(cudaMalloc(&c->dactive, 3 * slots * sizeof(unsigned)));
-    c->p.active = (unsigned*)c->dactive; c->p.longq = (unsigned*)c->dactive + slots; c->p.longq2 = (unsigned*)c->dactive + 2 * slots;
+    CK(cudaMalloc(&c->dactive, 2 * slots * sizeof(unsigned)));
+    c->p.active = (unsigned*)c->dactive; c->p.longq = (unsigned*)c->dactive + slots;
     return 0;
 }
 
@@ -691,7 +691,7 @@ void free_all(cudarl_ctx* c) {
     if (c->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->comm);
     void* bufs[] = {c->dci, c->dstate[0], c->dstate[1], c->dimport, c->dactive, c->dreward, c->ddone, c->dent, c->dctl, c->deps,
                     c->dtra, c->dtrr, c->dtrd, c->dsckey, c->dscval, c->dgather, c->dact,
-                    c->dub[0], c->dub[1], c->dub[2], c->dub[3], c->dub[4], c->dub[5], c->dub[6],
+                    c->dub,
                     c->dQ, c->drec[0], c->drec[1], c->darr[0], c->darr[1], c->dovf[0], c->dovf[1], c->dbmax[0], c->dbmax[1],
                     c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dhop, c->dtq, c->dpeer_ptrs, c->dbarrier_word, c->dgbar, c->dgcnt, c->dgmv, c->dgstate, c->dgbins, c->dwork[0], c->dwork[1]};
     for (void* b : bufs) if (b) cudaFree(b);
@@ -987,29 +987,61 @@ int cudarl_update_batch(cudarl_ctx* c, int64_t n, const int32_t* sx, const int32
     if (n == 0) return 0;
     if (!sx || !sy || !a || !r || !nx || !ny || !dn) return fail(c, -1, "null argument");
     if (n >= (1ll << 26)) return fail(c, -1, "batch too large (at most 2^26 - 1 transitions per call)");
-    const int W = c->p.W, H = c->p.H;
-    for (int64_t i = 0; i < n; ++i)   // src/q_learning.cu:192-194,212-214 reject these; the reference kernel would read out of bounds
-        if (sx[i] < 0 || sx[i] >= W || sy[i] < 0 || sy[i] >= H || a[i] < 0 || a[i] >= CUDARL_ACTIONS ||
-            nx[i] < 0 || nx[i] >= W || ny[i] < 0 || ny[i] >= H) return fail(c, -3, "Invalid state or action");
     CK(cudaSetDevice(c->cfg.device));
-    { int rl = leave_tiles(c); if (rl) return rl; }
-    int rc = ensure_entry_capacity(c, (size_t)n); if (rc) return rc;
-    if ((size_t)n > c->ub_cap) {
+    { int rc = close_kernel_segment(c); if (rc) return rc; }
+    const size_t N = (size_t)n;
+    if (n > (int64_t)UPDATE_SMALL) { int rc = ensure_entry_capacity(c, N); if (rc) return rc; }
+    // Checked and packed to 12 bytes a transition on the way: into the mapped stage while they fit it (the kernel reads them across the
+    // link), else through the ring to the device.
+    struct Source { const int32_t *sx, *sy, *a, *nx, *ny; const uint8_t* dn; uint32_t W, H; std::atomic<bool> bad{false}; } src;
+    src.sx = sx; src.sy = sy; src.a = a; src.nx = nx; src.ny = ny; src.dn = dn; src.W = (uint32_t)c->p.W; src.H = (uint32_t)c->p.H;
+    const Fill pack_at = [](void* dst, size_t first, size_t bytes, const void* arg) {
+        Source& s = *(Source*)arg;
+        uint32_t* const o = (uint32_t*)dst; const size_t i0 = first / 4, m = bytes / 4;
+        uint32_t bad = 0;
+        for (size_t k = 0; k < m; ++k) {
+            const uint32_t x = (uint32_t)s.sx[i0 + k], y = (uint32_t)s.sy[i0 + k], act = (uint32_t)s.a[i0 + k];
+            bad |= (uint32_t)(x >= s.W) | (uint32_t)(y >= s.H) | (uint32_t)(act >= (uint32_t)CUDARL_ACTIONS);
+            o[k] = ((y * s.W + x) << 2) | (act & 3u) | (s.dn[i0 + k] ? 0x80000000u : 0u);
+        }
+        if (bad) s.bad = true;
+    };
+    const Fill pack_next = [](void* dst, size_t first, size_t bytes, const void* arg) {
+        Source& s = *(Source*)arg;
+        uint32_t* const o = (uint32_t*)dst; const size_t i0 = first / 4, m = bytes / 4;
+        uint32_t bad = 0;
+        for (size_t k = 0; k < m; ++k) {
+            const uint32_t x = (uint32_t)s.nx[i0 + k], y = (uint32_t)s.ny[i0 + k];
+            bad |= (uint32_t)(x >= s.W) | (uint32_t)(y >= s.H);
+            o[k] = y * s.W + x;
+        }
+        if (bad) s.bad = true;
+    };
+    const size_t part = up16(N * 4);
+    const bool small = STAGE_DATA + 3 * part <= STAGE_BYTES;
+    if (!small && 3 * part > c->ub_cap) {
         CK(cudaStreamSynchronize(c->st));
-        for (auto& b : c->dub) { if (b) cudaFree(b); b = nullptr; }
-        c->ub_cap = 0;
-        size_t cap = pow2ceil((size_t)n);
-        for (int k = 0; k < 7; ++k) CK(cudaMalloc(&c->dub[k], cap * 4));
+        cudaFree(c->dub); c->dub = nullptr; c->ub_cap = 0;
+        const size_t cap = pow2ceil(3 * part);
+        CK(cudaMalloc(&c->dub, cap));
         c->ub_cap = cap;
     }
-    const void* src[7] = {sx, sy, a, r, nx, ny, dn};
-    for (int k = 0; k < 7; ++k) CK(cudaMemcpyAsync(c->dub[k], src[k], (size_t)n * (k == 6 ? 1 : 4), cudaMemcpyHostToDevice, c->st));
+    unsigned char* const dev = small ? c->stage.dev + STAGE_DATA : (unsigned char*)c->dub;
+    Segment in[3];
+    for (int k = 0; k < 3; ++k) {
+        in[k].bytes = N * 4; in[k].arg = &src; in[k].fill = k == 0 ? pack_at : k == 1 ? pack_next : nullptr;
+        if (small) { in[k].host = c->stage.host + STAGE_DATA + k * part; in[k].dev = k == 2 ? const_cast<float*>(r) : nullptr; }
+        else { in[k].dev = dev + k * part; in[k].host = k == 2 ? const_cast<float*>(r) : nullptr; }
+    }
+    if (small) copy_host(in, 3, true); else CK(copy_in(in, 3, c->cfg.device, c->st));
+    // src/q_learning.cu:192-194,212-214 reject these; the reference kernel would read out of bounds
+    if (src.bad) return fail(c, -3, "Invalid state or action");
     c->p.step = (unsigned long long)c->h_step;
-    launch_update_batch(c->p, (unsigned)n, (const int*)c->dub[0], (const int*)c->dub[1], (const int*)c->dub[2], (const float*)c->dub[3],
-                        (const int*)c->dub[4], (const int*)c->dub[5], (const unsigned char*)c->dub[6], c->st);
+    const Transitions tr{(const unsigned*)dev, (const unsigned*)(dev + part), (const float*)(dev + 2 * part)};
+    launch_update_batch(c->p, (unsigned)n, tr, handover(c), c->st);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(c->st));
-    return 0;
+    if (c->tile_mode) { launch_tile_border(c->p, c->st); CK(cudaGetLastError()); }       // the records stay in their tiles; the table under them has changed
+    return wait_box(c);
 }
 
 int cudarl_get_state(cudarl_ctx* c, int32_t* x, int32_t* y, int32_t* t) {
@@ -1064,9 +1096,10 @@ int cudarl_get_q(cudarl_ctx* c, float* q) {
 int cudarl_set_q(cudarl_ctx* c, const float* q) {
     if (!c || !q) return fail(c, -1, "null argument");
     CK(cudaSetDevice(c->cfg.device));
-    { int rl = leave_tiles(c); if (rl) return rl; }
+    { int rc = close_kernel_segment(c); if (rc) return rc; }
     const Segment in{const_cast<float*>(q), c->p.Q, (size_t)c->p.S * sizeof(float4)};
     CK(copy_in(&in, 1, c->cfg.device, c->st));
+    if (c->tile_mode) { c->p.step = (unsigned long long)c->h_step; launch_tile_border(c->p, c->st); CK(cudaGetLastError()); }
     return 0;
 }
 

@@ -26,7 +26,7 @@ constexpr int SLOTS = 12, MAX_WORKERS = 7, MAX_DEVICES = 64;
 // Below this the driver copies: it is as fast as the ring up to there (B200 box: 2 MB in 0.12 ms either way, 4 MB 0.23 and 0.16).
 constexpr size_t SHARED_MIN_OUT = (size_t)768 << 10, SHARED_MIN_IN = (size_t)3 << 20;
 
-struct Chunk { unsigned char* host; unsigned char* dev; size_t bytes; };
+struct Chunk { unsigned char* host; unsigned char* dev; size_t bytes; Fill fill; const void* arg; size_t first; };
 enum class Way { Out, In, Host, HostIn };        // device -> caller, caller -> device, stage -> caller, caller -> stage
 
 // One transfer.  The caller's thread alone talks to the driver (several threads asking for events and enqueueing copies hold each
@@ -83,6 +83,17 @@ void copy_past_caches(unsigned char* d, const unsigned char* s, size_t n) {
 #endif
 }
 
+// A chunk on its way to the device: copied, or made in pieces that fit the first-level cache.
+void send(unsigned char* dst, const unsigned char* src, const Chunk& c) {
+    if (!c.fill) { copy_past_caches(dst, src, c.bytes); return; }
+    alignas(64) unsigned char part[8192];
+    for (size_t k = 0; k < c.bytes; k += sizeof(part)) {
+        const size_t b = std::min(sizeof(part), c.bytes - k);
+        c.fill(part, c.first + k, b, c.arg);
+        copy_past_caches(dst + k, part, b);
+    }
+}
+
 // Take and copy one chunk if one is ready.
 bool copy_one(Job& j) {
     size_t k = j.next.load(std::memory_order_relaxed);
@@ -95,9 +106,9 @@ bool copy_one(Job& j) {
     unsigned char* const buf = pool().ring + slot * SLOT_BYTES;
     switch (j.way) {
         case Way::Out: std::memcpy(c.host, buf, c.bytes); j.turn[slot].store(k + SLOTS, std::memory_order_release); break;
-        case Way::In: copy_past_caches(buf, c.host, c.bytes); j.filled[slot].store(k + 1, std::memory_order_release); break;
+        case Way::In: send(buf, c.host, c); j.filled[slot].store(k + 1, std::memory_order_release); break;
         case Way::Host: std::memcpy(c.host, c.dev, c.bytes); break;
-        case Way::HostIn: copy_past_caches(c.host, c.dev, c.bytes); break;
+        case Way::HostIn: send(c.host, c.dev, c); break;
     }
     j.done.fetch_add(1, std::memory_order_release);
     return true;
@@ -150,10 +161,11 @@ void cut(Job& j, const Segment* segs, int n, size_t most, size_t least) {
     while (piece > least && total / piece < 2u * (MAX_WORKERS + 1)) piece >>= 1;
     for (int s = 0; s < n; ++s) {
         unsigned char* h = (unsigned char*)segs[s].host; unsigned char* d = (unsigned char*)segs[s].dev;
-        for (size_t left = segs[s].bytes; left;) {
-            const size_t to_edge = piece - ((uintptr_t)h & (piece - 1)), b = std::min(left, to_edge);
-            j.chunks.push_back(Chunk{h, d, b});
-            h += b; d += b; left -= b;
+        const bool made = segs[s].fill != nullptr;
+        for (size_t first = 0; first < segs[s].bytes;) {
+            const size_t edge = piece - ((made ? first : (uintptr_t)h + first) & (piece - 1)), b = std::min(segs[s].bytes - first, edge);
+            j.chunks.push_back(Chunk{made && !h ? nullptr : h + first, made && !d ? nullptr : d + first, b, segs[s].fill, segs[s].arg, first});
+            first += b;
         }
     }
 }
@@ -209,9 +221,10 @@ cudaError_t run_job(Job& j, int device, cudaStream_t st) {
 
 cudaError_t copy_all(const Segment* segs, int n, bool out, int device, cudaStream_t st) {
     size_t total = 0;
-    for (int s = 0; s < n; ++s) total += segs[s].bytes;
+    bool made = false;
+    for (int s = 0; s < n; ++s) { total += segs[s].bytes; made |= segs[s].fill != nullptr; }
     Pool& p = pool();
-    if (total >= (out ? SHARED_MIN_OUT : SHARED_MIN_IN) && device >= 0 && device < MAX_DEVICES) {
+    if ((made || total >= (out ? SHARED_MIN_OUT : SHARED_MIN_IN)) && device >= 0 && device < MAX_DEVICES) {
         std::unique_lock<std::mutex> lk(p.use, std::try_to_lock);      // another thread's transfer has the ring: let the driver do this one
         if (lk.owns_lock()) {
             cudaError_t e = cudaStreamSynchronize(st);                 // do not spin through work enqueued earlier
@@ -225,6 +238,14 @@ cudaError_t copy_all(const Segment* segs, int n, bool out, int device, cudaStrea
         }
     }
     for (int s = 0; s < n; ++s) {
+        if (segs[s].fill) {                      // through pageable memory of our own
+            std::vector<unsigned char> made(segs[s].bytes);
+            segs[s].fill(made.data(), 0, segs[s].bytes, segs[s].arg);
+            cudaError_t e = cudaMemcpyAsync(segs[s].dev, made.data(), segs[s].bytes, cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            if (e != cudaSuccess) return e;
+            continue;
+        }
         const cudaError_t e = out ? cudaMemcpyAsync(segs[s].host, segs[s].dev, segs[s].bytes, cudaMemcpyDeviceToHost, st)
                                   : cudaMemcpyAsync(segs[s].dev, segs[s].host, segs[s].bytes, cudaMemcpyHostToDevice, st);
         if (e != cudaSuccess) return e;
@@ -288,7 +309,7 @@ void copy_host(const Segment* segs, int n, bool into_stage) {
         }
     }
     for (int s = 0; s < n; ++s)
-        if (into_stage) copy_past_caches((unsigned char*)segs[s].host, (const unsigned char*)segs[s].dev, segs[s].bytes);
+        if (into_stage) send((unsigned char*)segs[s].host, (const unsigned char*)segs[s].dev, Chunk{nullptr, nullptr, segs[s].bytes, segs[s].fill, segs[s].arg, 0});
         else std::memcpy(segs[s].host, segs[s].dev, segs[s].bytes);
 }
 cudaError_t copy_out(const Segment* segs, int n, int device, cudaStream_t st) { return copy_all(segs, n, true, device, st); }

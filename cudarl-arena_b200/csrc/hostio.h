@@ -12,7 +12,10 @@
 
 namespace cudarl {
 
-struct Segment { void* host; void* dev; size_t bytes; };
+// One array of a copy.  With `fill`, the bytes on their way to the device do not lie in the caller's memory: fill(dst, first, bytes, arg)
+// makes `bytes` of them from offset `first` on (both multiples of 4), called from several threads for different parts.
+typedef void (*Fill)(void* dst, size_t first, size_t bytes, const void* arg);
+struct Segment { void* host; void* dev; size_t bytes; Fill fill = nullptr; const void* arg = nullptr; };
 
 // One pinned block mapped into the device, for the small results and inputs of a context.
 constexpr size_t STAGE_BYTES = (size_t)1 << 20;

@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
     __shared__ float s_vals[LONG_SMEM];
     __shared__ unsigned s_medlen[MED_CHUNKS];
     __shared__ unsigned s_nmed;
-    const unsigned nactive = p.ctl->active_count[p.step & 1ull];      // slots that received a chain in this step
+    const unsigned nactive = p.ctl->active_count;      // slots that received a chain in this call
   for (unsigned tile = blockIdx.x; tile * BLOCK < nactive; tile += gridDim.x) {
     if (threadIdx.x == 0) s_nmed = 0;
     __syncthreads();
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
     const unsigned slot = ai < nactive ? p.active[ai] : 0u;
     const unsigned head = ai < nactive ? p.mailbox[slot] : 0u;
     if (head) {
-        p.mailbox[slot] = 0u;                          // leave the mailbox empty for the next step
+        p.mailbox[slot] = 0u;                          // leave the mailbox empty for the next call
         unsigned long long k8[SHORT_MAX]; float v8[SHORT_MAX];
         unsigned q = head, pos = 0, rem = 0; bool fresh = false;
 #pragma unroll
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
                 s_medlen[chunk] = staged ? L : 0u;
             }
             if (!staged) {                              // hand the chain to k_fix_long
-                const unsigned li = atomicAdd(&p.ctl->long_count[p.step & 1ull], 1u);
+                const unsigned li = atomicAdd(&p.ctl->long_count, 1u);
                 p.longq[li] = head;
             }
         }
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
 // Long chains (more than 32 entries: cells crowded with environments).  First tier: one WARP per chain for up
 // to 256 entries -- lane 0 hops from run to run, all lanes copy the run's entries into the warp's slice of
 // shared memory, a warp-wide bitonic sort orders them by (cell, action, id), the first lane of every cell run
-// applies it.  Chains that do not fit are queued for k_fix_long2 (one block per chain).
+// applies it.  Chains that do not fit are left to the block.
 constexpr unsigned WARP_LONG = 256;
 
 __device__ bool process_long_warp(const Params& p, unsigned head, unsigned long long* keys, float* vals) {
@@ -346,29 +346,35 @@ __device__ bool process_long_warp(const Params& p, unsigned head, unsigned long 
     return true;
 }
 
-__global__ void __launch_bounds__(BLOCK) k_fix_long(Params p) {
-    __shared__ unsigned long long s_keys[(BLOCK / 32) * WARP_LONG];
-    __shared__ float s_vals[(BLOCK / 32) * WARP_LONG];
-    const unsigned n = p.ctl->long_count[p.step & 1ull];
+// Eight chains at a time, one per warp; those too long for a warp are then taken one after the other by the whole block: any length,
+// in shared memory up to 1024 entries, in the global scratch beyond.  The last kernel of an update_batch: it clears the call's counters
+// and posts the box.
+__global__ void __launch_bounds__(BLOCK) k_fix_long(Params p, Handover h) {
+    constexpr unsigned WARPS = BLOCK / 32;
+    __shared__ unsigned long long s_keys[WARPS * WARP_LONG];
+    __shared__ float s_vals[WARPS * WARP_LONG];
+    __shared__ unsigned s_left[WARPS], s_bcast[3];
+    const unsigned n = p.ctl->long_count;
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     unsigned done = 0;
-    for (unsigned c = blockIdx.x * (BLOCK / 32) + warp; c < n; c += gridDim.x * (BLOCK / 32)) {
-        const unsigned head = p.longq[c];
-        if (!process_long_warp(p, head, s_keys + warp * WARP_LONG, s_vals + warp * WARP_LONG)) {
-            if (lane == 0) p.longq2[atomicAdd(&p.ctl->long2_count[p.step & 1ull], 1u)] = head;
+    for (unsigned c0 = blockIdx.x * WARPS; c0 < n; c0 += gridDim.x * WARPS) {
+        const unsigned c = c0 + warp;
+        unsigned left = 0u;
+        if (c < n) {
+            const unsigned head = p.longq[c];
+            if (!process_long_warp(p, head, s_keys + warp * WARP_LONG, s_vals + warp * WARP_LONG)) left = head;
+            ++done;
         }
-        ++done;
+        if (lane == 0u) s_left[warp] = left;
+        __syncthreads();
+        for (unsigned k = 0; k < WARPS; ++k) if (s_left[k]) process_long(p, s_left[k], s_keys, s_vals, s_bcast);
+        __syncthreads();
     }
     if (lane == 0 && done) atomicAdd(&p.ctl->long_chains, (unsigned long long)done);
-}
-
-// Second tier: one block per chain, any length (shared memory up to 1024 entries, the global scratch beyond).
-__global__ void __launch_bounds__(BLOCK) k_fix_long2(Params p) {
-    __shared__ unsigned long long s_keys[LONG_SMEM];
-    __shared__ float s_vals[LONG_SMEM];
-    __shared__ unsigned s_bcast[3];
-    const unsigned n = p.ctl->long2_count[p.step & 1ull];
-    for (unsigned c = blockIdx.x; c < n; c += gridDim.x) process_long(p, p.longq2[c], s_keys, s_vals, s_bcast);
+    if (last_to_finish<false>(p)) {
+        p.ctl->active_count = 0u; p.ctl->long_count = 0u; p.ctl->scratch_cursor = 0u;
+        box_put_error(p, h);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -411,38 +417,92 @@ __global__ void k_step_one(Params p, int action, bool reset, Handover h) {
     box_put_error(p, h);
 }
 
-__global__ void k_active_reset(Params p) { p.ctl->active_count[p.step & 1ull] = 0; p.ctl->long_count[p.step & 1ull] = 0; p.ctl->long2_count[p.step & 1ull] = 0; }
+// The three words of a transition, all on their way at once: left to the compiler, the second waits behind the branch on the first, and a
+// look-up across the link takes 2 us.
+__device__ __forceinline__ void load_transition(const Transitions& tr, unsigned i, unsigned& at, unsigned& next, float& r) {
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(at) : "l"(tr.at + i));
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(next) : "l"(tr.next + i));
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(tr.r + i));
+}
+// The TD target of a transition, from the table as it is before the call.
+__device__ __forceinline__ float transition_target(const Params& p, unsigned at, unsigned next, float r) {
+    float m = 0.0f;
+    if (!(at >> 31)) {
+        m = max4(__ldcg(p.Q + next));
+        if (p.legacy_clamp && m < 0.0f) m = 0.0f;
+    }
+    return __fmaf_rn(p.gamma, m, r);
+}
 
-// update_batch, phase 1: TD target of every transition from the table as it is now; every
-// transition becomes a collision entry (index order = fold order).
-__global__ void k_update_main(Params p, unsigned n, const int* sx, const int* sy, const int* act, const float* rew,
-                              const int* nxs, const int* nys, const unsigned char* dn) {
+// update_batch, phase 1: the TD target of every transition; every transition becomes a collision entry (index order = fold order).
+__global__ void k_update_main(Params p, unsigned n, Transitions tr) {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned lane = threadIdx.x & 31u;
-    if (i == 0) { p.ctl->scratch_cursor = 0; }     // the long-chain scratch is per call; nobody reads it in this kernel
     bool first = false; unsigned slot = 0;
     if (i < n) {
-        int x = sx[i], y = sy[i], a = act[i], nx = nxs[i], ny = nys[i];
-        unsigned s = (unsigned)y * (unsigned)p.W + (unsigned)x;
-        unsigned s2 = (unsigned)ny * (unsigned)p.W + (unsigned)nx;
-        float m = 0.0f;
-        if (!dn[i]) {
-            m = max4(__ldcg(p.Q + s2));
-            if (p.legacy_clamp && m < 0.0f) m = 0.0f;
-        }
-        float d = __fmaf_rn(p.gamma, m, rew[i]);           // TD target
-        slot = mb_slot(p, s);
-        unsigned prev = atomicExch(p.mailbox + slot, i + 1u);          // a run of one entry
-        p.ent[i] = make_uint4((s << 3) | (unsigned)a, i, __float_as_uint(d), prev);
+        unsigned at, next; float r;
+        load_transition(tr, i, at, next, r);
+        const float d = transition_target(p, at, next, r);
+        const unsigned cell = (at & 0x7FFFFFFFu) >> 2;
+        slot = mb_slot(p, cell);
+        const unsigned prev = atomicExch(p.mailbox + slot, i + 1u);              // a run of one entry
+        p.ent[i] = make_uint4((cell << 3) | (at & 3u), i, __float_as_uint(d), prev);
         first = prev == 0u;
     }
     const unsigned fm = __ballot_sync(FULL, first);                  // list the slots that just became active
     if (fm) {
         unsigned base = 0;
-        if (lane == __ffs(fm) - 1u) base = atomicAdd(&p.ctl->active_count[p.step & 1ull], __popc(fm));
+        if (lane == __ffs(fm) - 1u) base = atomicAdd(&p.ctl->active_count, __popc(fm));
         base = __shfl_sync(FULL, base, __ffs(fm) - 1);
         if (first) p.active[base + __popc(fm & ((1u << lane) - 1u))] = slot;
     }
+}
+
+// update_batch of up to 1,024 transitions in one block: targets, a bitonic sort by (cell, action, index) -- strides below a warp by
+// shuffle -- and the first of every run folds it.  One launch instead of three and nothing but latency: the inputs across the link, one
+// look-up of the next rows, the sort, one read and write of the entries.  KEY: 32 bits hold cell, action and index of grids of up to
+// 2^20 cells and halve the sort's shuffles.
+template <class KEY>
+__global__ void __launch_bounds__(UPDATE_SMALL) k_update_small(const __grid_constant__ Params p, unsigned n, const __grid_constant__ Transitions tr, Handover h) {
+    __shared__ KEY s_key[UPDATE_SMALL];
+    __shared__ float s_target[UPDATE_SMALL];
+    constexpr unsigned IDX = 10u, IDX_MASK = (1u << IDX) - 1u;
+    static_assert(UPDATE_SMALL == 1u << IDX, "index bits of the key");
+    const unsigned i = threadIdx.x;
+    KEY key = ~(KEY)0;
+    if (i < n) {
+        unsigned at, next; float r;
+        load_transition(tr, i, at, next, r);
+        s_target[i] = transition_target(p, at, next, r);
+        key = ((KEY)(at & 0x7FFFFFFFu) << IDX) | i;
+    }
+    for (unsigned k = 2u; k <= blockDim.x; k <<= 1)
+        for (unsigned j = k >> 1; j; j >>= 1) {
+            KEY other;
+            if (j >= 32u) {
+                __syncthreads();
+                s_key[i] = key;
+                __syncthreads();
+                other = s_key[i ^ j];
+            } else other = __shfl_xor_sync(FULL, key, j);
+            const bool low = ((i & k) == 0u) == ((i & j) == 0u);     // this place keeps the smaller of the two
+            key = (other < key) == low ? other : key;
+        }
+    __syncthreads();
+    s_key[i] = key;
+    __syncthreads();
+    const KEY at = key >> IDX;
+    if (key != ~(KEY)0 && (i == 0u || s_key[i - 1u] >> IDX != at)) {
+        float* const q = reinterpret_cast<float*>(p.Q) + at;
+        float v = *q;
+        for (unsigned j = i; j < blockDim.x; ++j) {
+            const KEY e = s_key[j];
+            if (e >> IDX != at) break;
+            v = __fmaf_rn(p.lr, __fsub_rn(s_target[(unsigned)e & IDX_MASK], v), v);      // each sees the value the one before it left
+        }
+        *q = v;
+    }
+    if (i == 0u) box_put_error(p, h);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -491,14 +551,17 @@ void launch_step_actions(const Params& p, const int* a, float* r, unsigned char*
     if (p.N) k_step_actions<<<nblk(p.N), BLOCK, 0, st>>>(p, a, r, d, h);
 }
 void launch_step_one(const Params& p, int action, bool reset, Handover h, cudaStream_t st) { k_step_one<<<1, 1, 0, st>>>(p, action, reset, h); }
-void launch_update_batch(const Params& p, unsigned n, const int* sx, const int* sy, const int* a, const float* r,
-                         const int* nx, const int* ny, const unsigned char* dn, cudaStream_t st) {
-    if (!n) return;
-    k_active_reset<<<1, 1, 0, st>>>(p);
-    k_update_main<<<nblk(n), BLOCK, 0, st>>>(p, n, sx, sy, a, r, nx, ny, dn);
+void launch_update_batch(const Params& p, unsigned n, const Transitions& tr, Handover h, cudaStream_t st) {
+    if (n <= UPDATE_SMALL) {
+        unsigned threads = 32u; while (threads < n) threads <<= 1;
+        // strictly below 2^20 cells: no key of 32 bits is the padding's all-ones word
+        if (p.S < (1u << 20)) k_update_small<unsigned><<<1, threads, 0, st>>>(p, n, tr, h);
+        else k_update_small<unsigned long long><<<1, threads, 0, st>>>(p, n, tr, h);
+        return;
+    }
+    k_update_main<<<nblk(n), BLOCK, 0, st>>>(p, n, tr);
     k_fix<<<fix_blocks(p), BLOCK, 0, st>>>(p);
-    k_fix_long<<<296, BLOCK, 0, st>>>(p);
-    k_fix_long2<<<296, BLOCK, 0, st>>>(p);
+    k_fix_long<<<296, BLOCK, 0, st>>>(p, h);
 }
 void launch_q_init(const Params& p, int kind, float scale, cudaStream_t st) { k_q_init<<<nblk(p.S), BLOCK, 0, st>>>(p, kind, scale); }
 void launch_cell_set(const Params& p, unsigned cell, unsigned cls, int clear_goals, cudaStream_t st) {

@@ -29,10 +29,9 @@ struct Ctl {
     unsigned int eps_mode;          // 0 fixed index, 1 advance by one per step, 2 per-episode index
     unsigned int eps_len;           // table length (clamp)
     unsigned long long eps_base_k;  // per-episode mode: table[0] belongs to episodes/N == eps_base_k
-    unsigned int active_count[2];   // mailbox slots holding a chain, per step parity
-    unsigned int long_count[2];     // chains queued for the warp-per-chain kernel, per step parity
-    unsigned int long2_count[2];    // chains too long for a warp, queued for the block-per-chain kernel
-    unsigned int scratch_cursor;    // bump allocator of the long-chain scratch, reset every step
+    unsigned int active_count;      // update_batch: mailbox slots holding a chain,
+    unsigned int long_count;        // chains left to k_fix_long,
+    unsigned int scratch_cursor;    // bump allocator of the long-chain scratch: all zero between calls
     unsigned int error;             // sticky internal error bits
     unsigned int never;             // zero for good: what a wait that a test makes run out looks at
     float eps_used;                 // epsilon of the most recent step (for the stats call)
@@ -123,8 +122,7 @@ struct Params {
     unsigned* mailbox;     // update_batch: chain heads (0 = empty), power-of-two size
     unsigned mb_slots;     // mailbox slots (power of two, multiple of BLOCK)
     unsigned* active;      // list of the mailbox slots that hold a chain in this step (mb_slots entries)
-    unsigned* longq;       // heads of the chains left to the warp-per-chain kernel (mb_slots entries)
-    unsigned* longq2;      // heads of the chains left to the block-per-chain kernel (mb_slots entries)
+    unsigned* longq;       // heads of the chains left to k_fix_long (mb_slots entries)
     Ctl* ctl;
     const float* eps_tab;
     int* tr_a; float* tr_r; unsigned char* tr_d;   // optional trace of the last step, per ENVIRONMENT
@@ -149,8 +147,11 @@ void launch_import_state(const Params& p, const int* x, const int* y, const int*
 void launch_reset_all(const Params& p, cudaStream_t st);
 void launch_step_actions(const Params& p, const int* d_actions, float* d_rewards, unsigned char* d_dones, Handover h, cudaStream_t st);
 void launch_step_one(const Params& p, int action, bool reset, Handover h, cudaStream_t st);        // one environment: words 1-4 = x, y, reward bits, done
-void launch_update_batch(const Params& p, unsigned n, const int* sx, const int* sy, const int* a, const float* r,
-                         const int* nx, const int* ny, const unsigned char* dn, cudaStream_t st);
+// update_batch: transitions checked and packed by the host, in device memory or in the mapped stage -- cell * 4 + action with bit 31 =
+// the episode ended there; next cell; reward.  The box is posted when the table is updated.
+struct Transitions { const unsigned* at; const unsigned* next; const float* r; };
+constexpr unsigned UPDATE_SMALL = 1024u;
+void launch_update_batch(const Params& p, unsigned n, const Transitions& tr, Handover h, cudaStream_t st);
 void launch_q_init(const Params& p, int kind, float scale, cudaStream_t st);
 // greedy rollout (rollout.cu); hop: one word per cell, scratch; words 1-4 = environments that reached a goal, steps taken, low halves first
 void launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st);
