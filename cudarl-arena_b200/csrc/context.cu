@@ -96,7 +96,7 @@ struct cudarl_ctx {
     void *dci = nullptr, *dreward = nullptr, *ddone = nullptr;
     void *dstate[2] = {nullptr, nullptr};   // int4 {x,y,t,id} per environment, and a scratch copy of the same size
     void *dimport = nullptr;              // staging for caller state arrays (3 x N int32)
-    void *dactive = nullptr;
+    void *dmail = nullptr;                // update_batch: chain heads and work lists
     // tile engine (the layout the train step runs on)
     void *dQ = nullptr;                    // the table (padded so that it splits into equal slices for any number of ranks)
     void *drec[2] = {nullptr, nullptr}, *darr[2] = {nullptr, nullptr}, *dovf[2] = {nullptr, nullptr}, *dbmax[2] = {nullptr, nullptr};
@@ -223,34 +223,37 @@ int upload_cells(cudarl_ctx* c) {
     return 0;
 }
 
-// (Re)allocate the collision entry array and the long-chain scratch for `cap` entries.
-int ensure_entry_capacity(cudarl_ctx* c, size_t cap) {
-    if (cap <= c->ent_cap) return 0;
+// The work area of an update_batch of `n` transitions that one block does not hold: collision entries, chain heads and work lists,
+// the scratch of the longest chains.  Grown to the next power of two, kept until the context goes.  As many chain heads as transitions
+// (but no more than cells): a chain then holds one cell's transitions; with 65,536 heads for a million of them, 16 cells shared one and
+// the chains became long ones (320 us in k_fix_long for 1,000,003 transitions on 1024 x 1024 cells).
+int ensure_entry_capacity(cudarl_ctx* c, size_t n) {
+    if (n <= c->ent_cap) return 0;
     CK(cudaStreamSynchronize(c->st));
-    cudaFree(c->dent); cudaFree(c->dsckey); cudaFree(c->dscval);
-    c->dent = c->dsckey = c->dscval = nullptr; c->ent_cap = 0;
-    size_t sc = 2 * pow2ceil(cap); if (sc < 4096) sc = 4096;
+    cudaFree(c->dent); cudaFree(c->dsckey); cudaFree(c->dscval); cudaFree(c->dmail);
+    c->dent = c->dsckey = c->dscval = c->dmail = nullptr; c->ent_cap = 0;
+    const size_t cap = pow2ceil(std::max<size_t>(n, 4096)), scratch = 2 * cap;
+    size_t slots = std::min(cap, pow2ceil(c->p.S));
+    slots = std::min<size_t>(std::max<size_t>(slots, BLOCK), (size_t)1 << 24);
     CK(cudaMalloc(&c->dent, cap * sizeof(uint4)));
-    CK(cudaMalloc(&c->dsckey, sc * sizeof(unsigned long long)));
-    CK(cudaMalloc(&c->dscval, sc * sizeof(float)));
+    CK(cudaMalloc(&c->dsckey, scratch * sizeof(unsigned long long)));
+    CK(cudaMalloc(&c->dscval, scratch * sizeof(float)));
+    CK(cudaMalloc(&c->dmail, 3 * slots * sizeof(unsigned)));
+    CK(cudaMemsetAsync(c->dmail, 0, slots * sizeof(unsigned), c->st));
     c->p.ent = (uint4*)c->dent;
-    c->p.sc_key = (unsigned long long*)c->dsckey; c->p.sc_val = (float*)c->dscval; c->p.sc_cap = (unsigned)sc;
+    c->p.sc_key = (unsigned long long*)c->dsckey; c->p.sc_val = (float*)c->dscval; c->p.sc_cap = (unsigned)scratch;
+    c->p.mailbox = (unsigned*)c->dmail; c->p.mb_slots = (unsigned)slots;
+    c->p.active = c->p.mailbox + slots; c->p.longq = c->p.mailbox + 2 * slots;
     c->ent_cap = cap; c->p.ent_cap = (unsigned)cap;
     return 0;
 }
 
-// The per-cell class words, and the chain heads / work lists of update_batch.
-int alloc_hot(cudarl_ctx* c) {
-    const size_t S = c->p.S, N = c->p.N ? c->p.N : 1;
-    const size_t ci_bytes = (2 * S + 255) / 256 * 256;      // one 16-bit word per cell
-    size_t slots = pow2ceil(N) / 2; if (slots < (1u << 16)) slots = 1u << 16; if (slots > (1u << 24)) slots = 1u << 24;
-    const size_t total = ci_bytes + slots * sizeof(unsigned);
-    CK(cudaMalloc(&c->dci, total));
-    CK(cudaMemsetAsync(c->dci, 0, total, c->st));
+// The per-cell class words.
+int alloc_cells(cudarl_ctx* c) {
+    const size_t bytes = (2 * (size_t)c->p.S + 255) / 256 * 256;      // one 16-bit word per cell
+    CK(cudaMalloc(&c->dci, bytes));
+    CK(cudaMemsetAsync(c->dci, 0, bytes, c->st));
     c->p.cw = (unsigned short*)c->dci;
-    c->p.mailbox = (unsigned*)((char*)c->dci + ci_bytes); c->p.mb_slots = (unsigned)slots;
-    CK(cudaMalloc(&c->dactive, 2 * slots * sizeof(unsigned)));
-    c->p.active = (unsigned*)c->dactive; c->p.longq = (unsigned*)c->dactive + slots;
     return 0;
 }
 
@@ -689,7 +692,7 @@ void free_all(cudarl_ctx* c) {
     if (c->st) cudaStreamSynchronize(c->st);
     for (size_t r = 0; r < c->peer_tables.size(); ++r) if ((int)r != c->rank && c->peer_tables[r]) cudaIpcCloseMemHandle(c->peer_tables[r]);
     if (c->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->comm);
-    void* bufs[] = {c->dci, c->dstate[0], c->dstate[1], c->dimport, c->dactive, c->dreward, c->ddone, c->dent, c->dctl, c->deps,
+    void* bufs[] = {c->dci, c->dstate[0], c->dstate[1], c->dimport, c->dmail, c->dreward, c->ddone, c->dent, c->dctl, c->deps,
                     c->dtra, c->dtrr, c->dtrd, c->dsckey, c->dscval, c->dgather, c->dact,
                     c->dub,
                     c->dQ, c->drec[0], c->drec[1], c->darr[0], c->darr[1], c->dovf[0], c->dovf[1], c->dbmax[0], c->dbmax[1],
@@ -758,7 +761,7 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
             CK(cudaEventCreateWithFlags(&c->ev_eps, cudaEventDisableTiming));
             CK(cudaEventCreate(&c->ev0)); CK(cudaEventCreate(&c->ev1));
             const size_t N = p.N ? p.N : 1;
-            { int r0 = alloc_hot(c); if (r0) return r0; }
+            { int r0 = alloc_cells(c); if (r0) return r0; }
             for (int cp = 0; cp < 2; ++cp) { CK(cudaMalloc(&c->dstate[cp], N * 16)); CK(cudaMemsetAsync(c->dstate[cp], 0, N * 16, c->st)); }
             CK(cudaMalloc(&c->dctl, sizeof(Ctl)));
             CK(cudaMemsetAsync(c->dctl, 0, sizeof(Ctl), c->st));
@@ -767,7 +770,7 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
             hostio_retain(); c->retained = true;
             CK(stage_take(&c->stage));
             c->box = (HostBox*)c->stage.host;
-            int r2 = ensure_entry_capacity(c, N); if (r2) return r2;
+            int r2;
             r2 = alloc_table(c); if (r2) return r2;
             c->gather = use_gather(c);
             r2 = c->gather ? alloc_gather(c) : alloc_tiles(c); if (r2) return r2;
