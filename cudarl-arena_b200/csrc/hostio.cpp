@@ -15,14 +15,14 @@
 namespace cudarl {
 namespace {
 
-// A slot is one huge page of the caller's array where that is made of huge pages: each is faulted in by one core.  Twelve slots keep
-// eight cores and the copy engine busy.  Measured on the B200 box (16 cores, 268 MB into a fresh NumPy array): 56 ms through the
-// driver, 10 ms with 8 copying threads, no gain from 12 or 16.
+// A slot is one huge page of the caller's array where that is made of huge pages: each is faulted in by one core.  Twenty slots keep
+// twelve cores and the copy engine busy.  Measured on the B200 box (16 cores, 268 MB into a fresh NumPy array): 56 ms through the
+// driver, 9.6 ms with 8 copying threads, 7.5 with 12; into memory that has been written before 5.6 either way, the speed of the link.
 constexpr size_t SLOT_BYTES = (size_t)2 << 20;
 constexpr size_t PIECE_MIN = (size_t)128 << 10;
 // Copies within the host between a stage and the caller: shared from a quarter of a megabyte on.
 constexpr size_t HOST_MIN = (size_t)256 << 10, HOST_PIECE = (size_t)32 << 10;
-constexpr int SLOTS = 12, MAX_WORKERS = 7, MAX_DEVICES = 64;
+constexpr int SLOTS = 20, MAX_WORKERS = 11, MAX_DEVICES = 64;
 // Below this the driver copies: it is as fast as the ring up to there (B200 box: 2 MB in 0.12 ms either way, 4 MB 0.23 and 0.16).
 constexpr size_t SHARED_MIN_OUT = (size_t)768 << 10, SHARED_MIN_IN = (size_t)3 << 20;
 
@@ -142,7 +142,7 @@ void worker_main() {
 void ready_workers() {
     Pool& p = pool();
     if (!p.workers.empty()) return;
-    const int n = std::min(MAX_WORKERS, (int)std::thread::hardware_concurrency() / 2 - 1);
+    const int n = std::min(MAX_WORKERS, (int)std::thread::hardware_concurrency() * 3 / 4 - 1);      // with the caller three quarters of the cores
     p.stop = false;
     for (int k = 0; k < n; ++k) p.workers.emplace_back(worker_main);
 }
