@@ -9,8 +9,8 @@
 //   k_rollout_walk    one thread per environment draws its start cell and hops from tile to tile over those words; a path that
 //                     comes back to an earlier tile entry (Brent's cycle search over the hops) never ends.
 //
-// What bounds it: k_rollout_tiles streams the table once (16 bytes in, 4 out per cell) and the doubling (5-7 rounds of one
-// shared-memory look-up per cell: a round in which nothing changed is the last) runs behind other blocks' loads; k_rollout_walk
+// What bounds it: k_rollout_tiles streams the table once (16 bytes in, 4 out per cell) and the doubling (one
+// shared-memory look-up per cell and round, until a round finds no path to end) runs behind other blocks' loads; k_rollout_walk
 // is a few scattered 4-byte look-ups per environment.  B200, 4096 x 4096 cells, 4,194,304 environments, 1000 steps: see the
 // figures at the two kernels; the walk over single cells it replaces took 13.55 ms (1000 scattered byte loads per environment).
 //
@@ -23,24 +23,29 @@ namespace cudarl {
 // Word of a cell.  While the tile is folded: kind LIVE, bits 0-11 the cell reached after 2^round steps.  Final: EXIT with the number
 // of steps in bits 0-12, the edge it leaves by (0 up, 1 right, 2 down, 3 left) in bits 22-23 and the place along it in bits 16-21;
 // GOAL with the number of steps; or TRAPPED.  A path without a circle has at most 4096 steps inside a tile.
-constexpr unsigned RT_SHIFT = 6u, RT = 1u << RT_SHIFT, RT_CELLS = RT * RT, RT_THREADS = 512u, RT_PER = RT_CELLS / RT_THREADS;
+constexpr unsigned RT_SHIFT = 6u, RT = 1u << RT_SHIFT, RT_CELLS = RT * RT, RT_THREADS = 512u, RT_PER = RT_CELLS / RT_THREADS, RT_ROWS = RT_THREADS / RT;
 constexpr unsigned KIND_LIVE = 0u, KIND_EXIT = 1u << 30, KIND_GOAL = 2u << 30, KIND_MASK = 3u << 30, TRAPPED = 0u, STEPS_MASK = 0x1FFFu;
 
 __global__ void __launch_bounds__(RT_THREADS) k_rollout_tiles(const __grid_constant__ Params p, unsigned* __restrict__ hop) {
     __shared__ unsigned s_w[RT_CELLS];
     const int x0 = (int)(blockIdx.x << RT_SHIFT), y0 = (int)(blockIdx.y << RT_SHIFT);
     unsigned cur[RT_PER];
+    const unsigned lx = threadIdx.x & (RT - 1u), ly0 = threadIdx.x >> RT_SHIFT;          // a thread's cells lie below one another, 8 rows apart
+    const int x = x0 + (int)lx;
+    const float4* const q = p.Q + (size_t)(y0 + (int)ly0) * (size_t)p.W + (size_t)x;
+    const MoveColumn moves(p, (unsigned)x);
+    const bool inside = x0 + (int)RT <= p.W && y0 + (int)RT <= p.H;                       // the same for the whole block
 #pragma unroll
     for (unsigned k = 0; k < RT_PER; ++k) {
-        const unsigned ic = k * RT_THREADS + threadIdx.x, lx = ic & (RT - 1u), ly = ic >> RT_SHIFT;
-        const int x = x0 + (int)lx, y = y0 + (int)ly;
+        const unsigned ly = ly0 + k * RT_ROWS, ic = (ly << RT_SHIFT) | lx;
+        const int y = y0 + (int)ly;
         unsigned w = KIND_LIVE | ic;
-        if (x < p.W && y < p.H) {
-            const float4 row = __ldcs(p.Q + (size_t)y * (size_t)p.W + (size_t)x);
-            const unsigned mvb = move_byte(p, x, y);
-            const unsigned a = (unsigned)argmax4(row);
-            if ((mvb >> (4u + a)) & 1u) w = KIND_GOAL | 1u;
-            else if (!((mvb >> a) & 1u)) {
+        if (inside || (x < p.W && y < p.H)) {
+            const float4 row = __ldcs(q + (size_t)(k * RT_ROWS) * (size_t)p.W);
+            const unsigned mvb = moves.at((unsigned)y);
+            const unsigned a = (unsigned)argmax4(row), mv = mvb >> a;
+            if (mv & 16u) w = KIND_GOAL | 1u;
+            else if (!(mv & 1u)) {
                 const unsigned mx = lx + (a == 1u) - (a == 3u), my = ly + (a == 2u) - (a == 0u);       // wraps when the move leaves the tile
                 w = (mx | my) < RT ? (KIND_LIVE | (my << RT_SHIFT) | mx) : (KIND_EXIT | (a << 22) | (((a & 1u) ? ly : lx) << 16) | 1u);
             }
@@ -49,15 +54,17 @@ __global__ void __launch_bounds__(RT_THREADS) k_rollout_tiles(const __grid_const
     }
     __syncthreads();
     for (unsigned len = 1u; len <= RT_CELLS; len <<= 1) {
-        bool changed = false;
+        bool found = false;
 #pragma unroll
         for (unsigned k = 0; k < RT_PER; ++k) {
             if ((cur[k] & KIND_MASK) != KIND_LIVE) continue;
             const unsigned w = s_w[cur[k]], nw = (w & KIND_MASK) == KIND_LIVE ? w : w + len;
-            changed |= nw != cur[k];
+            found |= nw != w;
             cur[k] = nw;
         }
-        if (!__syncthreads_or(changed)) break;              // every path that is still inside stands still or runs in a circle
+        // No path was found to end: none of the rest does.  (Had a live cell a way out, some cell on that way would be between 1 and 2 times
+        // `len` steps from its end, and would have found it in this round.)
+        if (!__syncthreads_or(found)) break;
 #pragma unroll
         for (unsigned k = 0; k < RT_PER; ++k) s_w[k * RT_THREADS + threadIdx.x] = cur[k];
         __syncthreads();

@@ -50,14 +50,17 @@ __device__ __forceinline__ float u01(unsigned w) { return (float)(w >> 8) * 5.96
 
 __device__ __forceinline__ unsigned cw_load(const unsigned short* cw, unsigned cell) { return cw[cell]; }
 
-// The move byte of a cell (written tile by tile by k_te_cls, row by row by k_gather_moves, for the engine in use): bit a = a move in direction a is blocked, bit 4+a = the cell an
-// environment stands on after choosing a is a goal.
-__device__ __forceinline__ unsigned move_byte(const Params& p, int x, int y) {
-    if (p.gp.mv) return __ldg(p.gp.mv + (size_t)y * (size_t)p.W + (size_t)x);
-    const TileP& tp = p.tp;
-    const unsigned m = tp.T - 1u, tile = ((unsigned)y >> tp.tshift) * tp.tiles_x + ((unsigned)x >> tp.tshift);
-    return __ldg(tp.tcls + (size_t)tile * tp.cls_stride + ((((unsigned)y & m) << tp.tshift) | ((unsigned)x & m)));
-}
+// The move bytes of the cells of a column (written tile by tile by k_te_cls, row by row by k_gather_moves, for the engine in use): bit a
+// = a move in direction a is blocked, bit 4+a = the cell an environment stands on after choosing a is a goal.
+struct MoveColumn {
+    const unsigned char* at_x; unsigned tall, mask, shift;           // a row of tiles (or of cells) is `tall` bytes
+    __device__ __forceinline__ MoveColumn(const Params& p, unsigned x) {
+        const TileP& tp = p.tp;
+        if (p.gp.mv) { at_x = p.gp.mv + x; tall = (unsigned)p.W; mask = 0u; shift = 0u; }
+        else { mask = tp.T - 1u; shift = tp.tshift; tall = tp.tiles_x * tp.cls_stride; at_x = tp.tcls + (x >> shift) * tp.cls_stride + (x & mask); }
+    }
+    __device__ __forceinline__ unsigned at(unsigned y) const { return __ldg(at_x + ((y >> shift) * tall + ((y & mask) << shift))); }
+};
 
 __device__ __forceinline__ void box_put(const Handover& h, unsigned k, unsigned v) {
     *reinterpret_cast<volatile unsigned long long*>(&h.box->w[k]) = ((unsigned long long)h.ticket << 32) | v;
