@@ -8,7 +8,7 @@
 // What bounds it: one block's issue slots, about 300 instructions per warp and step.  B200, us per step, here / gather engine: one
 // environment 0.59 / 3.0, 200 on 20 x 20 cells 1.1 / 4.7, 1,000 on 32 x 32 2.2 / 4.7; 4,096 on 64 x 64 16 / 4.7.  The same spread over
 // the distributed shared memory of a cluster was no faster than L2 (4,096 on 64 x 64: 4.4 with 16 blocks; scattered 16-byte accesses to
-// other blocks' shared memory are served one by one).
+// other blocks' shared memory are served one by one), nor with a copy of the table in every block (3.9: every update is then stored 8 times).
 #include "step_loop.cuh"
 
 namespace cudarl {
@@ -19,6 +19,7 @@ constexpr unsigned ARENA_ENVS = 1024u;
 inline size_t arena_bytes(unsigned S) { return (size_t)S * 48u + (S + 15u) / 16u * 16u; }
 
 struct ArenaSpace {
+    static constexpr bool ALONE = true;
     float4* rows; unsigned* counters; const unsigned char* mv; unsigned S;
     __device__ __forceinline__ float4 row(unsigned s) const { return rows[s]; }
     __device__ __forceinline__ unsigned moves(unsigned s) const { return mv[s]; }
@@ -52,6 +53,11 @@ __global__ void __launch_bounds__(AB, 1) k_arena_steps(const __grid_constant__ P
     for (unsigned s = threadIdx.x; s < S; s += AB) p.Q[s] = rows[s];
 }
 
+template <unsigned AB>
+static bool allow() {
+    return cudaFuncSetAttribute((const void*)k_arena_steps<AB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ARENA_MOST) == cudaSuccess &&
+           cudaFuncSetAttribute((const void*)k_arena_steps<AB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ARENA_MOST) == cudaSuccess;
+}
 // One block holds up to 1,024 environments at one per thread; twice that takes longer than the gather engine.
 bool arena_plan(Params& p) {
     GatherP& gp = p.gp;
@@ -59,18 +65,15 @@ bool arena_plan(Params& p) {
     if (n > ARENA_ENVS || arena_bytes(p.S) > ARENA_MOST) return false;
     gp.threads = n <= 32u ? 32u : n <= 256u ? 256u : 1024u;
     gp.chunk = gp.threads; gp.grid = 1u; gp.arena = 1u;
-    return true;
+    return allow<32u>() && allow<256u>() && allow<1024u>();
 }
 
-template <unsigned AB, bool PLAIN>
-static cudaError_t launch_two(const Params& p, const StepLaunch& l, cudaStream_t st) {
-    const cudaError_t e = cudaFuncSetAttribute((const void*)k_arena_steps<AB, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ARENA_MOST);
-    if (e != cudaSuccess) return e;
-    k_arena_steps<AB, PLAIN><<<1, AB, arena_bytes(p.S), st>>>(p, l);
+template <unsigned AB>
+static cudaError_t launch_one(const Params& p, const StepLaunch& l, cudaStream_t st) {
+    if (plain(p, l)) k_arena_steps<AB, true><<<1, AB, arena_bytes(p.S), st>>>(p, l);
+    else             k_arena_steps<AB, false><<<1, AB, arena_bytes(p.S), st>>>(p, l);
     return cudaGetLastError();
 }
-template <unsigned AB>
-static cudaError_t launch_one(const Params& p, const StepLaunch& l, cudaStream_t st) { return plain(p, l) ? launch_two<AB, true>(p, l, st) : launch_two<AB, false>(p, l, st); }
 cudaError_t launch_arena_steps(const Params& p, const StepLaunch& l, cudaStream_t st) {
     return p.gp.threads == 32u ? launch_one<32u>(p, l, st) : p.gp.threads == 256u ? launch_one<256u>(p, l, st) : launch_one<1024u>(p, l, st);
 }

@@ -124,6 +124,10 @@ struct cudarl_ctx {
     int eps_mode = 0;                     // 0 one fixed value, 1 table indexed by step of the call, 2 per-episode (device index)
     float eps_used = 0.0f;
     double eps_running = 1.0;
+    // per-episode schedule: finished episodes as last seen, the step they were seen at; epsilon after so many decays; the table uploaded last
+    uint64_t ep_seen = 0; int64_t ep_seen_step = 0;
+    uint64_t eps_chain_k = 0; double eps_chain_e = 1.0;
+    uint64_t eps_base_k = 0; uint32_t eps_len = 1;
     int64_t eval_calls = 0;
     bool trace = false;
     // communicator
@@ -360,7 +364,9 @@ int check_posted_error(cudarl_ctx* c) {
 int wait_counters(cudarl_ctx* c) {
     launch_post(c->p, handover(c), c->st);
     CK(cudaGetLastError());
-    return wait_box(c, 13);
+    { int rw = wait_box(c, 13); if (rw) return rw; }
+    c->ep_seen = box64(c, 1); c->ep_seen_step = c->h_step;
+    return 0;
 }
 // Device arrays into the caller's: through the stage when they are small (one kernel, no copies), else through the pinned ring.
 int hand_out(cudarl_ctx* c, const Segment* segs, int n) {
@@ -652,7 +658,7 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         c->p.step = (unsigned long long)c->h_step;
         c->p.eps_idx = c->eps_mode == 1 ? (unsigned)k : 0u;
         StepLaunch l{};
-        l.steps = (unsigned)m; l.chunk = c->p.gp.chunk; l.barrier_base = c->barrier_base; l.eps_mode = c->eps_mode; l.trace = c->trace ? 1 : 0;
+        l.steps = (unsigned)m; l.chunk = c->p.gp.chunk; l.barrier_base = c->barrier_base; l.eps_mode = c->eps_mode; l.trace = c->trace ? 1 : 0; l.eps_len = c->eps_len; l.eps_base_k = c->eps_base_k;
         l.in = c->dealt >= 0 ? (const int4*)c->dwork[c->dealt] : c->p.st; l.out = deal ? (int4*)c->dwork[c->dealt == 0 ? 1 : 0] : c->p.st;
         CK(c->p.gp.arena ? launch_arena_steps(c->p, l, c->st) : launch_gather_steps(c->p, l, c->st));
         c->barrier_base += c->p.gp.grid * gather_barriers(l);
@@ -788,7 +794,7 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
         rc = body();
     } while (0);
     if (rc) { g_err = c->err; free_all(c); delete c; return rc; }
-    c->eps_running = (double)f->eps0;
+    c->eps_running = c->eps_chain_e = (double)f->eps0;
     *out = c;
     return 0;
 }
@@ -904,7 +910,7 @@ int cudarl_train_steps(cudarl_ctx* c, int64_t n) {
     if (f.eps_kind == CUDARL_EPS_FIXED) {
         if (!c->eps_fixed_valid) {
             float e = (float)f.eps0; rc = upload_eps(c, &e, 1); if (rc) return rc;
-            k_ctl_eps<<<1, 1, 0, c->st>>>(c->p.ctl, 0u, 1u, 0ull);
+            if (!c->gather) k_ctl_eps<<<1, 1, 0, c->st>>>(c->p.ctl, 0u, 1u, 0ull);
             c->eps_fixed_valid = true;
         }
         c->eps_mode = 0;
@@ -919,17 +925,20 @@ int cudarl_train_steps(cudarl_ctx* c, int64_t n) {
             }
         }
         rc = upload_eps(c, tab.data(), (size_t)n); if (rc) return rc;
-        k_ctl_eps<<<1, 1, 0, c->st>>>(c->p.ctl, 1u, (unsigned)n, 0ull);
+        if (!c->gather) k_ctl_eps<<<1, 1, 0, c->st>>>(c->p.ctl, 1u, (unsigned)n, 0ull);
         c->eps_mode = 1;
     } else {  // per episode: index = episodes finished / environments, resolved on the device every step
-        { int rw = wait_counters(c); if (rw) return rw; }
-        unsigned long long k0 = box64(c, 1) / (unsigned long long)c->p.N;
-        std::vector<float> tab((size_t)n + 1);
-        double e = (double)f.eps0;
-        for (unsigned long long j = 0; j < k0; ++j) e *= (double)f.eps_decay;
-        for (int64_t k = 0; k <= n; ++k) { tab[k] = (float)e; e *= (double)f.eps_decay; }
-        rc = upload_eps(c, tab.data(), (size_t)n + 1); if (rc) return rc;
-        k_ctl_eps<<<1, 1, 0, c->st>>>(c->p.ctl, 2u, (unsigned)(n + 1), k0);
+        // The table starts at the episodes the host last saw: they grow by at most one per environment and step, so it reaches far enough
+        // without asking the device -- unless that was long ago.  (The tile engine starts from index 0: it needs to know.)
+        if (!c->gather || c->h_step - c->ep_seen_step > 4096) { int rw = wait_counters(c); if (rw) return rw; }
+        const uint64_t k0 = c->ep_seen / (uint64_t)c->p.N;
+        for (; c->eps_chain_k < k0; ++c->eps_chain_k) c->eps_chain_e *= (double)f.eps_decay;
+        std::vector<float> tab((size_t)(c->h_step - c->ep_seen_step + n + 2));
+        double e = c->eps_chain_e;
+        for (auto& v : tab) { v = (float)e; e *= (double)f.eps_decay; }
+        rc = upload_eps(c, tab.data(), tab.size()); if (rc) return rc;
+        c->eps_base_k = k0; c->eps_len = (uint32_t)tab.size();
+        if (!c->gather) k_ctl_eps<<<1, 1, 0, c->st>>>(c->p.ctl, 2u, c->eps_len, k0);
         c->eps_mode = 2;
     }
     return run_steps(c, n);
@@ -940,7 +949,7 @@ int cudarl_train_steps_eps(cudarl_ctx* c, int64_t n, const float* eps_host) {
     if (n == 0 || c->p.N == 0) return 0;
     CK(cudaSetDevice(c->cfg.device));
     int rc = upload_eps(c, eps_host, (size_t)n); if (rc) return rc;
-    k_ctl_eps<<<1, 1, 0, c->st>>>(c->p.ctl, 1u, (unsigned)n, 0ull);
+    if (!c->gather) k_ctl_eps<<<1, 1, 0, c->st>>>(c->p.ctl, 1u, (unsigned)n, 0ull);
     c->eps_mode = 1;
     return run_steps(c, n);
 }

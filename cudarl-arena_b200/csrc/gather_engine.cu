@@ -26,6 +26,7 @@ constexpr unsigned long long GRID_WAIT_NS = 2000000000ull;
 // A barrier of all blocks of the launch: an arrival counter that only ever grows (the host passes its value at the launch).  Bounded
 // in time: a block that waits two seconds records the failure, and everybody leaves.
 struct GlobalTable {
+    static constexpr bool ALONE = false;
     const Params& p;
     __device__ __forceinline__ float4 row(unsigned s) const { return p.Q[s]; }
     __device__ __forceinline__ unsigned moves(unsigned s) const { return __ldg(p.gp.mv + s); }
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(CB, 1) k_cluster_steps(const __grid_constant__
 }
 
 // ------------------------------------------------------------------------------------------------
-// The move byte of every cell (see move_byte in rules.cuh), row by row.
+// The move byte of every cell (see MoveColumn in rules.cuh), row by row.
 __global__ void __launch_bounds__(BLOCK) k_gather_moves(Params p, unsigned char* __restrict__ mv) {
     for (unsigned s = blockIdx.x * BLOCK + threadIdx.x; s < p.S; s += gridDim.x * BLOCK) {
         const int y = (int)(s / (unsigned)p.W), x = (int)(s - (unsigned)y * (unsigned)p.W);

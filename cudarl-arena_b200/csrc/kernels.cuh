@@ -92,7 +92,12 @@ struct GatherP {
     unsigned deal_every;                    // steps between two dealings by cell; 0 = the environments stay in their order
     unsigned cluster, arena;                // all blocks in one cluster; the world in the shared memory of one block
 };
-struct StepLaunch { unsigned steps, chunk, barrier_base; int eps_mode, trace; const int4* in; int4* out; };    // in != out: deal by cell first
+struct StepLaunch {
+    unsigned steps, chunk, barrier_base;
+    int eps_mode, trace;
+    unsigned eps_len; unsigned long long eps_base_k;     // eps_mode 2: entries of the table, and the episodes / environments of its first
+    const int4* in; int4* out;                           // in != out: deal by cell first
+};
 
 // ---- everything a kernel needs, passed by value ------------------------------------------------
 struct Params {

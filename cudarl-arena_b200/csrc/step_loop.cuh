@@ -15,7 +15,7 @@
 // crowded ones 4.7 -> 5.5).  Counters alternate by step parity; who counted clears its counter in the next step's count phase, when
 // everybody has read it and nobody uses that parity.
 //
-// A Space gives: row(s), moves(s), add(par, idx, n) -> old count, count(par, idx, n), note(par, idx) -> marked before, clear(par, idx),
+// A Space gives: ALONE (the launch is one block), row(s), moves(s), add(par, idx, n) -> old count, count(par, idx, n), note(par, idx) -> marked before, clear(par, idx),
 // counts(par, s) -> uint4, store(idx, v), arrive(), wait() -> false when the launch has to be given up.
 #pragma once
 #include "kernels.cuh"
@@ -95,7 +95,15 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
         s = (unsigned)r.y * W + (unsigned)r.x; t = (unsigned)r.z; id = (unsigned)r.w;
         if (STREAM) { m_pos[j] = make_uint2(s, t); m_id[j] = id; m_own[j] = NOBODY; } else w = draw(id, g);
     }
-    unsigned eps_at = !PLAIN && l.eps_mode == 2 ? *reinterpret_cast<volatile unsigned*>(&ctl->eps_idx) : p.eps_idx;
+    // Epsilon by finished episodes: the index grows whenever their number passes the next multiple of the number of environments.
+    unsigned eps_at = p.eps_idx;
+    unsigned long long ep0 = 0ull, ep_next = ~0ull;
+    if (!PLAIN && l.eps_mode == 2) {
+        ep0 = *reinterpret_cast<volatile unsigned long long*>(&ctl->episodes);
+        const unsigned long long k = ep0 / p.N;
+        eps_at = (unsigned)min(k - l.eps_base_k, (unsigned long long)(l.eps_len - 1u));
+        ep_next = (k + 1ull) * p.N;
+    }
     float eps = __ldg(p.eps_tab + eps_at);
 
     for (unsigned step = 0; step < l.steps; ++step, ++g) {
@@ -150,7 +158,7 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
                 if (applies) m_tv[j] = make_float2(target, value);
             }
         }
-        if (!PLAIN && l.eps_mode == 2) {              // finished episodes of this step, before anybody can pass the barrier
+        if (!PLAIN && l.eps_mode == 2 && !Space::ALONE) {              // finished episodes of this step, before anybody can pass the barrier
             __syncthreads();
             if (tid == 0u && s_ep) { atomicAdd(&ctl->episodes, (unsigned long long)s_ep); s_ep = 0u; }
         }
@@ -185,9 +193,8 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
         // adds to them before everybody has passed the second)
         if (l.eps_mode == 1) ++eps_at;
         else if (!PLAIN && l.eps_mode == 2) {
-            const unsigned long long kk = *reinterpret_cast<volatile unsigned long long*>(&ctl->episodes) / (unsigned long long)p.N;
-            const unsigned long long rel = kk > ctl->eps_base_k ? kk - ctl->eps_base_k : 0ull;
-            eps_at = (unsigned)(rel < (unsigned long long)(ctl->eps_len - 1u) ? rel : (unsigned long long)(ctl->eps_len - 1u));
+            const unsigned long long ep = Space::ALONE ? ep0 + *reinterpret_cast<volatile unsigned*>(&s_ep) : *reinterpret_cast<volatile unsigned long long*>(&ctl->episodes);
+            while (ep >= ep_next) { ep_next += p.N; eps_at = min(eps_at + 1u, l.eps_len - 1u); }
         }
         space.arrive();
         if (l.eps_mode && step + 1u < l.steps) eps = __ldg(p.eps_tab + eps_at);
@@ -212,11 +219,11 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
     if (tid == 0u) {
         if (s_sum[0]) atomicAdd(&ctl->goals, (unsigned long long)s_sum[0]);
         if (s_sum[1]) atomicAdd(&ctl->timeouts, (unsigned long long)s_sum[1]);
-        if (l.eps_mode != 2 && s_sum[0] + s_sum[1]) atomicAdd(&ctl->episodes, (unsigned long long)(s_sum[0] + s_sum[1]));
+        if ((l.eps_mode != 2 || Space::ALONE) && s_sum[0] + s_sum[1]) atomicAdd(&ctl->episodes, (unsigned long long)(s_sum[0] + s_sum[1]));
         if (s_sum[2]) atomicAdd(&ctl->conflicts, (unsigned long long)s_sum[2]);
         if (s_sum[3]) atomicAdd(&ctl->long_chains, (unsigned long long)s_sum[3]);
         if (s_sum[4]) atomicAdd(&ctl->general, (unsigned long long)s_sum[4]);
-        if (blockIdx.x == 0u && l.eps_mode == 2) { ctl->eps_used = eps; ctl->eps_idx = eps_at; }
+        if (blockIdx.x == 0u && l.eps_mode == 2) ctl->eps_used = eps;
     }
 }
 
