@@ -14,8 +14,10 @@
 namespace cudarl {
 
 constexpr size_t ARENA_MOST = 226u * 1024u;      // dynamic shared memory of a block (227 KB less the static words of step_loop.cuh)
+constexpr size_t SOLO_MOST = 216u * 1024u;       // 8.3 KB go to the draws
 constexpr unsigned ARENA_ENVS = 1024u;
 // rows (16 bytes a cell), two rows of counters by step parity (16 bytes each), a move byte
+inline size_t solo_bytes(unsigned S) { return (size_t)S * 16u + (S + 15u) / 16u * 16u; }      // without the counters
 inline size_t arena_bytes(unsigned S) { return (size_t)S * 48u + (S + 15u) / 16u * 16u; }
 
 struct ArenaSpace {
@@ -53,6 +55,103 @@ __global__ void __launch_bounds__(AB, 1) k_arena_steps(const __grid_constant__ P
     for (unsigned s = threadIdx.x; s < S; s += AB) p.Q[s] = rows[s];
 }
 
+// Up to 32 environments: one warp steps them, without counters or a barrier in the step -- who stands on the same (cell, action) is found
+// with a match across the warp, and the lowest of them applies the update for all.  A second warp makes the random draws, which depend
+// on nothing, a chunk of steps ahead.  SHARED: the world in shared memory; else in global memory, where the rows the warp walks over stay in
+// its first-level cache.
+// What bounds it: the chain of dependent instructions of one step, 4 - 5 cycles each (B200, one environment, fixed epsilon: with the counters
+// and barriers of the block's step 0.58 us a step, with the match but the draws in the same warp 0.46).
+constexpr unsigned SOLO_CHUNK = 32u;
+
+template <bool SHARED, bool PLAIN>
+__global__ void __launch_bounds__(64, 1) k_solo_steps(const __grid_constant__ Params p, const __grid_constant__ StepLaunch l) {
+    extern __shared__ __align__(16) unsigned char arena[];
+    __shared__ unsigned s_flag, s_sum[5];
+    __shared__ unsigned s_draw[2][SOLO_CHUNK][32];   // per step and environment: the 24 bits compared with epsilon, above them the action to explore
+    __shared__ unsigned s_thr[2][SOLO_CHUNK];        // explore iff those 24 bits are below
+    if (!may_start(p, &s_flag)) return;
+    const unsigned tid = threadIdx.x, lane = tid & 31u, S = p.S, W = (unsigned)p.W;
+    const bool walker = tid < 32u;
+    if (tid < 5u) s_sum[tid] = 0u;
+    float4* const rows = SHARED ? reinterpret_cast<float4*>(arena) : p.Q;
+    unsigned char* const moves = SHARED ? arena + (size_t)S * 16u : p.gp.mv;
+    if (SHARED) {
+#pragma unroll 8
+        for (unsigned s = tid; s < S; s += 64u) { rows[s] = p.Q[s]; moves[s] = __ldg(p.gp.mv + s); }
+    }
+    const unsigned tmax = p.max_steps > 0 ? (unsigned)p.max_steps : 0x7FFFFFFFu;
+    const bool act = lane < p.N, crowd = p.N > 1u;
+    Tally tally{0u, 0u, 0u, 0u, 0u};
+    unsigned s = 0u, t = 0u, id = 0u, ended = 0u;
+    if (act) { const int4 r = l.out[lane]; s = (unsigned)r.y * W + (unsigned)r.x; t = (unsigned)r.z; id = (unsigned)r.w; }
+    EpsilonIndex eps_index(p, l, PLAIN);
+    float eps = __ldg(p.eps_tab + eps_index.at);
+    auto threshold = [](float e) -> unsigned { return !(e > 0.0f) ? 0u : e >= 1.0f ? (1u << 24) : (unsigned)ceilf(e * 16777216.0f); };
+    unsigned thr = threshold(eps);
+    auto make_draws = [&](unsigned first) {
+        const unsigned b = (first / SOLO_CHUNK) & 1u, m = min(SOLO_CHUNK, l.steps - first);
+        for (unsigned k = 0; k < m; ++k) {
+            const unsigned long long g = p.step + first + k;
+            const U4 r = philox4x32_10(p.env_offset + id, 0u, (unsigned)g, (unsigned)(g >> 32), p.policy_keys);
+            s_draw[b][k][lane] = (r.x >> 8) | (r.y << 24);
+        }
+        if (lane < m) s_thr[b][lane] = threshold(__ldg(p.eps_tab + (l.eps_mode == 1 ? p.eps_idx + first + lane : p.eps_idx)));
+    };
+    if (!walker) make_draws(0u);
+    __syncthreads();
+
+    for (unsigned first = 0; first < l.steps; first += SOLO_CHUNK) {
+        if (!walker) { if (first + SOLO_CHUNK < l.steps) make_draws(first + SOLO_CHUNK); }
+        else {
+            const unsigned b = (first / SOLO_CHUNK) & 1u, m = min(SOLO_CHUNK, l.steps - first);
+            for (unsigned k = 0; k < m; ++k) {
+                const float4 row = rows[s];
+                unsigned mv = moves[s];
+                const unsigned w = s_draw[b][k][lane];
+                if (PLAIN || l.eps_mode != 2) thr = s_thr[b][k];
+                const int a = (w & 0xFFFFFFu) < thr ? (int)(w >> 24) & 3 : argmax4(row);
+                mv >>= a;                             // bit 0: the move is blocked, bit 4: it ends on a goal
+                const unsigned cell = s, own = s * 4u + (unsigned)a, there = a == 0 ? s - W : a == 1 ? s + 1u : a == 2 ? s + W : s - 1u;
+                const bool blocked = (mv & 1u) != 0u, done = (mv & 16u) != 0u;
+                s = blocked ? s : there;
+                float m4 = max4(rows[s]);
+                unsigned n = 1u; bool applies = act;
+                if (crowd) {
+                    const unsigned mates = __match_any_sync(FULL, act ? own : NOBODY), here = __match_any_sync(FULL, act ? cell : NOBODY);
+                    n = (unsigned)__popc(mates); applies = act && lane == (unsigned)__ffs((int)mates) - 1u;
+                    const unsigned tot = act ? (unsigned)__popc(here) : 0u;
+                    if (tot > 1u) ++tally.conf;
+                    if (tot > CROWDED_CELL) { ++tally.on_crowded; if (lane == (unsigned)__ffs((int)here) - 1u) ++tally.crowded; }
+                }
+                if (!PLAIN && p.legacy_clamp && m4 < 0.0f) m4 = 0.0f;
+                float r = -0.01f;
+                if (!PLAIN && p.ntraps && blocked) { const unsigned y = cell / W; r = blocked_step_reward(p, (int)(cell - y * W), (int)y, a); }     // a trap charges its penalty
+                const float target = done ? 1.0f : __fmaf_rn(p.gamma, m4, r);
+                __syncwarp();                         // every lane has taken its target from Q_t
+                if (applies) reinterpret_cast<float*>(rows)[own] = apply_counted(pick(row, a), target, p.lr, n);
+                if (!PLAIN && act && l.trace && first + k + 1u == l.steps) { p.tr_a[id] = a; p.tr_r[id] = done ? 1.0f : r; p.tr_d[id] = done ? 1 : 0; }
+                t = min(t + 1u, STEP_SAT);
+                const bool over = act && (done || t >= tmax);
+                if (__any_sync(FULL, over)) {
+                    if (over) {
+                        s = sample_start(p, p.env_offset + id, p.step + first + k + 1ull, TAG_START); t = 0u;
+                        if (done) ++tally.goals; else ++tally.timeouts;
+                    }
+                    if (!PLAIN && l.eps_mode == 2) {
+                        ended += (unsigned)__popc(__ballot_sync(FULL, over));
+                        if (first + k + 1u < l.steps) { eps_index.next(p, l, PLAIN, ended, true); eps = __ldg(p.eps_tab + eps_index.at); thr = threshold(eps); }
+                    }
+                }
+                __syncwarp();                         // the entries are stored
+            }
+        }
+        __syncthreads();
+    }
+    if (SHARED) for (unsigned k = tid; k < S; k += 64u) p.Q[k] = rows[k];
+    if (walker && act) { const unsigned y = s / W; l.out[lane] = make_int4((int)(s - y * W), (int)y, (int)t, (int)id); }
+    add_tallies(p, l, tally, s_sum, true, eps);
+}
+
 template <unsigned AB>
 static bool allow() {
     return cudaFuncSetAttribute((const void*)k_arena_steps<AB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ARENA_MOST) == cudaSuccess &&
@@ -62,10 +161,15 @@ static bool allow() {
 bool arena_plan(Params& p) {
     GatherP& gp = p.gp;
     const unsigned n = p.N ? p.N : 1u;
+    if (n <= 32u) {
+        gp.threads = gp.chunk = 32u; gp.grid = 1u; gp.arena = 1u;
+        return cudaFuncSetAttribute((const void*)k_solo_steps<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLO_MOST) == cudaSuccess &&
+               cudaFuncSetAttribute((const void*)k_solo_steps<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLO_MOST) == cudaSuccess;
+    }
     if (n > ARENA_ENVS || arena_bytes(p.S) > ARENA_MOST) return false;
-    gp.threads = n <= 32u ? 32u : n <= 256u ? 256u : 1024u;
+    gp.threads = n <= 256u ? 256u : 1024u;
     gp.chunk = gp.threads; gp.grid = 1u; gp.arena = 1u;
-    return allow<32u>() && allow<256u>() && allow<1024u>();
+    return allow<256u>() && allow<1024u>();
 }
 
 template <unsigned AB>
@@ -75,7 +179,13 @@ static cudaError_t launch_one(const Params& p, const StepLaunch& l, cudaStream_t
     return cudaGetLastError();
 }
 cudaError_t launch_arena_steps(const Params& p, const StepLaunch& l, cudaStream_t st) {
-    return p.gp.threads == 32u ? launch_one<32u>(p, l, st) : p.gp.threads == 256u ? launch_one<256u>(p, l, st) : launch_one<1024u>(p, l, st);
+    if (p.gp.threads == 32u) {
+        const bool fits = solo_bytes(p.S) <= SOLO_MOST, pl = plain(p, l);
+        if (fits) { if (pl) k_solo_steps<true, true><<<1, 64, solo_bytes(p.S), st>>>(p, l); else k_solo_steps<true, false><<<1, 64, solo_bytes(p.S), st>>>(p, l); }
+        else { if (pl) k_solo_steps<false, true><<<1, 64, 0, st>>>(p, l); else k_solo_steps<false, false><<<1, 64, 0, st>>>(p, l); }
+        return cudaGetLastError();
+    }
+    return p.gp.threads == 256u ? launch_one<256u>(p, l, st) : launch_one<1024u>(p, l, st);
 }
 
 }  // namespace cudarl

@@ -54,6 +54,48 @@ __device__ __forceinline__ bool may_start(const Params& p, unsigned* s_flag) {
     return *s_flag != 0u;
 }
 
+// The index of a step's epsilon in the table: fixed, by step, or by finished episodes -- it grows whenever their number passes the next
+// multiple of the number of environments.
+struct EpsilonIndex {
+    unsigned at; unsigned long long ep0, ep_next;
+    __device__ __forceinline__ EpsilonIndex(const Params& p, const StepLaunch& l, bool plain) : at(p.eps_idx), ep0(0ull), ep_next(~0ull) {
+        if (plain || l.eps_mode != 2) return;
+        ep0 = *reinterpret_cast<volatile unsigned long long*>(&p.ctl->episodes);
+        const unsigned long long k = ep0 / p.N;
+        at = (unsigned)min(k - l.eps_base_k, (unsigned long long)(l.eps_len - 1u));
+        ep_next = (k + 1ull) * p.N;
+    }
+    // alone: `local` counts the episodes of this launch (one block), else the control block does
+    __device__ __forceinline__ void next(const Params& p, const StepLaunch& l, bool plain, unsigned local, bool alone) {
+        if (l.eps_mode == 1) ++at;
+        else if (!plain && l.eps_mode == 2) {
+            const unsigned long long ep = alone ? ep0 + local : *reinterpret_cast<volatile unsigned long long*>(&p.ctl->episodes);
+            while (ep >= ep_next) { ep_next += p.N; at = min(at + 1u, l.eps_len - 1u); }
+        }
+    }
+};
+// The sums of a launch: warp, block (s_sum: five zeroed words), control block.
+__device__ __forceinline__ void add_tallies(const Params& p, const StepLaunch& l, const Tally& tally, unsigned* s_sum, bool episodes, float eps) {
+    Ctl* const ctl = p.ctl;
+    const unsigned tid = threadIdx.x;
+    unsigned sums[5] = {tally.goals, tally.timeouts, tally.conf, tally.crowded, tally.on_crowded};
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const unsigned v = __reduce_add_sync(FULL, sums[k]);
+        if ((tid & 31u) == 0u && v) atomicAdd(&s_sum[k], v);
+    }
+    __syncthreads();
+    if (tid == 0u) {
+        if (s_sum[0]) atomicAdd(&ctl->goals, (unsigned long long)s_sum[0]);
+        if (s_sum[1]) atomicAdd(&ctl->timeouts, (unsigned long long)s_sum[1]);
+        if (episodes && s_sum[0] + s_sum[1]) atomicAdd(&ctl->episodes, (unsigned long long)(s_sum[0] + s_sum[1]));
+        if (s_sum[2]) atomicAdd(&ctl->conflicts, (unsigned long long)s_sum[2]);
+        if (s_sum[3]) atomicAdd(&ctl->long_chains, (unsigned long long)s_sum[3]);
+        if (s_sum[4]) atomicAdd(&ctl->general, (unsigned long long)s_sum[4]);
+        if (blockIdx.x == 0u && l.eps_mode == 2) ctl->eps_used = eps;
+    }
+}
+
 // Where the state of the environments of a block lives during a launch.
 enum class Home { Registers, Shared, Global };
 // One environment of a block: cell, steps of the episode, number; the (cell, action) owned in this step, its TD target and value.
@@ -95,16 +137,8 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
         s = (unsigned)r.y * W + (unsigned)r.x; t = (unsigned)r.z; id = (unsigned)r.w;
         if (STREAM) { m_pos[j] = make_uint2(s, t); m_id[j] = id; m_own[j] = NOBODY; } else w = draw(id, g);
     }
-    // Epsilon by finished episodes: the index grows whenever their number passes the next multiple of the number of environments.
-    unsigned eps_at = p.eps_idx;
-    unsigned long long ep0 = 0ull, ep_next = ~0ull;
-    if (!PLAIN && l.eps_mode == 2) {
-        ep0 = *reinterpret_cast<volatile unsigned long long*>(&ctl->episodes);
-        const unsigned long long k = ep0 / p.N;
-        eps_at = (unsigned)min(k - l.eps_base_k, (unsigned long long)(l.eps_len - 1u));
-        ep_next = (k + 1ull) * p.N;
-    }
-    float eps = __ldg(p.eps_tab + eps_at);
+    EpsilonIndex eps_index(p, l, PLAIN);
+    float eps = __ldg(p.eps_tab + eps_index.at);
 
     for (unsigned step = 0; step < l.steps; ++step, ++g) {
         const unsigned par = (unsigned)g & 1u;
@@ -189,15 +223,9 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
             }
             space.store(own, apply_counted(value, target, p.lr, n));
         }
-        // the index of the next step's epsilon: by step, or by the episodes finished so far (read between the two barriers: nobody
-        // adds to them before everybody has passed the second)
-        if (l.eps_mode == 1) ++eps_at;
-        else if (!PLAIN && l.eps_mode == 2) {
-            const unsigned long long ep = Space::ALONE ? ep0 + *reinterpret_cast<volatile unsigned*>(&s_ep) : *reinterpret_cast<volatile unsigned long long*>(&ctl->episodes);
-            while (ep >= ep_next) { ep_next += p.N; eps_at = min(eps_at + 1u, l.eps_len - 1u); }
-        }
+        eps_index.next(p, l, PLAIN, Space::ALONE ? *reinterpret_cast<volatile unsigned*>(&s_ep) : 0u, Space::ALONE);        // between the two barriers: nobody adds to the episodes before everybody has passed the second
         space.arrive();
-        if (l.eps_mode && step + 1u < l.steps) eps = __ldg(p.eps_tab + eps_at);
+        if (l.eps_mode && step + 1u < l.steps) eps = __ldg(p.eps_tab + eps_index.at);
         if (!space.wait()) return;
     }
 
@@ -209,22 +237,7 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
         const unsigned y = s / W;
         work[first + j] = make_int4((int)(s - y * W), (int)y, (int)t, (int)id);
     }
-    unsigned sums[5] = {tally.goals, tally.timeouts, tally.conf, tally.crowded, tally.on_crowded};
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const unsigned v = __reduce_add_sync(FULL, sums[k]);
-        if ((tid & 31u) == 0u && v) atomicAdd(&s_sum[k], v);
-    }
-    __syncthreads();
-    if (tid == 0u) {
-        if (s_sum[0]) atomicAdd(&ctl->goals, (unsigned long long)s_sum[0]);
-        if (s_sum[1]) atomicAdd(&ctl->timeouts, (unsigned long long)s_sum[1]);
-        if ((l.eps_mode != 2 || Space::ALONE) && s_sum[0] + s_sum[1]) atomicAdd(&ctl->episodes, (unsigned long long)(s_sum[0] + s_sum[1]));
-        if (s_sum[2]) atomicAdd(&ctl->conflicts, (unsigned long long)s_sum[2]);
-        if (s_sum[3]) atomicAdd(&ctl->long_chains, (unsigned long long)s_sum[3]);
-        if (s_sum[4]) atomicAdd(&ctl->general, (unsigned long long)s_sum[4]);
-        if (blockIdx.x == 0u && l.eps_mode == 2) ctl->eps_used = eps;
-    }
+    add_tallies(p, l, tally, s_sum, l.eps_mode != 2 || Space::ALONE, eps);
 }
 
 // Whether a launch needs none of the options PLAIN leaves out.

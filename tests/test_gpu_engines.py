@@ -20,7 +20,7 @@ def world(pkg, w, h, n, **kw):
     return pkg.make_config(w, h, n, **base)
 
 
-LIMITS = [1, 32, 33, 256, 257, 1024, 1025, 4096, 4097, 8193, 16384, 16385, SMS * 512, SMS * 512 + 1, SMS * 1024, SMS * 1024 + 1, 4 * SMS * 1024 + 77, 1300000]
+LIMITS = [1, 2, 31, 32, 33, 256, 257, 1024, 1025, 4096, 4097, 8193, 16384, 16385, SMS * 512, SMS * 512 + 1, SMS * 1024, SMS * 1024 + 1, 4 * SMS * 1024 + 77, 1300000]
 
 
 @pytest.mark.parametrize("n", LIMITS)
@@ -38,11 +38,11 @@ def test_population_limits(pkg, orc, n):
     assert (sa.conflicts, sa.goals, sa.timeouts, sa.device_error) == (sb.conflicts, sb.goals, sb.timeouts, 0)
 
 
-@pytest.mark.parametrize("n", [33, 5000, 80000])
+@pytest.mark.parametrize("n", [31, 33, 5000, 80000])
 def test_crowded_cells_are_counted_alike(pkg, orc, n):
     """Cells with more than 24 environments, whoever applies their updates: the number of such (cell, step) pairs and of the
     environment-steps on them, against a count of the states the oracle went through."""
-    cfg = world(pkg, 9, 8, n, num_goals=1, obstacle_p=0.0, max_steps=0)
+    cfg = world(pkg, 9, 8, n, num_goals=1, obstacle_p=0.0, max_steps=0, start_mode=pkg.START_CENTRE if n < 32 else pkg.START_RANDOM)
     gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
     cells = chained = 0
     for _ in range(12):
@@ -56,15 +56,15 @@ def test_crowded_cells_are_counted_alike(pkg, orc, n):
     assert_same(gpu, cpu, "crowded")
 
 
-@pytest.mark.parametrize("h", [4722, 4723])
-def test_largest_world_of_one_block(pkg, orc, h):
-    cfg = world(pkg, 1, h, 300)
+@pytest.mark.parametrize("h,n", [(4722, 300), (4723, 300), (13010, 20), (13011, 20), (13011, 1)])
+def test_largest_worlds_of_one_block_and_of_one_warp(pkg, orc, h, n):
+    cfg = world(pkg, 1, h, n)
     gpu, cpu = pair(pkg, orc, cfg)
     gpu.train_steps(40); cpu.train_steps(40)
     assert_same(gpu, cpu, "1 x %d" % h)
 
 
-@pytest.mark.parametrize("n,kw", [(700, {}), (3000, {}), (90000, {"legacy_clamp": 1}), (400000, {"start_mode": 0}), (2000, {"start_mode": 0, "max_steps": 0})])
+@pytest.mark.parametrize("n,kw", [(1, {}), (29, {}), (29, {"start_mode": 0}), (700, {}), (3000, {}), (90000, {"legacy_clamp": 1}), (400000, {"start_mode": 0}), (2000, {"start_mode": 0, "max_steps": 0})])
 def test_common_start_traps_and_episode_epsilon(pkg, orc, n, kw):
     """Everybody on one start cell (whole warps count once), traps, the clamp, and the epsilon that follows the finished episodes."""
     cfg = world(pkg, 91, 93, n, eps_kind=pkg.EPS_MULT_PER_EPISODE, eps0=1.0, eps_decay=0.9, **kw)
