@@ -31,13 +31,16 @@ struct Tally { unsigned goals, timeouts, conf, crowded, on_crowded; };
 
 // The update of (cell, action) `own` from the counted number of environments on it: the map q <- fma(lr, d - q, q) as often as counted.
 // It is a contraction, so a long run ends at its fixed point: once the value stops changing it never changes again.
+// Two at a time: a value that stands still shows at once, and half as many looks for one that does not.
 __device__ __forceinline__ float apply_counted(float v, float d, float lr, unsigned n) {
-    for (unsigned i = 0; i < n; ++i) {
-        const float w = __fmaf_rn(lr, __fsub_rn(d, v), v);
-        if (__float_as_uint(w) == __float_as_uint(v)) break;
-        v = w;
+    auto once = [&](float u) -> float { return __fmaf_rn(lr, __fsub_rn(d, u), u); };
+    for (;;) {
+        const float w = once(v);
+        if (n == 1u || __float_as_uint(w) == __float_as_uint(v)) return w;
+        const float x = once(w);
+        if (n == 2u || __float_as_uint(x) == __float_as_uint(w)) return x;
+        v = x; n -= 2u;
     }
-    return v;
 }
 
 // Whether a launch may start.  A context in which a wait has run out does nothing any more (its barrier counter is off); with a poll
