@@ -114,6 +114,7 @@ struct cudarl_ctx {
     void *dtra = nullptr, *dtrr = nullptr, *dtrd = nullptr, *dsckey = nullptr, *dscval = nullptr;
     void *dgather = nullptr;              // replica averaging: the other ranks' rows of this rank's slice
     void* dub = nullptr; size_t ub_cap = 0;                               // the arrays of a large update_batch, and their bytes
+    int32_t seen_x = 0, seen_y = 0;       // where the one environment of a context was when it was last stepped alone
     void* dact = nullptr;                 // actions of the host form of step_actions, where the stage is too small for them
     size_t ent_cap = 0, eps_cap = 0;
     float* h_eps = nullptr; size_t h_eps_cap = 0; cudaEvent_t ev_eps = nullptr; bool eps_inflight = false;
@@ -883,18 +884,21 @@ int cudarl_get_reward_done(cudarl_ctx* c, float* rewards, uint8_t* dones) {
 }  // extern "C"
 
 namespace cudarl {
-// One environment, everything a caller of the facade asks for from one launch.
-int step_single(cudarl_ctx* c, bool reset, int32_t action, SingleStep* out) {
-    if (!c || !out || c->p.N != 1) return fail(c, -1, "bad argument");
+// One environment, everything a caller of the facade asks for from one launch; `begin` launches, `end` waits.
+int step_single_begin(cudarl_ctx* c, bool reset, int32_t action) {
+    if (!c || c->p.N != 1) return fail(c, -1, "bad argument");
     CK(cudaSetDevice(c->cfg.device));
     { int rl = leave_tiles(c); if (rl) return rl; }
     int rc = ensure_step_buffers(c); if (rc) return rc;
     c->p.step = (unsigned long long)c->h_step;
-    launch_step_one(c->p, action, reset, handover(c), c->st);
+    launch_step_one(c->p, action, reset, c->seen_x, c->seen_y, handover(c), c->st);
     CK(cudaGetLastError());
-    { int rw = wait_box(c, 4); if (rw) return rw; }
     if (reset) c->epoch_step = c->h_step;
-    out->x = (int32_t)box32(c, 1); out->y = (int32_t)box32(c, 2); out->reward = boxf(c, 3); out->done = box32(c, 4) != 0;
+    return 0;
+}
+int step_single_end(cudarl_ctx* c, SingleStep* out) {
+    { int rw = wait_box(c, 4); if (rw) return rw; }
+    out->x = c->seen_x = (int32_t)box32(c, 1); out->y = c->seen_y = (int32_t)box32(c, 2); out->reward = boxf(c, 3); out->done = box32(c, 4) != 0;
     return check_posted_error(c);
 }
 }  // namespace cudarl

@@ -2,7 +2,7 @@
 #include "facade.h"
 #include "../../include/cudarl.h"
 #include "internal.h"
-#include <sstream>
+#include <string>
 #include <stdexcept>
 
 namespace {
@@ -46,17 +46,15 @@ void Environment::refresh_grid() {
     for (int32_t k = 0; k < nt; ++k) grid_[(size_t)tc[k]] = tpn[k];      // a trap shows its penalty, as src/kernels.cu:61 reads it
 }
 
-void Environment::reset() {
+void Environment::beginReset() { check(cudarl::step_single_begin(ctx_, true, 0), ctx_, "reset"); }
+void Environment::beginStep(int action) { check(cudarl::step_single_begin(ctx_, false, action), ctx_, "step"); }   // obstacles, goals and traps are looked up on the device
+void Environment::finish() {
     cudarl::SingleStep s;
-    check(cudarl::step_single(ctx_, true, 0, &s), ctx_, "reset");
-    x_ = s.x; y_ = s.y; reward_ = 0.0f; done_ = false;
-}
-
-void Environment::step(int action) {
-    cudarl::SingleStep s;
-    check(cudarl::step_single(ctx_, false, action, &s), ctx_, "step");       // obstacles, goals and traps are looked up on the device
+    check(cudarl::step_single_end(ctx_, &s), ctx_, "step");
     x_ = s.x; y_ = s.y; reward_ = s.reward; done_ = s.done;
 }
+void Environment::reset() { beginReset(); finish(); }
+void Environment::step(int action) { beginStep(action); finish(); }
 
 float Environment::getCellValue(int x, int y) const {
     if (x >= 0 && x < width_ && y >= 0 && y < height_) return grid_[(size_t)y * width_ + x];
@@ -75,9 +73,10 @@ EnvironmentBridge::EnvironmentBridge(int width, int height, int env_id) : width(
 std::vector<float> EnvironmentBridge::reset() { env->reset(); return getObservation(); }
 std::tuple<std::vector<float>, float, bool, std::string> EnvironmentBridge::step(int action) {
     env->step(action);
-    std::stringstream info;
-    info << "agent_pos: (" << env->getAgentX() << "," << env->getAgentY() << ")";   // src/environment_bridge.cu:30-31
-    return std::make_tuple(getObservation(), env->getReward(), env->isDone(), info.str());
+    return std::make_tuple(getObservation(), env->getReward(), env->isDone(), getInfo());
+}
+std::string EnvironmentBridge::getInfo() const {
+    return "agent_pos: (" + std::to_string(env->getAgentX()) + "," + std::to_string(env->getAgentY()) + ")";   // src/environment_bridge.cu:30-31
 }
 std::vector<float> EnvironmentBridge::getObservation() const { return env->getGrid(); }
 int EnvironmentBridge::getWidth() const { return width; }

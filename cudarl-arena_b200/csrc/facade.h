@@ -47,6 +47,12 @@ public:
     bool isDone() const { return done_; }
     float getCellValue(int x, int y) const;     // 0.0 outside the grid (src/environment.cu:127-132)
     std::vector<float> getGrid() const;         // free 0.0, goal 1.0, obstacle -1.0, trap = its penalty
+    const std::vector<float>& grid() const { return grid_; }
+
+    // reset() and step() in two halves, with room for the caller's own work between them
+    void beginReset();
+    void beginStep(int action);
+    void finish();
 
     // grid edits used by EnvironmentBridge
     void addObstacle(int x, int y);
@@ -70,6 +76,8 @@ public:
     std::vector<float> reset();
     std::tuple<std::vector<float>, float, bool, std::string> step(int action);
     std::vector<float> getObservation() const;
+    std::string getInfo() const;
+    Environment& environment() { return *env; }
     int getWidth() const;
     int getHeight() const;
     std::pair<int, int> getAgentPosition() const;

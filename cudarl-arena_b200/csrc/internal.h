@@ -5,7 +5,9 @@
 namespace cudarl {
 
 struct SingleStep { int32_t x, y; float reward; bool done; };
-// cudarl_step_actions (or cudarl_reset_all) of a context with one environment, with the environment's position: one launch, one wait.
-int step_single(cudarl_ctx* ctx, bool reset, int32_t action, SingleStep* out);
+// cudarl_step_actions (or cudarl_reset_all) of a context with one environment, with the environment's position: one launch, one wait, and the
+// caller's own work between the two.
+int step_single_begin(cudarl_ctx* ctx, bool reset, int32_t action);
+int step_single_end(cudarl_ctx* ctx, SingleStep* out);
 
 }  // namespace cudarl

@@ -19,23 +19,17 @@
 
 namespace cudarl {
 
-// Move from (x,y) by `action`; returns the new cell and its cell word.
-__device__ __forceinline__ unsigned move_cell(const Params& p, int x, int y, unsigned s, unsigned cw_s, int action,
-                                              unsigned& cw_new) {
-    int dx = (action == 1) - (action == 3), dy = (action == 2) - (action == 0);
-    int nx = x + dx, ny = y + dy;
-    bool inb = nx >= 0 && nx < p.W && ny >= 0 && ny < p.H;
-    unsigned tgt = inb ? (unsigned)ny * (unsigned)p.W + (unsigned)nx : s;
-    unsigned ct = (tgt != s) ? cw_load(p.cw, tgt) : cw_s;
-    bool moved = (tgt != s) && !(ct & CW_OBST);
-    cw_new = moved ? ct : cw_s;
-    return moved ? tgt : s;
+// The cell `action` leads to from (x, y) if nothing is in the way there (its own at the edge of the grid, or for any action but 0..3).
+__device__ __forceinline__ unsigned target_cell(const World& p, int x, int y, int action) {
+    const int nx = x + (action == 1) - (action == 3), ny = y + (action == 2) - (action == 0);
+    const bool inb = nx >= 0 && nx < p.W && ny >= 0 && ny < p.H;
+    return inb ? (unsigned)ny * (unsigned)p.W + (unsigned)nx : (unsigned)y * (unsigned)p.W + (unsigned)x;
 }
 
 // chain heads are indexed by the low bits of the cell: neighbouring cells -> neighbouring slots
 __device__ __forceinline__ unsigned mb_slot(const Params& p, unsigned cell) { return cell & (p.mb_slots - 1u); }
 
-__global__ void k_reset_all(Params p) {
+__global__ void k_reset_all(const __grid_constant__ World p) {
     unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.N) return;
     unsigned e = (unsigned)p.st[i].w;
@@ -44,12 +38,12 @@ __global__ void k_reset_all(Params p) {
     if (p.reward) { p.reward[e] = 0.0f; p.done[e] = 0; }
 }
 
-__global__ void k_ids_identity(Params p) {
+__global__ void k_ids_identity(const __grid_constant__ World p) {
     unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < p.N) p.st[i].w = (int)i;
 }
 // overwrite x / y / t of environment-ordered records from caller arrays (any of them may be null)
-__global__ void k_import_state(Params p, const int* x, const int* y, const int* t) {
+__global__ void k_import_state(const __grid_constant__ World p, const int* x, const int* y, const int* t) {
     unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.N) return;
     int4 r = p.st[i];
@@ -60,7 +54,7 @@ __global__ void k_import_state(Params p, const int* x, const int* y, const int* 
     p.st[i] = r;
 }
 // x[N] | y[N] | t[N] in environment order, into the spare copy or straight into the mapped stage
-__global__ void k_export_state(Params p, int* __restrict__ out, Handover h) {
+__global__ void k_export_state(const __grid_constant__ World p, int* __restrict__ out, Handover h) {
     unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < p.N) {
         const int4 r = p.st[i];
@@ -70,13 +64,13 @@ __global__ void k_export_state(Params p, int* __restrict__ out, Handover h) {
 }
 // Small results: device memory into mapped host memory, 16 bytes per thread and turn (both ends are 16-byte aligned, the tail is
 // copied to the next multiple of 16: every buffer of the context and the stage have that room).
-__global__ void k_copy_out(Params p, CopySpan a, CopySpan b, Handover h) {
+__global__ void k_copy_out(const __grid_constant__ World p, CopySpan a, CopySpan b, Handover h) {
     const unsigned n = gridDim.x * blockDim.x, i0 = blockIdx.x * blockDim.x + threadIdx.x;
     for (unsigned i = i0; i * 16u < a.bytes; i += n) reinterpret_cast<uint4*>(a.dst)[i] = reinterpret_cast<const uint4*>(a.src)[i];
     for (unsigned i = i0; i * 16u < b.bytes; i += n) reinterpret_cast<uint4*>(b.dst)[i] = reinterpret_cast<const uint4*>(b.src)[i];
     if (last_to_finish<true>(p)) box_put_error(p, h);
 }
-__global__ void k_post(Params p, Handover h) {
+__global__ void k_post(const __grid_constant__ World p, Handover h) {
     const unsigned long long* const c[6] = {&p.ctl->episodes, &p.ctl->goals, &p.ctl->timeouts, &p.ctl->conflicts, &p.ctl->long_chains, &p.ctl->general};
 #pragma unroll
     for (unsigned k = 0; k < 6u; ++k) if (threadIdx.x == k) box_put64(h, 1u + 2u * k, *c[k]);       // one counter per lane
@@ -380,38 +374,48 @@ __global__ void __launch_bounds__(BLOCK) k_fix_long(Params p, Handover h) {
 // ------------------------------------------------------------------------------------------------
 // Caller-driven step (no learning, sticky done, no auto-reset): Environment::step for all envs.
 // actions / rewards / dones are indexed by environment id.
-// The record of one environment after `a`; reward and sticky done flag in `r` and `dn`.
-__device__ __forceinline__ int4 stepped(const Params& p, const int4 rec, int a, float& r, unsigned char& dn) {
-    const int x = rec.x, y = rec.y;
-    const unsigned s = (unsigned)y * (unsigned)p.W + (unsigned)x;
-    unsigned cs = cw_load(p.cw, s), c2;
-    if (a < 0 || a > 3) a = -1;                         // any other value: no movement (src/gpu/environment.cu:31)
-    const unsigned s2 = move_cell(p, x, y, s, cs, a, c2);
-    r = (s2 == s && a >= 0) ? blocked_step_reward(p, x, y, a) : -0.01f;    // a trap charges its penalty (src/kernels.cu:61-63)
-    if (c2 & CW_GOAL) { r = 1.0f; dn = 1; }
+// The record of one environment after `a`, which leads towards cell `to`; cell words of its own cell and of `to`.  Reward and sticky done flag
+// in `r` and `dn`.
+__device__ __forceinline__ int4 stepped(const World& p, const int4 rec, int a, unsigned to, unsigned cw_own, unsigned cw_to, float& r, unsigned char& dn) {
+    const unsigned s = (unsigned)rec.y * (unsigned)p.W + (unsigned)rec.x;
+    const bool moved = to != s && !(cw_to & CW_OBST);
+    r = (!moved && a >= 0 && a <= 3) ? blocked_step_reward(p, rec.x, rec.y, a) : -0.01f;    // a trap charges its penalty (src/kernels.cu:61-63)
+    if ((moved ? cw_to : cw_own) & CW_GOAL) { r = 1.0f; dn = 1; }
+    const unsigned s2 = moved ? to : s;
     return make_int4((int)(s2 % (unsigned)p.W), (int)(s2 / (unsigned)p.W), rec.z + 1, rec.w);
 }
-__global__ void k_step_actions(Params p, const int* __restrict__ actions, float* __restrict__ rewards, unsigned char* __restrict__ dones, Handover h) {
+__global__ void k_step_actions(const __grid_constant__ World p, const int* __restrict__ actions, float* __restrict__ rewards, unsigned char* __restrict__ dones, Handover h) {
     unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < p.N) {
         const int4 rec = p.st[i];
         const unsigned e = (unsigned)rec.w;
+        const int a = actions[e];
         float r; unsigned char dn = p.done[e];
-        p.st[i] = stepped(p, rec, actions[e], r, dn);
+        const unsigned to = target_cell(p, rec.x, rec.y, a);
+        p.st[i] = stepped(p, rec, a, to, cw_load(p.cw, (unsigned)rec.y * (unsigned)p.W + (unsigned)rec.x), cw_load(p.cw, to), r, dn);
         p.reward[e] = r; p.done[e] = dn;
         if (rewards) rewards[e] = r;
         if (dones) dones[e] = dn;
     }
     if (h.box && last_to_finish<true>(p)) box_put_error(p, h);
 }
-// A context with one environment: the action comes with the launch, everything a caller asks for goes back in the box.
-__global__ void k_step_one(Params p, int action, bool reset, Handover h) {
+// A context with one environment: the action comes with the launch, everything a caller asks for goes back in the box.  (x, y) is where the
+// host last saw the environment: the cell words there are on their way while the record is, and nearly always the right ones.
+__global__ void k_step_one(const __grid_constant__ World p, int action, bool reset, int x, int y, Handover h) {
     int4 rec = p.st[0];
     float r = 0.0f; unsigned char dn = 0;
     if (reset) {
         const unsigned c = sample_start(p, p.env_offset + (unsigned)rec.w, p.step, TAG_START);
         rec = make_int4((int)(c % (unsigned)p.W), (int)(c / (unsigned)p.W), 0, rec.w);
-    } else { dn = p.done[0]; rec = stepped(p, rec, action, r, dn); }
+    } else {
+        unsigned to = target_cell(p, x, y, action), own = cw_load(p.cw, (unsigned)y * (unsigned)p.W + (unsigned)x), there = cw_load(p.cw, to);
+        dn = p.done[0];
+        if (rec.x != x || rec.y != y) {
+            to = target_cell(p, rec.x, rec.y, action);
+            own = cw_load(p.cw, (unsigned)rec.y * (unsigned)p.W + (unsigned)rec.x); there = cw_load(p.cw, to);
+        }
+        rec = stepped(p, rec, action, to, own, there, r, dn);
+    }
     p.st[0] = rec; p.reward[0] = r; p.done[0] = dn;
     box_put(h, 1u, (unsigned)rec.x); box_put(h, 2u, (unsigned)rec.y); box_put(h, 3u, __float_as_uint(r)); box_put(h, 4u, dn);
     box_put_error(p, h);
@@ -425,7 +429,7 @@ __device__ __forceinline__ void load_transition(const Transitions& tr, unsigned 
     asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(tr.r + i));
 }
 // The TD target of a transition, from the table as it is before the call.
-__device__ __forceinline__ float transition_target(const Params& p, unsigned at, unsigned next, float r) {
+__device__ __forceinline__ float transition_target(const World& p, unsigned at, unsigned next, float r) {
     float m = 0.0f;
     if (!(at >> 31)) {
         m = max4(__ldcg(p.Q + next));
@@ -463,7 +467,7 @@ __global__ void k_update_main(Params p, unsigned n, Transitions tr) {
 // look-up of the next rows, the sort, one read and write of the entries.  KEY: 32 bits hold cell, action and index of grids of up to
 // 2^20 cells and halve the sort's shuffles.
 template <class KEY>
-__global__ void __launch_bounds__(UPDATE_SMALL) k_update_small(const __grid_constant__ Params p, unsigned n, const __grid_constant__ Transitions tr, Handover h) {
+__global__ void __launch_bounds__(UPDATE_SMALL) k_update_small(const __grid_constant__ World p, unsigned n, const __grid_constant__ Transitions tr, Handover h) {
     __shared__ KEY s_key[UPDATE_SMALL];
     __shared__ float s_target[UPDATE_SMALL];
     constexpr unsigned IDX = 10u, IDX_MASK = (1u << IDX) - 1u;
@@ -506,7 +510,7 @@ __global__ void __launch_bounds__(UPDATE_SMALL) k_update_small(const __grid_cons
 }
 
 // ------------------------------------------------------------------------------------------------
-__global__ void k_q_init(Params p, int kind, float scale) {
+__global__ void k_q_init(const __grid_constant__ World p, int kind, float scale) {
     unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= p.S) return;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -517,7 +521,7 @@ __global__ void k_q_init(Params p, int kind, float scale) {
     }
     p.Q[s] = v;
 }
-__global__ void k_cell_set(Params p, unsigned cell, unsigned cls, int clear_goals) {
+__global__ void k_cell_set(const __grid_constant__ World p, unsigned cell, unsigned cls, int clear_goals) {
     unsigned* w32 = reinterpret_cast<unsigned*>(p.cw);
     if (clear_goals) {
         unsigned n2 = (p.S + 1u) / 2u;
@@ -550,7 +554,7 @@ void launch_reset_all(const Params& p, cudaStream_t st) {
 void launch_step_actions(const Params& p, const int* a, float* r, unsigned char* d, Handover h, cudaStream_t st) {
     if (p.N) k_step_actions<<<nblk(p.N), BLOCK, 0, st>>>(p, a, r, d, h);
 }
-void launch_step_one(const Params& p, int action, bool reset, Handover h, cudaStream_t st) { k_step_one<<<1, 1, 0, st>>>(p, action, reset, h); }
+void launch_step_one(const Params& p, int action, bool reset, int x, int y, Handover h, cudaStream_t st) { k_step_one<<<1, 1, 0, st>>>(p, action, reset, x, y, h); }
 void launch_update_batch(const Params& p, unsigned n, const Transitions& tr, Handover h, cudaStream_t st) {
     if (n <= UPDATE_SMALL) {
         unsigned threads = 32u; while (threads < n) threads <<= 1;

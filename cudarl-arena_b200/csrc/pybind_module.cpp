@@ -95,6 +95,20 @@ private:
     cudarl_ctx* ctx_ = nullptr;
 };
 
+// The grid as a list of floats.  Nearly every cell is free, an obstacle or a goal: those share three float objects instead of one being made
+// per cell.
+py::list observation(EnvironmentBridge& e) {
+    static PyObject* const zero = PyFloat_FromDouble(0.0); static PyObject* const one = PyFloat_FromDouble(1.0); static PyObject* const minus = PyFloat_FromDouble(-1.0);
+    const std::vector<float>& g = e.environment().grid();
+    py::list o(g.size());
+    for (size_t i = 0; i < g.size(); ++i) {
+        PyObject* v = g[i] == 0.0f ? zero : g[i] == 1.0f ? one : g[i] == -1.0f ? minus : nullptr;
+        if (v) Py_INCREF(v); else if (!(v = PyFloat_FromDouble((double)g[i]))) throw py::error_already_set();
+        PyList_SET_ITEM(o.ptr(), (py::ssize_t)i, v);
+    }
+    return o;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(cudarl_core, m) {
@@ -103,9 +117,19 @@ PYBIND11_MODULE(cudarl_core, m) {
     py::class_<EnvironmentBridge>(m, "Environment")
         .def(py::init<int, int>(), py::arg("width") = 10, py::arg("height") = 10)
         .def(py::init<int, int, int>(), py::arg("width"), py::arg("height"), py::arg("env_id"))
-        .def("reset", &EnvironmentBridge::reset)
-        .def("step", &EnvironmentBridge::step)
-        .def("get_observation", &EnvironmentBridge::getObservation)
+        .def("reset", [](EnvironmentBridge& e) {
+            e.environment().beginReset();
+            py::list o = observation(e);
+            e.environment().finish();
+            return o;
+        })
+        .def("step", [](EnvironmentBridge& e, int action) {
+            e.environment().beginStep(action);
+            py::list o = observation(e);                 // while the device steps
+            e.environment().finish();
+            return py::make_tuple(std::move(o), e.environment().getReward(), e.environment().isDone(), e.getInfo());
+        })
+        .def("get_observation", &observation)
         .def("get_width", &EnvironmentBridge::getWidth)
         .def("get_height", &EnvironmentBridge::getHeight)
         .def("get_agent_position", &EnvironmentBridge::getAgentPosition)
@@ -120,7 +144,7 @@ PYBIND11_MODULE(cudarl_core, m) {
         .def("is_done", &EnvironmentBridge::isDone)
         .def("get_agent_x", [](const EnvironmentBridge& e) { return e.getAgentPosition().first; })
         .def("get_agent_y", [](const EnvironmentBridge& e) { return e.getAgentPosition().second; })
-        .def("get_grid_data", &EnvironmentBridge::getObservation);
+        .def("get_grid_data", &observation);
 
     py::class_<CudaQLearning>(m, "CudaQLearning")
         .def(py::init<int, int, int, float, float>(), py::arg("width"), py::arg("height"), py::arg("action_space_size") = 4,

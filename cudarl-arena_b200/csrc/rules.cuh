@@ -66,11 +66,11 @@ __device__ __forceinline__ void box_put(const Handover& h, unsigned k, unsigned 
     *reinterpret_cast<volatile unsigned long long*>(&h.box->w[k]) = ((unsigned long long)h.ticket << 32) | v;
 }
 __device__ __forceinline__ void box_put64(const Handover& h, unsigned k, unsigned long long v) { box_put(h, k, (unsigned)v); box_put(h, k + 1u, (unsigned)(v >> 32)); }
-__device__ __forceinline__ void box_put_error(const Params& p, const Handover& h) { box_put(h, 0u, *reinterpret_cast<volatile unsigned*>(&p.ctl->error)); }
+__device__ __forceinline__ void box_put_error(const World& p, const Handover& h) { box_put(h, 0u, *reinterpret_cast<volatile unsigned*>(&p.ctl->error)); }
 // To be called by all threads of every block, after their writes: true in one thread of the last block to get here, which sees what
 // the other blocks have written -- and, when HOST, after which the host sees it too (arrays in the stage).
 template <bool HOST>
-__device__ __forceinline__ bool last_to_finish(const Params& p) {
+__device__ __forceinline__ bool last_to_finish(const World& p) {
     __syncthreads();
     if (threadIdx.x != 0u) return false;
     if (HOST) __threadfence_system(); else __threadfence();
@@ -83,7 +83,7 @@ __device__ __forceinline__ bool last_to_finish(const Params& p) {
 
 // Start cell of an episode.  CENTRE/FIXED: the configured cell (reference: src/environment.cu:9-10).
 // RANDOM: first free non-goal cell among 64 seeded candidates, else the precomputed fallback cell.
-__device__ __forceinline__ unsigned sample_start(const Params& p, unsigned gi, unsigned long long nonce, unsigned tag) {
+__device__ __forceinline__ unsigned sample_start(const World& p, unsigned gi, unsigned long long nonce, unsigned tag) {
     if (p.start_mode != 2) return p.start_cell;
 #pragma unroll 1            // restarts are rare: keep the inlined copies of this loop small (the step kernel's hot loop must fit the instruction cache)
     for (unsigned k = 0; k < 16; ++k) {
@@ -100,7 +100,7 @@ __device__ __forceinline__ unsigned sample_start(const Params& p, unsigned gi, u
 // Reward of a step that does not end on a goal, for an agent at (x, y) whose action `a` was blocked: the step cost, or -- when
 // the cell it walked into is a trap -- that trap's penalty (src/kernels.cu:47,61-63 of the reference: a trap is an obstacle, the
 // agent stays where it is and is charged the cell's value).  Binary search in the sparse trap table.
-__device__ __forceinline__ float blocked_step_reward(const Params& p, int x, int y, int a) {
+__device__ __forceinline__ float blocked_step_reward(const World& p, int x, int y, int a) {
     if (!p.ntraps) return -0.01f;
     const int nx = x + (a == 1) - (a == 3), ny = y + (a == 2) - (a == 0);
     if (nx < 0 || nx >= p.W || ny < 0 || ny >= p.H) return -0.01f;
