@@ -9,10 +9,10 @@
 //   k_rollout_walk    one thread per environment draws its start cell and hops from tile to tile over those words; a path that
 //                     comes back to an earlier tile entry (Brent's cycle search over the hops) never ends.
 //
-// What bounds it: k_rollout_tiles streams the table once (16 bytes in, 4 out per cell) and the doubling (one
-// shared-memory look-up per cell and round, until a round finds no path to end) runs behind other blocks' loads; k_rollout_walk
-// is a few scattered 4-byte look-ups per environment.  B200, 4096 x 4096 cells, 4,194,304 environments, 1000 steps: see the
-// figures at the two kernels; the walk over single cells it replaces took 13.55 ms (1000 scattered byte loads per environment).
+// What bounds it: k_rollout_tiles streams the table once (16 bytes in, 4 out per cell) and looks up one word in shared memory per cell and round,
+// until a round finds no path to end; k_rollout_walk makes a few scattered 4-byte look-ups per environment, one after the other.  B200,
+// 4096 x 4096 cells, 4,194,304 environments, 1000 steps: 97 + 76 us (doubling to the last round 138 us; one environment per thread, start cells
+// looked up in the cell words 89 us); the walk over single cells this replaces took 13.55 ms.
 //
 // Reference semantics: src/train.py:262-311 (evaluate), first-max argmax src/q_learning.cu:196-206.
 #include "kernels.cuh"
@@ -22,9 +22,9 @@ namespace cudarl {
 
 // Word of a cell.  While the tile is folded: kind LIVE, bits 0-11 the cell reached after 2^round steps.  Final: EXIT with the number
 // of steps in bits 0-12, the edge it leaves by (0 up, 1 right, 2 down, 3 left) in bits 22-23 and the place along it in bits 16-21;
-// GOAL with the number of steps; or TRAPPED.  A path without a circle has at most 4096 steps inside a tile.
+// GOAL with the number of steps; or TRAPPED.  Bit 29: an obstacle or a goal, where no episode starts.  A path without a circle has at most 4096 steps inside a tile.
 constexpr unsigned RT_SHIFT = 6u, RT = 1u << RT_SHIFT, RT_CELLS = RT * RT, RT_THREADS = 512u, RT_PER = RT_CELLS / RT_THREADS, RT_ROWS = RT_THREADS / RT;
-constexpr unsigned KIND_LIVE = 0u, KIND_EXIT = 1u << 30, KIND_GOAL = 2u << 30, KIND_MASK = 3u << 30, TRAPPED = 0u, STEPS_MASK = 0x1FFFu;
+constexpr unsigned KIND_LIVE = 0u, KIND_EXIT = 1u << 30, KIND_GOAL = 2u << 30, KIND_MASK = 3u << 30, TRAPPED = 3u << 30, NO_START = 1u << 29, STEPS_MASK = 0x1FFFu;
 
 __global__ void __launch_bounds__(RT_THREADS) k_rollout_tiles(const __grid_constant__ Params p, unsigned* __restrict__ hop) {
     __shared__ unsigned s_w[RT_CELLS];
@@ -34,6 +34,8 @@ __global__ void __launch_bounds__(RT_THREADS) k_rollout_tiles(const __grid_const
     const int x = x0 + (int)lx;
     const float4* const q = p.Q + (size_t)(y0 + (int)ly0) * (size_t)p.W + (size_t)x;
     const MoveColumn moves(p, (unsigned)x);
+    const unsigned short* const cw = p.cw + (size_t)(y0 + (int)ly0) * (size_t)p.W + (size_t)x;
+    unsigned no_start = 0u;
     const bool inside = x0 + (int)RT <= p.W && y0 + (int)RT <= p.H;                       // the same for the whole block
 #pragma unroll
     for (unsigned k = 0; k < RT_PER; ++k) {
@@ -43,6 +45,7 @@ __global__ void __launch_bounds__(RT_THREADS) k_rollout_tiles(const __grid_const
         if (inside || (x < p.W && y < p.H)) {
             const float4 row = __ldcs(q + (size_t)(k * RT_ROWS) * (size_t)p.W);
             const unsigned mvb = moves.at((unsigned)y);
+            if (__ldcs(cw + (size_t)(k * RT_ROWS) * (size_t)p.W) & (CW_OBST | CW_GOAL)) no_start |= NO_START >> k;
             const unsigned a = (unsigned)argmax4(row), mv = mvb >> a;
             if (mv & 16u) w = KIND_GOAL | 1u;
             else if (!(mv & 1u)) {
@@ -69,40 +72,71 @@ __global__ void __launch_bounds__(RT_THREADS) k_rollout_tiles(const __grid_const
         for (unsigned k = 0; k < RT_PER; ++k) s_w[k * RT_THREADS + threadIdx.x] = cur[k];
         __syncthreads();
     }
+    unsigned* const out = hop + (size_t)(y0 + (int)ly0) * (size_t)p.W + (size_t)x;
 #pragma unroll
     for (unsigned k = 0; k < RT_PER; ++k) {
-        const unsigned ic = k * RT_THREADS + threadIdx.x;
-        const int x = x0 + (int)(ic & (RT - 1u)), y = y0 + (int)(ic >> RT_SHIFT);
-        if (x < p.W && y < p.H) hop[(size_t)y * (size_t)p.W + (size_t)x] = (cur[k] & KIND_MASK) == KIND_LIVE ? TRAPPED : cur[k];
+        const unsigned w = ((cur[k] & KIND_MASK) == KIND_LIVE ? TRAPPED : cur[k]) | ((no_start << k) & NO_START);
+        if (inside || (x < p.W && y0 + (int)(ly0 + k * RT_ROWS) < p.H)) out[(size_t)(k * RT_ROWS) * (size_t)p.W] = w;
     }
 }
 
+// A start cell as sample_start draws it, and its word, which says whether an episode may start there.
+__device__ __forceinline__ unsigned walk_start(const Params& p, const unsigned* __restrict__ hop, unsigned gi, unsigned long long nonce, unsigned& word) {
+    if (p.start_mode == 2) {
+#pragma unroll 1
+        for (unsigned k = 0; k < 16u; ++k) {
+            const U4 w = philox4x32_10(gi, k, (unsigned)nonce, (unsigned)(nonce >> 32), p.k0, p.k1 ^ TAG_EVAL);
+            unsigned c;
+            c = __umulhi(w.x, p.S); word = __ldg(hop + c); if (!(word & NO_START)) return c;
+            c = __umulhi(w.y, p.S); word = __ldg(hop + c); if (!(word & NO_START)) return c;
+            c = __umulhi(w.z, p.S); word = __ldg(hop + c); if (!(word & NO_START)) return c;
+            c = __umulhi(w.w, p.S); word = __ldg(hop + c); if (!(word & NO_START)) return c;
+        }
+    }
+    const unsigned c = p.start_mode == 2 ? p.fallback_start : p.start_cell;
+    word = __ldg(hop + c);
+    return c;
+}
+
+// EPT environments per thread: their first look-ups are on the way at the same time.
+template <unsigned EPT>
 __global__ void __launch_bounds__(BLOCK) k_rollout_walk(const __grid_constant__ Params p, const unsigned* __restrict__ hop, unsigned max_steps,
                                                         unsigned long long nonce, Handover h) {
     __shared__ unsigned s_reached; __shared__ unsigned long long s_steps;
     if (threadIdx.x == 0) { s_reached = 0u; s_steps = 0ull; }
     __syncthreads();
-    const unsigned i = blockIdx.x * BLOCK + threadIdx.x;
-    unsigned steps = 0u; bool reached = false;
-    if (i < p.N) {
-        const unsigned s = sample_start(p, p.env_offset + i, nonce, TAG_EVAL);
-        unsigned y = s / (unsigned)p.W, x = s - y * (unsigned)p.W;
+    const unsigned i0 = blockIdx.x * (BLOCK * EPT) + threadIdx.x;
+    unsigned cell[EPT], word[EPT];
+#pragma unroll
+    for (unsigned k = 0; k < EPT; ++k) {
+        const unsigned i = i0 + k * BLOCK;
+        cell[k] = p.start_mode == 2 ? __umulhi(philox4x32_10(p.env_offset + i, 0u, (unsigned)nonce, (unsigned)(nonce >> 32), p.k0, p.k1 ^ TAG_EVAL).x, p.S) : p.start_cell;
+        word[k] = __ldg(hop + cell[k]);
+    }
+    unsigned nr = 0u; unsigned long long sum = 0ull;
+#pragma unroll
+    for (unsigned k = 0; k < EPT; ++k) {
+        const unsigned i = i0 + k * BLOCK;
+        if (i >= p.N) continue;
+        unsigned s = cell[k], w = word[k];
+        if (p.start_mode == 2 && (w & NO_START)) s = walk_start(p, hop, p.env_offset + i, nonce, w);
+        unsigned steps = 0u, y = s / (unsigned)p.W, x = s - y * (unsigned)p.W;
         unsigned cx = x, cy = y, hops = 0u, limit = 1u;      // the entry the path is compared with, moved up at 1, 3, 7, 15, ... hops
         for (;;) {
-            const unsigned w = __ldg(hop + (size_t)y * (size_t)p.W + (size_t)x);
-            if (w == TRAPPED) { steps = max_steps; break; }
+            if ((w & KIND_MASK) == TRAPPED) { steps = max_steps; break; }
             steps += w & STEPS_MASK;
-            if ((w & KIND_MASK) == KIND_GOAL) { reached = steps <= max_steps; if (!reached) steps = max_steps; break; }
+            if ((w & KIND_MASK) == KIND_GOAL) { if (steps <= max_steps) ++nr; else steps = max_steps; break; }
             if (steps >= max_steps) { steps = max_steps; break; }
             const unsigned e = (w >> 22) & 3u, at = (w >> 16) & (RT - 1u), tx = x & ~(RT - 1u), ty = y & ~(RT - 1u);
             x = (e & 1u) ? (e == 1u ? tx + RT : tx - 1u) : tx + at;
             y = (e & 1u) ? ty + at : (e == 2u ? ty + RT : ty - 1u);
             if (x == cx && y == cy) { steps = max_steps; break; }
             if (++hops == limit) { cx = x; cy = y; hops = 0u; limit <<= 1; }
+            w = __ldg(hop + (size_t)y * (size_t)p.W + (size_t)x);
         }
+        sum += steps;
     }
-    const unsigned nr = __popc(__ballot_sync(FULL, reached));
-    unsigned long long sum = steps;
+    nr = __reduce_add_sync(FULL, nr);
     for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
     if ((threadIdx.x & 31u) == 0u) { if (nr) atomicAdd(&s_reached, nr); atomicAdd(&s_steps, sum); }
     __syncthreads();
@@ -117,7 +151,9 @@ __global__ void __launch_bounds__(BLOCK) k_rollout_walk(const __grid_constant__ 
 void launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
     const dim3 tiles(((unsigned)p.W + RT - 1u) / RT, ((unsigned)p.H + RT - 1u) / RT);
     k_rollout_tiles<<<tiles, RT_THREADS, 0, st>>>(p, hop);
-    k_rollout_walk<<<(p.N + BLOCK - 1u) / BLOCK, BLOCK, 0, st>>>(p, hop, max_steps, nonce, h);
+    // four environments per thread where the chip is full with that
+    if (p.N >= 4u * 8u * BLOCK * 148u) k_rollout_walk<4u><<<(p.N + 4u * BLOCK - 1u) / (4u * BLOCK), BLOCK, 0, st>>>(p, hop, max_steps, nonce, h);
+    else k_rollout_walk<1u><<<(p.N + BLOCK - 1u) / BLOCK, BLOCK, 0, st>>>(p, hop, max_steps, nonce, h);
 }
 
 }  // namespace cudarl

@@ -117,3 +117,17 @@ def test_update_batch_limits(pkg, orc, w, h, n):
     assert np.array_equal(gpu.get_q(), cpu.get_q())
     gpu.update_batch(**b); cpu.update_batch(**b)
     assert np.array_equal(gpu.get_q(), cpu.get_q()) and gpu.get_stats().device_error == 0
+
+
+@pytest.mark.parametrize("w,h,n,warm", [(63, 65, 700, 300), (64, 64, 5000, 900), (200, 129, 9000, 1500), (1, 300, 40, 50), (700, 650, 1212415, 20), (700, 650, 1212416, 20),
+                                        (640, 641, 1300001, 20)])
+@pytest.mark.parametrize("start", [0, 2])
+def test_rollout_limits(pkg, orc, w, h, n, warm, start):
+    """The folded rollout: grids around the edge of its 64 x 64 tiles, one and four environments per thread, caps below, at and beyond the
+    lengths of the paths, a common start cell; the table is taken over from the GPU, so that only the rollout is compared."""
+    gpu, cpu = pair(pkg, orc, world(pkg, w, h, n, start_mode=start, max_steps=200, eps0=0.2), threads=THREADS)
+    gpu.train_steps(warm)
+    cpu.set_q(gpu.get_q())
+    for cap in (0, 1, 17, 60) if n > 100000 else (0, 1, 17, 64, 5000):
+        a, b = gpu.eval_rollout(cap), cpu.eval_rollout(cap)
+        assert (a.envs, a.reached, a.total_steps, a.reward_sum) == (b.envs, b.reached, b.total_steps, b.reward_sum), cap
