@@ -15,7 +15,7 @@ The line printed by rank 0 carries
   roofline   algorithmic bytes (60 B per env-step) x envs per launch / mean duration of the step kernel
              (k_tile_step; one CUDA event pair around every uninterrupted run of launches), against the
              measured HBM copy bandwidth of MEASURED_PEAKS.json,
-  eval       the greedy rollout of all environments that follows training in the workload (k_eval),
+  eval       the greedy rollout of all environments that follows training in the workload (k_rollout_tiles, k_rollout_walk),
   cpu_baseline  the CPU oracle (a C++ port of the same semantics) timed on this box's cores,
   cpu_baseline_reference_python  the reference's own Python loop at its default configuration, where its
              checkout is present,
@@ -37,7 +37,6 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 PKG_DIR = os.path.join(ROOT, "cudarl-arena_b200")
 ALGO_BYTES_TRAIN = 60      # 12 state in + 12 state out + 16 Q[s] row + 16 Q[s'] row + 4 Q[s,a] write
-ALGO_BYTES_EVAL = 40       # greedy rollout step: 24 state + 16 Q[s] row
 FALLBACK_HBM_GBS = 6650.0
 TRAFFIC_C5 = 455.5e6      # dram__bytes_read.sum + dram__bytes_write.sum of one k_tile_step launch on C5 (one ncu capture of one launch)
 
@@ -394,14 +393,14 @@ def main():
             tot = [(int(es.total_steps), int(es.reached))]
         ev_steps, ev_reached = sum(t[0] for t in tot), sum(t[1] for t in tot)
         ev_rate = ev_steps / (ev_ms * 1e-3)
+        eval_bytes = 17 * env.W * env.H + 4 * n_local
         ev = {"value": ev_rate, "unit": "env-steps/s", "ms": ev_ms, "step_cap": args.eval_steps, "env_steps": ev_steps,
               "reached_fraction": ev_reached / float(n_local * world),
-              "roofline": {"bound": "hbm", "kernel": "k_eval_policy + k_eval", "algorithmic_bytes_per_env_step": ALGO_BYTES_EVAL,
-                           "achieved": ALGO_BYTES_EVAL * ev_rate / world / 1e9, "peak": peak, "unit": "GB/s",
-                           "frac": ALGO_BYTES_EVAL * ev_rate / world / 1e9 / peak, "peak_kind": peak_kind,
-                           "note": "includes the host call and its synchronising read of the result; the rollout folds the table into a "
-                                   "one-byte-per-cell policy map once (k_eval_policy) and then reads one byte per environment-step, so "
-                                   "against the 40 B per env-step of a rollout that reads Q[s] every step frac can exceed 1"}}
+              "roofline": {"bound": "hbm", "kernel": "k_rollout_tiles + k_rollout_walk", "algorithmic_bytes_per_rollout": eval_bytes,
+                           "achieved": eval_bytes / (ev_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
+                           "frac": eval_bytes / (ev_ms * 1e-3) / 1e9 / peak, "peak_kind": peak_kind,
+                           "note": "includes the host call and its synchronising read of the result; the rollout folds the table into path lengths "
+                                   "tile by tile and hops over tiles: the table and the cell classes in once, a start cell per environment"}}
 
     peer_mem = env.comm_peer_memory() if world > 1 else False
     rebucket = int(cfg.rebucket_every) if int(cfg.rebucket_every) > 0 else 256      # the library's default period

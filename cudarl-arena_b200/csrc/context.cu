@@ -111,7 +111,7 @@ struct cudarl_ctx {
     bool cls_dirty = true;                // the per-tile class bytes must be rebuilt from the cell words
     int64_t bucket_every = 256, since_bucket = 0;
     void *dent = nullptr, *dctl = nullptr, *deps = nullptr;
-    void *dtra = nullptr, *dtrr = nullptr, *dtrd = nullptr, *dsckey = nullptr, *dscval = nullptr;
+    void *dtra = nullptr, *dtrr = nullptr, *dtrd = nullptr, *dsort = nullptr;
     void *dgather = nullptr;              // replica averaging: the other ranks' rows of this rank's slice
     void* dub = nullptr; size_t ub_cap = 0;                               // the arrays of a large update_batch, and their bytes
     int32_t seen_x = 0, seen_y = 0;       // where the one environment of a context was when it was last stepped alone
@@ -229,24 +229,28 @@ int upload_cells(cudarl_ctx* c) {
 }
 
 // The work area of an update_batch of `n` transitions that one block does not hold: collision entries, chain heads and work lists,
-// the scratch of the longest chains.  Grown to the next power of two, kept until the context goes.  As many chain heads as transitions
+// the sort of the crowded cells.  Grown to the next power of two, kept until the context goes.  As many chain heads as transitions
 // (but no more than cells): a chain then holds one cell's transitions; with 65,536 heads for a million of them, 16 cells shared one and
 // the chains became long ones (320 us in k_fix_long for 1,000,003 transitions on 1024 x 1024 cells).
 int ensure_entry_capacity(cudarl_ctx* c, size_t n) {
     if (n <= c->ent_cap) return 0;
     CK(cudaStreamSynchronize(c->st));
-    cudaFree(c->dent); cudaFree(c->dsckey); cudaFree(c->dscval); cudaFree(c->dmail);
-    c->dent = c->dsckey = c->dscval = c->dmail = nullptr; c->ent_cap = 0;
-    const size_t cap = pow2ceil(std::max<size_t>(n, 4096)), scratch = 2 * cap;
+    cudaFree(c->dent); cudaFree(c->dsort); cudaFree(c->dmail);
+    c->dent = c->dsort = c->dmail = nullptr; c->ent_cap = 0;
+    const size_t cap = pow2ceil(std::max<size_t>(n, 4096));
     size_t slots = std::min(cap, pow2ceil(c->p.S));
     slots = std::min<size_t>(std::max<size_t>(slots, BLOCK), (size_t)1 << 24);
     CK(cudaMalloc(&c->dent, cap * sizeof(uint4)));
-    CK(cudaMalloc(&c->dsckey, scratch * sizeof(unsigned long long)));
-    CK(cudaMalloc(&c->dscval, scratch * sizeof(float)));
+    CK(cudaMalloc(&c->dsort, 2 * cap * sizeof(uint2) + SORT_WORDS * sizeof(unsigned)));
+    SortP& so = c->p.so;
+    so.a = (uint2*)c->dsort; so.b = so.a + cap;
+    so.barrier = (unsigned*)(so.b + cap); so.part = so.barrier + 1; so.total = so.part + SORT_MOST_BLOCKS; so.hist = so.total + 512;
+    CK(cudaMemsetAsync(so.barrier, 0, sizeof(unsigned), c->st));
+    int sms = 0; CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
+    so.blocks = std::min<unsigned>((unsigned)std::max(sms, 1), SORT_MOST_BLOCKS);
     CK(cudaMalloc(&c->dmail, 3 * slots * sizeof(unsigned)));
     CK(cudaMemsetAsync(c->dmail, 0, slots * sizeof(unsigned), c->st));
     c->p.ent = (uint4*)c->dent;
-    c->p.sc_key = (unsigned long long*)c->dsckey; c->p.sc_val = (float*)c->dscval; c->p.sc_cap = (unsigned)scratch;
     c->p.mailbox = (unsigned*)c->dmail; c->p.mb_slots = (unsigned)slots;
     c->p.active = c->p.mailbox + slots; c->p.longq = c->p.mailbox + 2 * slots;
     c->ent_cap = cap; c->p.ent_cap = (unsigned)cap;
@@ -700,7 +704,7 @@ void free_all(cudarl_ctx* c) {
     for (size_t r = 0; r < c->peer_tables.size(); ++r) if ((int)r != c->rank && c->peer_tables[r]) cudaIpcCloseMemHandle(c->peer_tables[r]);
     if (c->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->comm);
     void* bufs[] = {c->dci, c->dstate[0], c->dstate[1], c->dimport, c->dmail, c->dreward, c->ddone, c->dent, c->dctl, c->deps,
-                    c->dtra, c->dtrr, c->dtrd, c->dsckey, c->dscval, c->dgather, c->dact,
+                    c->dtra, c->dtrr, c->dtrd, c->dsort, c->dgather, c->dact,
                     c->dub,
                     c->dQ, c->drec[0], c->drec[1], c->darr[0], c->darr[1], c->dovf[0], c->dovf[1], c->dbmax[0], c->dbmax[1],
                     c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dhop, c->dtq, c->dpeer_ptrs, c->dbarrier_word, c->dgbar, c->dgcnt, c->dgmv, c->dgstate, c->dgbins, c->dwork[0], c->dwork[1]};

@@ -17,14 +17,13 @@
 //
 // Reference semantics: those of tile_engine.cu.
 #include "step_loop.cuh"
+#include "grid_barrier.cuh"
 #include <cstring>
 
 namespace cudarl {
 
-constexpr unsigned long long GRID_WAIT_NS = 2000000000ull;
 
-// A barrier of all blocks of the launch: an arrival counter that only ever grows (the host passes its value at the launch).  Bounded
-// in time: a block that waits two seconds records the failure, and everybody leaves.
+// The table and the counters in global memory.
 struct GlobalTable {
     static constexpr bool ALONE = false;
     const Params& p;
@@ -38,31 +37,10 @@ struct GlobalTable {
     __device__ __forceinline__ void store(unsigned idx, float v) const { reinterpret_cast<float*>(p.Q)[idx] = v; }
 };
 struct GridSpace : GlobalTable {
-    unsigned target; unsigned* s_flag;
-    __device__ __forceinline__ GridSpace(const Params& q, unsigned base, unsigned* flag) : GlobalTable{q}, target(base), s_flag(flag) {}
-    __device__ __forceinline__ void arrive() {      // this block's writes are visible to whoever sees the arrival
-        __syncthreads();
-        target += gridDim.x;
-        if (threadIdx.x == 0u) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(p.gp.barrier) : "memory");
-    }
-    __device__ __forceinline__ bool wait() {
-        if (threadIdx.x == 0u) {
-            unsigned v, ok = 1u;
-            unsigned long long t0 = 0ull;
-            for (unsigned it = 1u;; ++it) {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.gp.barrier) : "memory");
-                if ((int)(v - target) >= 0) break;
-                if ((it & 1023u) == 0u) {
-                    unsigned long long now; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-                    if (t0 == 0ull) t0 = now;
-                    else if (now - t0 > GRID_WAIT_NS) { atomicOr(&p.ctl->error, ERR_COPY_TIMEOUT); ok = 0u; break; }
-                }
-            }
-            *s_flag = ok;
-        }
-        __syncthreads();
-        return *s_flag != 0u;
-    }
+    GridBarrier barrier;
+    __device__ __forceinline__ GridSpace(const Params& q, unsigned base, unsigned* flag) : GlobalTable{q}, barrier{q.gp.barrier, q.ctl, base, flag} {}
+    __device__ __forceinline__ void arrive() { barrier.arrive(); }
+    __device__ __forceinline__ bool wait() { return barrier.wait(); }
 };
 
 // Deal the environments to the blocks by cell: the records of l.in, sorted by lines of eight cells (128 bytes of the table) in the

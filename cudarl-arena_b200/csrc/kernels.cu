@@ -15,6 +15,7 @@
 //   TD update   src/kernels.cu:96-114 (true max as in src/gpu/kernels.cu:36-45, src/train.py:134)
 #include "kernels.cuh"
 #include "rules.cuh"
+#include "grid_barrier.cuh"
 #include <cstdio>
 
 namespace cudarl {
@@ -84,23 +85,6 @@ __device__ __forceinline__ void cswap(unsigned long long& ka, float& va, unsigne
     if (ka > kb) { unsigned long long tk = ka; ka = kb; kb = tk; float tv = va; va = vb; vb = tv; }
 }
 
-// Block-wide bitonic sort of n2 (power of two) key/value pairs in shared or global memory.
-__device__ void block_bitonic(unsigned long long* keys, float* vals, unsigned n2) {
-    for (unsigned k = 2; k <= n2; k <<= 1) {
-        for (unsigned j = k >> 1; j > 0; j >>= 1) {
-            for (unsigned i = threadIdx.x; i < n2; i += blockDim.x) {
-                unsigned ixj = i ^ j;
-                if (ixj > i) {
-                    unsigned long long a = keys[i], b = keys[ixj];
-                    bool up = (i & k) == 0;
-                    if ((a > b) == up) { keys[i] = b; keys[ixj] = a; float t = vals[i]; vals[i] = vals[ixj]; vals[ixj] = t; }
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
-
 // Fold a sorted run (same cell) starting at index j of keys/vals; returns nothing, writes Q_{t+1}.
 __device__ void apply_run(const Params& p, const unsigned long long* keys, const float* vals, unsigned j, unsigned n) {
     unsigned w0 = (unsigned)(keys[j] >> 32);
@@ -115,73 +99,12 @@ __device__ void apply_run(const Params& p, const unsigned long long* keys, const
     p.Q[cell] = row;          // in place: the targets were taken before this kernel started, and one thread owns the cell
 }
 
-constexpr unsigned LONG_SMEM = 1024;   // chain entries sorted in shared memory; longer chains use the global scratch
+constexpr unsigned STAGE_ENTRIES = 1024;   // chain entries a block stages in shared memory
+constexpr unsigned LONG_MARK = 0xFFFFFFFFu;   // in a mailbox slot: its chain is long
 constexpr int SHORT_MAX = 8;           // chain entries folded in registers by one thread
 
-// One long chain, whole block: count its entries (one hop per run), pick shared memory or a slice of the
-// global scratch, copy the runs (one warp per run, batches of 256 runs), bitonic-sort by (cell, action, id)
-// and let the first thread of every cell run fold it.
-__device__ void process_long(const Params& p, unsigned head1, unsigned long long* s_keys, float* s_vals,
-                             unsigned* s_bcast) {
-    __shared__ unsigned s_run[BLOCK], s_off[BLOCK];
-    if (threadIdx.x == 0) {
-        unsigned q = head1, L = 0, hops = 0;
-        while (q && hops <= p.ent_cap) {          // a chain can never have more runs than the entry array has slots
-            L += (q >> LINK_POS_BITS) + 1u; ++hops;
-            q = p.ent[(q & LINK_POS_MASK) - 1u].w;
-        }
-        unsigned n2 = 1; while (n2 < L) n2 <<= 1;
-        unsigned base = 0xFFFFFFFFu;
-        if (q || L > p.ent_cap) { atomicOr(&p.ctl->error, ERR_CHAIN_CYCLE); base = 0xFFFFFFFEu; }
-        else if (L > LONG_SMEM) {
-            base = atomicAdd(&p.ctl->scratch_cursor, n2);
-            if (base + n2 > p.sc_cap) { atomicOr(&p.ctl->error, ERR_SCRATCH_OVERFLOW); base = 0xFFFFFFFEu; }
-        }
-        s_bcast[0] = L; s_bcast[1] = n2; s_bcast[2] = base;
-    }
-    __syncthreads();
-    const unsigned L = s_bcast[0], n2 = s_bcast[1], base = s_bcast[2];
-    if (base != 0xFFFFFFFEu) {
-        unsigned long long* keys = (base == 0xFFFFFFFFu) ? s_keys : p.sc_key + base;
-        float* vals = (base == 0xFFFFFFFFu) ? s_vals : p.sc_val + base;
-        __shared__ unsigned s_q, s_nb, s_done_entries;
-        if (threadIdx.x == 0) { s_q = head1; s_done_entries = 0; }
-        __syncthreads();
-        while (true) {                               // batches of up to 256 runs; ends when the chain is exhausted
-            if (threadIdx.x == 0) {
-                unsigned q = s_q, nb = 0, off = s_done_entries;
-                while (q && nb < (unsigned)BLOCK) {
-                    s_run[nb] = q; s_off[nb] = off; off += (q >> LINK_POS_BITS) + 1u; ++nb;
-                    q = p.ent[(q & LINK_POS_MASK) - 1u].w;
-                }
-                s_q = q; s_nb = nb; s_done_entries = off;
-            }
-            __syncthreads();
-            const unsigned nb = s_nb;
-            if (nb == 0u) break;
-            for (unsigned r = threadIdx.x >> 5; r < nb; r += BLOCK / 32) {
-                const unsigned link = s_run[r], pos0 = (link & LINK_POS_MASK) - 1u, len = (link >> LINK_POS_BITS) + 1u;
-                const unsigned j = threadIdx.x & 31u;
-                if (j < len && s_off[r] + j < L) {
-                    const uint4 e = p.ent[pos0 + j];
-                    keys[s_off[r] + j] = ((unsigned long long)e.x << 32) | e.y; vals[s_off[r] + j] = __uint_as_float(e.z);
-                }
-            }
-            __syncthreads();
-        }
-        for (unsigned i = L + threadIdx.x; i < n2; i += blockDim.x) { keys[i] = ~0ull; vals[i] = 0.0f; }
-        __syncthreads();
-        block_bitonic(keys, vals, n2);
-        for (unsigned j = threadIdx.x; j < L; j += blockDim.x) {
-            unsigned cp = (unsigned)(keys[j] >> 34);
-            if (j == 0 || (unsigned)(keys[j - 1] >> 34) != cp) apply_run(p, keys, vals, j, L);
-        }
-    }
-    __syncthreads();
-}
-
 constexpr unsigned MED_MAX = 32;                         // chain entries ranked by one warp with shuffles
-constexpr unsigned MED_CHUNKS = LONG_SMEM / MED_MAX;     // medium chains a block can stage in shared memory
+constexpr unsigned MED_CHUNKS = STAGE_ENTRIES / MED_MAX;     // medium chains a block can stage in shared memory
 
 // One warp orders a staged chain of L <= 32 entries by (cell, action, index) with a shuffle ranking
 // (indices are unique, so ranks are a permutation), then the first lane of every cell run folds it.
@@ -211,12 +134,12 @@ __device__ void process_medium(const Params& p, unsigned long long* keys, float*
 // the chain's entries:
 //   <= 8 entries   in registers, ordered by a sorting network and folded by that thread;
 //   <= 32 entries  staged in shared memory by that thread, ordered and folded by one warp;
-//   longer         queued for k_fix_long (one warp per chain up to 256 entries, then one block per chain).
+//   longer         marked, and left to k_fix_long.
 __device__ __forceinline__ void flush_row(const Params& p, unsigned cellpar, const float4& row) { p.Q[cellpar >> 1] = row; }
 
 __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
-    __shared__ unsigned long long s_keys[LONG_SMEM];
-    __shared__ float s_vals[LONG_SMEM];
+    __shared__ unsigned long long s_keys[STAGE_ENTRIES];
+    __shared__ float s_vals[STAGE_ENTRIES];
     __shared__ unsigned s_medlen[MED_CHUNKS];
     __shared__ unsigned s_nmed;
     const unsigned nactive = p.ctl->active_count;      // slots that received a chain in this call
@@ -279,9 +202,10 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
                 staged = (rem == 0u && q == 0u);
                 s_medlen[chunk] = staged ? L : 0u;
             }
-            if (!staged) {                              // hand the chain to k_fix_long
+            if (!staged) {                              // leave the chain's cells to k_fix_long
                 const unsigned li = atomicAdd(&p.ctl->long_count, 1u);
-                p.longq[li] = head;
+                p.longq[li] = slot;
+                p.mailbox[slot] = LONG_MARK;
             }
         }
     }
@@ -298,75 +222,124 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
 
 }
 
-// Long chains (more than 32 entries: cells crowded with environments).  First tier: one WARP per chain for up
-// to 256 entries -- lane 0 hops from run to run, all lanes copy the run's entries into the warp's slice of
-// shared memory, a warp-wide bitonic sort orders them by (cell, action, id), the first lane of every cell run
-// applies it.  Chains that do not fit are left to the block.
-constexpr unsigned WARP_LONG = 256;
+// Entries of long chains (more than 32: cells crowded with transitions).  Following such a chain is one look-up after the other -- 10,000
+// transitions of a cell took 5 ms -- so it is not followed: the entries of marked slots are picked out of the entry array in order, sorted
+// by cell and action with a stable radix sort, which keeps the order of the transitions, and every (cell, action) is folded by one warp.
+// One cooperative launch; without long chains it ends at once.  The last kernel of an update_batch: it clears the call's counters and posts
+// the box.
+// What bounds it: the sort's three barriers per pass of 9 bits and three sweeps over the entries, then the longest (cell, action) at about
+// 10 cycles a transition.
+constexpr unsigned SORT_THREADS = 512u, SORT_WARPS = SORT_THREADS / 32u, SORT_BITS = 9u, SORT_BINS = 1u << SORT_BITS;
+static_assert(SORT_BINS == SORT_THREADS, "one bin per thread");
 
-__device__ bool process_long_warp(const Params& p, unsigned head, unsigned long long* keys, float* vals) {
-    const unsigned lane = threadIdx.x & 31u;
-    unsigned q = head, L = 0, hops = 0; bool fits = true;
-    while (q && hops <= p.ent_cap) {                  // q is warp-uniform
-        const unsigned pos0 = (q & LINK_POS_MASK) - 1u, len = (q >> LINK_POS_BITS) + 1u;
-        if (L + len > WARP_LONG) { fits = false; break; }
-        uint4 e = make_uint4(0u, 0u, 0u, 0u);
-        if (lane < len) { e = __ldcg(p.ent + pos0 + lane); keys[L + lane] = ((unsigned long long)e.x << 32) | e.y; vals[L + lane] = __uint_as_float(e.z); }
-        q = __shfl_sync(FULL, e.w, 0);                // the run's first entry carries the link to the next run
-        L += len; ++hops;
+__device__ void fold_crowded(const Params& p, unsigned n, GridBarrier& bar) {
+    __shared__ unsigned s_count[SORT_WARPS][SORT_BINS];
+    __shared__ unsigned s_base[SORT_BINS], s_warp[33];
+    const SortP& so = p.so;
+    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, lt = (1u << lane) - 1u, blocks = gridDim.x, b = blockIdx.x;
+    auto share = [&](unsigned m, unsigned& first, unsigned& last) { const unsigned per = (m + blocks - 1u) / blocks; first = min(b * per, m); last = min(first + per, m); };
+    unsigned first, last, total = 0u;
+
+    // ---- pick out, in order ----
+    share(n, first, last);
+    auto chosen = [&](unsigned i, uint4& e) -> bool { if (i >= last) return false; e = p.ent[i]; return p.mailbox[mb_slot(p, e.x >> 3)] == LONG_MARK; };
+    unsigned mine = 0u; uint4 e;
+    for (unsigned i = first + tid; i < last; i += SORT_THREADS) if (chosen(i, e)) ++mine;
+    block_scan_excl(mine, s_warp, &total);
+    if (tid == 0u) so.part[b] = total;
+    if (!bar.pass()) return;
+    unsigned before = 0u, all = 0u;
+    for (unsigned k = tid; k < blocks; k += SORT_THREADS) { const unsigned v = so.part[k]; all += v; if (k < b) before += v; }
+    block_scan_excl(before, s_warp, &before);
+    block_scan_excl(all, s_warp, &all);
+    for (unsigned i0 = first; i0 < last; i0 += SORT_THREADS) {
+        const bool take = chosen(i0 + tid, e);
+        const unsigned at = before + block_scan_excl(take ? 1u : 0u, s_warp, &total);
+        if (take) so.a[at] = make_uint2(((e.x >> 3) << 2) | (e.x & 3u), e.z);
+        before += total;
     }
-    if (!fits || q) return false;
-    unsigned n2 = 32; while (n2 < L) n2 <<= 1;
-    for (unsigned i = L + lane; i < n2; i += 32u) { keys[i] = ~0ull; vals[i] = 0.0f; }
-    __syncwarp();
-    for (unsigned k = 2; k <= n2; k <<= 1) {
-        for (unsigned j = k >> 1; j > 0; j >>= 1) {
-            for (unsigned i = lane; i < n2; i += 32u) {
-                const unsigned ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = keys[i], b = keys[ixj];
-                    const bool up = (i & k) == 0;
-                    if ((a > b) == up) { keys[i] = b; keys[ixj] = a; const float t = vals[i]; vals[i] = vals[ixj]; vals[ixj] = t; }
-                }
+    if (!bar.pass()) return;
+    for (unsigned k = b * SORT_THREADS + tid; k < p.ctl->long_count; k += blocks * SORT_THREADS) p.mailbox[p.longq[k]] = 0u;
+
+    // ---- sort, least significant digit first ----
+    uint2 *from = so.a, *to = so.b;
+    const unsigned key_bits = 32u - (unsigned)__clz((int)(p.S * 4u - 1u)), passes = (key_bits + SORT_BITS - 1u) / SORT_BITS, bits = (key_bits + passes - 1u) / passes;
+    share(all, first, last);
+    for (unsigned pass = 0; pass < passes; ++pass) {
+        const unsigned shift = pass * bits, mask = (1u << bits) - 1u;
+        s_base[tid] = 0u;
+        __syncthreads();
+        for (unsigned i = first + tid; i < last; i += SORT_THREADS) atomicAdd(&s_base[(from[i].x >> shift) & mask], 1u);
+        __syncthreads();
+        so.hist[tid * blocks + b] = s_base[tid];
+        if (!bar.pass()) return;
+        for (unsigned d = b * SORT_WARPS + warp; d < SORT_BINS; d += blocks * SORT_WARPS) {       // a warp per digit: where each block's part of it starts
+            unsigned run = 0u;
+            for (unsigned k0 = 0; k0 < blocks; k0 += 32u) {
+                const unsigned k = k0 + lane, v = k < blocks ? so.hist[d * blocks + k] : 0u;
+                unsigned inc = v;
+                for (int o = 1; o < 32; o <<= 1) { const unsigned u = __shfl_up_sync(FULL, inc, o); if (lane >= (unsigned)o) inc += u; }
+                if (k < blocks) so.hist[d * blocks + k] = run + inc - v;
+                run += __shfl_sync(FULL, inc, 31);
             }
-            __syncwarp();
+            if (lane == 0u) so.total[d] = run;
         }
+        if (!bar.pass()) return;
+        const unsigned start = block_scan_excl(so.total[tid], s_warp, &total) + so.hist[tid * blocks + b];
+        s_base[tid] = start;
+        for (unsigned i0 = first; i0 < last; i0 += SORT_THREADS) {
+            for (unsigned w = 0; w < SORT_WARPS; ++w) s_count[w][tid] = 0u;
+            __syncthreads();
+            const unsigned i = i0 + tid;
+            const bool act = i < last;
+            const uint2 v = act ? from[i] : make_uint2(0u, 0u);
+            const unsigned d = act ? (v.x >> shift) & mask : SORT_BINS;
+            const unsigned mates = __match_any_sync(FULL, d), rank = __popc(mates & lt);
+            if (act && rank == 0u) s_count[warp][d] = __popc(mates);
+            __syncthreads();
+            unsigned run = s_base[tid];
+            for (unsigned w = 0; w < SORT_WARPS; ++w) { const unsigned c = s_count[w][tid]; s_count[w][tid] = run; run += c; }
+            s_base[tid] = run;
+            __syncthreads();
+            if (act) to[s_count[warp][d] + rank] = v;
+            __syncthreads();
+        }
+        uint2* const t = from; from = to; to = t;
+        if (!bar.pass()) return;
     }
-    for (unsigned j = lane; j < L; j += 32u) {
-        const unsigned cp = (unsigned)(keys[j] >> 34);
-        if (j == 0 || (unsigned)(keys[j - 1] >> 34) != cp) apply_run(p, keys, vals, j, L);
-    }
-    __syncwarp();
-    return true;
-}
 
-// Eight chains at a time, one per warp; those too long for a warp are then taken one after the other by the whole block: any length,
-// in shared memory up to 1024 entries, in the global scratch beyond.  The last kernel of an update_batch: it clears the call's counters
-// and posts the box.
-__global__ void __launch_bounds__(BLOCK) k_fix_long(Params p, Handover h) {
-    constexpr unsigned WARPS = BLOCK / 32;
-    __shared__ unsigned long long s_keys[WARPS * WARP_LONG];
-    __shared__ float s_vals[WARPS * WARP_LONG];
-    __shared__ unsigned s_left[WARPS], s_bcast[3];
-    const unsigned n = p.ctl->long_count;
-    const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    unsigned done = 0;
-    for (unsigned c0 = blockIdx.x * WARPS; c0 < n; c0 += gridDim.x * WARPS) {
-        const unsigned c = c0 + warp;
-        unsigned left = 0u;
-        if (c < n) {
-            const unsigned head = p.longq[c];
-            if (!process_long_warp(p, head, s_keys + warp * WARP_LONG, s_vals + warp * WARP_LONG)) left = head;
-            ++done;
+    // ---- fold: the warp whose window a (cell, action) starts in takes all of it ----
+    unsigned crowded = 0u;
+    for (unsigned i0 = (b * SORT_WARPS + warp) * 32u; i0 < all; i0 += blocks * SORT_WARPS * 32u) {
+        const unsigned i = i0 + lane, key = i < all ? from[i].x : 0xFFFFFFFFu, prev = i && i < all ? from[i - 1u].x : 0xFFFFFFFFu;
+        if (i < all && (key >> 2) != (prev >> 2) && i + 32u < all && (from[i + 32u].x >> 2) == (key >> 2)) ++crowded;      // a cell with more than 32 transitions
+        unsigned starts = __ballot_sync(FULL, i < all && key != prev);
+        while (starts) {
+            const unsigned l = (unsigned)__ffs((int)starts) - 1u, k = __shfl_sync(FULL, key, l);
+            starts &= starts - 1u;
+            float q = reinterpret_cast<const float*>(p.Q)[k];
+            unsigned j = i0 + l + lane;
+            uint2 cur = j < all ? from[j] : make_uint2(0xFFFFFFFFu, 0u);
+            for (;;) {
+                const unsigned m = __ballot_sync(FULL, cur.x == k), cnt = m == FULL ? 32u : (unsigned)__ffs((int)~m) - 1u;
+                const float target = __uint_as_float(cur.y);
+                j += 32u;
+                cur = cnt == 32u && j < all ? from[j] : make_uint2(0xFFFFFFFFu, 0u);          // on its way while these are folded
+                for (unsigned u = 0; u < cnt; ++u) q = __fmaf_rn(p.lr, __fsub_rn(__shfl_sync(FULL, target, u), q), q);      // each sees the value the one before it left
+                if (cnt < 32u) break;
+            }
+            if (lane == 0u) reinterpret_cast<float*>(p.Q)[k] = q;
         }
-        if (lane == 0u) s_left[warp] = left;
-        __syncthreads();
-        for (unsigned k = 0; k < WARPS; ++k) if (s_left[k]) process_long(p, s_left[k], s_keys, s_vals, s_bcast);
-        __syncthreads();
     }
-    if (lane == 0 && done) atomicAdd(&p.ctl->long_chains, (unsigned long long)done);
+    crowded = __reduce_add_sync(FULL, crowded);
+    if (lane == 0u && crowded) atomicAdd(&p.ctl->long_chains, (unsigned long long)crowded);
+}
+__global__ void __launch_bounds__(SORT_THREADS) k_fix_long(const __grid_constant__ Params p, unsigned n, Handover h) {
+    __shared__ unsigned s_flag;
+    GridBarrier bar{p.so.barrier, p.ctl, 0u, &s_flag};
+    if (p.ctl->long_count && !(*reinterpret_cast<volatile unsigned*>(&p.ctl->error) & ERR_COPY_TIMEOUT)) fold_crowded(p, n, bar);
     if (last_to_finish<false>(p)) {
-        p.ctl->active_count = 0u; p.ctl->long_count = 0u; p.ctl->scratch_cursor = 0u;
+        p.ctl->active_count = 0u; p.ctl->long_count = 0u; *p.so.barrier = 0u;
         box_put_error(p, h);
     }
 }
@@ -565,7 +538,9 @@ void launch_update_batch(const Params& p, unsigned n, const Transitions& tr, Han
     }
     k_update_main<<<nblk(n), BLOCK, 0, st>>>(p, n, tr);
     k_fix<<<fix_blocks(p), BLOCK, 0, st>>>(p);
-    k_fix_long<<<296, BLOCK, 0, st>>>(p, h);
+    void* args[3] = {const_cast<Params*>(&p), &n, &h};
+    const unsigned blocks = (n + 2u * SORT_THREADS - 1u) / (2u * SORT_THREADS);
+    cudaLaunchCooperativeKernel((const void*)k_fix_long, dim3(blocks < p.so.blocks ? blocks : p.so.blocks), dim3(SORT_THREADS), args, 0, st);
 }
 void launch_q_init(const Params& p, int kind, float scale, cudaStream_t st) { k_q_init<<<nblk(p.S), BLOCK, 0, st>>>(p, kind, scale); }
 void launch_cell_set(const Params& p, unsigned cell, unsigned cls, int clear_goals, cudaStream_t st) {

@@ -30,8 +30,7 @@ struct Ctl {
     unsigned int eps_len;           // table length (clamp)
     unsigned long long eps_base_k;  // per-episode mode: table[0] belongs to episodes/N == eps_base_k
     unsigned int active_count;      // update_batch: mailbox slots holding a chain,
-    unsigned int long_count;        // chains left to k_fix_long,
-    unsigned int scratch_cursor;    // bump allocator of the long-chain scratch: all zero between calls
+    unsigned int long_count;        // chains left to k_fix_long: zero between calls
     unsigned int error;             // sticky internal error bits
     unsigned int never;             // zero for good: what a wait that a test makes run out looks at
     float eps_used;                 // epsilon of the most recent step (for the stats call)
@@ -125,6 +124,14 @@ struct World {
     Ctl* ctl;
     unsigned long long step;   // set by the host per launch: global batched step index g (keys the policy stream, selects the counter plane)
 };
+constexpr unsigned SORT_MOST_BLOCKS = 256u;
+struct SortP {
+    unsigned* barrier;     // zero between calls
+    uint2 *a, *b;          // {cell * 4 + action, target}: as many as transitions
+    unsigned *part, *total, *hist;     // per block, per digit, per digit and block
+    unsigned blocks;       // of the launch: all run at the same time
+};
+constexpr size_t SORT_WORDS = 1u + SORT_MOST_BLOCKS + 512u + 512u * (size_t)SORT_MOST_BLOCKS;      // barrier, part, total, hist
 struct Params : World {
     unsigned policy_keys[20];   // the ten round keys of the policy stream, two words each: operands straight from the constant bank
     uint4* ent;            // collision entries
@@ -132,10 +139,10 @@ struct Params : World {
     unsigned* mailbox;     // update_batch: chain heads (0 = empty), power-of-two size
     unsigned mb_slots;     // mailbox slots (power of two, multiple of BLOCK)
     unsigned* active;      // list of the mailbox slots that hold a chain in this step (mb_slots entries)
-    unsigned* longq;       // heads of the chains left to k_fix_long (mb_slots entries)
+    unsigned* longq;       // slots of the chains left to k_fix_long (mb_slots entries)
     const float* eps_tab;
     int* tr_a; float* tr_r; unsigned char* tr_d;   // optional trace of the last step, per ENVIRONMENT
-    unsigned long long* sc_key; float* sc_val; unsigned sc_cap;   // long-chain scratch (global)
+    SortP so;              // update_batch: the sort of k_fix_long
     // per-launch values set by the host
     unsigned eps_idx;          // index of this step's epsilon in eps_tab
     int eps_from_ctl;          // 1: take the index from ctl (per-episode schedule)

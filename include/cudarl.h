@@ -84,7 +84,7 @@ typedef struct cudarl_config {
     int32_t  sync_every;    /* average the replicas every this many train steps; 0 = never */
     int32_t  rebucket_every;/* re-size the per-tile record regions every this many train steps (0 = default 256, <0 = only when
                                training starts); results never depend on it */
-    int32_t  tile_edge;     /* tile edge of the train step in cells: 0 = chosen from the population density, or 8 / 16;
+    int32_t  tile_edge;     /* 0 = how the train step runs is chosen from the sizes; 8 / 16 = always in tiles of that many cells;
                                results never depend on it */
     int32_t  avg_over_nccl; /* 1: the replica averaging always moves its slices by NCCL send / receive, never over IPC-mapped
                                peer memory (same results; must be the same on every rank) */

@@ -131,3 +131,22 @@ def test_rollout_limits(pkg, orc, w, h, n, warm, start):
     for cap in (0, 1, 17, 60) if n > 100000 else (0, 1, 17, 64, 5000):
         a, b = gpu.eval_rollout(cap), cpu.eval_rollout(cap)
         assert (a.envs, a.reached, a.total_steps, a.reward_sum) == (b.envs, b.reached, b.total_steps, b.reward_sum), cap
+
+
+@pytest.mark.parametrize("w,h,n", [(1, 1, 1025), (1, 2, 300000), (10, 10, 1 << 20), (64, 64, 200000), (300, 200, 1300), (2000, 1500, 70001)])
+def test_update_batch_crowded_cells(pkg, orc, w, h, n):
+    """Cells with more transitions than a chain is followed for: none, some and all of the batch, one to three passes of the sort."""
+    rng = np.random.RandomState(n)
+    gpu, cpu = pair(pkg, orc, pkg.make_config(w, h, 1, lr=0.05, gamma=0.95, q_init_kind=pkg.QINIT_UNIFORM, q_init_scale=1.0))
+    hot = rng.rand(n) < 0.4
+    b = dict(sx=np.where(hot, np.minimum(w - 1, rng.geometric(0.3, n)), rng.randint(0, w, n)), sy=np.where(hot, h // 2, rng.randint(0, h, n)),
+             a=rng.randint(0, 4, n), r=rng.choice([-0.01, 1.0, 0.25], n).astype(np.float32), nx=rng.randint(0, w, n), ny=rng.randint(0, h, n),
+             dn=(rng.rand(n) < 0.2).astype(np.uint8))
+    for _ in range(2):
+        gpu.update_batch(**b)
+        assert cpu.update_batch(**b) == 0
+        assert np.array_equal(gpu.get_q(), cpu.get_q())
+    cells = np.bincount(b["sy"] * w + b["sx"])
+    if w * h <= 4096:                                    # no two cells share a chain
+        assert gpu.get_stats().long_chains == 2 * int((cells > 32).sum())
+    assert gpu.get_stats().device_error == 0
