@@ -773,7 +773,7 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
             CK(cudaEventCreate(&c->ev0)); CK(cudaEventCreate(&c->ev1));
             const size_t N = p.N ? p.N : 1;
             { int r0 = alloc_cells(c); if (r0) return r0; }
-            for (int cp = 0; cp < 2; ++cp) { CK(cudaMalloc(&c->dstate[cp], N * 16)); CK(cudaMemsetAsync(c->dstate[cp], 0, N * 16, c->st)); }
+            for (int cp = 0; cp < 2; ++cp) { CK(cudaMalloc(&c->dstate[cp], N * 16 + 64)); CK(cudaMemsetAsync(c->dstate[cp], 0, N * 16 + 64, c->st)); }
             CK(cudaMalloc(&c->dctl, sizeof(Ctl)));
             CK(cudaMemsetAsync(c->dctl, 0, sizeof(Ctl), c->st));
             p.st = (int4*)c->dstate[0]; p.st2 = (int4*)c->dstate[1];
@@ -1068,16 +1068,16 @@ int cudarl_get_state(cudarl_ctx* c, int32_t* x, int32_t* y, int32_t* t) {
     if (!c) return -1;
     CK(cudaSetDevice(c->cfg.device));
     { int rl = records_in_order(c); if (rl) return rl; }
-    const size_t N = c->p.N, b = N * 4;
-    // the export kernel writes x[N] | y[N] | t[N] in environment order: into the stage when there is room, else into the spare copy
-    const bool small = 3 * b <= STAGE_ROOM;
-    launch_export_state(c->p, small ? (int*)(c->stage.dev + STAGE_DATA) : (int*)c->p.st2, handover(c), c->st);
+    const size_t N = c->p.N, b = N * 4, row = up16(b);
+    // the export kernel writes x | y | t in environment order: into the stage when there is room, else into the spare copy
+    const bool small = 3 * row <= STAGE_ROOM;
+    launch_export_state(c->p, small ? (int*)(c->stage.dev + STAGE_DATA) : (int*)c->p.st2, (unsigned)(row / 4), handover(c), c->st);
     CK(cudaGetLastError());
     unsigned char* const base = small ? c->stage.host + STAGE_DATA : (unsigned char*)c->p.st2;
     Segment out[3]; int n = 0;
     if (x) out[n++] = Segment{x, base, b};
-    if (y) out[n++] = Segment{y, base + b, b};
-    if (t) out[n++] = Segment{t, base + 2 * b, b};
+    if (y) out[n++] = Segment{y, base + row, b};
+    if (t) out[n++] = Segment{t, base + 2 * row, b};
     if (!small) CK(copy_out(out, n, c->cfg.device, c->st));
     { int rw = wait_box(c); if (rw) return rw; }
     if (small) copy_host(out, n, false);

@@ -54,12 +54,15 @@ __global__ void k_import_state(const __grid_constant__ World p, const int* x, co
     r.w = (int)i;
     p.st[i] = r;
 }
-// x[N] | y[N] | t[N] in environment order, into the spare copy or straight into the mapped stage
-__global__ void k_export_state(const __grid_constant__ World p, int* __restrict__ out, Handover h) {
-    unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+// x | y | t in environment order (rows of `stride` >= N words, a multiple of 4), into the spare copy or straight into the mapped stage: four
+// environments per thread, whole 16-byte words out.
+__global__ void k_export_state(const __grid_constant__ World p, int* __restrict__ out, unsigned stride, Handover h) {
+    const unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) * 4u;
     if (i < p.N) {
-        const int4 r = p.st[i];
-        out[r.w] = r.x; out[p.N + r.w] = r.y; out[2u * p.N + r.w] = r.z;
+        const int4 r0 = p.st[i], r1 = p.st[min(i + 1u, p.N - 1u)], r2 = p.st[min(i + 2u, p.N - 1u)], r3 = p.st[min(i + 3u, p.N - 1u)];
+        *reinterpret_cast<int4*>(out + i) = make_int4(r0.x, r1.x, r2.x, r3.x);
+        *reinterpret_cast<int4*>(out + stride + i) = make_int4(r0.y, r1.y, r2.y, r3.y);
+        *reinterpret_cast<int4*>(out + 2u * stride + i) = make_int4(r0.z, r1.z, r2.z, r3.z);
     }
     if (last_to_finish<true>(p)) box_put_error(p, h);
 }
@@ -357,15 +360,26 @@ __device__ __forceinline__ int4 stepped(const World& p, const int4 rec, int a, u
     const unsigned s2 = moved ? to : s;
     return make_int4((int)(s2 % (unsigned)p.W), (int)(s2 / (unsigned)p.W), rec.z + 1, rec.w);
 }
+__device__ __forceinline__ void step_record(const World& p, unsigned i, int a, float& r, unsigned char& dn) {
+    const int4 rec = p.st[i];                               // record i is environment i
+    dn = p.done[i];
+    const unsigned to = target_cell(p, rec.x, rec.y, a);
+    p.st[i] = stepped(p, rec, a, to, cw_load(p.cw, (unsigned)rec.y * (unsigned)p.W + (unsigned)rec.x), cw_load(p.cw, to), r, dn);
+}
+// VEC: four environments per thread, so that what crosses the link does so in 16-byte words a thread; else any alignment.
+template <bool VEC>
 __global__ void k_step_actions(const __grid_constant__ World p, const int* __restrict__ actions, float* __restrict__ rewards, unsigned char* __restrict__ dones, Handover h) {
-    unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < p.N) {
-        const int4 rec = p.st[i];
-        const unsigned e = (unsigned)rec.w;
-        const int a = actions[e];
-        float r; unsigned char dn = p.done[e];
-        const unsigned to = target_cell(p, rec.x, rec.y, a);
-        p.st[i] = stepped(p, rec, a, to, cw_load(p.cw, (unsigned)rec.y * (unsigned)p.W + (unsigned)rec.x), cw_load(p.cw, to), r, dn);
+    const unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) * (VEC ? 4u : 1u);
+    if (VEC && i + 4u <= p.N) {
+        const int4 a = *reinterpret_cast<const int4*>(actions + i);
+        float4 r; uchar4 d;
+        step_record(p, i, a.x, r.x, d.x); step_record(p, i + 1u, a.y, r.y, d.y); step_record(p, i + 2u, a.z, r.z, d.z); step_record(p, i + 3u, a.w, r.w, d.w);
+        *reinterpret_cast<float4*>(p.reward + i) = r; *reinterpret_cast<uchar4*>(p.done + i) = d;
+        if (rewards) *reinterpret_cast<float4*>(rewards + i) = r;
+        if (dones) *reinterpret_cast<uchar4*>(dones + i) = d;
+    } else for (unsigned e = i; e < p.N && e < i + (VEC ? 4u : 1u); ++e) {
+        float r; unsigned char dn;
+        step_record(p, e, actions[e], r, dn);
         p.reward[e] = r; p.done[e] = dn;
         if (rewards) rewards[e] = r;
         if (dones) dones[e] = dn;
@@ -513,7 +527,7 @@ static inline unsigned fix_blocks(const Params& p) { unsigned b = p.mb_slots / B
 static inline unsigned sweep_blocks(unsigned S) { unsigned b = nblk((2u * S + 15u) / 16u); return b < 1u ? 1u : (b > 1184u ? 1184u : b); }
 
 void launch_identity_ids(const Params& p, cudaStream_t st) { if (p.N) k_ids_identity<<<nblk(p.N), BLOCK, 0, st>>>(p); }
-void launch_export_state(const Params& p, int* out, Handover h, cudaStream_t st) { k_export_state<<<p.N ? nblk(p.N) : 1u, BLOCK, 0, st>>>(p, out, h); }
+void launch_export_state(const Params& p, int* out, unsigned stride, Handover h, cudaStream_t st) { k_export_state<<<p.N ? nblk((p.N + 3u) / 4u) : 1u, BLOCK, 0, st>>>(p, out, stride, h); }
 void launch_copy_out(const Params& p, const CopySpan* spans, int n, Handover h, cudaStream_t st) {
     const CopySpan none{nullptr, nullptr, 0u}, a = n > 0 ? spans[0] : none, b = n > 1 ? spans[1] : none;
     const unsigned blocks = nblk(((a.bytes > b.bytes ? a.bytes : b.bytes) + 15u) / 16u);
@@ -525,7 +539,10 @@ void launch_reset_all(const Params& p, cudaStream_t st) {
     if (p.N) k_reset_all<<<nblk(p.N), BLOCK, 0, st>>>(p);
 }
 void launch_step_actions(const Params& p, const int* a, float* r, unsigned char* d, Handover h, cudaStream_t st) {
-    if (p.N) k_step_actions<<<nblk(p.N), BLOCK, 0, st>>>(p, a, r, d, h);
+    if (!p.N) return;
+    const bool vec = (((uintptr_t)a | (uintptr_t)r) & 15u) == 0u && ((uintptr_t)d & 3u) == 0u;
+    if (vec) k_step_actions<true><<<nblk((p.N + 3u) / 4u), BLOCK, 0, st>>>(p, a, r, d, h);
+    else k_step_actions<false><<<nblk(p.N), BLOCK, 0, st>>>(p, a, r, d, h);
 }
 void launch_step_one(const Params& p, int action, bool reset, int x, int y, Handover h, cudaStream_t st) { k_step_one<<<1, 1, 0, st>>>(p, action, reset, x, y, h); }
 void launch_update_batch(const Params& p, unsigned n, const Transitions& tr, Handover h, cudaStream_t st) {

@@ -154,7 +154,7 @@ constexpr int BLOCK = 256;
 
 // launch wrappers (kernels.cu); all asynchronous on `st`
 void launch_identity_ids(const Params& p, cudaStream_t st);
-void launch_export_state(const Params& p, int* out, Handover h, cudaStream_t st);                 // out = x[N]|y[N]|t[N] in environment order
+void launch_export_state(const Params& p, int* out, unsigned stride, Handover h, cudaStream_t st);   // out = x | y | t in environment order, rows of `stride` words (a multiple of 4)
 struct CopySpan { const void* src; void* dst; unsigned bytes; };
 void launch_copy_out(const Params& p, const CopySpan* spans, int n, Handover h, cudaStream_t st); // up to two spans of device memory into mapped host memory
 void launch_post(const Params& p, Handover h, cudaStream_t st);                                   // words 1.. = the counters of the control block, in the order of cudarl_stats, low half first; then epsilon
