@@ -346,7 +346,18 @@ inline float boxf(const cudarl_ctx* c, unsigned k) { const uint32_t b = box32(c,
 // The next kernel's hand-over: where it puts small results, and under which number it reports them.
 Handover handover(cudarl_ctx* c) { return Handover{(HostBox*)c->stage.dev, ++c->ticket}; }
 // Arrays in the stage, behind the box.
-constexpr size_t STAGE_DATA = 256, STAGE_ROOM = STAGE_BYTES - STAGE_DATA;
+constexpr size_t STAGE_DATA = 256;
+// How large a stage: room for the states of all environments and for the table, each up to 4 MB: so far a kernel's own accesses across the
+// link are faster than copies through the ring (B200, states of 131,072 environments 145 -> 65 us, a table of 1 MB 100 -> 59 us, of 4 MB
+// 193 -> 134 us); 64 KB for a single small environment, of which a program may keep many.
+constexpr size_t UPDATE_MOST = (size_t)1 << 20;
+size_t stage_bytes(const Params& p) {
+    if (p.N == 1u && p.S <= 2048u) return (size_t)64 << 10;
+    const size_t most = (size_t)4 << 20, states = STAGE_DATA + 12 * ((size_t)p.N + 4), table = STAGE_DATA + 16 * (size_t)p.S;
+    size_t b = (size_t)1 << 20;
+    for (const size_t want : {states, table}) while (want <= most && b < want) b += (size_t)1 << 20;
+    return b;
+}
 inline size_t up16(size_t b) { return (b + 15) / 16 * 16; }
 
 // After the box has been posted: has any kernel recorded an internal failure (a copy that never landed, a full
@@ -377,7 +388,7 @@ int wait_counters(cudarl_ctx* c) {
 int hand_out(cudarl_ctx* c, const Segment* segs, int n) {
     size_t room = 0;
     for (int k = 0; k < n; ++k) room += up16(segs[k].bytes);
-    if (room <= STAGE_ROOM && n <= 2) {
+    if (STAGE_DATA + room <= c->stage.bytes && n <= 2) {
         CopySpan spans[2]; size_t off = STAGE_DATA;
         for (int k = 0; k < n; ++k) { spans[k] = CopySpan{segs[k].dev, c->stage.dev + off, (unsigned)segs[k].bytes}; off += up16(segs[k].bytes); }
         launch_copy_out(c->p, spans, n, handover(c), c->st);
@@ -779,7 +790,7 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
             p.st = (int4*)c->dstate[0]; p.st2 = (int4*)c->dstate[1];
             p.ctl = (Ctl*)c->dctl;
             hostio_retain(); c->retained = true;
-            CK(stage_take(&c->stage));
+            CK(stage_take(&c->stage, stage_bytes(p)));
             c->box = (HostBox*)c->stage.host;
             int r2;
             r2 = alloc_table(c); if (r2) return r2;
@@ -854,7 +865,7 @@ int cudarl_step_actions(cudarl_ctx* c, const int32_t* actions, float* rewards, u
     const size_t N = c->p.N;
     if (N == 0) return 0;
     const size_t off_r = STAGE_DATA + up16(N * 4), off_d = off_r + up16(N * 4);
-    if (off_d + N <= STAGE_BYTES) {
+    if (off_d + N <= c->stage.bytes) {
         // actions read, rewards and flags written by the kernel itself across the link: one launch and one wait instead of three copies
         const Segment in{c->stage.host + STAGE_DATA, const_cast<int32_t*>(actions), N * 4};
         copy_host(&in, 1, true);
@@ -1038,7 +1049,7 @@ int cudarl_update_batch(cudarl_ctx* c, int64_t n, const int32_t* sx, const int32
         if (bad) s.bad = true;
     };
     const size_t part = up16(N * 4);
-    const bool small = STAGE_DATA + 3 * part <= STAGE_BYTES;
+    const bool small = STAGE_DATA + 3 * part <= std::min(c->stage.bytes, UPDATE_MOST);
     if (!small && 3 * part > c->ub_cap) {
         CK(cudaStreamSynchronize(c->st));
         cudaFree(c->dub); c->dub = nullptr; c->ub_cap = 0;
@@ -1070,7 +1081,7 @@ int cudarl_get_state(cudarl_ctx* c, int32_t* x, int32_t* y, int32_t* t) {
     { int rl = records_in_order(c); if (rl) return rl; }
     const size_t N = c->p.N, b = N * 4, row = up16(b);
     // the export kernel writes x | y | t in environment order: into the stage when there is room, else into the spare copy
-    const bool small = 3 * row <= STAGE_ROOM;
+    const bool small = STAGE_DATA + 3 * row <= c->stage.bytes;
     launch_export_state(c->p, small ? (int*)(c->stage.dev + STAGE_DATA) : (int*)c->p.st2, (unsigned)(row / 4), handover(c), c->st);
     CK(cudaGetLastError());
     unsigned char* const base = small ? c->stage.host + STAGE_DATA : (unsigned char*)c->p.st2;

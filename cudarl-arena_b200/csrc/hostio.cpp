@@ -20,25 +20,29 @@ namespace {
 // twelve cores and the copy engine busy.  Measured on the B200 box (16 cores, 268 MB into a fresh NumPy array): 56 ms through the
 // driver, 9.6 ms with 8 copying threads, 7.5 with 12; into memory that has been written before 5.6 either way, the speed of the link.
 constexpr size_t SLOT_BYTES = (size_t)2 << 20;
-constexpr size_t PIECE_MIN = (size_t)128 << 10;
+constexpr size_t CHUNK_MIN = (size_t)64 << 10, PIECE_MIN = (size_t)256 << 10, HOST_CHUNK_MOST = (size_t)128 << 10;
 // Copies within the host between a stage and the caller: shared from a quarter of a megabyte on.
 constexpr size_t HOST_MIN = (size_t)256 << 10, HOST_PIECE = (size_t)32 << 10;
 constexpr int SLOTS = 20, MAX_WORKERS = 11, MAX_DEVICES = 64;
 // Below this the driver copies: it is as fast as the ring up to there (B200 box: 2 MB in 0.12 ms either way, 4 MB 0.23 and 0.16).
 constexpr size_t SHARED_MIN_OUT = (size_t)768 << 10, SHARED_MIN_IN = (size_t)3 << 20;
 
-struct Chunk { unsigned char* host; unsigned char* dev; size_t bytes; Fill fill; const void* arg; size_t first; };
+// What one core copies at a time; `at`: where it lies in the slot of its piece.
+struct Chunk { unsigned char* host; unsigned char* dev; size_t bytes; Fill fill; const void* arg; size_t first; size_t piece, at; };
+// What the copy engine moves at a time: chunks [chunk, chunk + count).  Enqueueing one takes the caller's thread about 8 us, so they are
+// larger than what is best for the cores: 4 MB in 32 pieces took 290 us.
+struct Piece { unsigned char* dev; size_t bytes, chunk, count; };
 enum class Way { Out, In, Host, HostIn };        // device -> caller, caller -> device, stage -> caller, caller -> stage
 
 // One transfer.  The caller's thread alone talks to the driver (several threads asking for events and enqueueing copies hold each
 // other up in it) and copies when it has nothing else to do; the workers only copy.
 struct Job {
-    std::vector<Chunk> chunks;
+    std::vector<Chunk> chunks; std::vector<Piece> pieces;
     Way way = Way::Host;
     std::atomic<size_t> next{0};                 // first chunk nobody has taken
-    std::atomic<size_t> landed{0};               // Out: chunks whose device copy is complete
-    std::atomic<size_t> turn[SLOTS];             // the chunk the slot is free for
-    std::atomic<size_t> filled[SLOTS];           // In: 1 + the last chunk copied into the slot
+    std::atomic<size_t> landed{0};               // Out: chunks whose piece is complete
+    std::atomic<size_t> turn[SLOTS];             // the piece the slot is free for
+    std::atomic<size_t> copied[SLOTS];           // chunks of the slot's piece copied out of it, or into it
     std::atomic<size_t> done{0};                 // chunks copied by a thread
     std::atomic<bool> failed{false};
     std::atomic<int> busy{0};                    // workers inside the job
@@ -99,15 +103,18 @@ void send(unsigned char* dst, const unsigned char* src, const Chunk& c) {
 bool copy_one(Job& j) {
     size_t k = j.next.load(std::memory_order_relaxed);
     if (k >= j.chunks.size()) return false;
-    const size_t slot = k % SLOTS;
-    if (j.way == Way::Out && k >= j.landed.load(std::memory_order_acquire)) return false;
-    if (j.way == Way::In && j.turn[slot].load(std::memory_order_acquire) != k) return false;
-    if (!j.next.compare_exchange_strong(k, k + 1)) return true;          // another thread was quicker: look again
     const Chunk& c = j.chunks[k];
-    unsigned char* const buf = pool().ring + slot * SLOT_BYTES;
+    const size_t slot = c.piece % SLOTS;
+    if (j.way == Way::Out && k >= j.landed.load(std::memory_order_acquire)) return false;
+    if (j.way == Way::In && j.turn[slot].load(std::memory_order_acquire) != c.piece) return false;
+    if (!j.next.compare_exchange_strong(k, k + 1)) return true;          // another thread was quicker: look again
+    unsigned char* const buf = pool().ring + slot * SLOT_BYTES + c.at;
     switch (j.way) {
-        case Way::Out: std::memcpy(c.host, buf, c.bytes); j.turn[slot].store(k + SLOTS, std::memory_order_release); break;
-        case Way::In: send(buf, c.host, c); j.filled[slot].store(k + 1, std::memory_order_release); break;
+        case Way::Out:
+            std::memcpy(c.host, buf, c.bytes);
+            if (j.copied[slot].fetch_add(1, std::memory_order_acq_rel) + 1 == j.pieces[c.piece].count) { j.copied[slot] = 0; j.turn[slot].store(c.piece + SLOTS, std::memory_order_release); }
+            break;
+        case Way::In: send(buf, c.host, c); j.copied[slot].fetch_add(1, std::memory_order_release); break;
         case Way::Host: std::memcpy(c.host, c.dev, c.bytes); break;
         case Way::HostIn: send(c.host, c.dev, c); break;
     }
@@ -147,17 +154,23 @@ void ready_workers() {
     p.stop = false;
     for (int k = 0; k < n; ++k) p.workers.emplace_back(worker_main);
 }
-// Cut into pieces of `most` bytes, or of less (but not below `least`) so that a short transfer still has two for every core.
-void cut(Job& j, const Segment* segs, int n, size_t most, size_t least) {
-    size_t total = 0, piece = most;
+// Cut into chunks of at most `most` bytes, or of less (but not below `least`) so that a short transfer still has two for every core; for the
+// copy engine (`pieces`) into eight pieces or more, of up to a slot, each of whole chunks.
+void cut(Job& j, const Segment* segs, int n, size_t most, size_t least, bool pieces) {
+    size_t total = 0, chunk = most, piece = SLOT_BYTES;
     for (int s = 0; s < n; ++s) total += segs[s].bytes;
-    while (piece > least && total / piece < 2u * (MAX_WORKERS + 1)) piece >>= 1;
+    while (chunk > least && total / chunk < 2u * (MAX_WORKERS + 1)) chunk >>= 1;
+    while (piece > PIECE_MIN && total / piece < 8u) piece >>= 1;
     for (int s = 0; s < n; ++s) {
         unsigned char* h = (unsigned char*)segs[s].host; unsigned char* d = (unsigned char*)segs[s].dev;
         const bool made = segs[s].fill != nullptr;
+        const uintptr_t base = made ? 0u : (uintptr_t)h;
         for (size_t first = 0; first < segs[s].bytes;) {
-            const size_t edge = piece - ((made ? first : (uintptr_t)h + first) & (piece - 1)), b = std::min(segs[s].bytes - first, edge);
-            j.chunks.push_back(Chunk{made && !h ? nullptr : h + first, made && !d ? nullptr : d + first, b, segs[s].fill, segs[s].arg, first});
+            if (pieces && (first == 0 || ((base + first) & (piece - 1)) == 0)) j.pieces.push_back(Piece{d + first, 0, j.chunks.size(), 0});
+            const size_t edge = chunk - ((base + first) & (chunk - 1)), b = std::min(segs[s].bytes - first, edge);
+            Chunk c{made && !h ? nullptr : h + first, made && !d ? nullptr : d + first, b, segs[s].fill, segs[s].arg, first, 0, 0};
+            if (pieces) { Piece& p = j.pieces.back(); c.piece = j.pieces.size() - 1; c.at = p.bytes; p.bytes += b; ++p.count; }
+            j.chunks.push_back(c);
             first += b;
         }
     }
@@ -185,7 +198,7 @@ cudaError_t ready_ring(int device) {
         const Segment all{ring, nullptr, bytes, [](void* d, size_t, size_t n, const void*) { std::memset(d, 0, n); }, nullptr};
         Job j;
         j.way = Way::HostIn;
-        cut(j, &all, 1, SLOT_BYTES, SLOT_BYTES);
+        cut(j, &all, 1, SLOT_BYTES, SLOT_BYTES, false);
         publish(j);
         help(j);
         withdraw(j);
@@ -201,33 +214,35 @@ cudaError_t ready_ring(int device) {
 cudaError_t run_job(Job& j, int device, cudaStream_t st) {
     Pool& p = pool();
     cudaEvent_t* const ev = p.events[device];
-    const size_t n = j.chunks.size();
-    for (size_t k = 0; k < SLOTS; ++k) { j.turn[k] = k; j.filled[k] = 0; }
+    const size_t n = j.pieces.size();
+    for (size_t k = 0; k < SLOTS; ++k) { j.turn[k] = k; j.copied[k] = 0; }
     publish(j);
-    size_t issued = 0, complete = 0;             // device copies enqueued, and known to be complete, in order
+    size_t issued = 0, complete = 0;             // pieces enqueued, and known to be complete, in order
     cudaError_t e = cudaSuccess;
-    while (e == cudaSuccess && (complete < n || j.done.load(std::memory_order_acquire) < n)) {
+    while (e == cudaSuccess && (complete < n || j.done.load(std::memory_order_acquire) < j.chunks.size())) {
+        // what has landed first: the other threads wait for it
+        if (complete < issued) {
+            const size_t slot = complete % SLOTS;
+            const cudaError_t q = cudaEventQuery(ev[slot]);
+            if (q == cudaSuccess) {
+                if (j.way == Way::In) { j.copied[slot] = 0; j.turn[slot].store(complete + SLOTS, std::memory_order_release); }
+                else j.landed.store(j.pieces[complete].chunk + j.pieces[complete].count, std::memory_order_release);
+                ++complete;
+                continue;
+            }
+            if (q != cudaErrorNotReady) { e = q; break; }
+        }
         if (issued < n) {
             const size_t slot = issued % SLOTS;
-            const Chunk& c = j.chunks[issued];
+            const Piece& c = j.pieces[issued];
             unsigned char* const buf = p.ring + slot * SLOT_BYTES;
-            const bool ready = j.way == Way::Out ? j.turn[slot].load(std::memory_order_acquire) == issued : j.filled[slot].load(std::memory_order_acquire) == issued + 1;
+            const bool ready = j.turn[slot].load(std::memory_order_acquire) == issued && (j.way == Way::Out || j.copied[slot].load(std::memory_order_acquire) == c.count);
             if (ready) {
                 e = j.way == Way::Out ? cudaMemcpyAsync(buf, c.dev, c.bytes, cudaMemcpyDeviceToHost, st) : cudaMemcpyAsync(c.dev, buf, c.bytes, cudaMemcpyHostToDevice, st);
                 if (e == cudaSuccess) e = cudaEventRecord(ev[slot], st);
                 ++issued;
                 continue;
             }
-        }
-        if (complete < issued) {
-            const cudaError_t q = cudaEventQuery(ev[complete % SLOTS]);
-            if (q == cudaSuccess) {
-                if (j.way == Way::In) j.turn[complete % SLOTS].store(complete + SLOTS, std::memory_order_release);
-                ++complete;
-                if (j.way == Way::Out) j.landed.store(complete, std::memory_order_release);
-                continue;
-            }
-            if (q != cudaErrorNotReady) { e = q; break; }
         }
         // In: a thread that copies does not send off what the others have filled, and the link idles meanwhile
         if (j.way == Way::Out || p.workers.empty()) copy_one(j); else cpu_relax();
@@ -252,7 +267,7 @@ cudaError_t copy_all(const Segment* segs, int n, bool out, int device, cudaStrea
             if (e != cudaSuccess) return e;
             Job j;
             j.way = out ? Way::Out : Way::In;
-            cut(j, segs, n, SLOT_BYTES, PIECE_MIN);
+            cut(j, segs, n, SLOT_BYTES, CHUNK_MIN, true);
             return run_job(j, device, st);
         }
     }
@@ -291,13 +306,15 @@ void hostio_release() {
     p.spare.clear();
 }
 
-cudaError_t stage_take(Stage* s) {
+cudaError_t stage_take(Stage* s, size_t bytes) {
     Pool& p = pool();
     {
         std::lock_guard<std::mutex> lk(p.mu);
-        if (!p.spare.empty()) { *s = p.spare.back(); p.spare.pop_back(); std::memset(s->host, 0, 256); return cudaSuccess; }
+        for (size_t k = 0; k < p.spare.size(); ++k)
+            if (p.spare[k].bytes == bytes) { *s = p.spare[k]; p.spare.erase(p.spare.begin() + (long)k); std::memset(s->host, 0, 256); return cudaSuccess; }
     }
-    cudaError_t e = cudaHostAlloc((void**)&s->host, STAGE_BYTES, cudaHostAllocPortable | cudaHostAllocMapped);
+    s->bytes = bytes;
+    cudaError_t e = cudaHostAlloc((void**)&s->host, bytes, cudaHostAllocPortable | cudaHostAllocMapped);
     if (e != cudaSuccess) { s->host = nullptr; return e; }
     std::memset(s->host, 0, 256);
     e = cudaHostGetDevicePointer((void**)&s->dev, s->host, 0);
@@ -320,7 +337,7 @@ void copy_host(const Segment* segs, int n, bool into_stage) {
             ready_workers();
             Job j;
             j.way = into_stage ? Way::HostIn : Way::Host;
-            cut(j, segs, n, PIECE_MIN, HOST_PIECE);
+            cut(j, segs, n, HOST_CHUNK_MOST, HOST_PIECE, false);
             publish(j);
             help(j);
             withdraw(j);                         // every worker has left: every chunk is copied

@@ -18,12 +18,11 @@ typedef void (*Fill)(void* dst, size_t first, size_t bytes, const void* arg);
 struct Segment { void* host; void* dev; size_t bytes; Fill fill = nullptr; const void* arg = nullptr; };
 
 // One pinned block mapped into the device, for the small results and inputs of a context.
-constexpr size_t STAGE_BYTES = (size_t)1 << 20;
-struct Stage { unsigned char* host = nullptr; unsigned char* dev = nullptr; };
+struct Stage { unsigned char* host = nullptr; unsigned char* dev = nullptr; size_t bytes = 0; };
 
 void hostio_retain();                         // one per context: keeps the process-wide parts alive
 void hostio_release();
-cudaError_t stage_take(Stage* s);             // zeroed first 256 bytes
+cudaError_t stage_take(Stage* s, size_t bytes);      // zeroed first 256 bytes
 void stage_give(Stage* s);
 
 // Device -> host: everything enqueued on `st` before has been waited for and the data is in the caller's arrays on return.

@@ -531,7 +531,7 @@ void launch_export_state(const Params& p, int* out, unsigned stride, Handover h,
 void launch_copy_out(const Params& p, const CopySpan* spans, int n, Handover h, cudaStream_t st) {
     const CopySpan none{nullptr, nullptr, 0u}, a = n > 0 ? spans[0] : none, b = n > 1 ? spans[1] : none;
     const unsigned blocks = nblk(((a.bytes > b.bytes ? a.bytes : b.bytes) + 15u) / 16u);
-    k_copy_out<<<blocks < 1u ? 1u : (blocks > 64u ? 64u : blocks), BLOCK, 0, st>>>(p, a, b, h);
+    k_copy_out<<<blocks < 1u ? 1u : (blocks > 296u ? 296u : blocks), BLOCK, 0, st>>>(p, a, b, h);
 }
 void launch_post(const Params& p, Handover h, cudaStream_t st) { k_post<<<1, 32, 0, st>>>(p, h); }
 void launch_import_state(const Params& p, const int* x, const int* y, const int* t, cudaStream_t st) { if (p.N) k_import_state<<<nblk(p.N), BLOCK, 0, st>>>(p, x, y, t); }
