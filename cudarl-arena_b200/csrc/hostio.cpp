@@ -21,6 +21,8 @@ namespace {
 // driver, 9.6 ms with 8 copying threads, 7.5 with 12; into memory that has been written before 5.6 either way, the speed of the link.
 constexpr size_t SLOT_BYTES = (size_t)2 << 20;
 constexpr size_t CHUNK_MIN = (size_t)64 << 10, PIECE_MIN = (size_t)256 << 10, HOST_CHUNK_MOST = (size_t)128 << 10;
+// From here on a result array is likely to be fresh memory.
+constexpr size_t TOUCH_MIN = (size_t)4 << 20;
 // Copies within the host between a stage and the caller: shared from a quarter of a megabyte on.
 constexpr size_t HOST_MIN = (size_t)256 << 10, HOST_PIECE = (size_t)32 << 10;
 constexpr int SLOTS = 20, MAX_WORKERS = 11, MAX_DEVICES = 64;
@@ -32,7 +34,7 @@ struct Chunk { unsigned char* host; unsigned char* dev; size_t bytes; Fill fill;
 // What the copy engine moves at a time: chunks [chunk, chunk + count).  Enqueueing one takes the caller's thread about 8 us, so they are
 // larger than what is best for the cores: 4 MB in 32 pieces took 290 us.
 struct Piece { unsigned char* dev; size_t bytes, chunk, count; };
-enum class Way { Out, In, Host, HostIn };        // device -> caller, caller -> device, stage -> caller, caller -> stage
+enum class Way { Out, In, Host, HostIn, Touch }; // device -> caller, caller -> device, stage -> caller, caller -> stage; pages of the caller faulted in
 
 // One transfer.  The caller's thread alone talks to the driver (several threads asking for events and enqueueing copies hold each
 // other up in it) and copies when it has nothing else to do; the workers only copy.
@@ -117,6 +119,7 @@ bool copy_one(Job& j) {
         case Way::In: send(buf, c.host, c); j.copied[slot].fetch_add(1, std::memory_order_release); break;
         case Way::Host: std::memcpy(c.host, c.dev, c.bytes); break;
         case Way::HostIn: send(c.host, c.dev, c); break;
+        case Way::Touch: for (size_t b = 0; b < c.bytes; b += 4096) *(volatile unsigned char*)(c.host + b) = 0; break;
     }
     j.done.fetch_add(1, std::memory_order_release);
     return true;
@@ -260,9 +263,18 @@ cudaError_t copy_all(const Segment* segs, int n, bool out, int device, cudaStrea
     if ((made || total >= (out ? SHARED_MIN_OUT : SHARED_MIN_IN)) && device >= 0 && device < MAX_DEVICES) {
         std::unique_lock<std::mutex> lk(p.use, std::try_to_lock);      // another thread's transfer has the ring: let the driver do this one
         if (lk.owns_lock()) {
+            ready_workers();
+            if (out && total >= TOUCH_MIN && cudaStreamQuery(st) == cudaErrorNotReady) {
+                // the device is still at work enqueued earlier: the pages the results go to are faulted in meanwhile
+                Job t;
+                t.way = Way::Touch;
+                cut(t, segs, n, SLOT_BYTES, SLOT_BYTES, false);
+                publish(t);
+                help(t);
+                withdraw(t);
+            }
             cudaError_t e = cudaStreamSynchronize(st);                 // do not spin through work enqueued earlier
             if (e != cudaSuccess) return e;
-            ready_workers();
             e = ready_ring(device);
             if (e != cudaSuccess) return e;
             Job j;
