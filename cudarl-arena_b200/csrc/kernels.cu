@@ -449,23 +449,62 @@ __global__ void k_update_main(Params p, unsigned n, Transitions tr) {
     }
 }
 
-// update_batch of up to 1,024 transitions in one block: targets, a bitonic sort by (cell, action, index) -- strides below a warp by
-// shuffle -- and the first of every run folds it.  One launch instead of three and nothing but latency: the inputs across the link, one
-// look-up of the next rows, the sort, one read and write of the entries.  KEY: 32 bits hold cell, action and index of grids of up to
-// 2^20 cells and halve the sort's shuffles.
+// update_batch of up to 1,024 transitions in one block, one launch, nothing but latency: the inputs across the link, one look-up of the next
+// rows, one read and write of the entries.  Transitions of one (cell, action) find each other in a hash table in shared memory; the first
+// there folds their list, by index, when no list is longer than 8 -- else the block sorts them all (bitonic by (cell, action, index), strides
+// below a warp by shuffle) and the first of every run folds it.  KEY: 32 bits hold cell, action and index of grids of up to 2^20 cells and
+// halve the sort's shuffles.
+constexpr unsigned UPDATE_SLOTS = 2u * UPDATE_SMALL, UPDATE_LIST = 8u;
 template <class KEY>
 __global__ void __launch_bounds__(UPDATE_SMALL) k_update_small(const __grid_constant__ World p, unsigned n, const __grid_constant__ Transitions tr, Handover h) {
     __shared__ KEY s_key[UPDATE_SMALL];
     __shared__ float s_target[UPDATE_SMALL];
+    __shared__ unsigned s_slot[UPDATE_SLOTS], s_head[UPDATE_SLOTS], s_next[UPDATE_SMALL];       // (cell, action) + 1; list of its transitions: index + 1, 0 = end
     constexpr unsigned IDX = 10u, IDX_MASK = (1u << IDX) - 1u;
     static_assert(UPDATE_SMALL == 1u << IDX, "index bits of the key");
     const unsigned i = threadIdx.x;
     KEY key = ~(KEY)0;
+    unsigned at = 0u, next = 0u; float r = 0.0f;
+    if (i < n) load_transition(tr, i, at, next, r);
+    for (unsigned k = i; k < UPDATE_SLOTS; k += blockDim.x) { s_slot[k] = 0u; s_head[k] = 0u; }
+    __syncthreads();
+    bool first = false; unsigned slot = 0u;
     if (i < n) {
-        unsigned at, next; float r;
-        load_transition(tr, i, at, next, r);
-        s_target[i] = transition_target(p, at, next, r);
-        key = ((KEY)(at & 0x7FFFFFFFu) << IDX) | i;
+        const unsigned own = at & 0x7FFFFFFFu;
+        key = ((KEY)own << IDX) | i;
+        slot = (own * 0x9E3779B1u) >> (32u - IDX - 1u);
+        for (;; slot = (slot + 1u) & (UPDATE_SLOTS - 1u)) {
+            const unsigned was = atomicCAS(&s_slot[slot], 0u, own + 1u);
+            first = was == 0u;
+            if (first || was == own + 1u) break;
+        }
+        s_next[i] = atomicExch(&s_head[slot], i + 1u);
+    }
+    float v = 0.0f;
+    float* const q = reinterpret_cast<float*>(p.Q) + (at & 0x7FFFFFFFu);
+    if (first) v = *q;
+    if (i < n) s_target[i] = transition_target(p, at, next, r);
+    __syncthreads();
+    unsigned list[UPDATE_LIST], len = 0u;
+    if (first) {
+        unsigned e = s_head[slot];
+#pragma unroll
+        for (unsigned k = 0; k < UPDATE_LIST; ++k) { list[k] = e ? e : 0xFFFFFFFFu; if (e) { ++len; e = s_next[e - 1u]; } }
+        if (e) len = UPDATE_LIST + 1u;
+    }
+    if (!__syncthreads_or(len > UPDATE_LIST)) {
+        if (first) {
+            for (unsigned last = 0u; len; --len) {
+                unsigned m = list[0] > last ? list[0] : 0xFFFFFFFFu;
+#pragma unroll
+                for (unsigned k = 1; k < UPDATE_LIST; ++k) if (list[k] > last && list[k] < m) m = list[k];
+                v = __fmaf_rn(p.lr, __fsub_rn(s_target[m - 1u], v), v);          // each sees the value the one before it left
+                last = m;
+            }
+            *q = v;
+        }
+        if (i == 0u) box_put_error(p, h);
+        return;
     }
     for (unsigned k = 2u; k <= blockDim.x; k <<= 1)
         for (unsigned j = k >> 1; j; j >>= 1) {
@@ -482,17 +521,21 @@ __global__ void __launch_bounds__(UPDATE_SMALL) k_update_small(const __grid_cons
     __syncthreads();
     s_key[i] = key;
     __syncthreads();
-    const KEY at = key >> IDX;
-    if (key != ~(KEY)0 && (i == 0u || s_key[i - 1u] >> IDX != at)) {
-        float* const q = reinterpret_cast<float*>(p.Q) + at;
-        float v = *q;
+    const KEY own = key >> IDX;
+    if (key != ~(KEY)0 && (i == 0u || s_key[i - 1u] >> IDX != own)) {
+        float* const entry = reinterpret_cast<float*>(p.Q) + own;
+        float u = *entry;
         for (unsigned j = i; j < blockDim.x; ++j) {
             const KEY e = s_key[j];
-            if (e >> IDX != at) break;
-            v = __fmaf_rn(p.lr, __fsub_rn(s_target[(unsigned)e & IDX_MASK], v), v);      // each sees the value the one before it left
+            if (e >> IDX != own) break;
+            u = __fmaf_rn(p.lr, __fsub_rn(s_target[(unsigned)e & IDX_MASK], u), u);
         }
-        *q = v;
+        *entry = u;
     }
+    // a cell with more than 32 transitions
+    const KEY cell = key >> (IDX + 2u);
+    if (key != ~(KEY)0 && (i == 0u || s_key[i - 1u] >> (IDX + 2u) != cell) && i + 32u < blockDim.x && s_key[i + 32u] != ~(KEY)0 && s_key[i + 32u] >> (IDX + 2u) == cell)
+        atomicAdd(&p.ctl->long_chains, 1ull);
     if (i == 0u) box_put_error(p, h);
 }
 

@@ -133,9 +133,10 @@ def test_rollout_limits(pkg, orc, w, h, n, warm, start):
         assert (a.envs, a.reached, a.total_steps, a.reward_sum) == (b.envs, b.reached, b.total_steps, b.reward_sum), cap
 
 
-@pytest.mark.parametrize("w,h,n", [(1, 1, 1025), (1, 2, 300000), (10, 10, 1 << 20), (64, 64, 200000), (300, 200, 1300), (2000, 1500, 70001)])
+@pytest.mark.parametrize("w,h,n", [(5, 5, 33), (9, 3, 700), (40, 40, 1000), (3000, 2000, 1024), (1, 1, 1024), (1, 1, 1025), (1, 2, 300000), (10, 10, 1 << 20), (64, 64, 200000), (300, 200, 1300), (2000, 1500, 70001)])
 def test_update_batch_crowded_cells(pkg, orc, w, h, n):
-    """Cells with more transitions than a chain is followed for: none, some and all of the batch, one to three passes of the sort."""
+    """Cells with more transitions than a chain is followed for: none, some and all of the batch, one
+    block with its lists or its sort, one to three passes of the sort across blocks."""
     rng = np.random.RandomState(n)
     gpu, cpu = pair(pkg, orc, pkg.make_config(w, h, 1, lr=0.05, gamma=0.95, q_init_kind=pkg.QINIT_UNIFORM, q_init_scale=1.0))
     hot = rng.rand(n) < 0.4
