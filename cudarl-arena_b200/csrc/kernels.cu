@@ -146,10 +146,12 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
     __shared__ unsigned s_medlen[MED_CHUNKS];
     __shared__ unsigned s_nmed;
     const unsigned nactive = p.ctl->active_count;      // slots that received a chain in this call
-  for (unsigned tile = blockIdx.x; tile * BLOCK < nactive; tile += gridDim.x) {
+    // few slots are spread over all blocks, a warp's worth each: a block stages no more than 32 chains of medium length
+    const unsigned per = min((unsigned)BLOCK, ((nactive + gridDim.x - 1u) / gridDim.x + 31u) & ~31u);
+  for (unsigned tile = blockIdx.x; tile * per < nactive; tile += gridDim.x) {
     if (threadIdx.x == 0) s_nmed = 0;
     __syncthreads();
-    const unsigned ai = tile * BLOCK + threadIdx.x;
+    const unsigned ai = threadIdx.x < per ? tile * per + threadIdx.x : nactive;
     const unsigned slot = ai < nactive ? p.active[ai] : 0u;
     const unsigned head = ai < nactive ? p.mailbox[slot] : 0u;
     if (head) {
@@ -566,7 +568,7 @@ __global__ void k_cell_set(const __grid_constant__ World p, unsigned cell, unsig
 
 // ------------------------------------------------------------------------------------------------
 static inline unsigned nblk(unsigned n) { return (n + BLOCK - 1) / BLOCK; }
-static inline unsigned fix_blocks(const Params& p) { unsigned b = p.mb_slots / BLOCK; return b > 1184u ? 1184u : b; }
+static inline unsigned fix_blocks(const Params& p) { const unsigned b = p.mb_slots / 32u; return b > 1184u ? 1184u : b; }
 static inline unsigned sweep_blocks(unsigned S) { unsigned b = nblk((2u * S + 15u) / 16u); return b < 1u ? 1u : (b > 1184u ? 1184u : b); }
 
 void launch_identity_ids(const Params& p, cudaStream_t st) { if (p.N) k_ids_identity<<<nblk(p.N), BLOCK, 0, st>>>(p); }
