@@ -353,12 +353,12 @@ constexpr size_t STAGE_DATA = 256;
 constexpr size_t UPDATE_MOST = (size_t)1 << 20;
 size_t stage_bytes(const Params& p) {
     if (p.N == 1u && p.S <= 2048u) return (size_t)64 << 10;
-    const size_t most = (size_t)4 << 20, states = STAGE_DATA + 12 * ((size_t)p.N + 4), table = STAGE_DATA + 16 * (size_t)p.S;
+    const size_t most = (size_t)4 << 20, states = STAGE_DATA + 12 * ((size_t)p.N + 16), table = STAGE_DATA + 16 * (size_t)p.S;
     size_t b = (size_t)1 << 20;
     for (const size_t want : {states, table}) while (want <= most && b < want) b += (size_t)1 << 20;
     return b;
 }
-inline size_t up16(size_t b) { return (b + 15) / 16 * 16; }
+inline size_t up64(size_t b) { return (b + 63) / 64 * 64; }
 
 // After the box has been posted: has any kernel recorded an internal failure (a copy that never landed, a full
 // scratch area, a record outside its tile)?  The word is sticky; the results of the context are not to be trusted.
@@ -387,16 +387,16 @@ int wait_counters(cudarl_ctx* c) {
 // Device arrays into the caller's: through the stage when they are small (one kernel, no copies), else through the pinned ring.
 int hand_out(cudarl_ctx* c, const Segment* segs, int n) {
     size_t room = 0;
-    for (int k = 0; k < n; ++k) room += up16(segs[k].bytes);
+    for (int k = 0; k < n; ++k) room += up64(segs[k].bytes);
     if (STAGE_DATA + room <= c->stage.bytes && n <= 2) {
         CopySpan spans[2]; size_t off = STAGE_DATA;
-        for (int k = 0; k < n; ++k) { spans[k] = CopySpan{segs[k].dev, c->stage.dev + off, (unsigned)segs[k].bytes}; off += up16(segs[k].bytes); }
+        for (int k = 0; k < n; ++k) { spans[k] = CopySpan{segs[k].dev, c->stage.dev + off, (unsigned)segs[k].bytes}; off += up64(segs[k].bytes); }
         launch_copy_out(c->p, spans, n, handover(c), c->st);
         CK(cudaGetLastError());
         { int rw = wait_box(c); if (rw) return rw; }
         off = STAGE_DATA;
         Segment parts[2];
-        for (int k = 0; k < n; ++k) { parts[k] = Segment{segs[k].host, c->stage.host + off, segs[k].bytes}; off += up16(segs[k].bytes); }
+        for (int k = 0; k < n; ++k) { parts[k] = Segment{segs[k].host, c->stage.host + off, segs[k].bytes}; off += up64(segs[k].bytes); }
         copy_host(parts, n, false);
         return 0;
     }
@@ -864,7 +864,7 @@ int cudarl_step_actions(cudarl_ctx* c, const int32_t* actions, float* rewards, u
     int rc = ensure_step_buffers(c); if (rc) return rc;
     const size_t N = c->p.N;
     if (N == 0) return 0;
-    const size_t off_r = STAGE_DATA + up16(N * 4), off_d = off_r + up16(N * 4);
+    const size_t off_r = STAGE_DATA + up64(N * 4), off_d = off_r + up64(N * 4);
     if (off_d + N <= c->stage.bytes) {
         // actions read, rewards and flags written by the kernel itself across the link: one launch and one wait instead of three copies
         const Segment in{c->stage.host + STAGE_DATA, const_cast<int32_t*>(actions), N * 4};
@@ -1048,7 +1048,7 @@ int cudarl_update_batch(cudarl_ctx* c, int64_t n, const int32_t* sx, const int32
         }
         if (bad) s.bad = true;
     };
-    const size_t part = up16(N * 4);
+    const size_t part = up64(N * 4);
     const bool small = STAGE_DATA + 3 * part <= std::min(c->stage.bytes, UPDATE_MOST);
     if (!small && 3 * part > c->ub_cap) {
         CK(cudaStreamSynchronize(c->st));
@@ -1079,7 +1079,7 @@ int cudarl_get_state(cudarl_ctx* c, int32_t* x, int32_t* y, int32_t* t) {
     if (!c) return -1;
     CK(cudaSetDevice(c->cfg.device));
     { int rl = records_in_order(c); if (rl) return rl; }
-    const size_t N = c->p.N, b = N * 4, row = up16(b);
+    const size_t N = c->p.N, b = N * 4, row = up64(b);
     // the export kernel writes x | y | t in environment order: into the stage when there is room, else into the spare copy
     const bool small = STAGE_DATA + 3 * row <= c->stage.bytes;
     launch_export_state(c->p, small ? (int*)(c->stage.dev + STAGE_DATA) : (int*)c->p.st2, (unsigned)(row / 4), handover(c), c->st);

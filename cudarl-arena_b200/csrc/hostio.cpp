@@ -71,19 +71,23 @@ inline void cpu_relax() {
 }
 
 // Into memory that the device reads next: past the caches.  The device's reads of lines that lie modified in a core's cache run at
-// about 5 GB/s on the B200 box (16 MB took 1.3 ms, 0.45 ms this way).
-void copy_past_caches(unsigned char* d, const unsigned char* s, size_t n) {
+// about 5 GB/s on the B200 box (16 MB took 1.3 ms, 0.45 ms this way).  line_end: the rest of the line that the last
+// byte lies in is nobody's and may be written.
+void copy_past_caches(unsigned char* d, const unsigned char* s, size_t n, bool line_end) {
 #if defined(__x86_64__)
-    const size_t head = std::min(n, (size_t)(-(intptr_t)d & 15));
-    std::memcpy(d, s, head);
-    size_t k = head;
+    size_t k = std::min(n, (size_t)(-(intptr_t)d & 15));
+    std::memcpy(d, s, k);
     for (; k + 64 <= n; k += 64) {
         const __m128i a = _mm_loadu_si128((const __m128i*)(s + k)), b = _mm_loadu_si128((const __m128i*)(s + k + 16)),
                       c = _mm_loadu_si128((const __m128i*)(s + k + 32)), e = _mm_loadu_si128((const __m128i*)(s + k + 48));
         _mm_stream_si128((__m128i*)(d + k), a); _mm_stream_si128((__m128i*)(d + k + 16), b);
         _mm_stream_si128((__m128i*)(d + k + 32), c); _mm_stream_si128((__m128i*)(d + k + 48), e);
     }
-    std::memcpy(d + k, s + k, n - k);
+    if (k < n && line_end && ((uintptr_t)(d + k) & 63u) == 0u) {      // a whole line again, so that it stays out of this core's cache
+        alignas(16) unsigned char rest[64] = {};
+        std::memcpy(rest, s + k, n - k);
+        for (int b = 0; b < 64; b += 16) _mm_stream_si128((__m128i*)(d + k + b), _mm_load_si128((const __m128i*)(rest + b)));
+    } else std::memcpy(d + k, s + k, n - k);
     _mm_sfence();
 #else
     std::memcpy(d, s, n);
@@ -91,13 +95,13 @@ void copy_past_caches(unsigned char* d, const unsigned char* s, size_t n) {
 }
 
 // A chunk on its way to the device: copied, or made in pieces that fit the first-level cache.
-void send(unsigned char* dst, const unsigned char* src, const Chunk& c) {
-    if (!c.fill) { copy_past_caches(dst, src, c.bytes); return; }
+void send(unsigned char* dst, const unsigned char* src, const Chunk& c, bool line_end) {
+    if (!c.fill) { copy_past_caches(dst, src, c.bytes, line_end); return; }
     alignas(64) unsigned char part[8192];
     for (size_t k = 0; k < c.bytes; k += sizeof(part)) {
         const size_t b = std::min(sizeof(part), c.bytes - k);
         c.fill(part, c.first + k, b, c.arg);
-        copy_past_caches(dst + k, part, b);
+        copy_past_caches(dst + k, part, b, line_end);
     }
 }
 
@@ -116,9 +120,9 @@ bool copy_one(Job& j) {
             std::memcpy(c.host, buf, c.bytes);
             if (j.copied[slot].fetch_add(1, std::memory_order_acq_rel) + 1 == j.pieces[c.piece].count) { j.copied[slot] = 0; j.turn[slot].store(c.piece + SLOTS, std::memory_order_release); }
             break;
-        case Way::In: send(buf, c.host, c); j.copied[slot].fetch_add(1, std::memory_order_release); break;
+        case Way::In: send(buf, c.host, c, false); j.copied[slot].fetch_add(1, std::memory_order_release); break;
         case Way::Host: std::memcpy(c.host, c.dev, c.bytes); break;
-        case Way::HostIn: send(c.host, c.dev, c); break;
+        case Way::HostIn: send(c.host, c.dev, c, true); break;
         case Way::Touch: for (size_t b = 0; b < c.bytes; b += 4096) *(volatile unsigned char*)(c.host + b) = 0; break;
     }
     j.done.fetch_add(1, std::memory_order_release);
@@ -357,7 +361,7 @@ void copy_host(const Segment* segs, int n, bool into_stage) {
         }
     }
     for (int s = 0; s < n; ++s)
-        if (into_stage) send((unsigned char*)segs[s].host, (const unsigned char*)segs[s].dev, Chunk{nullptr, nullptr, segs[s].bytes, segs[s].fill, segs[s].arg, 0});
+        if (into_stage) send((unsigned char*)segs[s].host, (const unsigned char*)segs[s].dev, Chunk{nullptr, nullptr, segs[s].bytes, segs[s].fill, segs[s].arg, 0}, true);
         else std::memcpy(segs[s].host, segs[s].dev, segs[s].bytes);
 }
 cudaError_t copy_out(const Segment* segs, int n, int device, cudaStream_t st) { return copy_all(segs, n, true, device, st); }

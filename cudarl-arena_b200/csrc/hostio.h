@@ -30,7 +30,8 @@ cudaError_t copy_out(const Segment* segs, int n, int device, cudaStream_t st);
 // Host -> device, ordered on `st`: the caller's arrays may be reused on return.
 cudaError_t copy_in(const Segment* segs, int n, int device, cudaStream_t st);
 
-// Between a stage and the caller: `dev` is the source, `host` the destination, both host memory; into_stage: the device reads it next.
+// Between a stage and the caller: `dev` is the source, `host` the destination, both host memory; into_stage: the device reads it next, and the destination owns its
+// cache lines to the end of the last one.
 void copy_host(const Segment* segs, int n, bool into_stage);
 
 }  // namespace cudarl
