@@ -1024,31 +1024,8 @@ int cudarl_update_batch(cudarl_ctx* c, int64_t n, const int32_t* sx, const int32
     if (n > (int64_t)UPDATE_SMALL) { int rc = ensure_entry_capacity(c, N); if (rc) return rc; }
     // Checked and packed to 12 bytes a transition on the way: into the mapped stage while they fit it (the kernel reads them across the
     // link), else through the ring to the device.
-    struct Source { const int32_t *sx, *sy, *a, *nx, *ny; const uint8_t* dn; uint32_t W, H; std::atomic<bool> bad{false}; } src;
-    src.sx = sx; src.sy = sy; src.a = a; src.nx = nx; src.ny = ny; src.dn = dn; src.W = (uint32_t)c->p.W; src.H = (uint32_t)c->p.H;
-    const Fill pack_at = [](void* dst, size_t first, size_t bytes, const void* arg) {
-        Source& s = *(Source*)arg;
-        uint32_t* const o = (uint32_t*)dst; const size_t i0 = first / 4, m = bytes / 4;
-        uint32_t bad = 0;
-        for (size_t k = 0; k < m; ++k) {
-            const uint32_t x = (uint32_t)s.sx[i0 + k], y = (uint32_t)s.sy[i0 + k], act = (uint32_t)s.a[i0 + k];
-            bad |= (uint32_t)(x >= s.W) | (uint32_t)(y >= s.H) | (uint32_t)(act >= (uint32_t)CUDARL_ACTIONS);
-            o[k] = ((y * s.W + x) << 2) | (act & 3u) | (s.dn[i0 + k] ? 0x80000000u : 0u);
-        }
-        if (bad) s.bad = true;
-    };
-    const Fill pack_next = [](void* dst, size_t first, size_t bytes, const void* arg) {
-        Source& s = *(Source*)arg;
-        uint32_t* const o = (uint32_t*)dst; const size_t i0 = first / 4, m = bytes / 4;
-        uint32_t bad = 0;
-        for (size_t k = 0; k < m; ++k) {
-            const uint32_t x = (uint32_t)s.nx[i0 + k], y = (uint32_t)s.ny[i0 + k];
-            bad |= (uint32_t)(x >= s.W) | (uint32_t)(y >= s.H);
-            o[k] = y * s.W + x;
-        }
-        if (bad) s.bad = true;
-    };
-    const size_t part = up64(N * 4);
+    TransitionSource src{sx, sy, a, nx, ny, dn, (uint32_t)c->p.W, (uint32_t)c->p.H};
+    const size_t part = (N * 4 + 255) / 256 * 256;
     const bool small = STAGE_DATA + 3 * part <= std::min(c->stage.bytes, UPDATE_MOST);
     if (!small && 3 * part > c->ub_cap) {
         CK(cudaStreamSynchronize(c->st));
@@ -1060,7 +1037,7 @@ int cudarl_update_batch(cudarl_ctx* c, int64_t n, const int32_t* sx, const int32
     unsigned char* const dev = small ? c->stage.dev + STAGE_DATA : (unsigned char*)c->dub;
     Segment in[3];
     for (int k = 0; k < 3; ++k) {
-        in[k].bytes = N * 4; in[k].arg = &src; in[k].fill = k == 0 ? pack_at : k == 1 ? pack_next : nullptr;
+        in[k].bytes = N * 4; in[k].arg = &src; in[k].fill = k == 0 ? pack_cell_action : k == 1 ? pack_next_cell : nullptr;
         if (small) { in[k].host = c->stage.host + STAGE_DATA + k * part; in[k].dev = k == 2 ? const_cast<float*>(r) : nullptr; }
         else { in[k].dev = dev + k * part; in[k].host = k == 2 ? const_cast<float*>(r) : nullptr; }
     }

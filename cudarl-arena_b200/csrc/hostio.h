@@ -8,7 +8,9 @@
 // given back when the last context goes.  Every function may be called from several threads at once.
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstddef>
+#include <cstdint>
 
 namespace cudarl {
 
@@ -19,6 +21,16 @@ struct Segment { void* host; void* dev; size_t bytes; Fill fill = nullptr; const
 
 // One pinned block mapped into the device, for the small results and inputs of a context.
 struct Stage { unsigned char* host = nullptr; unsigned char* dev = nullptr; size_t bytes = 0; };
+
+// Fills for the transitions of an update_batch: one word each, checked (`bad`: one was outside the grid or the action set).
+struct TransitionSource {
+    const int32_t *sx, *sy, *a, *nx, *ny; const uint8_t* dn; uint32_t W, H;
+    std::atomic<bool> bad{false};
+    TransitionSource(const int32_t* sx_, const int32_t* sy_, const int32_t* a_, const int32_t* nx_, const int32_t* ny_, const uint8_t* dn_, uint32_t W_, uint32_t H_)
+        : sx(sx_), sy(sy_), a(a_), nx(nx_), ny(ny_), dn(dn_), W(W_), H(H_) {}
+};
+void pack_cell_action(void* dst, size_t first, size_t bytes, const void* source);      // cell * 4 + action, bit 31 = the episode ended there
+void pack_next_cell(void* dst, size_t first, size_t bytes, const void* source);
 
 void hostio_retain();                         // one per context: keeps the process-wide parts alive
 void hostio_release();
