@@ -3,7 +3,7 @@
 // The table does not change during a rollout, so the greedy policy is a map from cells to cells, and the length of an episode is
 // the length of a path in that map.  Nobody has to walk it cell by cell:
 //
-//   k_rollout_tiles   one block per 64 x 64 cells folds the policy of its tile by pointer doubling in shared memory: for every
+//   k_rollout_tiles   one block per 64 x 64 (small grids: 32 x 32) cells folds the policy of its tile by pointer doubling in shared memory: for every
 //                     cell the number of steps until the path ends on a goal or leaves the tile (and where), or "never" when it
 //                     runs in a circle inside the tile.  One 4-byte word per cell.
 //   k_rollout_walk    one thread per environment draws its start cell and hops from tile to tile over those words; a path that
@@ -12,21 +12,27 @@
 // What bounds it: k_rollout_tiles streams the table once (16 bytes in, 4 out per cell) and looks up one word in shared memory per cell and round,
 // until a round finds no path to end; k_rollout_walk makes a few scattered 4-byte look-ups per environment, one after the other.  B200,
 // 4096 x 4096 cells, 4,194,304 environments, 1000 steps: 97 + 76 us (doubling to the last round 138 us; one environment per thread, start cells
-// looked up in the cell words 89 us); the walk over single cells this replaces took 13.55 ms.
+// looked up in the cell words 89 us); the walk over single cells this replaces took 13.55 ms.  256 x 256 cells, 65,536 environments: the
+// call takes 17.6 us; 24.4 us with 64 x 64 tiles (16 blocks, 8 cells per thread and 3 more rounds than the 64 blocks of 32 x 32) and the walk
+// started after the last fold had ended.
 //
 // Reference semantics: src/train.py:262-311 (evaluate), first-max argmax src/q_learning.cu:196-206.
 #include "kernels.cuh"
 #include "rules.cuh"
+#include <cstring>
 
 namespace cudarl {
 
 // Word of a cell.  While the tile is folded: kind LIVE, bits 0-11 the cell reached after 2^round steps.  Final: EXIT with the number
 // of steps in bits 0-12, the edge it leaves by (0 up, 1 right, 2 down, 3 left) in bits 22-23 and the place along it in bits 16-21;
 // GOAL with the number of steps; or TRAPPED.  Bit 29: an obstacle or a goal, where no episode starts.  A path without a circle has at most 4096 steps inside a tile.
-constexpr unsigned RT_SHIFT = 6u, RT = 1u << RT_SHIFT, RT_CELLS = RT * RT, RT_THREADS = 512u, RT_PER = RT_CELLS / RT_THREADS, RT_ROWS = RT_THREADS / RT;
+constexpr unsigned RT_ROWS = 8u;                 // rows of a tile that its threads take at a time
 constexpr unsigned KIND_LIVE = 0u, KIND_EXIT = 1u << 30, KIND_GOAL = 2u << 30, KIND_MASK = 3u << 30, TRAPPED = 3u << 30, NO_START = 1u << 29, STEPS_MASK = 0x1FFFu;
 
-__global__ void __launch_bounds__(RT_THREADS) k_rollout_tiles(const __grid_constant__ Params p, unsigned* __restrict__ hop) {
+template <unsigned RT_SHIFT>
+__global__ void __launch_bounds__(RT_ROWS << RT_SHIFT) k_rollout_tiles(const __grid_constant__ Params p, unsigned* __restrict__ hop) {
+    constexpr unsigned RT = 1u << RT_SHIFT, RT_CELLS = RT * RT, RT_THREADS = RT * RT_ROWS, RT_PER = RT_CELLS / RT_THREADS;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");       // the walk's blocks may take the slots that free up, and draw
     __shared__ unsigned s_w[RT_CELLS];
     const int x0 = (int)(blockIdx.x << RT_SHIFT), y0 = (int)(blockIdx.y << RT_SHIFT);
     unsigned cur[RT_PER];
@@ -80,6 +86,8 @@ __global__ void __launch_bounds__(RT_THREADS) k_rollout_tiles(const __grid_const
     }
 }
 
+// (no read-only loads: the words are written while the walk's first instructions already run)
+__device__ __forceinline__ unsigned ld_word(const unsigned* p) { unsigned v; asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
 // A start cell as sample_start draws it, and its word, which says whether an episode may start there.
 __device__ __forceinline__ unsigned walk_start(const Params& p, const unsigned* __restrict__ hop, unsigned gi, unsigned long long nonce, unsigned& word) {
     if (p.start_mode == 2) {
@@ -87,21 +95,22 @@ __device__ __forceinline__ unsigned walk_start(const Params& p, const unsigned* 
         for (unsigned k = 0; k < 16u; ++k) {
             const U4 w = philox4x32_10(gi, k, (unsigned)nonce, (unsigned)(nonce >> 32), p.k0, p.k1 ^ TAG_EVAL);
             unsigned c;
-            c = __umulhi(w.x, p.S); word = __ldg(hop + c); if (!(word & NO_START)) return c;
-            c = __umulhi(w.y, p.S); word = __ldg(hop + c); if (!(word & NO_START)) return c;
-            c = __umulhi(w.z, p.S); word = __ldg(hop + c); if (!(word & NO_START)) return c;
-            c = __umulhi(w.w, p.S); word = __ldg(hop + c); if (!(word & NO_START)) return c;
+            c = __umulhi(w.x, p.S); word = ld_word(hop + c); if (!(word & NO_START)) return c;
+            c = __umulhi(w.y, p.S); word = ld_word(hop + c); if (!(word & NO_START)) return c;
+            c = __umulhi(w.z, p.S); word = ld_word(hop + c); if (!(word & NO_START)) return c;
+            c = __umulhi(w.w, p.S); word = ld_word(hop + c); if (!(word & NO_START)) return c;
         }
     }
     const unsigned c = p.start_mode == 2 ? p.fallback_start : p.start_cell;
-    word = __ldg(hop + c);
+    word = ld_word(hop + c);
     return c;
 }
 
 // EPT environments per thread: their first look-ups are on the way at the same time.
-template <unsigned EPT>
+template <unsigned EPT, unsigned RT_SHIFT>
 __global__ void __launch_bounds__(BLOCK) k_rollout_walk(const __grid_constant__ Params p, const unsigned* __restrict__ hop, unsigned max_steps,
                                                         unsigned long long nonce, Handover h) {
+    constexpr unsigned RT = 1u << RT_SHIFT;
     __shared__ unsigned s_reached; __shared__ unsigned long long s_steps;
     if (threadIdx.x == 0) { s_reached = 0u; s_steps = 0ull; }
     __syncthreads();
@@ -111,8 +120,10 @@ __global__ void __launch_bounds__(BLOCK) k_rollout_walk(const __grid_constant__ 
     for (unsigned k = 0; k < EPT; ++k) {
         const unsigned i = i0 + k * BLOCK;
         cell[k] = p.start_mode == 2 ? __umulhi(philox4x32_10(p.env_offset + i, 0u, (unsigned)nonce, (unsigned)(nonce >> 32), p.k0, p.k1 ^ TAG_EVAL).x, p.S) : p.start_cell;
-        word[k] = __ldg(hop + cell[k]);
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");                    // the words are written
+#pragma unroll
+    for (unsigned k = 0; k < EPT; ++k) word[k] = ld_word(hop + cell[k]);
     unsigned nr = 0u; unsigned long long sum = 0ull;
 #pragma unroll
     for (unsigned k = 0; k < EPT; ++k) {
@@ -132,7 +143,7 @@ __global__ void __launch_bounds__(BLOCK) k_rollout_walk(const __grid_constant__ 
             y = (e & 1u) ? ty + at : (e == 2u ? ty + RT : ty - 1u);
             if (x == cx && y == cy) { steps = max_steps; break; }
             if (++hops == limit) { cx = x; cy = y; hops = 0u; limit <<= 1; }
-            w = __ldg(hop + (size_t)y * (size_t)p.W + (size_t)x);
+            w = ld_word(hop + (size_t)y * (size_t)p.W + (size_t)x);
         }
         sum += steps;
     }
@@ -148,12 +159,27 @@ __global__ void __launch_bounds__(BLOCK) k_rollout_walk(const __grid_constant__ 
     }
 }
 
-void launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
+template <unsigned RT_SHIFT>
+static void launch_tiled(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
+    constexpr unsigned RT = 1u << RT_SHIFT;
     const dim3 tiles(((unsigned)p.W + RT - 1u) / RT, ((unsigned)p.H + RT - 1u) / RT);
-    k_rollout_tiles<<<tiles, RT_THREADS, 0, st>>>(p, hop);
+    k_rollout_tiles<RT_SHIFT><<<tiles, RT * RT_ROWS, 0, st>>>(p, hop);
     // four environments per thread where the chip is full with that
-    if (p.N >= 4u * 8u * BLOCK * 148u) k_rollout_walk<4u><<<(p.N + 4u * BLOCK - 1u) / (4u * BLOCK), BLOCK, 0, st>>>(p, hop, max_steps, nonce, h);
-    else k_rollout_walk<1u><<<(p.N + BLOCK - 1u) / BLOCK, BLOCK, 0, st>>>(p, hop, max_steps, nonce, h);
+    const unsigned ept = p.N >= 4u * 8u * BLOCK * 148u ? 4u : 1u;
+    cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((p.N + ept * BLOCK - 1u) / (ept * BLOCK)); cfg.blockDim = dim3(BLOCK); cfg.stream = st;
+    cudaLaunchAttribute at;                              // the walk is set up, and draws its start cells, while the last tiles are folded
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, ept == 4u ? k_rollout_walk<4u, RT_SHIFT> : k_rollout_walk<1u, RT_SHIFT>, p, (const unsigned*)hop, max_steps, nonce, h);
+}
+void launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
+    // A 64 x 64 tile takes 512 threads, four of them fill an SM.  Where they do not fill every SM (the chain of rounds in one block is then what
+    // takes the time) tiles of a quarter of that size are folded by four times as many blocks; beyond, the larger tile saves hops.  Call with 64 /
+    // 32: 256^2 cells 24.0 / 20.4 us, 700^2 24.2 / 21.7, 1024^2 38.3 / 37.5, 1500^2 35.0 / 34.3, 2048^2 52.9 / 54.6.
+    const unsigned big = (((unsigned)p.W + 63u) / 64u) * (((unsigned)p.H + 63u) / 64u);
+    if (big < 4u * 148u) launch_tiled<5u>(p, hop, max_steps, nonce, h, st);
+    else launch_tiled<6u>(p, hop, max_steps, nonce, h, st);
 }
 
 }  // namespace cudarl

@@ -120,10 +120,12 @@ def test_update_batch_limits(pkg, orc, w, h, n):
 
 
 @pytest.mark.parametrize("w,h,n,warm", [(63, 65, 700, 300), (64, 64, 5000, 900), (200, 129, 9000, 1500), (1, 300, 40, 50), (700, 650, 1212415, 20), (700, 650, 1212416, 20),
-                                        (640, 641, 1300001, 20)])
+                                        (640, 641, 1300001, 20), (31, 33, 500, 300), (1, 37824, 400, 60), (1, 37825, 400, 60), (1537, 1500, 9000, 300),
+                                        (1537, 1500, 1212416, 20)])
 @pytest.mark.parametrize("start", [0, 2])
 def test_rollout_limits(pkg, orc, w, h, n, warm, start):
-    """The folded rollout: grids around the edge of its 64 x 64 tiles, one and four environments per thread, caps below, at and beyond the
+    """The folded rollout: grids around the edges of its 32 x 32 and 64 x 64 tiles and
+    between the two, one and four environments per thread, caps below, at and beyond the
     lengths of the paths, a common start cell; the table is taken over from the GPU, so that only the rollout is compared."""
     gpu, cpu = pair(pkg, orc, world(pkg, w, h, n, start_mode=start, max_steps=200, eps0=0.2), threads=THREADS)
     gpu.train_steps(warm)
