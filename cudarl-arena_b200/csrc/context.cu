@@ -89,7 +89,7 @@ struct cudarl_ctx {
     std::map<uint32_t, float> traps;      // cell -> penalty; mirrored on the device as a table sorted by cell
     void* dtraps = nullptr; size_t traps_cap = 0;
     void* dtq = nullptr;                    // ticket counters of the step kernel's tile queues
-    void* dhop = nullptr;                   // folded greedy policy of the evaluation rollout (one word per cell), allocated on first use
+    unsigned* hop = nullptr;                // folded greedy policy of the evaluation rollout: one word per cell, behind the table
     Stage stage; bool retained = false;     // pinned, mapped block: the box for small results at its head, small arrays behind it
     HostBox* box = nullptr; unsigned ticket = 0;                                    // the box, and the last call's ticket
     // device buffers
@@ -480,7 +480,8 @@ int alloc_tiles(cudarl_ctx* c) {
 
 int alloc_table(cudarl_ctx* c) {
     const size_t S = c->p.S;
-    CK(cudaMalloc(&c->dQ, (S + 64) * sizeof(float4)));
+    CK(cudaMalloc(&c->dQ, (S + 64) * sizeof(float4) + S * sizeof(unsigned)));
+    c->hop = (unsigned*)((float4*)c->dQ + S + 64);      // (its own allocation, made by the first rollout, cost that one up to a millisecond)
     CK(cudaMemsetAsync(c->dQ, 0, (S + 64) * sizeof(float4), c->st));
     c->p.Q = (float4*)c->dQ;
     return 0;
@@ -718,7 +719,7 @@ void free_all(cudarl_ctx* c) {
                     c->dtra, c->dtrr, c->dtrd, c->dsort, c->dgather, c->dact,
                     c->dub,
                     c->dQ, c->drec[0], c->drec[1], c->darr[0], c->darr[1], c->dovf[0], c->dovf[1], c->dbmax[0], c->dbmax[1],
-                    c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dhop, c->dtq, c->dpeer_ptrs, c->dbarrier_word, c->dgbar, c->dgcnt, c->dgmv, c->dgstate, c->dgbins, c->dwork[0], c->dwork[1]};
+                    c->dtmeta, c->dtscratch, c->dtcls, c->dtraps, c->dtq, c->dpeer_ptrs, c->dbarrier_word, c->dgbar, c->dgcnt, c->dgmv, c->dgstate, c->dgbins, c->dwork[0], c->dwork[1]};
     for (void* b : bufs) if (b) cudaFree(b);
     if (c->h_eps) cudaFreeHost(c->h_eps);
     stage_give(&c->stage);
@@ -1001,8 +1002,7 @@ int cudarl_eval_rollout(cudarl_ctx* c, int32_t max_steps, cudarl_eval_stats* out
     out->envs = c->p.N; out->reached = 0; out->total_steps = 0;
     if (c->p.N) {                                        // the records stay where they are: a rollout reads the table and the grid only
         refresh_moves(c);                                // it reads the move bytes
-        if (!c->dhop) CK(cudaMalloc(&c->dhop, (size_t)c->p.S * sizeof(unsigned)));           // kept until the context goes
-        launch_rollout(c->p, (unsigned*)c->dhop, (unsigned)max_steps, (unsigned long long)c->eval_calls, handover(c), c->st);
+        launch_rollout(c->p, c->hop, (unsigned)max_steps, (unsigned long long)c->eval_calls, handover(c), c->st);
         CK(cudaGetLastError());
         { int rw = wait_box(c, 4); if (rw) return rw; }
         out->reached = (int64_t)box64(c, 1); out->total_steps = (int64_t)box64(c, 3);
