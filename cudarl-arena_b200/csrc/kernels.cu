@@ -374,8 +374,17 @@ __global__ void k_step_actions(const __grid_constant__ World p, const int* __res
     const unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) * (VEC ? 4u : 1u);
     if (VEC && i + 4u <= p.N) {
         const int4 a = *reinterpret_cast<const int4*>(actions + i);
-        float4 r; uchar4 d;
-        step_record(p, i, a.x, r.x, d.x); step_record(p, i + 1u, a.y, r.y, d.y); step_record(p, i + 2u, a.z, r.z, d.z); step_record(p, i + 3u, a.w, r.w, d.w);
+        float4 r; uchar4 d = *reinterpret_cast<const uchar4*>(p.done + i);
+        const int acts[4] = {a.x, a.y, a.z, a.w};
+        int4 rec[4]; unsigned to[4], own[4], there[4]; float rr[4]; unsigned char dd[4] = {d.x, d.y, d.z, d.w};
+        // all loads of one kind before the first store: the four environments' look-ups are on their way together
+#pragma unroll
+        for (unsigned k = 0; k < 4u; ++k) rec[k] = p.st[i + k];
+#pragma unroll
+        for (unsigned k = 0; k < 4u; ++k) { to[k] = target_cell(p, rec[k].x, rec[k].y, acts[k]); own[k] = cw_load(p.cw, (unsigned)rec[k].y * (unsigned)p.W + (unsigned)rec[k].x); there[k] = cw_load(p.cw, to[k]); }
+#pragma unroll
+        for (unsigned k = 0; k < 4u; ++k) p.st[i + k] = stepped(p, rec[k], acts[k], to[k], own[k], there[k], rr[k], dd[k]);
+        r = make_float4(rr[0], rr[1], rr[2], rr[3]); d = make_uchar4(dd[0], dd[1], dd[2], dd[3]);
         *reinterpret_cast<float4*>(p.reward + i) = r; *reinterpret_cast<uchar4*>(p.done + i) = d;
         if (rewards) *reinterpret_cast<float4*>(rewards + i) = r;
         if (dones) *reinterpret_cast<uchar4*>(dones + i) = d;
@@ -586,7 +595,8 @@ void launch_reset_all(const Params& p, cudaStream_t st) {
 void launch_step_actions(const Params& p, const int* a, float* r, unsigned char* d, Handover h, cudaStream_t st) {
     if (!p.N) return;
     const bool vec = (((uintptr_t)a | (uintptr_t)r) & 15u) == 0u && ((uintptr_t)d & 3u) == 0u;
-    if (vec) k_step_actions<true><<<nblk((p.N + 3u) / 4u), BLOCK, 0, st>>>(p, a, r, d, h);
+    // results that go across the link; within the device one environment per thread is the better spread: 4,194,304 environments 57 us, four per thread 62
+    if (vec && h.box) k_step_actions<true><<<nblk((p.N + 3u) / 4u), BLOCK, 0, st>>>(p, a, r, d, h);
     else k_step_actions<false><<<nblk(p.N), BLOCK, 0, st>>>(p, a, r, d, h);
 }
 void launch_step_one(const Params& p, int action, bool reset, int x, int y, Handover h, cudaStream_t st) { k_step_one<<<1, 1, 0, st>>>(p, action, reset, x, y, h); }
