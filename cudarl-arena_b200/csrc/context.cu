@@ -349,12 +349,13 @@ Handover handover(cudarl_ctx* c) { return Handover{(HostBox*)c->stage.dev, ++c->
 constexpr size_t STAGE_DATA = 256;
 // How large a stage: room for the states of all environments and for the table, each up to 4 MB: so far a kernel's own accesses across the
 // link are faster than copies through the ring (B200, states of 131,072 environments 145 -> 65 us, a table of 1 MB 100 -> 59 us, of 4 MB
-// 193 -> 134 us); 64 KB for a single small environment, of which a program may keep many.
-constexpr size_t UPDATE_MOST = (size_t)1 << 20;
+// 193 -> 134 us); 64 KB for a single small environment, of which a program may keep many; all 4 MB without environments, where transitions
+// are what comes in (100,000 on 1024 x 1024 cells 109 -> 86 us, 300,000 216 -> 156 us; ring / stage).
 size_t stage_bytes(const Params& p) {
     if (p.N == 1u && p.S <= 2048u) return (size_t)64 << 10;
     const size_t most = (size_t)4 << 20, states = STAGE_DATA + 12 * ((size_t)p.N + 16), table = STAGE_DATA + 16 * (size_t)p.S;
     size_t b = (size_t)1 << 20;
+    if (p.N == 0u) return most;
     for (const size_t want : {states, table}) while (want <= most && b < want) b += (size_t)1 << 20;
     return b;
 }
@@ -1026,7 +1027,7 @@ int cudarl_update_batch(cudarl_ctx* c, int64_t n, const int32_t* sx, const int32
     // link), else through the ring to the device.
     TransitionSource src{sx, sy, a, nx, ny, dn, (uint32_t)c->p.W, (uint32_t)c->p.H};
     const size_t part = (N * 4 + 255) / 256 * 256;
-    const bool small = STAGE_DATA + 3 * part <= std::min(c->stage.bytes, UPDATE_MOST);
+    const bool small = STAGE_DATA + 3 * part <= c->stage.bytes;
     if (!small && 3 * part > c->ub_cap) {
         CK(cudaStreamSynchronize(c->st));
         cudaFree(c->dub); c->dub = nullptr; c->ub_cap = 0;
