@@ -95,12 +95,12 @@ def test_tile_engine_forced(pkg, orc, edge, w, h, n, kw):
 
 
 @pytest.mark.parametrize("w,h", [(7, 5), (1024, 1023), (1025, 1024)])
-@pytest.mark.parametrize("n", [1, 33, 1024, 1025, 87000, 90001, 300000])
+@pytest.mark.parametrize("n", [1, 33, 1024, 1025, 87000, 90001, 300000, 349504, 349505])
 def test_update_batch_limits(pkg, orc, w, h, n):
-    """update_batch on both sides of its limits -- one block, the mapped stage, the ring; 32-bit and 64-bit sort keys -- and a transition
+    """update_batch on both sides of its limits -- one block, the mapped stage (of a context without environments, too), the ring; 32-bit and 64-bit sort keys -- and a transition
     out of range anywhere in the batch, which must leave the table as it was."""
     rng = np.random.RandomState(n + w)
-    gpu, cpu = pair(pkg, orc, pkg.make_config(w, h, 1, lr=0.3, gamma=0.95, q_init_kind=pkg.QINIT_UNIFORM, q_init_scale=1.0))
+    gpu, cpu = pair(pkg, orc, pkg.make_config(w, h, 1 if n <= 300000 else 0, lr=0.3, gamma=0.95, q_init_kind=pkg.QINIT_UNIFORM, q_init_scale=1.0))
     spot = rng.rand(n) < 0.3                             # a third of the batch on few cells
     b = dict(sx=np.where(spot, rng.randint(0, 3, n), rng.randint(0, w, n)), sy=np.where(spot, h - 1, rng.randint(0, h, n)), a=rng.randint(0, 4, n),
              r=rng.choice([-0.01, 1.0, 0.25], n).astype(np.float32), nx=rng.randint(0, w, n), ny=rng.randint(0, h, n), dn=(rng.rand(n) < 0.2).astype(np.uint8))
