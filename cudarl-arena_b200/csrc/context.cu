@@ -1003,8 +1003,8 @@ int cudarl_eval_rollout(cudarl_ctx* c, int32_t max_steps, cudarl_eval_stats* out
     out->envs = c->p.N; out->reached = 0; out->total_steps = 0;
     if (c->p.N) {                                        // the records stay where they are: a rollout reads the table and the grid only
         refresh_moves(c);                                // it reads the move bytes
-        launch_rollout(c->p, c->hop, (unsigned)max_steps, (unsigned long long)c->eval_calls, handover(c), c->st);
         CK(cudaGetLastError());
+        CK(launch_rollout(c->p, c->hop, (unsigned)max_steps, (unsigned long long)c->eval_calls, handover(c), c->st));
         { int rw = wait_box(c, 4); if (rw) return rw; }
         out->reached = (int64_t)box64(c, 1); out->total_steps = (int64_t)box64(c, 3);
     }

@@ -170,7 +170,7 @@ constexpr unsigned UPDATE_SMALL = 1024u;
 void launch_update_batch(const Params& p, unsigned n, const Transitions& tr, Handover h, cudaStream_t st);
 void launch_q_init(const Params& p, int kind, float scale, cudaStream_t st);
 // greedy rollout (rollout.cu); hop: one word per cell, scratch; words 1-4 = environments that reached a goal, steps taken, low halves first
-void launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st);
+cudaError_t launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st);
 // tile engine (tile_engine.cu)
 size_t tile_step_smem(const Params& p);
 int  tile_engine_configure(Params& p, int device);                  // opt in to the dynamic shared memory the step needs; sets tp.grid

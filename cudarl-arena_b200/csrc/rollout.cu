@@ -30,11 +30,12 @@ constexpr unsigned RT_ROWS = 8u;                 // rows of a tile that its thre
 constexpr unsigned KIND_LIVE = 0u, KIND_EXIT = 1u << 30, KIND_GOAL = 2u << 30, KIND_MASK = 3u << 30, TRAPPED = 3u << 30, NO_START = 1u << 29, STEPS_MASK = 0x1FFFu;
 
 template <unsigned RT_SHIFT>
-__global__ void __launch_bounds__(RT_ROWS << RT_SHIFT) k_rollout_tiles(const __grid_constant__ Params p, unsigned* __restrict__ hop) {
+__global__ void __launch_bounds__(RT_ROWS << RT_SHIFT) k_rollout_tiles(const __grid_constant__ Params p, unsigned* __restrict__ hop, unsigned tiles_x) {
     constexpr unsigned RT = 1u << RT_SHIFT, RT_CELLS = RT * RT, RT_THREADS = RT * RT_ROWS, RT_PER = RT_CELLS / RT_THREADS;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");       // the walk's blocks may take the slots that free up, and draw
     __shared__ unsigned s_w[RT_CELLS];
-    const int x0 = (int)(blockIdx.x << RT_SHIFT), y0 = (int)(blockIdx.y << RT_SHIFT);
+    const unsigned ty = blockIdx.x / tiles_x, tx = blockIdx.x - ty * tiles_x;            // tiles in one dimension: a second one of the launch ends at 65,535, a grid's height at 2^28
+    const int x0 = (int)(tx << RT_SHIFT), y0 = (int)(ty << RT_SHIFT);
     unsigned cur[RT_PER];
     const unsigned lx = threadIdx.x & (RT - 1u), ly0 = threadIdx.x >> RT_SHIFT;          // a thread's cells lie below one another, 8 rows apart
     const int x = x0 + (int)lx;
@@ -160,10 +161,12 @@ __global__ void __launch_bounds__(BLOCK) k_rollout_walk(const __grid_constant__ 
 }
 
 template <unsigned RT_SHIFT>
-static void launch_tiled(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
+static cudaError_t launch_tiled(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
     constexpr unsigned RT = 1u << RT_SHIFT;
-    const dim3 tiles(((unsigned)p.W + RT - 1u) / RT, ((unsigned)p.H + RT - 1u) / RT);
-    k_rollout_tiles<RT_SHIFT><<<tiles, RT * RT_ROWS, 0, st>>>(p, hop);
+    const unsigned tiles_x = ((unsigned)p.W + RT - 1u) / RT, tiles_y = ((unsigned)p.H + RT - 1u) / RT;
+    k_rollout_tiles<RT_SHIFT><<<tiles_x * tiles_y, RT * RT_ROWS, 0, st>>>(p, hop, tiles_x);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;                      // no walk over words that nobody has written
     // four environments per thread where the chip is full with that
     const unsigned ept = p.N >= 4u * 8u * BLOCK * 148u ? 4u : 1u;
     cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof(cfg));
@@ -171,15 +174,14 @@ static void launch_tiled(const Params& p, unsigned* hop, unsigned max_steps, uns
     cudaLaunchAttribute at;                              // the walk is set up, and draws its start cells, while the last tiles are folded
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at; cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, ept == 4u ? k_rollout_walk<4u, RT_SHIFT> : k_rollout_walk<1u, RT_SHIFT>, p, (const unsigned*)hop, max_steps, nonce, h);
+    return cudaLaunchKernelEx(&cfg, ept == 4u ? k_rollout_walk<4u, RT_SHIFT> : k_rollout_walk<1u, RT_SHIFT>, p, (const unsigned*)hop, max_steps, nonce, h);
 }
-void launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
+cudaError_t launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
     // A 64 x 64 tile takes 512 threads, four of them fill an SM.  Where they do not fill every SM (the chain of rounds in one block is then what
     // takes the time) tiles of a quarter of that size are folded by four times as many blocks; beyond, the larger tile saves hops.  Call with 64 /
     // 32: 256^2 cells 24.0 / 20.4 us, 700^2 24.2 / 21.7, 1024^2 38.3 / 37.5, 1500^2 35.0 / 34.3, 2048^2 52.9 / 54.6.
     const unsigned big = (((unsigned)p.W + 63u) / 64u) * (((unsigned)p.H + 63u) / 64u);
-    if (big < 4u * 148u) launch_tiled<5u>(p, hop, max_steps, nonce, h, st);
-    else launch_tiled<6u>(p, hop, max_steps, nonce, h, st);
+    return big < 4u * 148u ? launch_tiled<5u>(p, hop, max_steps, nonce, h, st) : launch_tiled<6u>(p, hop, max_steps, nonce, h, st);
 }
 
 }  // namespace cudarl

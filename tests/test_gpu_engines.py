@@ -153,3 +153,19 @@ def test_update_batch_crowded_cells(pkg, orc, w, h, n):
     if w * h <= 4096:                                    # no two cells share a chain
         assert gpu.get_stats().long_chains == 2 * int((cells > 32).sum())
     assert gpu.get_stats().device_error == 0
+
+
+@pytest.mark.parametrize("w,h", [(1, 65535 * 64), (1, 65535 * 64 + 1), (1, 65536 * 64 + 65), (2, 65536 * 64 + 1)])
+@pytest.mark.parametrize("down", [True, False])
+def test_rollout_on_tall_grids(pkg, orc, w, h, down):
+    """Grids of more than 65,535 rows of tiles, and the tallest below: everybody walks straight to the goal at one end, through every row of tiles
+    on the way, for the whole height and for caps that end some of the walks."""
+    cfg = world(pkg, w, h, 20, obstacle_p=0.0, obstacle_kind=pkg.OBST_NONE, goal_mode=pkg.GOAL_LIST, goals=[(x, h - 1 if down else 0) for x in range(w)], num_goals=w)
+    gpu, cpu = pair(pkg, orc, cfg)
+    q = np.zeros((h, w, 4), np.float32)
+    q[..., 2 if down else 0] = 1.0
+    gpu.set_q(q); cpu.set_q(q)
+    for cap in (h, h // 2, 70):
+        a, b = gpu.eval_rollout(cap), cpu.eval_rollout(cap)
+        assert (a.envs, a.reached, a.total_steps) == (b.envs, b.reached, b.total_steps), cap
+        assert cap < h or a.reached == 20
