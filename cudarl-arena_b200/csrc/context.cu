@@ -878,7 +878,7 @@ int cudarl_step_actions(cudarl_ctx* c, const int32_t* actions, float* rewards, u
         if (rewards) out[n++] = Segment{rewards, c->stage.host + off_r, N * 4};
         if (dones) out[n++] = Segment{dones, c->stage.host + off_d, N};
         copy_host(out, n, false);
-        return 0;
+        return check_posted_error(c);
     }
     if (!c->dact) CK(cudaMalloc(&c->dact, N * sizeof(int)));
     const Segment in{const_cast<int32_t*>(actions), c->dact, N * 4};
@@ -895,7 +895,8 @@ int cudarl_get_reward_done(cudarl_ctx* c, float* rewards, uint8_t* dones) {
     Segment out[2]; int n = 0;
     if (rewards) out[n++] = Segment{rewards, c->dreward, (size_t)c->p.N * 4};
     if (dones) out[n++] = Segment{dones, c->ddone, (size_t)c->p.N};
-    return hand_out(c, out, n);
+    { int ro = hand_out(c, out, n); if (ro) return ro; }
+    return check_posted_error(c);
 }
 
 }  // extern "C"
@@ -994,7 +995,8 @@ int cudarl_get_trace(cudarl_ctx* c, int32_t* a, float* r, uint8_t* d) {
     if (a) out[n++] = Segment{a, c->dtra, N * 4};
     if (r) out[n++] = Segment{r, c->dtrr, N * 4};
     if (d) out[n++] = Segment{d, c->dtrd, N};
-    return hand_out(c, out, n);
+    { int ro = hand_out(c, out, n); if (ro) return ro; }
+    return check_posted_error(c);
 }
 
 int cudarl_eval_rollout(cudarl_ctx* c, int32_t max_steps, cudarl_eval_stats* out) {
@@ -1006,6 +1008,7 @@ int cudarl_eval_rollout(cudarl_ctx* c, int32_t max_steps, cudarl_eval_stats* out
         CK(cudaGetLastError());
         CK(launch_rollout(c->p, c->hop, (unsigned)max_steps, (unsigned long long)c->eval_calls, handover(c), c->st));
         { int rw = wait_box(c, 4); if (rw) return rw; }
+        { int re = check_posted_error(c); if (re) return re; }
         out->reached = (int64_t)box64(c, 1); out->total_steps = (int64_t)box64(c, 3);
     }
     c->eval_calls += 1;
@@ -1050,7 +1053,8 @@ int cudarl_update_batch(cudarl_ctx* c, int64_t n, const int32_t* sx, const int32
     launch_update_batch(c->p, (unsigned)n, tr, handover(c), c->st);
     CK(cudaGetLastError());
     if (c->tile_mode) { launch_tile_border(c->p, c->st); CK(cudaGetLastError()); }       // the records stay in their tiles; the table under them has changed
-    return wait_box(c);
+    { int rw = wait_box(c); if (rw) return rw; }
+    return check_posted_error(c);                        // a fold that gave up has left the table half updated
 }
 
 int cudarl_get_state(cudarl_ctx* c, int32_t* x, int32_t* y, int32_t* t) {

@@ -13,7 +13,8 @@
  * Return value of every `int` function: 0 = ok, <0 = bad argument / bad state,
  * >0 = CUDA (1000+cudaError) or NCCL (2000+ncclResult) failure, or CUDARL_ERR_DEVICE + bits when a
  * kernel of this library recorded an internal failure (see CUDARL_DEVERR_*; reported by the next call
- * that waits for the device: cudarl_synchronize, cudarl_get_stats, cudarl_get_q, cudarl_get_state).
+ * that waits for the device: cudarl_synchronize, every cudarl_get_* of device data, cudarl_step_actions,
+ * cudarl_eval_rollout, cudarl_update_batch).
  * A text for the last failure is kept per context (cudarl_last_error) and per thread for
  * failures of cudarl_create (cudarl_last_global_error).
  *
@@ -56,7 +57,7 @@ enum { CUDARL_QINIT_ZERO = 0,           /* src/q_learning.cu:13 */
 enum { CUDARL_DEVERR_SCRATCH_OVERFLOW = 1, /* a work area was too small for the step */
        CUDARL_DEVERR_BAD_STATE = 2,        /* a record outside its tile or outside the grid */
        CUDARL_DEVERR_CHAIN_CYCLE = 8,      /* update_batch: a collision chain longer than the batch */
-       CUDARL_DEVERR_COPY_TIMEOUT = 32 };  /* train step: a tile copy did not land within its wait bound */
+       CUDARL_DEVERR_COPY_TIMEOUT = 32 };  /* a wait inside a kernel (for a tile copy, for the other blocks of a launch) ran out */
 
 typedef struct cudarl_config {
     uint32_t struct_size;   /* = sizeof(cudarl_config); checked */

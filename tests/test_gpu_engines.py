@@ -169,3 +169,27 @@ def test_rollout_on_tall_grids(pkg, orc, w, h, down):
         a, b = gpu.eval_rollout(cap), cpu.eval_rollout(cap)
         assert (a.envs, a.reached, a.total_steps) == (b.envs, b.reached, b.total_steps), cap
         assert cap < h or a.reached == 20
+
+
+@pytest.mark.parametrize("n", [20, 2000, 300000])
+def test_calls_that_wait_report_a_failure_of_the_device(pkg, n):
+    """A wait inside a kernel has run out (the tests' poll bound): every call that hands results back says so, instead of returning what a
+    kernel left half done as if it were whole -- update_batch in one block and with its sort, results through the stage and through the ring."""
+    g = pkg.VecGridWorld(world(pkg, 90, 80, n))
+    g.set_trace(True)
+    g.train_steps(1); g.synchronize()
+    g.debug_set_copy_wait_polls(1)
+    g.train_steps(1)
+    g.debug_set_copy_wait_polls(0)
+    rng = np.random.RandomState(n)
+
+    def batch(m):
+        return dict(sx=np.full(m, 3), sy=np.full(m, 4), a=rng.randint(0, 4, m), r=np.ones(m, np.float32), nx=np.full(m, 3), ny=np.full(m, 5), dn=np.zeros(m, np.uint8))
+    calls = dict(update_small=lambda: g.update_batch(**batch(100)), update_sorted=lambda: g.update_batch(**batch(5000)), rollout=lambda: g.eval_rollout(50),
+                 step=lambda: g.step_actions(np.zeros(n, np.int32)), reward_done=g.get_reward_done, trace=g.get_trace, state=g.get_state, q=g.get_q,
+                 synchronize=g.synchronize, stats=g.get_stats)
+    for name, call in calls.items():
+        with pytest.raises(pkg.CudarlError) as ei:
+            call()
+            pytest.fail(name)
+        assert ei.value.code == 3000 + 32, name
