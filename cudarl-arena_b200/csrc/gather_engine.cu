@@ -157,7 +157,7 @@ void gather_plan(Params& p, int sms) {
     gp.grid = (n + gp.chunk - 1u) / gp.chunk;
     gp.bins_x = ((unsigned)p.W + 7u) / 8u; gp.nbins = gp.bins_x * (((unsigned)p.H + 7u) / 8u) * 8u;
 }
-unsigned gather_barriers(const StepLaunch& l) { return 2u * l.steps + (l.in != l.out ? 4u : 0u); }
+unsigned gather_barriers(const StepLaunch& l) { return 2u * l.steps + (l.in != l.out ? 4u : 0u) + (l.eps_mode == 2 ? 1u : 0u); }
 void launch_gather_export(const Params& p, const int4* work, cudaStream_t st) {
     if (p.N) k_gather_export<<<(p.N + BLOCK - 1u) / BLOCK, BLOCK, 0, st>>>(p, work);
 }

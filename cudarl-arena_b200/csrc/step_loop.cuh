@@ -142,6 +142,10 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
     }
     EpsilonIndex eps_index(p, l, PLAIN);
     float eps = __ldg(p.eps_tab + eps_index.at);
+    if (!PLAIN && l.eps_mode == 2 && !Space::ALONE) {       // every block has read the finished episodes before any adds those of the first step
+        space.arrive();
+        if (!space.wait()) return;
+    }
 
     for (unsigned step = 0; step < l.steps; ++step, ++g) {
         const unsigned par = (unsigned)g & 1u;

@@ -193,3 +193,15 @@ def test_calls_that_wait_report_a_failure_of_the_device(pkg, n):
             call()
             pytest.fail(name)
         assert ei.value.code == 3000 + 32, name
+
+
+@pytest.mark.parametrize("n", [5000, 16384, 60000, SMS * 512, 90000, 4 * SMS * 1024 + 77])
+def test_episode_epsilon_when_everybody_ends_in_the_first_step_of_a_launch(pkg, orc, n):
+    """The epsilon of a step follows the episodes finished before it.  All environments reach the step cap in the first step of a launch of many:
+    no block may see the episodes of that step when it looks up the epsilon it begins with.  One cluster, the whole GPU, dealt by cell or not."""
+    cfg = world(pkg, 120, 97, n, num_goals=1, max_steps=8, eps_kind=pkg.EPS_MULT_PER_EPISODE, eps0=1.0, eps_decay=0.6)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    for k in (7, 8, 8, 8, 8, 8, 64) if n < 100000 else (7, 8, 8):
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert_same(gpu, cpu, "n=%d after +%d" % (n, k))
+        assert gpu.get_stats().epsilon == cpu.get_stats().epsilon
