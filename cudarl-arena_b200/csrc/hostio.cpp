@@ -5,6 +5,7 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <sys/mman.h>
 #include <thread>
@@ -159,7 +160,9 @@ void ready_workers() {
     if (!p.workers.empty()) return;
     const int n = std::min(MAX_WORKERS, (int)std::thread::hardware_concurrency() * 3 / 4 - 1);      // with the caller three quarters of the cores
     p.stop = false;
-    for (int k = 0; k < n; ++k) p.workers.emplace_back(worker_main);
+    try {
+        for (int k = 0; k < n; ++k) p.workers.emplace_back(worker_main);
+    } catch (const std::exception&) {}           // a limit on threads: those that exist do, or the caller's alone
 }
 // Cut into chunks of at most `most` bytes, or of less (but not below `least`) so that a short transfer still has two for every core; for the
 // copy engine (`pieces`) into eight pieces or more, of up to a slot, each of whole chunks.
