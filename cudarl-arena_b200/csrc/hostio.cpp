@@ -368,12 +368,15 @@ cudaError_t stage_take(Stage* s, size_t bytes) {
         for (size_t k = 0; k < p.spare.size(); ++k)
             if (p.spare[k].bytes == bytes) { *s = p.spare[k]; p.spare.erase(p.spare.begin() + (long)k); std::memset(s->host, 0, 256); return cudaSuccess; }
     }
-    s->bytes = bytes;
-    cudaError_t e = cudaHostAlloc((void**)&s->host, bytes, cudaHostAllocPortable | cudaHostAllocMapped);
-    if (e != cudaSuccess) { s->host = nullptr; return e; }
-    std::memset(s->host, 0, 256);
-    e = cudaHostGetDevicePointer((void**)&s->dev, s->host, 0);
-    return e;
+    Stage t;
+    t.bytes = bytes;
+    cudaError_t e = cudaHostAlloc((void**)&t.host, bytes, cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) return e;
+    e = cudaHostGetDevicePointer((void**)&t.dev, t.host, 0);
+    if (e != cudaSuccess) { cudaFreeHost(t.host); return e; }
+    std::memset(t.host, 0, 256);
+    *s = t;
+    return cudaSuccess;
 }
 void stage_give(Stage* s) {
     if (!s->host) return;

@@ -13,6 +13,7 @@ namespace fake {
 std::mutex mu;
 std::map<unsigned char*, size_t> pinned;                     // registered and allocated ranges
 std::atomic<int> threads_left{1 << 30};
+std::atomic<bool> no_device_pointer{false};
 std::atomic<long> direct{0}, through_ring{0};                // copies from or to memory that is not pinned, and that is
 std::atomic<cudaError_t> last{cudaSuccess};
 cudaError_t set(cudaError_t e) { if (e != cudaSuccess && e != cudaErrorNotReady) last = e; return e; }
@@ -30,7 +31,7 @@ cudaError_t cudaHostRegister(void* p, size_t n, unsigned) { std::lock_guard<std:
 cudaError_t cudaHostUnregister(void* p) { std::lock_guard<std::mutex> lk(fake::mu); return fake::pinned.erase((unsigned char*)p) ? cudaSuccess : cudaErrorHostMemoryNotRegistered; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::aligned_alloc(4096, (n + 4095) / 4096 * 4096); return cudaHostRegister(*p, n, 0); }
 cudaError_t cudaFreeHost(void* p) { cudaHostUnregister(p); std::free(p); return cudaSuccess; }
-cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) { *d = h; return cudaSuccess; }
+cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) { if (fake::no_device_pointer) return fake::set(cudaErrorInvalidValue); *d = h; return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)1; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
@@ -94,9 +95,21 @@ static void callers() {
 // No thread can be started, or only some.
 static void no_threads() { fake::threads_left = 0; round_trips(); }
 static void few_threads() { fake::threads_left = 3; round_trips(); fake::threads_left = 0; round_trips(); }
+// A block whose device address cannot be had is not handed out, now or later.
+static void stage() {
+    Stage a, b;
+    fake::no_device_pointer = true;
+    EXPECT(stage_take(&a, 1 << 20) == cudaErrorInvalidValue);
+    stage_give(&a);
+    fake::no_device_pointer = false;
+    EXPECT(stage_take(&b, 1 << 20) == cudaSuccess && b.host && b.dev == b.host && b.bytes == (1u << 20));
+    stage_give(&b);
+    EXPECT(stage_take(&a, 1 << 20) == cudaSuccess && a.host && a.dev == a.host);
+    stage_give(&a);
+}
 
 int main(int argc, char** argv) {
-    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}};
+    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}, {"stage", stage}};
     const auto it = argc > 1 ? all.find(argv[1]) : all.end();
     if (it == all.end()) { for (auto& s : all) std::puts(s.first.c_str()); return 2; }
     hostio_retain();
