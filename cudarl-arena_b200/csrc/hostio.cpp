@@ -6,7 +6,9 @@
 #include <cstdint>
 #include <cstring>
 #include <exception>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <sys/mman.h>
 #include <thread>
 #include <vector>
@@ -282,21 +284,27 @@ cudaError_t copy_all(const Segment* segs, int n, bool out, int device, cudaStrea
             }
             cudaError_t e = cudaStreamSynchronize(st);                 // do not spin through work enqueued earlier
             if (e != cudaSuccess) return e;
-            e = ready_ring(device);
-            if (e != cudaSuccess) return e;
-            Job j;
-            j.way = out ? Way::Out : Way::In;
-            cut(j, segs, n, SLOT_BYTES, CHUNK_MIN, true);
-            return run_job(j, device, st);
+            if (ready_ring(device) == cudaSuccess) {
+                Job j;
+                j.way = out ? Way::Out : Way::In;
+                cut(j, segs, n, SLOT_BYTES, CHUNK_MIN, true);
+                return run_job(j, device, st);
+            }
+            cudaGetLastError();                  // no pinned memory to be had: the driver's copies do without
         }
     }
     for (int s = 0; s < n; ++s) {
         if (segs[s].fill) {                      // through pageable memory of our own
-            std::vector<unsigned char> made(segs[s].bytes);
-            segs[s].fill(made.data(), 0, segs[s].bytes, segs[s].arg);
-            cudaError_t e = cudaMemcpyAsync(segs[s].dev, made.data(), segs[s].bytes, cudaMemcpyHostToDevice, st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess) return e;
+            const size_t room = std::min(segs[s].bytes, SLOT_BYTES);
+            const std::unique_ptr<unsigned char[]> made(new (std::nothrow) unsigned char[room]);
+            if (!made) return cudaErrorMemoryAllocation;
+            for (size_t first = 0; first < segs[s].bytes; first += room) {
+                const size_t b = std::min(room, segs[s].bytes - first);
+                segs[s].fill(made.get(), first, b, segs[s].arg);
+                cudaError_t e = cudaMemcpyAsync((unsigned char*)segs[s].dev + first, made.get(), b, cudaMemcpyHostToDevice, st);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                if (e != cudaSuccess) return e;
+            }
             continue;
         }
         const cudaError_t e = out ? cudaMemcpyAsync(segs[s].host, segs[s].dev, segs[s].bytes, cudaMemcpyDeviceToHost, st)

@@ -13,7 +13,7 @@ namespace fake {
 std::mutex mu;
 std::map<unsigned char*, size_t> pinned;                     // registered and allocated ranges
 std::atomic<int> threads_left{1 << 30};
-std::atomic<bool> no_device_pointer{false};
+std::atomic<bool> no_device_pointer{false}, no_register{false};
 std::atomic<long> direct{0}, through_ring{0};                // copies from or to memory that is not pinned, and that is
 std::atomic<cudaError_t> last{cudaSuccess};
 cudaError_t set(cudaError_t e) { if (e != cudaSuccess && e != cudaErrorNotReady) last = e; return e; }
@@ -27,7 +27,7 @@ size_t pinned_bytes() { std::lock_guard<std::mutex> lk(mu); size_t b = 0; for (a
 
 extern "C" {
 cudaError_t cudaGetLastError(void) { return fake::last.exchange(cudaSuccess); }
-cudaError_t cudaHostRegister(void* p, size_t n, unsigned) { std::lock_guard<std::mutex> lk(fake::mu); fake::pinned[(unsigned char*)p] = n; return cudaSuccess; }
+cudaError_t cudaHostRegister(void* p, size_t n, unsigned) { if (fake::no_register) return fake::set(cudaErrorMemoryAllocation); std::lock_guard<std::mutex> lk(fake::mu); fake::pinned[(unsigned char*)p] = n; return cudaSuccess; }
 cudaError_t cudaHostUnregister(void* p) { std::lock_guard<std::mutex> lk(fake::mu); return fake::pinned.erase((unsigned char*)p) ? cudaSuccess : cudaErrorHostMemoryNotRegistered; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::aligned_alloc(4096, (n + 4095) / 4096 * 4096); return cudaHostRegister(*p, n, 0); }
 cudaError_t cudaFreeHost(void* p) { cudaHostUnregister(p); std::free(p); return cudaSuccess; }
@@ -107,9 +107,18 @@ static void stage() {
     EXPECT(stage_take(&a, 1 << 20) == cudaSuccess && a.host && a.dev == a.host);
     stage_give(&a);
 }
+// No memory can be pinned: the driver's own copies, and no error left behind for the next check.
+static void no_ring() {
+    fake::no_register = true;
+    round_trips();
+    EXPECT(fake::through_ring == 0 && cudaGetLastError() == cudaSuccess);
+    fake::no_register = false;
+    round_trips();
+    EXPECT(fake::through_ring > 0);
+}
 
 int main(int argc, char** argv) {
-    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}, {"stage", stage}};
+    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}, {"stage", stage}, {"no_ring", no_ring}};
     const auto it = argc > 1 ? all.find(argv[1]) : all.end();
     if (it == all.end()) { for (auto& s : all) std::puts(s.first.c_str()); return 2; }
     hostio_retain();
