@@ -13,7 +13,8 @@ namespace fake {
 std::mutex mu;
 std::map<unsigned char*, size_t> pinned;                     // registered and allocated ranges
 std::atomic<int> threads_left{1 << 30};
-std::atomic<bool> no_device_pointer{false}, no_register{false};
+std::atomic<bool> no_device_pointer{false}, no_register{false}, fails{false};
+std::atomic<bool> busy[2];                                  // streams 0 and 1 still at work
 std::atomic<long> direct{0}, through_ring{0};                // copies from or to memory that is not pinned, and that is
 std::atomic<cudaError_t> last{cudaSuccess};
 cudaError_t set(cudaError_t e) { if (e != cudaSuccess && e != cudaErrorNotReady) last = e; return e; }
@@ -36,8 +37,8 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaStreamQuery(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamQuery(cudaStream_t s) { return fake::busy[(size_t)s] ? cudaErrorNotReady : cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { if (fake::fails) return fake::set(cudaErrorLaunchFailure); while (fake::busy[(size_t)s]) std::this_thread::yield(); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kind, cudaStream_t) {
     (fake::is_pinned(kind == cudaMemcpyDeviceToHost ? d : s) ? fake::through_ring : fake::direct)++;
     std::memcpy(d, s, n);
@@ -116,9 +117,18 @@ static void no_ring() {
     round_trips();
     EXPECT(fake::through_ring > 0);
 }
+// What the device does before a result fails: the caller's array is as it was.
+static void failed_work() {
+    fake::busy[0] = true; fake::fails = true;
+    const Bytes before = noise((9u << 20) + 5, 3); Bytes host = before, dev(before.size(), 1);
+    const Segment s{host.data(), dev.data(), host.size()};
+    EXPECT(copy_out(&s, 1, 0, nullptr) == cudaErrorLaunchFailure);
+    EXPECT(host == before);
+    fake::busy[0] = false; fake::fails = false;
+}
 
 int main(int argc, char** argv) {
-    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}, {"stage", stage}, {"no_ring", no_ring}};
+    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}, {"stage", stage}, {"no_ring", no_ring}, {"failed_work", failed_work}};
     const auto it = argc > 1 ? all.find(argv[1]) : all.end();
     if (it == all.end()) { for (auto& s : all) std::puts(s.first.c_str()); return 2; }
     hostio_retain();
