@@ -280,11 +280,11 @@ cudaError_t copy_all(const Segment* segs, int n, bool out, int device, cudaStrea
     for (int s = 0; s < n; ++s) { total += segs[s].bytes; made |= segs[s].fill != nullptr; }
     Pool& p = pool();
     if ((made || total >= (out ? SHARED_MIN_OUT : SHARED_MIN_IN)) && device >= 0 && device < MAX_DEVICES) {
-        std::unique_lock<std::mutex> lk(p.use, std::try_to_lock);      // another thread's transfer has the ring: let the driver do this one
-        if (lk.owns_lock()) {
-            ready_workers();
-            if (out && total >= TOUCH_MIN && cudaStreamQuery(st) == cudaErrorNotReady) {
-                // the device is still at work enqueued earlier: the pages the results go to are faulted in meanwhile
+        if (out && total >= TOUCH_MIN && cudaStreamQuery(st) == cudaErrorNotReady) {
+            // the device is still at work enqueued earlier: the pages the results go to are faulted in meanwhile
+            std::unique_lock<std::mutex> lk(p.use, std::try_to_lock);
+            if (lk.owns_lock()) {
+                ready_workers();
                 Job t;
                 t.way = Way::Touch;
                 cut(t, segs, n, SLOT_BYTES, SLOT_BYTES, false);
@@ -292,8 +292,12 @@ cudaError_t copy_all(const Segment* segs, int n, bool out, int device, cudaStrea
                 help(t);
                 withdraw(t);
             }
-            cudaError_t e = cudaStreamSynchronize(st);                 // do not spin through work enqueued earlier
-            if (e != cudaSuccess) return e;
+        }
+        const cudaError_t e = cudaStreamSynchronize(st);               // without the ring: the wait may be as long as a training run
+        if (e != cudaSuccess) return e;
+        std::unique_lock<std::mutex> lk(p.use, std::try_to_lock);      // another thread's transfer has the ring: let the driver do this one
+        if (lk.owns_lock()) {
+            ready_workers();
             if (ready_ring(device) == cudaSuccess) {
                 Job j;
                 j.way = out ? Way::Out : Way::In;

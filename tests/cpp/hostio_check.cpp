@@ -2,6 +2,7 @@
 // answered by the stand-ins below, "device" memory is host memory, and what cannot be had in earnest (a thread that does not start, memory that
 // cannot be pinned, a stream that fails) is had by a switch.  One scenario per run, named on the command line; 0 = as it should be.
 #include "../../cudarl-arena_b200/csrc/hostio.cpp"
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <dlfcn.h>
@@ -126,9 +127,22 @@ static void failed_work() {
     EXPECT(host == before);
     fake::busy[0] = false; fake::fails = false;
 }
+// While one caller waits for its stream, another has the ring.
+static void long_wait() {
+    const Bytes dev = noise(9u << 20, 5); Bytes a(dev.size(), 0), b(dev.size(), 0), d = dev;
+    const Segment sa{a.data(), d.data(), d.size()}, sb{b.data(), d.data(), d.size()};
+    fake::busy[0] = true;
+    std::thread waits([&] { EXPECT(copy_out(&sa, 1, 0, (cudaStream_t)0) == cudaSuccess); });
+    std::this_thread::sleep_for(std::chrono::milliseconds(200));
+    EXPECT(copy_out(&sb, 1, 0, (cudaStream_t)1) == cudaSuccess);
+    EXPECT(fake::through_ring > 0 && fake::direct == 0 && b == dev);
+    fake::busy[0] = false;
+    waits.join();
+    EXPECT(fake::direct == 0 && a == dev);
+}
 
 int main(int argc, char** argv) {
-    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}, {"stage", stage}, {"no_ring", no_ring}, {"failed_work", failed_work}};
+    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}, {"stage", stage}, {"no_ring", no_ring}, {"failed_work", failed_work}, {"long_wait", long_wait}};
     const auto it = argc > 1 ? all.find(argv[1]) : all.end();
     if (it == all.end()) { for (auto& s : all) std::puts(s.first.c_str()); return 2; }
     hostio_retain();
