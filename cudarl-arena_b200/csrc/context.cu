@@ -503,11 +503,14 @@ int alloc_gather(cudarl_ctx* c) {
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
     CK(cudaMalloc(&c->dgbar, 256)); CK(cudaMemsetAsync(c->dgbar, 0, 256, c->st));
-    CK(cudaMalloc(&c->dgcnt, 8 * S * sizeof(unsigned))); CK(cudaMemsetAsync(c->dgcnt, 0, 8 * S * sizeof(unsigned), c->st));
     CK(cudaMalloc(&c->dgmv, S));
-    if (!arena_plan(p)) { gp = GatherP{}; gather_plan(p, sms); }
+    if (!arena_plan(p)) {
+        gp = GatherP{}; gather_plan(p, sms);
+        // 32 bytes a cell, twice the table: only for the launches that count in global memory, not for one block's worlds (or none)
+        CK(cudaMalloc(&c->dgcnt, 8 * S * sizeof(unsigned))); CK(cudaMemsetAsync(c->dgcnt, 0, 8 * S * sizeof(unsigned), c->st));
+        gp.cnt[0] = (unsigned*)c->dgcnt; gp.cnt[1] = gp.cnt[0] + 4 * S;
+    }
     gp.barrier = (unsigned*)c->dgbar;
-    gp.cnt[0] = (unsigned*)c->dgcnt; gp.cnt[1] = gp.cnt[0] + 4 * S;
     gp.mv = (unsigned char*)c->dgmv;
     if (gp.home == 2u) { CK(cudaMalloc(&c->dgstate, N * 24u)); gp.state = (unsigned char*)c->dgstate; }
     if (gp.deal_every) {

@@ -205,3 +205,17 @@ def test_episode_epsilon_when_everybody_ends_in_the_first_step_of_a_launch(pkg, 
         gpu.train_steps(k); cpu.train_steps(k)
         assert_same(gpu, cpu, "n=%d after +%d" % (n, k))
         assert gpu.get_stats().epsilon == cpu.get_stats().epsilon
+
+
+@pytest.mark.parametrize("n", [0, 1, 32])
+def test_memory_of_contexts_that_need_no_counters(pkg, n):
+    """A table with no or few environments: 16 bytes a cell, 4 for the rollout, 2 for the cell's class and 1 for its moves."""
+    import torch
+    side = 6000
+    pkg.VecGridWorld(world(pkg, 8, 8, 1)).close()            # what the process needs once
+    free = torch.cuda.mem_get_info()[0]
+    w = pkg.VecGridWorld(world(pkg, side, side, n))
+    used = free - torch.cuda.mem_get_info()[0]
+    assert used < 23 * side * side + (32 << 20)
+    w.train_steps(3); w.eval_rollout(5); w.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] < 23 * side * side + (32 << 20)
