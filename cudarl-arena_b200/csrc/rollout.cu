@@ -27,15 +27,18 @@ namespace cudarl {
 // of steps in bits 0-12, the edge it leaves by (0 up, 1 right, 2 down, 3 left) in bits 22-23 and the place along it in bits 16-21;
 // GOAL with the number of steps; or TRAPPED.  Bit 29: an obstacle or a goal, where no episode starts.  A path without a circle has at most 4096 steps inside a tile.
 constexpr unsigned RT_ROWS = 8u;                 // rows of a tile that its threads take at a time
+// Rows of tiles in a launch's second dimension, which ends at 65,535, while a grid's height ends at 2^28; the third takes the rest.
+constexpr unsigned GRID_ROWS = 32768u;
 constexpr unsigned KIND_LIVE = 0u, KIND_EXIT = 1u << 30, KIND_GOAL = 2u << 30, KIND_MASK = 3u << 30, TRAPPED = 3u << 30, NO_START = 1u << 29, STEPS_MASK = 0x1FFFu;
 
 template <unsigned RT_SHIFT>
-__global__ void __launch_bounds__(RT_ROWS << RT_SHIFT) k_rollout_tiles(const __grid_constant__ Params p, unsigned* __restrict__ hop, unsigned tiles_x) {
+// (32 registers, so that an SM is full: with 38 it held three blocks of 64 x 64 cells instead of four, 4096 x 4096 cells 173 -> 180 us)
+__global__ void __launch_bounds__(RT_ROWS << RT_SHIFT, 2048u / (RT_ROWS << RT_SHIFT)) k_rollout_tiles(const __grid_constant__ Params p, unsigned* __restrict__ hop) {
     constexpr unsigned RT = 1u << RT_SHIFT, RT_CELLS = RT * RT, RT_THREADS = RT * RT_ROWS, RT_PER = RT_CELLS / RT_THREADS;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");       // the walk's blocks may take the slots that free up, and draw
     __shared__ unsigned s_w[RT_CELLS];
-    const unsigned ty = blockIdx.x / tiles_x, tx = blockIdx.x - ty * tiles_x;            // tiles in one dimension: a second one of the launch ends at 65,535, a grid's height at 2^28
-    const int x0 = (int)(tx << RT_SHIFT), y0 = (int)(ty << RT_SHIFT);
+    const int x0 = (int)(blockIdx.x << RT_SHIFT), y0 = (int)((blockIdx.z * GRID_ROWS + blockIdx.y) << RT_SHIFT);
+    if (y0 >= p.H) return;
     unsigned cur[RT_PER];
     const unsigned lx = threadIdx.x & (RT - 1u), ly0 = threadIdx.x >> RT_SHIFT;          // a thread's cells lie below one another, 8 rows apart
     const int x = x0 + (int)lx;
@@ -164,7 +167,8 @@ template <unsigned RT_SHIFT>
 static cudaError_t launch_tiled(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
     constexpr unsigned RT = 1u << RT_SHIFT;
     const unsigned tiles_x = ((unsigned)p.W + RT - 1u) / RT, tiles_y = ((unsigned)p.H + RT - 1u) / RT;
-    k_rollout_tiles<RT_SHIFT><<<tiles_x * tiles_y, RT * RT_ROWS, 0, st>>>(p, hop, tiles_x);
+    const dim3 tiles(tiles_x, tiles_y < GRID_ROWS ? tiles_y : GRID_ROWS, (tiles_y + GRID_ROWS - 1u) / GRID_ROWS);
+    k_rollout_tiles<RT_SHIFT><<<tiles, RT * RT_ROWS, 0, st>>>(p, hop);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;                      // no walk over words that nobody has written
     // four environments per thread where the chip is full with that
