@@ -10,7 +10,7 @@
 //
 // All updates of one (cell, action) within a step are the same map, so only their number matters (see tile_engine.cu).  Who applies
 // it: with OWNERS the first to count there, which needs the counter's old value -- right where latency counts and crowds are common;
-// without, everybody who counted (all compute and store the same bits), so that the atomics need no answer -- right where their rate
+// without, everybody who counted (all compute and store the same bits; of a crowd in a streamed population the first), so that the atomics need no answer -- right where their rate
 // counts (1024 x 1024 cells, 1,048,576 environments: 25.0 -> 24.0 us a step; 1001 x 613, 150,001: 7.6 -> 6.8; but 64 x 64 with 4,096
 // crowded ones 4.7 -> 5.5).  Counters alternate by step parity; who counted clears its counter in the next step's count phase, when
 // everybody has read it and nobody uses that parity.
@@ -111,6 +111,11 @@ template <Home HOME, unsigned GB, bool PLAIN, bool OWNERS, class Space>
 __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, Space& space, int4* __restrict__ work, unsigned char* arrays) {
     __shared__ unsigned s_sum[5], s_ep;
     constexpr bool STREAM = HOME != Home::Registers;
+    // Without OWNERS, who applies what a crowd has counted: with one turn a step everybody (all at the same time, and the answer to the question who came
+    // first would take 0.6 us of the step's 7); with many turns the first to mark the counter, since the others' rounds would follow one another.
+    // 1024 x 1024 cells, everybody on one start cell, everybody / the first, us a step: 1,048,576 environments at lr 0.1 160 / 108, at 0.001 1,963 /
+    // 273, at 1e-5 107,000 / 10,170; 4,194,304 on 512 x 512, random starts 196 / 142.
+    constexpr bool FIRST = !OWNERS && STREAM;
     const unsigned tid = threadIdx.x, first = blockIdx.x * l.chunk, count = first < p.N ? min(l.chunk, p.N - first) : 0u;
     Ctl* const ctl = p.ctl;
     const unsigned W = (unsigned)p.W;
@@ -210,25 +215,32 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
         // ---- apply ----
         for (unsigned j = tid; j < end; j += GB) {
             if (STREAM) own = j < count ? m_own[j] : NOBODY;
-            if (own == NOBODY) continue;
-            if (STREAM) { const float2 q = m_tv[j]; target = q.x; value = q.y; }
-            uint4 c = space.counts(par, own >> 2);
-            const unsigned a = own & 3u;
-            unsigned n = a == 0u ? c.x : a == 1u ? c.y : a == 2u ? c.z : c.w;
-            const unsigned tot = c.x + c.y + c.z + c.w;
-            if (tot > 1u) tally.conf += OWNERS ? n : 1u;
-            if (tot > CROWDED_CELL) {                 // the lowest chosen action speaks for the cell
-                if (!OWNERS) {                        // the first to get here, that is; its mark on the counter looks like a huge count to the others
-                    c.x &= ~NOTED; c.y &= ~NOTED; c.z &= ~NOTED; c.w &= ~NOTED; n &= ~NOTED;
-                    ++tally.on_crowded;
-                }
-                const unsigned below = a == 0u ? 0u : a == 1u ? c.x : a == 2u ? c.x + c.y : c.x + c.y + c.z;
-                if (below == 0u) {
-                    if (OWNERS) { ++tally.crowded; tally.on_crowded += tot; }
-                    else if (!space.note(par, own)) ++tally.crowded;
+            unsigned n = 0u;
+            bool applies = own != NOBODY;
+            if (applies) {
+                if (STREAM) { const float2 q = m_tv[j]; target = q.x; value = q.y; }
+                uint4 c = space.counts(par, own >> 2);
+                const unsigned a = own & 3u;
+                n = a == 0u ? c.x : a == 1u ? c.y : a == 2u ? c.z : c.w;
+                const unsigned tot = c.x + c.y + c.z + c.w;
+                if (tot > 1u) tally.conf += OWNERS ? n : 1u;
+                if (tot > CROWDED_CELL) {             // (marks on the counters make the sum larger, or leave it as it is: it stays above)
+                    unsigned marked = 0u;
+                    if (!OWNERS) { marked = n & NOTED; c.x &= ~NOTED; c.y &= ~NOTED; c.z &= ~NOTED; n &= ~NOTED; ++tally.on_crowded; }
+                    const unsigned below = a == 0u ? 0u : a == 1u ? c.x : a == 2u ? c.x + c.y : c.x + c.y + c.z;       // the lowest chosen action speaks for the cell
+                    if (OWNERS) { if (below == 0u) { ++tally.crowded; tally.on_crowded += tot; } }
+                    else if (!FIRST) { if (below == 0u && !space.note(par, own)) ++tally.crowded; }
+                    else if (below == 0u || n > CROWDED_CELL) {
+                        bool one = !marked;              // one lane of a warp tries
+                        if (one && n > CROWDED_CELL) one = (tid & 31u) == (unsigned)__ffs((int)__match_any_sync(__activemask(), own)) - 1u;
+                        one = one && !space.note(par, own);
+                        if (one && below == 0u) ++tally.crowded;
+                        applies = one || n <= CROWDED_CELL;
+                    }
                 }
             }
-            space.store(own, apply_counted(value, target, p.lr, n));
+            if (FIRST) __syncwarp();                  // the lanes' rounds side by side, however they got here
+            if (applies) space.store(own, apply_counted(value, target, p.lr, n));
         }
         eps_index.next(p, l, PLAIN, Space::ALONE ? *reinterpret_cast<volatile unsigned*>(&s_ep) : 0u, Space::ALONE);        // between the two barriers: nobody adds to the episodes before everybody has passed the second
         space.arrive();
