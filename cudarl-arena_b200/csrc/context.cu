@@ -105,6 +105,7 @@ struct cudarl_ctx {
     bool gather = false;                   // the engine of this context's train steps: gather, or the tiles
     void *dgbar = nullptr, *dgcnt = nullptr, *dgmv = nullptr, *dgstate = nullptr, *dgbins = nullptr;
     int dealt = -1;                        // the work buffer the records are in, dealt by cell; -1: in environment order
+    unsigned since_deal = 0;               // steps since then
     void* dwork[2] = {nullptr, nullptr};
     uint32_t barrier_base = 0;             // arrivals at the grid barrier by all launches so far
     bool tile_mode = false;               // true: the records live in tile regions (train steps), false: in environment order
@@ -674,16 +675,19 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         int64_t m = std::min(n - k, most);
         if (c->cfg.sync_every > 0 && c->comm) m = std::min<int64_t>(m, c->cfg.sync_every - c->h_step % c->cfg.sync_every);
         const unsigned deal = c->p.gp.deal_every;
-        if (deal) m = std::min<int64_t>(m, deal);
+        const bool dealing = deal && (c->dealt < 0 || c->since_deal >= deal);
+        if (deal) m = std::min<int64_t>(m, dealing ? deal : deal - c->since_deal);
         { int rc = open_kernel_segment(c); if (rc) return rc; }
         c->p.step = (unsigned long long)c->h_step;
         c->p.eps_idx = c->eps_mode == 1 ? (unsigned)k : 0u;
         StepLaunch l{};
         l.steps = (unsigned)m; l.chunk = c->p.gp.chunk; l.barrier_base = c->barrier_base; l.eps_mode = c->eps_mode; l.trace = c->trace ? 1 : 0; l.eps_len = c->eps_len; l.eps_base_k = c->eps_base_k;
-        l.in = c->dealt >= 0 ? (const int4*)c->dwork[c->dealt] : c->p.st; l.out = deal ? (int4*)c->dwork[c->dealt == 0 ? 1 : 0] : c->p.st;
+        l.in = c->dealt >= 0 ? (const int4*)c->dwork[c->dealt] : c->p.st;
+        l.out = dealing ? (int4*)c->dwork[c->dealt == 0 ? 1 : 0] : const_cast<int4*>(l.in);
         CK(c->p.gp.arena ? launch_arena_steps(c->p, l, c->st) : launch_gather_steps(c->p, l, c->st));
         c->barrier_base += c->p.gp.grid * gather_barriers(l);
-        if (deal) c->dealt = c->dealt == 0 ? 1 : 0;
+        if (dealing) { c->dealt = c->dealt == 0 ? 1 : 0; c->since_deal = 0; }
+        c->since_deal += (unsigned)m;
         c->h_step += m; c->kseg_count += m; k += m;
         if (c->eps_mode != 2 && c->h_eps) c->eps_used = c->h_eps[c->eps_mode == 1 ? k - 1 : 0];
         if (c->cfg.sync_every > 0 && c->comm && (c->h_step % c->cfg.sync_every) == 0) { int rc = average_now(c); if (rc) return rc; }

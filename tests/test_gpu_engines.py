@@ -235,3 +235,30 @@ def test_a_crowd_of_slow_learners(pkg, orc, n, lr):
     cpu.train_steps(16)
     assert_same(gpu, cpu, "n=%d lr=%g" % (n, lr))
     assert t < 0.8
+
+
+def test_one_step_a_call_does_not_deal_every_step(pkg, orc):
+    """Dealt by cell every 64 steps, however many calls those are (a dealing in every launch took 13 us a step on top of the step's 7, a launch
+    alone takes 5); calls of any length in a row, and with the records read and replaced between them, leave the same world."""
+    cfg = world(pkg, 300, 290, 100000, max_steps=150)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    for k in (1, 1, 61, 1, 1, 64, 65, 3, 127, 1):
+        gpu.train_steps(k); cpu.train_steps(k)
+        if k in (61, 65, 3):
+            assert_same(gpu, cpu, "+%d" % k)
+        if k == 64:
+            x, y, t = gpu.get_state()
+            gpu.set_state(t=t); cpu.set_state(t=t)       # back to the order of the environments
+    assert_same(gpu, cpu, "after all")
+
+    def best(calls, steps):
+        times = []
+        for _ in range(15):
+            gpu.synchronize()
+            t = time.perf_counter()
+            for _ in range(calls):
+                gpu.train_steps(steps)
+            gpu.synchronize()
+            times.append(time.perf_counter() - t)
+        return min(times)
+    assert best(64, 1) < best(1, 64) + 64 * 9e-6
