@@ -1086,20 +1086,28 @@ int cudarl_get_state(cudarl_ctx* c, int32_t* x, int32_t* y, int32_t* t) {
 
 int cudarl_set_state(cudarl_ctx* c, const int32_t* x, const int32_t* y, const int32_t* t) {
     if (!c) return -1;
-    const size_t N = c->p.N;
-    if (x) for (size_t i = 0; i < N; ++i) if (x[i] < 0 || x[i] >= c->p.W) return fail(c, -3, "Invalid state");
-    if (y) for (size_t i = 0; i < N; ++i) if (y[i] < 0 || y[i] >= c->p.H) return fail(c, -3, "Invalid state");
-    if (t) for (size_t i = 0; i < N; ++i) if (t[i] < 0 || t[i] > 0xFFFFFE) return fail(c, -3, "Invalid state (an episode's step count lies in 0 .. 16,777,214)");
     CK(cudaSetDevice(c->cfg.device));
-    { int rl = leave_tiles(c); if (rl) return rl; }
-    if (!c->dimport) CK(cudaMalloc(&c->dimport, (N ? N : 1) * 12));
-    int* dx = (int*)c->dimport; int* dy = dx + N; int* dt = dy + N;
+    const size_t N = c->p.N, row = up64(N * 4);
+    // Checked on the way, by the cores that copy: into the mapped stage while the arrays fit it, else through the ring.  1,048,576 environments
+    // took 2.2 ms with three passes of one core first.
+    BoundedSource src[3] = {{x, (uint32_t)c->p.W - 1u}, {y, (uint32_t)c->p.H - 1u}, {t, STEP_SAT}};
+    const bool small = STAGE_DATA + 3 * row <= c->stage.bytes;
+    if (!small && !c->dimport) CK(cudaMalloc(&c->dimport, 3 * row));
+    unsigned char* const dev = small ? c->stage.dev + STAGE_DATA : (unsigned char*)c->dimport;
+    const int* to[3] = {nullptr, nullptr, nullptr};
     Segment in[3]; int n = 0;
-    if (x) in[n++] = Segment{const_cast<int32_t*>(x), dx, N * 4};
-    if (y) in[n++] = Segment{const_cast<int32_t*>(y), dy, N * 4};
-    if (t) in[n++] = Segment{const_cast<int32_t*>(t), dt, N * 4};
-    CK(copy_in(in, n, c->cfg.device, c->st));
-    launch_import_state(c->p, x ? dx : nullptr, y ? dy : nullptr, t ? dt : nullptr, c->st);
+    for (int k = 0; k < 3; ++k) {
+        if (!src[k].from) continue;
+        to[k] = (const int*)(dev + k * row);
+        in[n].bytes = N * 4; in[n].fill = copy_bounded; in[n].arg = &src[k];
+        if (small) in[n].host = c->stage.host + STAGE_DATA + k * row; else in[n].dev = dev + k * row;
+        ++n;
+    }
+    if (small) copy_host(in, n, true); else CK(copy_in(in, n, c->cfg.device, c->st));
+    if (src[0].bad || src[1].bad) return fail(c, -3, "Invalid state");
+    if (src[2].bad) return fail(c, -3, "Invalid state (an episode's step count lies in 0 .. 16,777,214)");
+    { int rl = leave_tiles(c); if (rl) return rl; }
+    launch_import_state(c->p, to[0], to[1], to[2], c->st);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->st));
     return 0;

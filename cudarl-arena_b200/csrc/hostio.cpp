@@ -355,6 +355,15 @@ VECTORISED static uint32_t cells(uint32_t* __restrict o, const int32_t* __restri
     }
     return bad;
 }
+VECTORISED static uint32_t bounded(uint32_t* __restrict o, const int32_t* __restrict v, size_t n, uint32_t most) {
+    uint32_t bad = 0;
+    for (size_t k = 0; k < n; ++k) { const uint32_t u = (uint32_t)v[k]; bad |= (uint32_t)(u > most); o[k] = u; }
+    return bad;
+}
+void copy_bounded(void* dst, size_t first, size_t bytes, const void* source) {
+    BoundedSource& s = *(BoundedSource*)source;
+    if (bounded((uint32_t*)dst, s.from + first / 4, bytes / 4, s.most)) s.bad = true;
+}
 void pack_cell_action(void* dst, size_t first, size_t bytes, const void* source) {
     TransitionSource& s = *(TransitionSource*)source;
     const size_t i = first / 4;

@@ -32,6 +32,14 @@ struct TransitionSource {
 void pack_cell_action(void* dst, size_t first, size_t bytes, const void* source);      // cell * 4 + action, bit 31 = the episode ended there
 void pack_next_cell(void* dst, size_t first, size_t bytes, const void* source);
 
+// Values of 0 .. most, checked on the way (`bad`: one was not).
+struct BoundedSource {
+    const int32_t* from; uint32_t most;
+    std::atomic<bool> bad{false};
+    BoundedSource(const int32_t* from_, uint32_t most_) : from(from_), most(most_) {}
+};
+void copy_bounded(void* dst, size_t first, size_t bytes, const void* source);
+
 void hostio_retain();                         // one per context: keeps the process-wide parts alive
 void hostio_release();
 cudaError_t stage_take(Stage* s, size_t bytes);      // zeroed first 256 bytes

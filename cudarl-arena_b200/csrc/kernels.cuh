@@ -152,6 +152,7 @@ struct Params : World {
 };
 
 constexpr int BLOCK = 256;
+constexpr unsigned STEP_SAT = 0xFFFFFEu;    // an episode's step counter saturates here (the tile records keep 24 bits of it)
 
 // launch wrappers (kernels.cu); all asynchronous on `st`
 void launch_identity_ids(const Params& p, cudaStream_t st);

@@ -13,7 +13,6 @@ namespace cudarl {
 
 constexpr unsigned FULL = 0xFFFFFFFFu;
 constexpr unsigned CROWDED_CELL = 24;       // a cell with more environments than this counts as "crowded" in the run statistics
-constexpr unsigned STEP_SAT = 0xFFFFFEu;    // an episode's step counter saturates here (the tile records keep 24 bits of it)
 
 // ------------------------------------------------------------------------------------------------
 // Philox4x32-10, counter-based: no generator state is stored anywhere.

@@ -140,9 +140,27 @@ static void long_wait() {
     waits.join();
     EXPECT(fake::direct == 0 && a == dev);
 }
+// Values checked on their way, into a stage and through the ring: the only one out of bounds is found wherever it is.
+static void bounded() {
+    for (size_t n : {(size_t)1, (size_t)77, (size_t)70001, (size_t)1500003}) {
+        std::vector<int32_t> v(n); std::vector<uint32_t> to((n + 31) / 16 * 16);
+        std::minstd_rand r((unsigned)n);
+        for (auto& u : v) u = (int32_t)(r() % 1000);
+        for (int way = 0; way < 2; ++way)
+            for (int32_t wrong : {0, 999, 1000, -1, INT32_MIN, INT32_MAX}) {
+                const size_t at = r() % n; const int32_t was = v[at];
+                v[at] = wrong;
+                BoundedSource src(v.data(), 999u);
+                Segment s; s.bytes = n * 4; s.fill = copy_bounded; s.arg = &src;
+                if (way) { s.host = to.data(); copy_host(&s, 1, true); } else { s.dev = to.data(); EXPECT(copy_in(&s, 1, 0, nullptr) == cudaSuccess); }
+                EXPECT(src.bad == (wrong < 0 || wrong > 999) && std::memcmp(to.data(), v.data(), n * 4) == 0);
+                v[at] = was;
+            }
+    }
+}
 
 int main(int argc, char** argv) {
-    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}, {"stage", stage}, {"no_ring", no_ring}, {"failed_work", failed_work}, {"long_wait", long_wait}};
+    const std::map<std::string, void (*)()> all = {{"plain", plain}, {"callers", callers}, {"no_threads", no_threads}, {"few_threads", few_threads}, {"stage", stage}, {"no_ring", no_ring}, {"failed_work", failed_work}, {"long_wait", long_wait}, {"bounded", bounded}};
     const auto it = argc > 1 ? all.find(argv[1]) : all.end();
     if (it == all.end()) { for (auto& s : all) std::puts(s.first.c_str()); return 2; }
     hostio_retain();

@@ -262,3 +262,31 @@ def test_one_step_a_call_does_not_deal_every_step(pkg, orc):
             times.append(time.perf_counter() - t)
         return min(times)
     assert best(64, 1) < best(1, 64) + 64 * 9e-6
+
+
+@pytest.mark.parametrize("n", [1, 300, 21800, 349504, 349505, 1 << 20])
+def test_set_state_limits(pkg, n):
+    """States in through the mapped stage and through the ring, all or some of the arrays, and one value out of range anywhere, which must leave the
+    states as they were.  (Checked by one core before it was copied, the largest took 2.2 ms.)"""
+    g = pkg.VecGridWorld(world(pkg, 1000, 777, n, obstacle_p=0.0, obstacle_kind=pkg.OBST_NONE, max_steps=0))
+    g.train_steps(2)
+    rng = np.random.RandomState(n)
+    x, y, t = rng.randint(0, 1000, n).astype(np.int32), rng.randint(0, 777, n).astype(np.int32), rng.randint(0, 0xFFFFFE + 1, n).astype(np.int32)
+    g.set_state(x, y, t)
+    assert all(np.array_equal(a, b) for a, b in zip(g.get_state(), (x, y, t)))
+    for k, bad in ((0, 1000), (0, -1), (1, 777), (1, -5), (2, 0xFFFFFF), (2, -1)):
+        wrong = [x.copy(), y.copy(), t.copy()]
+        wrong[k][rng.randint(0, n)] = bad
+        with pytest.raises(pkg.CudarlError) as ei:
+            g.set_state(*wrong)
+        assert ei.value.code == -3 and ("step count" in str(ei.value)) == (k == 2)
+    assert all(np.array_equal(a, b) for a, b in zip(g.get_state(), (x, y, t)))
+    y = y[::-1].copy()
+    g.set_state(y=y)
+    assert all(np.array_equal(a, b) for a, b in zip(g.get_state(), (x, y, t)))
+    times = []
+    for _ in range(15):
+        s = time.perf_counter()
+        g.set_state(x, y, t)
+        times.append(time.perf_counter() - s)
+    assert min(times) < 1.2e-3

@@ -17,7 +17,7 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["plain", "callers", "no_threads", "few_threads", "stage", "no_ring", "failed_work", "long_wait"])
+@pytest.mark.parametrize("scenario", ["plain", "callers", "no_threads", "few_threads", "stage", "no_ring", "failed_work", "long_wait", "bounded"])
 def test_copies(check, scenario):
     r = subprocess.run([check, scenario], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
