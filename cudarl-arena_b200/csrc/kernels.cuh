@@ -134,6 +134,7 @@ struct SortP {
 constexpr size_t SORT_WORDS = 1u + SORT_MOST_BLOCKS + 512u + 512u * (size_t)SORT_MOST_BLOCKS;      // barrier, part, total, hist
 struct Params : World {
     unsigned policy_keys[20];   // the ten round keys of the policy stream, two words each: operands straight from the constant bank
+    unsigned policy_pre[4];     // k_tile_step: what its step and the keys alone make of the first two rounds
     uint4* ent;            // collision entries
     unsigned ent_cap;      // slots in ent
     unsigned* mailbox;     // update_batch: chain heads (0 = empty), power-of-two size
@@ -177,7 +178,7 @@ int  tile_engine_configure(Params& p, int device);                  // opt in to
 void launch_tile_bucket(const Params& p, cudaStream_t st);         // p.st (any slot order) -> tile regions of parity p.step & 1
 void launch_tile_classes(const Params& p, cudaStream_t st);       // cell words -> per-tile class bytes (after any change of the grid)
 void launch_tile_export(const Params& p, cudaStream_t st);         // tile regions -> p.st in environment order
-void launch_tile_step(const Params& p, bool trace, cudaStream_t st);
+void launch_tile_step(Params& p, bool trace, cudaStream_t st);
 unsigned tile_cls_stride(unsigned tshift);                         // bytes of one tile's class block
 void launch_tile_border(const Params& p, cudaStream_t st);         // border array of parity p.step & 1 from the table (after any change of the table outside train steps)
 // gather engine (gather_engine.cu)

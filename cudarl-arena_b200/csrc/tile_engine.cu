@@ -31,7 +31,8 @@
 //
 // What bounds the kernel (B200, 4096 x 4096 cells, 4,194,304 environments): a tile is ~1,100 dependent instructions at ~10
 // cycles each for its warp; the 451 MB a step moves are hidden behind the other resident warps (28 per SM: 72 registers,
-// 7.75 KB of shared memory each).  The tile loop is rolled and reads its records from shared memory on purpose: unrolled
+// 7.75 KB of shared memory each).  Instructions taken out of that chain (the draw's common first rounds from the host, the move's offsets by
+// byte picks, the border value without a chain of comparisons: some 30 a tile) gave 105.7 -> 104.8 us a step.  The tile loop is rolled and reads its records from shared memory on purpose: unrolled
 // over register-held records it outgrew the instruction cache.
 //
 // Reference semantics (paths relative to the CudaRL-Arena project root):
@@ -108,6 +109,8 @@ __device__ __forceinline__ uint2 lds_u32x2(unsigned a) { uint2 v; asm volatile("
 __device__ __forceinline__ void sts_f32(unsigned a, float v) { asm volatile("st.shared.f32 [%0], %1;" :: "r"(a), "f"(v) : "memory"); }
 __device__ __forceinline__ void sts_zero8(unsigned a) { asm volatile("st.shared.v2.u32 [%0], {%1, %1};" :: "r"(a), "r"(0u) : "memory"); }
 __device__ __forceinline__ unsigned atoms_add(unsigned a, unsigned v) { unsigned o; asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(o) : "r"(a), "r"(v) : "memory"); return o; }
+// The bytes of v (0-3) or of zero (4-7) that sel's four digits name; with 8 added, that byte's sign bit eight times.
+__device__ __forceinline__ unsigned byte_pick(unsigned v, unsigned sel) { unsigned o; asm("prmt.b32 %0, %1, %2, %3;" : "=r"(o) : "r"(v), "r"(0u), "r"(sel)); return o; }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t;
@@ -426,20 +429,21 @@ __global__ void __launch_bounds__(WPB * 32u, MINB) k_tile_step(const __grid_cons
                 if (act && (lx | ly) >= T) { s_acc[5] = 1u; act = false; }             // never seen: the record does not lie in this tile
                 uint2 nrec = make_uint2(id, 0u); bool stays = false; unsigned key = 0u; float dd = 0.0f;
                 if (act) {
-                    const U4 w = philox4x32_10(p.env_offset + id, 0u, (unsigned)g, (unsigned)(g >> 32), p.policy_keys);
+                    const U4 w = policy_philox(p.env_offset + id, p.policy_keys, p.policy_pre);
                     const unsigned ic = (ly << TSH) | lx;
                     const float4 row = lds_f4(sq + ic * 16u);
                     const unsigned mvb = lds_u8(smv + ic);
                     int a = argmax4(row);
                     if ((w.x >> 8) < c.eps_thr) a = (int)(w.y & 3u);
-                    const bool blocked = (mvb >> a) & 1u, done = (mvb >> (a + 4)) & 1u;
-                    // per action: dx = {0, 1, 0, -1}, dy = {-1, 0, 1, 0}, one signed byte each
-                    const int dx = blocked ? 0 : (int)(signed char)(0xFF000100u >> (8 * a)), dy = blocked ? 0 : (int)(signed char)(0x000100FFu >> (8 * a));
-                    const unsigned mx = lx + (unsigned)dx, my = ly + (unsigned)dy;      // wraps when the move leaves the tile
+                    const unsigned mva = mvb >> a;
+                    const bool blocked = mva & 1u, done = mva & 16u;
+                    // per action: dx = {0, 1, 0, -1}, dy = {-1, 0, 1, 0}, one signed byte each; a blocked move takes a byte of zeros
+                    const unsigned sel = (blocked ? 4u : (unsigned)a) * 0x1111u + 0x8880u;      // that byte, and its sign three times
+                    const unsigned mx = lx + byte_pick(0xFF000100u, sel), my = ly + byte_pick(0x000100FFu, sel);      // wraps when the move leaves the tile
                     stays = (mx | my) < T;
-                    float m;
-                    if (stays) m = max4(lds_f4(sq + ((my << TSH) | mx) * 16u));
-                    else m = lds_f32(shalo + 4u * ((int)my < 0 ? lx : my >= T ? T + lx : (int)mx < 0 ? 2u * T + ly : 3u * T + ly));
+                    // the cell the move ends on: one of the tile's, or -- by the action -- one of the border values (north, south, west, east)
+                    float m = max4(lds_f4(sq + (((my << TSH) | mx) & (T2 - 1u)) * 16u));
+                    if (!stays) m = lds_f32(shalo + 4u * (((a & 1) ? ly : lx) + T * ((0x2130u >> (4 * a)) & 3u)));
                     if (p.legacy_clamp && m < 0.0f) m = 0.0f;
                     const float r = (blocked && p.ntraps) ? blocked_step_reward(p, tx0 + (int)lx, ty0 + (int)ly, a) : -0.01f;     // a trap charges its penalty
                     dd = done ? 1.0f : __fmaf_rn(p.gamma, m, r);                     // the TD target of (cell, a), from Q_t
@@ -907,7 +911,8 @@ static void launch_step_one(const Params& p, bool trace, unsigned grid, size_t s
     else if (p.tp.wait_polls) cudaLaunchKernelEx(&cfg, k_tile_step<false, TSH, MINB, true>, p);     // tests only: the waits run out
     else                      cudaLaunchKernelEx(&cfg, k_tile_step<false, TSH, MINB, false>, p);
 }
-void launch_tile_step(const Params& p, bool trace, cudaStream_t st) {
+void launch_tile_step(Params& p, bool trace, cudaStream_t st) {
+    policy_prefix(p.policy_keys, p.step, p.policy_pre);
     const size_t smem = tile_step_smem(p);
     const unsigned grid = tile_step_grid(p);
     if (p.tp.tshift == 3u) launch_step_one<3, MINB8>(p, trace, grid, smem, st);
