@@ -247,14 +247,13 @@ int ensure_entry_capacity(cudarl_ctx* c, size_t n) {
     so.a = (uint2*)c->dsort; so.b = so.a + cap;
     so.barrier = (unsigned*)(so.b + cap); so.part = so.barrier + 1; so.total = so.part + SORT_MOST_BLOCKS; so.hist = so.total + 512;
     CK(cudaMemsetAsync(so.barrier, 0, sizeof(unsigned), c->st));
-    int sms = 0; CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
-    so.blocks = std::min<unsigned>((unsigned)std::max(sms, 1), SORT_MOST_BLOCKS);
+    so.blocks = std::min<unsigned>(c->p.sms, SORT_MOST_BLOCKS);
     CK(cudaMalloc(&c->dmail, 3 * slots * sizeof(unsigned)));
     CK(cudaMemsetAsync(c->dmail, 0, slots * sizeof(unsigned), c->st));
     c->p.ent = (uint4*)c->dent;
     c->p.mailbox = (unsigned*)c->dmail; c->p.mb_slots = (unsigned)slots;
     c->p.active = c->p.mailbox + slots; c->p.longq = c->p.mailbox + 2 * slots;
-    c->ent_cap = cap; c->p.ent_cap = (unsigned)cap;
+    c->ent_cap = cap;
     return 0;
 }
 
@@ -368,8 +367,7 @@ int check_posted_error(cudarl_ctx* c) {
     const unsigned err = box32(c, 0);
     if (err) return fail(c, CUDARL_ERR_DEVICE + (int)err, "device error bits " + std::to_string(err) +
                          ((err & ERR_COPY_TIMEOUT) ? " (a wait of a kernel ran out)" : "") +
-                         ((err & ERR_SCRATCH_OVERFLOW) ? " (scratch area full)" : "") + ((err & ERR_BAD_STATE) ? " (a record outside its tile or the grid)" : "") +
-                         ((err & ERR_CHAIN_CYCLE) ? " (update_batch chain longer than the batch)" : ""));
+                         ((err & ERR_SCRATCH_OVERFLOW) ? " (scratch area full)" : "") + ((err & ERR_BAD_STATE) ? " (a record outside its tile or the grid)" : ""));
     if (c->comm && g_nccl.CommGetAsyncError) {               // a collective that failed after it was enqueued (a peer that went away)
         ncclResult_t ar = ncclSuccess;
         const ncclResult_t qr = g_nccl.CommGetAsyncError(c->comm, &ar);
@@ -471,7 +469,7 @@ int alloc_tiles(cudarl_ctx* c) {
     CK(cudaMalloc(&c->dtscratch, scratch_cap * sizeof(uint2)));
     tp.scratch = (uint2*)c->dtscratch; tp.scratch_cap = (unsigned)scratch_cap;
     tp.wait_polls = 0;
-    { int sms = 0; CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device)); tp.nq = (unsigned)(sms > 0 ? sms : 1); }
+    tp.nq = p.sms;
     CK(cudaMalloc(&c->dtq, 3 * (size_t)tp.nq * sizeof(unsigned)));
     CK(cudaMemsetAsync(c->dtq, 0, 3 * (size_t)tp.nq * sizeof(unsigned), c->st));
     tp.tq = (unsigned*)c->dtq;
@@ -501,12 +499,10 @@ bool use_gather(const cudarl_ctx* c) {
 int alloc_gather(cudarl_ctx* c) {
     Params& p = c->p; GatherP& gp = p.gp;
     const size_t S = p.S, N = p.N ? p.N : 1;
-    int sms = 0;
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
     CK(cudaMalloc(&c->dgbar, 256)); CK(cudaMemsetAsync(c->dgbar, 0, 256, c->st));
     CK(cudaMalloc(&c->dgmv, S));
     if (!arena_plan(p)) {
-        gp = GatherP{}; gather_plan(p, sms);
+        gp = GatherP{}; gather_plan(p);
         // 32 bytes a cell, twice the table: only for the launches that count in global memory, not for one block's worlds (or none)
         CK(cudaMalloc(&c->dgcnt, 8 * S * sizeof(unsigned))); CK(cudaMemsetAsync(c->dgcnt, 0, 8 * S * sizeof(unsigned), c->st));
         gp.cnt[0] = (unsigned*)c->dgcnt; gp.cnt[1] = gp.cnt[0] + 4 * S;
@@ -791,6 +787,7 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
             CK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
             CK(cudaEventCreateWithFlags(&c->ev_eps, cudaEventDisableTiming));
             CK(cudaEventCreate(&c->ev0)); CK(cudaEventCreate(&c->ev1));
+            { int sms = 0; CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device)); p.sms = (unsigned)std::max(sms, 1); }
             const size_t N = p.N ? p.N : 1;
             { int r0 = alloc_cells(c); if (r0) return r0; }
             for (int cp = 0; cp < 2; ++cp) { CK(cudaMalloc(&c->dstate[cp], N * 16 + 64)); CK(cudaMemsetAsync(c->dstate[cp], 0, N * 16 + 64, c->st)); }

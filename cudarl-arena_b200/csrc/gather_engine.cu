@@ -149,9 +149,9 @@ void launch_gather_moves(const Params& p, cudaStream_t st) {
 // How the population is spread over the launch: one environment per thread in registers while the blocks of one launch hold them all,
 // else streamed from shared memory, or from global memory where that is too small.
 constexpr unsigned SHARED_MOST = 200u * 1024u;
-void gather_plan(Params& p, int sms) {
+void gather_plan(Params& p) {
     GatherP& gp = p.gp;
-    const unsigned n = p.N ? p.N : 1u, s = (unsigned)(sms > 0 ? sms : 1);
+    const unsigned n = p.N ? p.N : 1u, s = p.sms;
     if (n <= 16u * 1024u) {
         gp.cluster = 1u;
         gp.threads = n <= 16u * 256u ? 256u : n <= 16u * 512u ? 512u : 1024u;

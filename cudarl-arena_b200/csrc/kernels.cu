@@ -90,13 +90,11 @@ __device__ __forceinline__ void cswap(unsigned long long& ka, float& va, unsigne
 
 // Fold a sorted run (same cell) starting at index j of keys/vals; returns nothing, writes Q_{t+1}.
 __device__ void apply_run(const Params& p, const unsigned long long* keys, const float* vals, unsigned j, unsigned n) {
-    unsigned w0 = (unsigned)(keys[j] >> 32);
-    unsigned cellp = w0 >> 2;              // (cell << 1) | parity
-    unsigned cell = w0 >> 3;
+    const unsigned cell = (unsigned)(keys[j] >> 34);
     float4 row = __ldcg(p.Q + cell);
     for (; j < n; ++j) {
         unsigned wj = (unsigned)(keys[j] >> 32);
-        if ((wj >> 2) != cellp) break;
+        if ((wj >> 2) != cell) break;
         fold(row, (int)(wj & 3u), p.lr, vals[j]);
     }
     p.Q[cell] = row;          // in place: the targets were taken before this kernel started, and one thread owns the cell
@@ -132,14 +130,11 @@ __device__ void process_medium(const Params& p, unsigned long long* keys, float*
 }
 
 // Collision folding, one thread per ACTIVE mailbox slot (the producers list every slot they were the
-// first to hook a chain into, so this kernel only visits slots that have work).  A slot's chain links
-// RUNS of consecutive entries (one run = the lanes of one warp on one cell).  The owning thread gathers
+// first to hook a chain into, so this kernel only visits slots that have work).  The owning thread gathers
 // the chain's entries:
 //   <= 8 entries   in registers, ordered by a sorting network and folded by that thread;
 //   <= 32 entries  staged in shared memory by that thread, ordered and folded by one warp;
 //   longer         marked, and left to k_fix_long.
-__device__ __forceinline__ void flush_row(const Params& p, unsigned cellpar, const float4& row) { p.Q[cellpar >> 1] = row; }
-
 __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
     __shared__ unsigned long long s_keys[STAGE_ENTRIES];
     __shared__ float s_vals[STAGE_ENTRIES];
@@ -157,18 +152,16 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
     if (head) {
         p.mailbox[slot] = 0u;                          // leave the mailbox empty for the next call
         unsigned long long k8[SHORT_MAX]; float v8[SHORT_MAX];
-        unsigned q = head, pos = 0, rem = 0; bool fresh = false;
+        unsigned q = head;                             // index of the next entry + 1
 #pragma unroll
         for (int j = 0; j < SHORT_MAX; ++j) {
-            if (rem == 0u && q) { pos = (q & LINK_POS_MASK) - 1u; rem = (q >> LINK_POS_BITS) + 1u; fresh = true; }
-            if (rem) {
-                const uint4 e = __ldcg(p.ent + pos);
+            if (q) {
+                const uint4 e = __ldcg(p.ent + (q - 1u));
                 k8[j] = ((unsigned long long)e.x << 32) | e.y; v8[j] = __uint_as_float(e.z);
-                if (fresh) { q = e.w; fresh = false; }
-                ++pos; --rem;
+                q = e.w;
             } else { k8[j] = ~0ull; v8[j] = 0.0f; }
         }
-        if (rem == 0u && q == 0u) {
+        if (q == 0u) {
             cswap(k8[0],v8[0],k8[1],v8[1]); cswap(k8[2],v8[2],k8[3],v8[3]); cswap(k8[4],v8[4],k8[5],v8[5]); cswap(k8[6],v8[6],k8[7],v8[7]);
             cswap(k8[0],v8[0],k8[2],v8[2]); cswap(k8[1],v8[1],k8[3],v8[3]); cswap(k8[4],v8[4],k8[6],v8[6]); cswap(k8[5],v8[5],k8[7],v8[7]);
             cswap(k8[1],v8[1],k8[2],v8[2]); cswap(k8[5],v8[5],k8[6],v8[6]); cswap(k8[0],v8[0],k8[4],v8[4]); cswap(k8[3],v8[3],k8[7],v8[7]);
@@ -176,19 +169,19 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
             cswap(k8[1],v8[1],k8[4],v8[4]); cswap(k8[3],v8[3],k8[6],v8[6]);
             cswap(k8[2],v8[2],k8[4],v8[4]); cswap(k8[3],v8[3],k8[5],v8[5]);
             cswap(k8[3],v8[3],k8[4],v8[4]);
-            unsigned curcp = 0xFFFFFFFFu; float4 row = make_float4(0.f, 0.f, 0.f, 0.f);
+            unsigned cur = 0xFFFFFFFFu; float4 row = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int j = 0; j < SHORT_MAX; ++j) {
                 if (k8[j] != ~0ull) {
-                    const unsigned w0 = (unsigned)(k8[j] >> 32), cp = w0 >> 2;
-                    if (cp != curcp) {
-                        if (curcp != 0xFFFFFFFFu) flush_row(p, curcp, row);
-                        curcp = cp; row = __ldcg(p.Q + (cp >> 1));
+                    const unsigned w0 = (unsigned)(k8[j] >> 32), cell = w0 >> 2;
+                    if (cell != cur) {
+                        if (cur != 0xFFFFFFFFu) p.Q[cur] = row;
+                        cur = cell; row = __ldcg(p.Q + cell);
                     }
                     fold(row, (int)(w0 & 3u), p.lr, v8[j]);
                 }
             }
-            if (curcp != 0xFFFFFFFFu) flush_row(p, curcp, row);
+            if (cur != 0xFFFFFFFFu) p.Q[cur] = row;
         } else {
             const unsigned chunk = atomicAdd(&s_nmed, 1u);
             bool staged = false;
@@ -197,14 +190,12 @@ __global__ void __launch_bounds__(BLOCK) k_fix(Params p) {
 #pragma unroll
                 for (int j = 0; j < SHORT_MAX; ++j) { mk[j] = k8[j]; mv[j] = v8[j]; }
                 unsigned L = SHORT_MAX;
-                while ((rem || q) && L < MED_MAX) {
-                    if (rem == 0u) { pos = (q & LINK_POS_MASK) - 1u; rem = (q >> LINK_POS_BITS) + 1u; fresh = true; }
-                    const uint4 e = __ldcg(p.ent + pos);
+                for (; q && L < MED_MAX; ++L) {
+                    const uint4 e = __ldcg(p.ent + (q - 1u));
                     mk[L] = ((unsigned long long)e.x << 32) | e.y; mv[L] = __uint_as_float(e.z);
-                    if (fresh) { q = e.w; fresh = false; }
-                    ++pos; --rem; ++L;
+                    q = e.w;
                 }
-                staged = (rem == 0u && q == 0u);
+                staged = q == 0u;
                 s_medlen[chunk] = staged ? L : 0u;
             }
             if (!staged) {                              // leave the chain's cells to k_fix_long
@@ -247,7 +238,7 @@ __device__ void fold_crowded(const Params& p, unsigned n, GridBarrier& bar) {
 
     // ---- pick out, in order ----
     share(n, first, last);
-    auto chosen = [&](unsigned i, uint4& e) -> bool { if (i >= last) return false; e = p.ent[i]; return p.mailbox[mb_slot(p, e.x >> 3)] == LONG_MARK; };
+    auto chosen = [&](unsigned i, uint4& e) -> bool { if (i >= last) return false; e = p.ent[i]; return p.mailbox[mb_slot(p, e.x >> 2)] == LONG_MARK; };
     unsigned mine = 0u; uint4 e;
     for (unsigned i = first + tid; i < last; i += SORT_THREADS) if (chosen(i, e)) ++mine;
     block_scan_excl(mine, s_warp, &total);
@@ -260,7 +251,7 @@ __device__ void fold_crowded(const Params& p, unsigned n, GridBarrier& bar) {
     for (unsigned i0 = first; i0 < last; i0 += SORT_THREADS) {
         const bool take = chosen(i0 + tid, e);
         const unsigned at = before + block_scan_excl(take ? 1u : 0u, s_warp, &total);
-        if (take) so.a[at] = make_uint2(((e.x >> 3) << 2) | (e.x & 3u), e.z);
+        if (take) so.a[at] = make_uint2(e.x, e.z);
         before += total;
     }
     if (!bar.pass()) return;
@@ -445,10 +436,10 @@ __global__ void k_update_main(Params p, unsigned n, Transitions tr) {
         unsigned at, next; float r;
         load_transition(tr, i, at, next, r);
         const float d = transition_target(p, at, next, r);
-        const unsigned cell = (at & 0x7FFFFFFFu) >> 2;
-        slot = mb_slot(p, cell);
-        const unsigned prev = atomicExch(p.mailbox + slot, i + 1u);              // a run of one entry
-        p.ent[i] = make_uint4((cell << 3) | (at & 3u), i, __float_as_uint(d), prev);
+        const unsigned own = at & 0x7FFFFFFFu;                                   // cell * 4 + action
+        slot = mb_slot(p, own >> 2);
+        const unsigned prev = atomicExch(p.mailbox + slot, i + 1u);
+        p.ent[i] = make_uint4(own, i, __float_as_uint(d), prev);
         first = prev == 0u;
     }
     const unsigned fm = __ballot_sync(FULL, first);                  // list the slots that just became active

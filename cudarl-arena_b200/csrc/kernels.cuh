@@ -14,11 +14,6 @@ enum : unsigned {
     CW_TRAP = 4u,      // an obstacle whose penalty replaces the step cost of an agent that walks into it (src/kernels.cu:61-63)
 };
 
-// A chain link names a run of consecutive collision entries: low 26 bits = position of the first entry + 1
-// (0 = end of chain), bits 26-30 = run length - 1 (a run never exceeds one warp).
-constexpr unsigned LINK_POS_BITS = 26u;
-constexpr unsigned LINK_POS_MASK = (1u << LINK_POS_BITS) - 1u;
-
 // ---- control block in device memory ------------------------------------------------------------
 struct Ctl {
     unsigned long long episodes, goals, timeouts, conflicts, long_chains;
@@ -36,7 +31,7 @@ struct Ctl {
     float eps_used;                 // epsilon of the most recent step (for the stats call)
 };
 
-enum : unsigned { ERR_SCRATCH_OVERFLOW = 1u, ERR_BAD_STATE = 2u, ERR_CHAIN_CYCLE = 8u, ERR_COPY_TIMEOUT = 32u };   // = CUDARL_DEVERR_* of cudarl.h
+enum : unsigned { ERR_SCRATCH_OVERFLOW = 1u, ERR_BAD_STATE = 2u, ERR_COPY_TIMEOUT = 32u };   // = CUDARL_DEVERR_* of cudarl.h
 
 // ---- results handed to the host without a copy ---------------------------------------------------
 // One per context, at the head of its pinned, mapped stage block.  A word carries 32 bits of a result and, above them, the number of
@@ -133,10 +128,11 @@ struct SortP {
 };
 constexpr size_t SORT_WORDS = 1u + SORT_MOST_BLOCKS + 512u + 512u * (size_t)SORT_MOST_BLOCKS;      // barrier, part, total, hist
 struct Params : World {
-    unsigned policy_keys[20];   // the ten round keys of the policy stream, two words each: operands straight from the constant bank
+    unsigned policy_keys[20];   // the ten round keys of the policy stream, two words each: operands straight from the constant bank (on an 8-byte
+                                // boundary: 4 bytes further a step on 8 x 8 tiles took 302 us instead of 297)
     unsigned policy_pre[4];     // k_tile_step: what its step and the keys alone make of the first two rounds
-    uint4* ent;            // collision entries
-    unsigned ent_cap;      // slots in ent
+    uint4* ent;            // update_batch, by transition: cell * 4 + action, index, target, index + 1 of the next in its chain (0 = end)
+    unsigned sms;          // multiprocessors of the device
     unsigned* mailbox;     // update_batch: chain heads (0 = empty), power-of-two size
     unsigned mb_slots;     // mailbox slots (power of two, multiple of BLOCK)
     unsigned* active;      // list of the mailbox slots that hold a chain in this step (mb_slots entries)
@@ -182,7 +178,7 @@ void launch_tile_step(Params& p, bool trace, cudaStream_t st);
 unsigned tile_cls_stride(unsigned tshift);                         // bytes of one tile's class block
 void launch_tile_border(const Params& p, cudaStream_t st);         // border array of parity p.step & 1 from the table (after any change of the table outside train steps)
 // gather engine (gather_engine.cu)
-void gather_plan(Params& p, int sms);
+void gather_plan(Params& p);
 unsigned gather_barriers(const StepLaunch& l);                      // arrivals per block of a launch
 void launch_gather_export(const Params& p, const int4* work, cudaStream_t st);      // records in any order -> p.st
 void launch_gather_moves(const Params& p, cudaStream_t st);         // cell words -> move bytes

@@ -172,7 +172,7 @@ static cudaError_t launch_tiled(const Params& p, unsigned* hop, unsigned max_ste
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;                      // no walk over words that nobody has written
     // four environments per thread where the chip is full with that
-    const unsigned ept = p.N >= 4u * 8u * BLOCK * 148u ? 4u : 1u;
+    const unsigned ept = p.N >= 4u * 8u * BLOCK * p.sms ? 4u : 1u;
     cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((p.N + ept * BLOCK - 1u) / (ept * BLOCK)); cfg.blockDim = dim3(BLOCK); cfg.stream = st;
     cudaLaunchAttribute at;                              // the walk is set up, and draws its start cells, while the last tiles are folded
@@ -185,7 +185,7 @@ cudaError_t launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, u
     // takes the time) tiles of a quarter of that size are folded by four times as many blocks; beyond, the larger tile saves hops.  Call with 64 /
     // 32: 256^2 cells 24.0 / 20.4 us, 700^2 24.2 / 21.7, 1024^2 38.3 / 37.5, 1500^2 35.0 / 34.3, 2048^2 52.9 / 54.6.
     const unsigned big = (((unsigned)p.W + 63u) / 64u) * (((unsigned)p.H + 63u) / 64u);
-    return big < 4u * 148u ? launch_tiled<5u>(p, hop, max_steps, nonce, h, st) : launch_tiled<6u>(p, hop, max_steps, nonce, h, st);
+    return big < 4u * p.sms ? launch_tiled<5u>(p, hop, max_steps, nonce, h, st) : launch_tiled<6u>(p, hop, max_steps, nonce, h, st);
 }
 
 }  // namespace cudarl
