@@ -32,13 +32,12 @@ constexpr unsigned GRID_ROWS = 32768u;
 constexpr unsigned KIND_LIVE = 0u, KIND_EXIT = 1u << 30, KIND_GOAL = 2u << 30, KIND_MASK = 3u << 30, TRAPPED = 3u << 30, NO_START = 1u << 29, STEPS_MASK = 0x1FFFu;
 
 template <unsigned RT_SHIFT>
-// (32 registers, so that an SM is full: with 38 it held three blocks of 64 x 64 cells instead of four, 4096 x 4096 cells 173 -> 180 us)
+// (32 registers, so that an SM is full: with 38 it held three blocks of 64 x 64 cells instead of four, 4096 x 4096 cells 173 -> 180 us; 171 now)
 __global__ void __launch_bounds__(RT_ROWS << RT_SHIFT, 2048u / (RT_ROWS << RT_SHIFT)) k_rollout_tiles(const __grid_constant__ Params p, unsigned* __restrict__ hop) {
     constexpr unsigned RT = 1u << RT_SHIFT, RT_CELLS = RT * RT, RT_THREADS = RT * RT_ROWS, RT_PER = RT_CELLS / RT_THREADS;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");       // the walk's blocks may take the slots that free up, and draw
     __shared__ unsigned s_w[RT_CELLS];
-    const int x0 = (int)(blockIdx.x << RT_SHIFT), y0 = (int)((blockIdx.z * GRID_ROWS + blockIdx.y) << RT_SHIFT);
-    if (y0 >= p.H) return;
+    const int x0 = (int)(blockIdx.x << RT_SHIFT), y0 = (int)((blockIdx.z * gridDim.y + blockIdx.y) << RT_SHIFT);
     unsigned cur[RT_PER];
     const unsigned lx = threadIdx.x & (RT - 1u), ly0 = threadIdx.x >> RT_SHIFT;          // a thread's cells lie below one another, 8 rows apart
     const int x = x0 + (int)lx;
@@ -167,7 +166,8 @@ template <unsigned RT_SHIFT>
 static cudaError_t launch_tiled(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
     constexpr unsigned RT = 1u << RT_SHIFT;
     const unsigned tiles_x = ((unsigned)p.W + RT - 1u) / RT, tiles_y = ((unsigned)p.H + RT - 1u) / RT;
-    const dim3 tiles(tiles_x, tiles_y < GRID_ROWS ? tiles_y : GRID_ROWS, (tiles_y + GRID_ROWS - 1u) / GRID_ROWS);
+    const unsigned layers = (tiles_y + GRID_ROWS - 1u) / GRID_ROWS;
+    const dim3 tiles(tiles_x, (tiles_y + layers - 1u) / layers, layers);     // (a tile beyond the last row has no cell of the grid in it)
     k_rollout_tiles<RT_SHIFT><<<tiles, RT * RT_ROWS, 0, st>>>(p, hop);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;                      // no walk over words that nobody has written
