@@ -1,12 +1,12 @@
-// arena_engine.cu -- the fused train step for the smallest worlds: the whole world in the shared memory of one block, many steps per
-// launch.
+// arena_engine.cu -- the fused train step for the smallest worlds: the whole world in the shared memory of one block (k_arena_steps), up to 32
+// environments in one warp (k_solo_steps), many steps per launch.
 //
 // A small world is latency, nothing else: in the gather engine (gather_engine.cu) a step is two barriers between blocks and several
 // dependent accesses to L2.  Here the table, the counters and the move bytes lie in shared memory, the environments in registers, and
-// the barrier is the block's.  The step itself is step_loop.cuh.
+// the barrier is the block's.  The step of k_arena_steps is step_loop.cuh; k_solo_steps, further down, has neither counters nor barriers.
 //
-// What bounds it: one block's issue slots, about 300 instructions per warp and step.  B200, us per step, here / gather engine: one
-// environment 0.59 / 3.0, 200 on 20 x 20 cells 1.1 / 4.7, 1,000 on 32 x 32 2.2 / 4.7; 4,096 on 64 x 64 16 / 4.7.  The same spread over
+// What bounds k_arena_steps: one block's issue slots, about 300 instructions per warp and step.  B200, us per step, here / gather engine: 200
+// on 20 x 20 cells 1.1 / 4.7, 1,000 on 32 x 32 2.2 / 4.7; 4,096 on 64 x 64 16 / 4.7.  The same spread over
 // the distributed shared memory of a cluster was no faster than L2 (4,096 on 64 x 64: 4.4 with 16 blocks; scattered 16-byte accesses to
 // other blocks' shared memory are served one by one), nor with a copy of the table in every block (3.9: every update is then stored 8 times).
 #include "step_loop.cuh"
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(AB, 1) k_arena_steps(const __grid_constant__ P
 // on nothing, a chunk of steps ahead.  SHARED: the world in shared memory; else in global memory, where the rows the warp walks over stay in
 // its first-level cache.
 // What bounds it: the chain of dependent instructions of one step, 4 - 5 cycles each (B200, one environment, fixed epsilon: with the counters
-// and barriers of the block's step 0.58 us a step, with the match but the draws in the same warp 0.46).
+// and barriers of the block's step 0.58 us a step, with the match but the draws in the same warp 0.46; as it is 0.36).
 constexpr unsigned SOLO_CHUNK = 32u;
 
 template <bool SHARED, bool PLAIN>

@@ -348,9 +348,9 @@ Handover handover(cudarl_ctx* c) { return Handover{(HostBox*)c->stage.dev, ++c->
 // Arrays in the stage, behind the box.
 constexpr size_t STAGE_DATA = 256;
 // How large a stage: room for the states of all environments and for the table, each up to 4 MB: so far a kernel's own accesses across the
-// link are faster than copies through the ring (B200, states of 131,072 environments 145 -> 65 us, a table of 1 MB 100 -> 59 us, of 4 MB
-// 193 -> 134 us); 64 KB for a single small environment, of which a program may keep many; all 4 MB without environments, where transitions
-// are what comes in (100,000 on 1024 x 1024 cells 109 -> 86 us, 300,000 216 -> 156 us; ring / stage).
+// link are faster than copies through the ring (B200, us a call, ring / stage: states of 131,072 environments 117 / 68, a table of 1 MB 74 / 58,
+// of 3.9 MB 211 / 129); 64 KB for a single small environment, of which a program may keep many; all 4 MB without environments, where
+// transitions are what comes in (100,000 on 1024 x 1024 cells 108 / 82, 300,000 209 / 152).
 size_t stage_bytes(const Params& p) {
     if (p.N == 1u && p.S <= 2048u) return (size_t)64 << 10;
     const size_t most = (size_t)4 << 20, states = STAGE_DATA + 12 * ((size_t)p.N + 16), table = STAGE_DATA + 16 * (size_t)p.S;

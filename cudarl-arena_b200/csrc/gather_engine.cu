@@ -8,11 +8,12 @@
 //
 // A population that fits the threads stays in registers for the whole launch, a larger one is streamed from shared memory (24 bytes an
 // environment), the largest from global memory.  Up to 16,384 environments run in the blocks of one cluster, whose barrier takes 0.28 us
-// where one of the grid takes 1.3 - 1.7.  Large populations are dealt to the blocks by cell every 64 steps (deal_by_cell).
+// where one of the grid takes 1.3 - 2.4.  Large populations are dealt to the blocks by cell every 64 steps (deal_by_cell), whether those are one
+// call or many.
 //
 // What bounds it (B200): small populations, the chain of a step -- two barriers and four dependent accesses to L2 (300 - 500 ns each with
-// the whole GPU at it): 256 x 256 cells with 65,536 environments 5.9 us a step.  Large ones, the rate of atomics on L2: about 117 G per
-// second, 9 of the 24 us that 1,048,576 environments on 1024 x 1024 cells take (packing the counters into 16 or 8 bits changed little:
+// the whole GPU at it): 256 x 256 cells with 65,536 environments 6.0 us a step.  Large ones, the rate of atomics on L2: about 117 G per
+// second, 9 of the 22 us that 1,048,576 environments on 1024 x 1024 cells take (packing the counters into 16 or 8 bits changed little:
 // it is atomics, not sectors).
 //
 // Reference semantics: those of tile_engine.cu.

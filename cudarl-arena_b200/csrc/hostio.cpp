@@ -20,7 +20,7 @@ namespace cudarl {
 namespace {
 
 // A slot is one huge page of the caller's array where that is made of huge pages: each is faulted in by one core.  Twenty slots keep
-// twelve cores and the copy engine busy.  Measured on the B200 box (16 cores, 268 MB into a fresh NumPy array): 56 ms through the
+// twelve cores and the copy engine busy.  Measured on a B200 machine (16 cores, 268 MB into a fresh NumPy array): 56 ms through the
 // driver, 9.6 ms with 8 copying threads, 7.5 with 12; into memory that has been written before 5.6 either way, the speed of the link.
 constexpr size_t SLOT_BYTES = (size_t)2 << 20;
 constexpr size_t CHUNK_MIN = (size_t)64 << 10, PIECE_MIN = (size_t)256 << 10, HOST_CHUNK_MOST = (size_t)128 << 10;
@@ -29,7 +29,10 @@ constexpr size_t TOUCH_MIN = (size_t)4 << 20;
 // Copies within the host between a stage and the caller: shared from a quarter of a megabyte on.
 constexpr size_t HOST_MIN = (size_t)256 << 10, HOST_PIECE = (size_t)32 << 10;
 constexpr int SLOTS = 20, MAX_WORKERS = 11, MAX_DEVICES = 64;
-// Below this the driver copies: it is as fast as the ring up to there (B200 box: 2 MB in 0.12 ms either way, 4 MB 0.23 and 0.16).
+// Below this the driver copies, although a ring that is there is the faster from half a megabyte on (B200 machine, us, ring / driver: in 512 KB 34 / 40,
+// 3 MB 124 / 178, 8 MB 223 / 434; out into memory written before 768 KB 48 / 65, 4 MB 178 / 226, into fresh memory 112 / 362 and 420 / 1,830): a
+// process that only has such transfers is spared the ring's set-up, 3 ms whatever its size (registering takes 0.5 - 4 ms a call), and the stages of
+// the contexts take most of them anyway.
 constexpr size_t SHARED_MIN_OUT = (size_t)768 << 10, SHARED_MIN_IN = (size_t)3 << 20;
 
 // What one core copies at a time; `at`: where it lies in the slot of its piece.
@@ -84,7 +87,7 @@ inline void fault_in(unsigned char* b) {
 }
 
 // Into memory that the device reads next: past the caches.  The device's reads of lines that lie modified in a core's cache run at
-// about 5 GB/s on the B200 box (16 MB took 1.3 ms, 0.45 ms this way).  line_end: the rest of the line that the last
+// about 5 GB/s on a B200 machine (16 MB took 1.3 ms, 0.45 ms this way).  line_end: the rest of the line that the last
 // byte lies in is nobody's and may be written.
 void copy_past_caches(unsigned char* d, const unsigned char* s, size_t n, bool line_end) {
 #if defined(__x86_64__)

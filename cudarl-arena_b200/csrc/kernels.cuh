@@ -36,7 +36,7 @@ enum : unsigned { ERR_SCRATCH_OVERFLOW = 1u, ERR_BAD_STATE = 2u, ERR_COPY_TIMEOU
 // ---- results handed to the host without a copy ---------------------------------------------------
 // One per context, at the head of its pinned, mapped stage block.  A word carries 32 bits of a result and, above them, the number of
 // the call it belongs to: the host waits for each word it needs by its number, so the words need no order among themselves and no
-// fence (launch to seen result 7.3 us on the B200 box, 9.3 with values, fence and flag, 9 - 10 for a copy or a synchronisation of
+// fence (launch to seen result 7.3 us on a B200 machine, 9.3 with values, fence and flag, 9 - 10 for a copy or a synchronisation of
 // the stream).  Word 0 carries Ctl::error and is also the flag behind arrays in the stage, which do take a fence.
 struct HostBox { unsigned long long w[32]; };
 struct Handover { HostBox* box; unsigned ticket; };              // box == nullptr: nothing to hand over

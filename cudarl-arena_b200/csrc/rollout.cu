@@ -11,10 +11,10 @@
 //
 // What bounds it: k_rollout_tiles streams the table once (16 bytes in, 4 out per cell) and looks up one word in shared memory per cell and round,
 // until a round finds no path to end; k_rollout_walk makes a few scattered 4-byte look-ups per environment, one after the other.  B200,
-// 4096 x 4096 cells, 4,194,304 environments, 1000 steps: 97 + 76 us (doubling to the last round 138 us; one environment per thread, start cells
-// looked up in the cell words 89 us); the walk over single cells this replaces took 13.55 ms.  256 x 256 cells, 65,536 environments: the
-// call takes 17.6 us; 24.4 us with 64 x 64 tiles (16 blocks, 8 cells per thread and 3 more rounds than the 64 blocks of 32 x 32) and the walk
-// started after the last fold had ended.
+// 4096 x 4096 cells, 4,194,304 environments, 1000 steps: the call 171 us, of which 95 + 75 (doubling to the last round 138 us; one environment per thread, start cells
+// looked up in the cell words 89 us); the walk over single cells this replaces took 13.6 ms.  256 x 256 cells, 65,536 environments: one call after
+// the other 17.8 us each (a call from Python with its own overhead 21), 24.4 with 64 x 64 tiles (16 blocks, 8 cells per thread and 3 more rounds than the 64 blocks of 32 x 32)
+// and the walk started after the last fold had ended.
 //
 // Reference semantics: src/train.py:262-311 (evaluate), first-max argmax src/q_learning.cu:196-206.
 #include "kernels.cuh"
@@ -182,7 +182,7 @@ static cudaError_t launch_tiled(const Params& p, unsigned* hop, unsigned max_ste
 }
 cudaError_t launch_rollout(const Params& p, unsigned* hop, unsigned max_steps, unsigned long long nonce, Handover h, cudaStream_t st) {
     // A 64 x 64 tile takes 512 threads, four of them fill an SM.  Where they do not fill every SM (the chain of rounds in one block is then what
-    // takes the time) tiles of a quarter of that size are folded by four times as many blocks; beyond, the larger tile saves hops.  Call with 64 /
+    // takes the time) tiles of a quarter of that size are folded by four times as many blocks; beyond, the larger tile saves hops.  A call from Python with 64 /
     // 32: 256^2 cells 24.0 / 20.4 us, 700^2 24.2 / 21.7, 1024^2 38.3 / 37.5, 1500^2 35.0 / 34.3, 2048^2 52.9 / 54.6.
     const unsigned big = (((unsigned)p.W + 63u) / 64u) * (((unsigned)p.H + 63u) / 64u);
     return big < 4u * p.sms ? launch_tiled<5u>(p, hop, max_steps, nonce, h, st) : launch_tiled<6u>(p, hop, max_steps, nonce, h, st);

@@ -24,7 +24,7 @@ def load_package():
 
 
 def pytest_configure(config):
-    config.addinivalue_line("markers", "gpu: needs a CUDA device (run on the B200 box)")
+    config.addinivalue_line("markers", "gpu: needs a CUDA device (run on a B200)")
 
 
 @pytest.fixture(scope="session")
