@@ -11,7 +11,7 @@
 //
 // What bounds it: k_rollout_tiles streams the table once (16 bytes in, 4 out per cell) and looks up one word in shared memory per cell and round,
 // until a round finds no path to end; k_rollout_walk makes a few scattered 4-byte look-ups per environment, one after the other.  B200,
-// 4096 x 4096 cells, 4,194,304 environments, 1000 steps: the call 171 us, of which 95 + 75 (doubling to the last round 138 us; one environment per thread, start cells
+// 4096 x 4096 cells, 4,194,304 environments, 1000 steps: the call 171 us, of which 94 + 74 under ncu (doubling to the last round 138 us; one environment per thread, start cells
 // looked up in the cell words 89 us); the walk over single cells this replaces took 13.6 ms.  256 x 256 cells, 65,536 environments: one call after
 // the other 17.8 us each (a call from Python with its own overhead 21), 24.4 with 64 x 64 tiles (16 blocks, 8 cells per thread and 3 more rounds than the 64 blocks of 32 x 32)
 // and the walk started after the last fold had ended.
