@@ -142,6 +142,13 @@ __device__ __forceinline__ int argmax4(float4 r) {   // first maximum wins
     if (r.w > bv) { bv = r.w; b = 3; }
     return b;
 }
+// The same in two levels instead of three, for where it is part of a chain: the first of a pair unless the second is larger -- or, in the second pair, the first
+// is no number (argmax4 passes over those, except in r.x).
+__device__ __forceinline__ int argmax4_pairs(float4 r) {
+    const bool y = r.y > r.x;
+    const float lo = y ? r.y : r.x, hi = fmaxf(r.z, r.w);
+    return hi > lo ? (r.z == hi ? 2 : 3) : (int)y;
+}
 __device__ __forceinline__ float max4(float4 r) {
     float m = r.x;
     m = r.y > m ? r.y : m; m = r.z > m ? r.z : m; m = r.w > m ? r.w : m;
