@@ -8,8 +8,8 @@
 //
 // A population that fits the threads stays in registers for the whole launch, a larger one is streamed from shared memory (24 bytes an
 // environment), the largest from global memory.  Up to 16,384 environments run in the blocks of one cluster, whose barrier takes 0.28 us
-// where one of the grid takes 1.3 - 2.4.  Large populations are dealt to the blocks by cell every 64 steps (deal_by_cell), whether those are one
-// call or many.
+// where one of the grid takes 1.3 - 2.4 (those that patch_engine.cu takes, only in launches of fewer than 16 steps).  Large populations are dealt to the
+// blocks by cell every 64 steps (deal_by_cell), whether those are one call or many.
 //
 // What bounds it (B200): small populations, the chain of a step -- two barriers and four dependent accesses to L2 (300 - 500 ns each with
 // the whole GPU at it): 256 x 256 cells with 65,536 environments 6.0 us a step.  Large ones, the rate of atomics on L2: about 117 G per
@@ -17,32 +17,10 @@
 // it is atomics, not sectors).
 //
 // Reference semantics: those of tile_engine.cu.
-#include "step_loop.cuh"
-#include "grid_barrier.cuh"
+#include "global_table.cuh"
 #include <cstring>
 
 namespace cudarl {
-
-
-// The table and the counters in global memory.
-struct GlobalTable {
-    static constexpr bool ALONE = false;
-    const Params& p;
-    __device__ __forceinline__ float4 row(unsigned s) const { return p.Q[s]; }
-    __device__ __forceinline__ unsigned moves(unsigned s) const { return __ldg(p.gp.mv + s); }
-    __device__ __forceinline__ unsigned add(unsigned par, unsigned idx, unsigned n) const { return atomicAdd(p.gp.cnt[par] + idx, n); }
-    __device__ __forceinline__ void count(unsigned par, unsigned idx, unsigned n) const { atomicAdd(p.gp.cnt[par] + idx, n); }
-    __device__ __forceinline__ bool note(unsigned par, unsigned idx) const { return (atomicOr(p.gp.cnt[par] + idx, NOTED) & NOTED) != 0u; }
-    __device__ __forceinline__ void clear(unsigned par, unsigned idx) const { p.gp.cnt[par][idx] = 0u; }
-    __device__ __forceinline__ uint4 counts(unsigned par, unsigned s) const { return *reinterpret_cast<const uint4*>(p.gp.cnt[par] + 4u * s); }
-    __device__ __forceinline__ void store(unsigned idx, float v) const { reinterpret_cast<float*>(p.Q)[idx] = v; }
-};
-struct GridSpace : GlobalTable {
-    GridBarrier barrier;
-    __device__ __forceinline__ GridSpace(const Params& q, unsigned base, unsigned* flag) : GlobalTable{q}, barrier{q.gp.barrier, q.ctl, base, flag} {}
-    __device__ __forceinline__ void arrive() { barrier.arrive(); }
-    __device__ __forceinline__ bool wait() { return barrier.wait(); }
-};
 
 // Deal the environments to the blocks by cell: the records of l.in, sorted by lines of eight cells (128 bytes of the table) in the
 // order of 8 x 8 tiles, into l.out.  The lanes of a warp then stand on a few lines instead of on 32: the rows, counters and move
@@ -112,10 +90,6 @@ __global__ void __launch_bounds__(BLOCK) k_gather_export(Params p, const int4* _
 }
 
 // The same with all blocks in one cluster: its barrier takes 0.28 us.
-struct ClusterSpace : GlobalTable {
-    __device__ __forceinline__ void arrive() const { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-    __device__ __forceinline__ bool wait() const { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); return true; }
-};
 template <unsigned CB, bool PLAIN>
 __global__ void __launch_bounds__(CB, 1) k_cluster_steps(const __grid_constant__ Params p, const __grid_constant__ StepLaunch l) {
     __shared__ unsigned s_flag;

@@ -86,6 +86,17 @@ struct GatherP {
     unsigned deal_every;                    // steps between two dealings by cell; 0 = the environments stay in their order
     unsigned cluster, arena;                // all blocks in one cluster; the world in the shared memory of one block
 };
+// ---- patch engine (patch_engine.cu): the world in the shared memory of a cluster's blocks, for launches of many steps ----
+constexpr unsigned PT_BLOCKS = 16u, PT_MOST_ENVS = 12288u, PT_DENSE_ENVS = 10240u, PT_BIN_WEIGHT = 128u;      // 16 for each of a bin's cells
+struct PatchP {
+    unsigned blocks, threads;  // 0 blocks: the world does not fit
+    unsigned shift, bins;      // rows of a band = 1 << shift; bins of eight cells
+    unsigned cells, slots, limit, ghosts;   // most cells, slots, environments and edge values of a patch
+    unsigned w_env, shared;    // weight of an environment; bytes of shared memory
+    unsigned bits, w_rcp;      // cells in the map of start cells (all or none); floor(2^32 / W): umulhi(n, w_rcp) is n / W or one less, for every n < 2^32
+    unsigned *count, *part, *rank, *cut;    // the counting sort: per bin (zero between launches), per block, per environment; first bin of every patch
+    int4* dealt;               // the records sorted by bin
+};
 struct StepLaunch {
     unsigned steps, chunk, barrier_base;
     int eps_mode, trace;
@@ -183,6 +194,9 @@ unsigned gather_barriers(const StepLaunch& l);                      // arrivals 
 void launch_gather_export(const Params& p, const int4* work, cudaStream_t st);      // records in any order -> p.st
 void launch_gather_moves(const Params& p, cudaStream_t st);         // cell words -> move bytes
 cudaError_t launch_gather_steps(const Params& p, const StepLaunch& l, cudaStream_t st);
+// patch engine (patch_engine.cu)
+bool patch_plan(const Params& p, PatchP& pp);                       // false: the world does not fit
+cudaError_t launch_patch_steps(const Params& p, const StepLaunch& l, const PatchP& pp, cudaStream_t st);      // p.st -> p.st (or from l.in)
 // arena engine (arena_engine.cu)
 bool arena_plan(Params& p);                                         // false: the world does not fit
 cudaError_t launch_arena_steps(const Params& p, const StepLaunch& l, cudaStream_t st);

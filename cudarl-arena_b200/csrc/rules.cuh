@@ -103,18 +103,22 @@ __device__ __forceinline__ bool last_to_finish(const World& p) {
 
 // Start cell of an episode.  CENTRE/FIXED: the configured cell (reference: src/environment.cu:9-10).
 // RANDOM: first free non-goal cell among 64 seeded candidates, else the precomputed fallback cell.
-__device__ __forceinline__ unsigned sample_start(const World& p, unsigned gi, unsigned long long nonce, unsigned tag) {
+template <class Closed>
+__device__ __forceinline__ unsigned sample_start_if(const World& p, unsigned gi, unsigned long long nonce, unsigned tag, Closed closed) {
     if (p.start_mode != 2) return p.start_cell;
 #pragma unroll 1            // restarts are rare: keep the inlined copies of this loop small (the step kernel's hot loop must fit the instruction cache)
     for (unsigned k = 0; k < 16; ++k) {
         U4 w = philox4x32_10(gi, k, (unsigned)nonce, (unsigned)(nonce >> 32), p.k0, p.k1 ^ tag);
         unsigned c;
-        c = __umulhi(w.x, p.S); if (!(cw_load(p.cw, c) & (CW_OBST | CW_GOAL))) return c;
-        c = __umulhi(w.y, p.S); if (!(cw_load(p.cw, c) & (CW_OBST | CW_GOAL))) return c;
-        c = __umulhi(w.z, p.S); if (!(cw_load(p.cw, c) & (CW_OBST | CW_GOAL))) return c;
-        c = __umulhi(w.w, p.S); if (!(cw_load(p.cw, c) & (CW_OBST | CW_GOAL))) return c;
+        c = __umulhi(w.x, p.S); if (!closed(c)) return c;
+        c = __umulhi(w.y, p.S); if (!closed(c)) return c;
+        c = __umulhi(w.z, p.S); if (!closed(c)) return c;
+        c = __umulhi(w.w, p.S); if (!closed(c)) return c;
     }
     return p.fallback_start;
+}
+__device__ __forceinline__ unsigned sample_start(const World& p, unsigned gi, unsigned long long nonce, unsigned tag) {
+    return sample_start_if(p, gi, nonce, tag, [&](unsigned c) { return cw_load(p.cw, c) & (CW_OBST | CW_GOAL); });
 }
 
 // Reward of a step that does not end on a goal, for an agent at (x, y) whose action `a` was blocked: the step cost, or -- when

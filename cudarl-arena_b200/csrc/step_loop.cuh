@@ -104,11 +104,11 @@ enum class Home { Registers, Shared, Global };
 // One environment of a block: cell, steps of the episode, number; the (cell, action) owned in this step, its TD target and value.
 constexpr unsigned STATE_BYTES = 24u;
 
-// The steps of one launch, GB threads per block.  A block owns `count` slots of the records in `work` from `first` on: one per thread,
+// The steps of one launch from step `skip` on, GB threads per block.  A block owns `count` slots of the records in `work` from `first` on: one per thread,
 // in registers, or streamed turn by turn from shared (`arrays`: chunk x STATE_BYTES) or global memory (gp.state: N x STATE_BYTES).
 // PLAIN: no traps, no clamp, no trace, epsilon by step -- the options are left out of the code, not skipped in it.
 template <Home HOME, unsigned GB, bool PLAIN, bool OWNERS, class Space>
-__device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, Space& space, int4* __restrict__ work, unsigned char* arrays) {
+__device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, Space& space, int4* __restrict__ work, unsigned char* arrays, unsigned skip = 0u) {
     __shared__ unsigned s_sum[5], s_ep;
     constexpr bool STREAM = HOME != Home::Registers;
     // Without OWNERS, who applies what a crowd has counted: with one turn a step everybody (all at the same time, and the answer to the question who came
@@ -138,7 +138,7 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
         const U4 r = philox4x32_10(p.env_offset + i, 0u, (unsigned)g, (unsigned)(g >> 32), p.policy_keys);
         return make_uint2(r.x, r.y);
     };
-    unsigned long long g = p.step;
+    unsigned long long g = p.step + skip;
     for (unsigned j = tid; j < end; j += GB) {
         if (j >= count) continue;
         const int4 r = work[first + j];
@@ -146,13 +146,14 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
         if (STREAM) { m_pos[j] = make_uint2(s, t); m_id[j] = id; m_own[j] = NOBODY; } else w = draw(id, g);
     }
     EpsilonIndex eps_index(p, l, PLAIN);
+    if (l.eps_mode == 1) eps_index.at += skip;
     float eps = __ldg(p.eps_tab + eps_index.at);
     if (!PLAIN && l.eps_mode == 2 && !Space::ALONE) {       // every block has read the finished episodes before any adds those of the first step
         space.arrive();
         if (!space.wait()) return;
     }
 
-    for (unsigned step = 0; step < l.steps; ++step, ++g) {
+    for (unsigned step = skip; step < l.steps; ++step, ++g) {
         const unsigned par = (unsigned)g & 1u;
         const unsigned thr = !(eps > 0.0f) ? 0u : eps >= 1.0f ? (1u << 24) : (unsigned)ceilf(eps * 16777216.0f);   // explore iff (w0 >> 8) < thr
 

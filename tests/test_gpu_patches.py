@@ -1,0 +1,124 @@
+"""The patch engine of the train step against the oracle: launches of many steps of worlds cut into patches of every shape, and the ways out of it in the
+middle of a launch -- a patch with more environments than slots, more records in a step than the receiver has room for."""
+import os
+
+import numpy as np
+import pytest
+
+from test_gpu_engines import world
+from test_gpu_parity import assert_same, pair
+
+pytestmark = pytest.mark.gpu
+THREADS = min(8, os.cpu_count() or 1)
+
+
+def same_stats(gpu, cpu):
+    a, b = gpu.get_stats(), cpu.get_stats()
+    assert (a.conflicts, a.goals, a.timeouts, a.episodes, a.epsilon, a.device_error) == (b.conflicts, b.goals, b.timeouts, b.episodes, b.epsilon, 0)
+
+
+@pytest.mark.parametrize("w,h,n", [
+    (40, 30, 1100), (64, 64, 4096), (120, 97, 1025),
+    (97, 120, 2048), (97, 120, 2049), (97, 120, 4097), (97, 120, 10240), (97, 120, 10241),       # both sides of 256 and 512 threads; the most environments
+    (160, 161, 12288), (160, 161, 12289),            # on crowded and on other grids, and one more
+    (5000, 1, 33), (1, 5000, 1025), (7, 3000, 6000), (3000, 9, 6000),        # one cell wide, one high: most of a band is empty
+    (3, 2, 5000), (2, 1, 1500),  # fewer bins of cells than blocks: patches without a cell
+    (340, 330, 1500), (420, 400, 1500),              # the map of start cells does not fit; nor the patches: the gather engine
+])
+def test_worlds_cut_into_patches(pkg, orc, w, h, n):
+    cfg = world(pkg, w, h, n, num_goals=1 if w * h < 100 else 3, obstacle_p=0.0 if w * h < 100 else 0.15, max_steps=37, env_offset=3)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    for k in (15, 16, 2, 90):        # one less than the fewest steps of such a launch, the fewest, a launch of the other engine between
+        gpu.set_trace(k != 90)                       # with and without the options
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert_same(gpu, cpu, "+%d" % k)
+        assert k == 90 or all(np.array_equal(a, b) for a, b in zip(gpu.get_trace(), cpu.get_trace()))
+    same_stats(gpu, cpu)
+
+
+@pytest.mark.parametrize("w,h,n", [(91, 93, 3000), (201, 199, 8000)])
+@pytest.mark.parametrize("kw", [{"eps_kind": 2, "eps0": 1.0, "eps_decay": 0.9}, {"eps_kind": 1, "eps0": 1.0, "eps_decay": 0.99},
+                                {"eps_kind": 3, "eps0": 1.0, "eps_end": 0.1, "eps_steps": 60, "legacy_clamp": 1}])
+def test_epsilons_traps_and_clamp(pkg, orc, w, h, n, kw):
+    """The epsilon of a step that follows the episodes all blocks have finished before it; by step, in launches that start anywhere in its table."""
+    cfg = world(pkg, w, h, n, **kw)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    cells = gpu.get_cells()
+    for k in np.flatnonzero(cells == 1)[:60]:
+        gpu.add_trap(int(k % w), int(k // w), -0.3); cpu.add_trap(int(k % w), int(k // w), -0.3)
+    for k in (16, 1, 33, 47):
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert_same(gpu, cpu, "+%d" % k)
+        same_stats(gpu, cpu)
+
+
+def crowd_world(pkg, n, **kw):
+    return world(pkg, 200, 190, n, num_goals=1, obstacle_p=0.0, obstacle_kind=pkg.OBST_NONE, goal_mode=pkg.GOAL_LIST, goals=[(199, 189)], **kw)
+
+
+@pytest.mark.parametrize("n", [3000, 12000])
+@pytest.mark.parametrize("together", [False, True])
+def test_crowds_that_no_patch_holds(pkg, orc, n, together):
+    """Everybody on one cell when a launch begins, or -- the rows lead all of them there -- by its middle; spread out again later."""
+    cfg = crowd_world(pkg, n, max_steps=90, eps0=0.02, lr=0.05)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    y, x = np.mgrid[0:190, 0:200]
+    q = np.zeros((190, 200, 4), np.float32)
+    q[..., 1] = x < 100; q[..., 3] = x > 100             # towards the middle column, along it towards the middle
+    q[..., 2] = (x == 100) & (y < 95); q[..., 0] = (x == 100) & (y >= 95)
+    gpu.set_q(q); cpu.set_q(q)
+    if together:
+        for m in (gpu, cpu):
+            m.set_state(np.full(n, 20, np.int32), np.full(n, 30, np.int32), None)
+    for k in (16, 150, 30):
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert_same(gpu, cpu, "+%d" % k)
+        same_stats(gpu, cpu)
+
+
+@pytest.mark.parametrize("n", [2500, 10000])
+def test_many_cross_at_once(pkg, orc, n):
+    """All environments of a few cells walk abreast: more records in a step than their receiver has room for."""
+    cfg = crowd_world(pkg, n, max_steps=0, eps0=0.0, lr=0.001)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    rng = np.random.RandomState(n)
+    q = np.zeros((190, 200, 4), np.float32); q[..., 1] = 1000.0
+    x, y = rng.randint(0, 8, n).astype(np.int32), (rng.randint(0, 3, n) * 60).astype(np.int32)
+    for m in (gpu, cpu):
+        m.set_q(q); m.set_state(x, y, np.zeros(n, np.int32))
+    for k in (16, 100, 40):
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert_same(gpu, cpu, "+%d" % k)
+    same_stats(gpu, cpu)
+
+
+def test_table_and_states_changed_between_launches(pkg, orc):
+    """Nothing of a launch is left in the next: the table set and updated, states set, cells changed in between."""
+    cfg = world(pkg, 150, 140, 9000, max_steps=60)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    rng = np.random.RandomState(5)
+    for turn in range(4):
+        gpu.train_steps(16); cpu.train_steps(16)
+        assert_same(gpu, cpu, "turn %d" % turn)
+        q = rng.uniform(0, 1, (140, 150, 4)).astype(np.float32)
+        x, y = rng.randint(0, 150, 9000).astype(np.int32), rng.randint(0, 140, 9000).astype(np.int32)
+        b = dict(sx=rng.randint(0, 150, 2000), sy=rng.randint(0, 140, 2000), a=rng.randint(0, 4, 2000), r=np.ones(2000, np.float32),
+                 nx=rng.randint(0, 150, 2000), ny=rng.randint(0, 140, 2000), dn=np.zeros(2000, np.uint8))
+        for m in (gpu, cpu):
+            m.set_q(q); m.set_state(x, y, None); m.update_batch(**b); m.add_obstacle(3 + turn, 4); m.set_goal(100 + turn, 20)
+    gpu.train_steps(30); cpu.train_steps(30)
+    assert_same(gpu, cpu, "last")
+    same_stats(gpu, cpu)
+
+
+def test_a_failed_wait_ends_the_launch(pkg):
+    """With the tests' poll bound a launch records the failure and leaves; every later launch does nothing."""
+    g = pkg.VecGridWorld(world(pkg, 120, 97, 5000))
+    g.train_steps(20); g.synchronize()
+    g.debug_set_copy_wait_polls(1)
+    g.train_steps(20)
+    g.debug_set_copy_wait_polls(0)
+    g.train_steps(20)
+    with pytest.raises(pkg.CudarlError) as ei:
+        g.synchronize()
+    assert ei.value.code == 3000 + 32
