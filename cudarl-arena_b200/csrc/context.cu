@@ -108,7 +108,7 @@ struct cudarl_ctx {
     unsigned since_deal = 0;               // steps since then
     void* dwork[2] = {nullptr, nullptr};
     PatchP patch{};                        // patch engine: launches of many steps of those of the gather engine's worlds that it takes
-    void* dpatch = nullptr;
+    void* dpatch = nullptr; size_t patch_zero = 0; uint32_t patch_epoch = 1;
     uint32_t barrier_base = 0;             // arrivals at the grid barrier by all launches so far
     bool tile_mode = false;               // true: the records live in tile regions (train steps), false: in environment order
     bool cls_dirty = true;                // the per-tile class bytes must be rebuilt from the cell words
@@ -500,11 +500,20 @@ bool use_gather(const cudarl_ctx* c) {
 }
 int alloc_patch(cudarl_ctx* c) {
     PatchP& pp = c->patch;
-    if (!c->p.gp.cluster || !c->p.N || !patch_plan(c->p, pp)) { pp = PatchP{}; return 0; }
-    const size_t N = c->p.N, words = (size_t)pp.bins + pp.blocks + (pp.blocks + 1) + N;
-    CK(cudaMalloc(&c->dpatch, N * sizeof(int4) + words * sizeof(unsigned)));
-    pp.dealt = (int4*)c->dpatch; pp.count = (unsigned*)(pp.dealt + N); pp.part = pp.count + pp.bins; pp.cut = pp.part + pp.blocks; pp.rank = pp.cut + pp.blocks + 1;
-    CK(cudaMemsetAsync(pp.count, 0, (size_t)pp.bins * sizeof(unsigned), c->st));
+    if (c->p.gp.arena || !c->p.N || !patch_plan(c->p, pp)) { pp = PatchP{}; return 0; }
+    const size_t N = c->p.N, G = pp.blocks;
+    size_t off = 0;
+    auto take = [&](size_t bytes) { const size_t at = off; off += (bytes + 255) / 256 * 256; return at; };
+    const size_t count = take(pp.bins * sizeof(unsigned)), barrier = take(pp.grid ? 1024 : 0), listed = take(pp.grid ? 3 * G * 4 : 0),
+                 list = take(pp.grid ? 3 * G * pp.threads * 16 : 0), edge = take(pp.grid ? 2 * (size_t)pp.keys * 8 : 0);
+    c->patch_zero = off;                                 // zero before the first launch: no step has the number 0
+    const size_t part = take(G * 4), cut = take((G + 1) * 4), rank = take(N * 4), dealt = take(N * sizeof(int4));
+    CK(cudaMalloc(&c->dpatch, off));
+    CK(cudaMemsetAsync(c->dpatch, 0, c->patch_zero, c->st));
+    unsigned char* const m = (unsigned char*)c->dpatch;
+    pp.count = (unsigned*)(m + count); pp.barrier = (unsigned*)(m + barrier); pp.listed = (unsigned*)(m + listed);
+    pp.list = (unsigned long long*)(m + list); pp.edge = (unsigned long long*)(m + edge);
+    pp.part = (unsigned*)(m + part); pp.cut = (unsigned*)(m + cut); pp.rank = (unsigned*)(m + rank); pp.dealt = (int4*)(m + dealt);
     return 0;
 }
 int alloc_gather(cudarl_ctx* c) {
@@ -673,9 +682,11 @@ int open_kernel_segment(cudarl_ctx* c) {
     return 0;
 }
 
-// A launch of patches costs 10 us more to begin than one of the gather engine's: 4,096 environments on 64 x 64 cells, 16 steps a call 5.0 us a step without, 4.6 with, 32 a call
-// 4.5 / 3.6.  Cut anew every 1,024 steps (every 256: 1 - 5 % slower).
-constexpr int64_t PATCH_FEWEST = 16, PATCH_MOST = 1024;
+// A launch of patches takes longer to begin than one of the gather engine: 4,096 environments on 64 x 64 cells (a cluster), 16 steps a call 5.0 us a step without, 4.6 with, 32 a
+// call 4.5 / 3.6; 65,536 on 256 x 256 (the whole GPU), 16 a call 7.1 / 7.2.  The population drifts, so they are cut anew: 30,000 on 150 x 150 with one goal every 1,024 steps
+// 5.7, every 256 5.0, but 65,536 on 256 x 256 4.30 / 4.39; in a cluster every 256 is 1 - 5 % slower.
+struct PatchSteps { int64_t fewest, most; };
+inline PatchSteps patch_steps(const PatchP& pp) { return pp.grid ? PatchSteps{32, 512} : PatchSteps{16, 1024}; }
 // n steps in launches of many: up to the next averaging of the replicas, and not so many that a launch keeps the GPU for long or
 // that a block's 32-bit sums could overflow.
 int run_gather(cudarl_ctx* c, int64_t n) {
@@ -684,9 +695,10 @@ int run_gather(cudarl_ctx* c, int64_t n) {
     for (int64_t k = 0; k < n;) {
         int64_t m = std::min(n - k, most);
         if (c->cfg.sync_every > 0 && c->comm) m = std::min<int64_t>(m, c->cfg.sync_every - c->h_step % c->cfg.sync_every);
-        const bool patches = c->patch.blocks && m >= PATCH_FEWEST;
-        if (patches) m = std::min(m, PATCH_MOST);
-        const unsigned deal = c->p.gp.deal_every;
+        const PatchSteps ps = patch_steps(c->patch);
+        const bool patches = c->patch.blocks && m >= ps.fewest;
+        if (patches) m = std::min(m, ps.most);
+        const unsigned deal = patches ? 0u : c->p.gp.deal_every;
         const bool dealing = deal && (c->dealt < 0 || c->since_deal >= deal);
         if (deal) m = std::min<int64_t>(m, dealing ? deal : deal - c->since_deal);
         { int rc = open_kernel_segment(c); if (rc) return rc; }
@@ -696,9 +708,15 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         l.steps = (unsigned)m; l.chunk = c->p.gp.chunk; l.barrier_base = c->barrier_base; l.eps_mode = c->eps_mode; l.trace = c->trace ? 1 : 0; l.eps_len = c->eps_len; l.eps_base_k = c->eps_base_k;
         l.in = c->dealt >= 0 ? (const int4*)c->dwork[c->dealt] : c->p.st;
         l.out = dealing ? (int4*)c->dwork[c->dealt == 0 ? 1 : 0] : const_cast<int4*>(l.in);
-        if (patches) {                                       // (p.st in and out: the worlds it takes are never dealt)
-            l.chunk = (c->p.N + c->patch.blocks - 1u) / c->patch.blocks;
+        if (patches) {                                       // from wherever the records are to the order of the environments
+            if (c->patch_epoch > 0xFFFFFFFFu - 4096u) {      // every number has been used
+                CK(cudaMemsetAsync(c->dpatch, 0, c->patch_zero, c->st));
+                c->patch_epoch = 1;
+            }
+            l.chunk = (c->p.N + c->patch.blocks - 1u) / c->patch.blocks; l.epoch = c->patch_epoch;
+            if (l.chunk > c->patch.threads) l.chunk = (l.chunk + 31u) / 32u * 32u;
             CK(launch_patch_steps(c->p, l, c->patch, c->st));
+            c->patch_epoch += (uint32_t)m + 2u; c->dealt = -1;
         } else {
             CK(c->p.gp.arena ? launch_arena_steps(c->p, l, c->st) : launch_gather_steps(c->p, l, c->st));
             c->barrier_base += c->p.gp.grid * gather_barriers(l);

@@ -8,7 +8,7 @@
 //
 // A population that fits the threads stays in registers for the whole launch, a larger one is streamed from shared memory (24 bytes an
 // environment), the largest from global memory.  Up to 16,384 environments run in the blocks of one cluster, whose barrier takes 0.28 us
-// where one of the grid takes 1.3 - 2.4 (those that patch_engine.cu takes, only in launches of fewer than 16 steps).  Large populations are dealt to the
+// where one of the grid takes 1.3 - 2.4 (patch_engine.cu takes most worlds of up to 110,000, in launches of 16 or 32 steps and more).  Large populations are dealt to the
 // blocks by cell every 64 steps (deal_by_cell), whether those are one call or many.
 //
 // What bounds it (B200): small populations, the chain of a step -- two barriers and four dependent accesses to L2 (300 - 500 ns each with
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_gather_steps(const __grid_consta
     extern __shared__ __align__(16) unsigned char arrays[];
     __shared__ unsigned s_flag;
     if (!may_start(p, &s_flag)) return;
-    GridSpace space(p, l.barrier_base, &s_flag);
+    GridSpace space(p, p.gp.barrier, l.barrier_base, &s_flag);
     if (l.in != l.out && !deal_by_cell<THREADS>(p, l, space)) return;
     run_steps<HOME, THREADS, PLAIN, OWNERS>(p, l, space, l.out, arrays);
 }

@@ -20,7 +20,7 @@ struct GlobalTable {
 };
 struct GridSpace : GlobalTable {
     GridBarrier barrier;
-    __device__ __forceinline__ GridSpace(const Params& q, unsigned base, unsigned* flag) : GlobalTable{q}, barrier{q.gp.barrier, q.ctl, base, flag} {}
+    __device__ __forceinline__ GridSpace(const Params& q, unsigned* counter, unsigned base, unsigned* flag) : GlobalTable{q}, barrier{counter, q.ctl, base, flag} {}
     __device__ __forceinline__ void arrive() { barrier.arrive(); }
     __device__ __forceinline__ bool wait() { return barrier.wait(); }
 };

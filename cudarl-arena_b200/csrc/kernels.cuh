@@ -86,19 +86,24 @@ struct GatherP {
     unsigned deal_every;                    // steps between two dealings by cell; 0 = the environments stay in their order
     unsigned cluster, arena;                // all blocks in one cluster; the world in the shared memory of one block
 };
-// ---- patch engine (patch_engine.cu): the world in the shared memory of a cluster's blocks, for launches of many steps ----
-constexpr unsigned PT_BLOCKS = 16u, PT_MOST_ENVS = 12288u, PT_DENSE_ENVS = 10240u, PT_BIN_WEIGHT = 128u;      // 16 for each of a bin's cells
+// ---- patch engine (patch_engine.cu): the world in the shared memory of several blocks, for launches of many steps ----
+constexpr unsigned PT_MOST_THREADS = 768u, PT_BLOCKS = 16u, PT_MOST_BLOCKS = 256u, PT_MOST_ENVS = 12288u, PT_DENSE_ENVS = 10240u, PT_BIN_WEIGHT = 128u;      // 16 for each of a bin's cells
 struct PatchP {
     unsigned blocks, threads;  // 0 blocks: the world does not fit
-    unsigned shift, bins;      // rows of a band = 1 << shift; bins of eight cells
+    bool grid;                 // on all multiprocessors instead of in a cluster
+    unsigned shift, keys, bins;             // rows of a band = 1 << shift; cells of all bands; bins of eight cells
     unsigned cells, slots, limit, ghosts;   // most cells, slots, environments and edge values of a patch
     unsigned w_env, shared;    // weight of an environment; bytes of shared memory
     unsigned bits, w_rcp;      // cells in the map of start cells (all or none); floor(2^32 / W): umulhi(n, w_rcp) is n / W or one less, for every n < 2^32
     unsigned *count, *part, *rank, *cut;    // the counting sort: per bin (zero between launches), per block, per environment; first bin of every patch
     int4* dealt;               // the records sorted by bin
+    // grid: words under the number of their step
+    unsigned* barrier;         // a barrier of the grid; from word 64 on, two counters 256 bytes apart; zero between launches
+    unsigned* listed;          // 3 x blocks: records in a block's list, by step modulo 3; zero before they are for
+    unsigned long long *list, *edge;        // 3 x blocks x threads records of two words; 2 x keys: max_a Q of the cells along the patches' edges
 };
 struct StepLaunch {
-    unsigned steps, chunk, barrier_base;
+    unsigned steps, chunk, barrier_base, epoch;          // epoch: the number of the first step for the patch engine's words, used once
     int eps_mode, trace;
     unsigned eps_len; unsigned long long eps_base_k;     // eps_mode 2: entries of the table, and the episodes / environments of its first
     const int4* in; int4* out;                           // in != out: deal by cell first

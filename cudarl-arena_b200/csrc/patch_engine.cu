@@ -1,17 +1,22 @@
-// patch_engine.cu -- the fused train step for worlds of a few thousand environments: cut into patches, one per block of a cluster, many steps per launch.
+// patch_engine.cu -- the fused train step for worlds that fit the shared memory of several blocks: cut into patches, one per block, many steps per launch.
 //
 // In the gather engine (gather_engine.cu) the table and the counters of a step lie in L2, and a step is two barriers and four dependent accesses there.
-// Here every block of one cluster owns a patch of the grid and the environments that stand on it: their rows, counters, move bytes and records are
-// in its shared memory.  What blocks have to tell one another in a step they write into one another's shared memory:
+// Here every block owns a patch of the grid and the environments that stand on it: their rows, counters, move bytes and records are in its shared
+// memory.  What blocks have to tell one another in a step is little:
 //
 //   * the environments that walk out of a patch, or whose next episode starts on another, as 8-byte records;
 //   * max_a Q of the cells along the patches' edges, for the TD targets of moves across them.
 //
-// One barrier of the cluster a step, and no access to L2:
-//
 //   look      every environment draws, reads its row, chooses, reads the row it moves to; one that goes gets its place in the receiver's list    (while the barrier is under way)
 //   commit    every environment counts itself, and is put back or sent
 //   apply     the first on a (cell, action) applies its update as often as it was counted; edge values out
+//
+// Up to some 10,000 environments the blocks are one cluster and write into one another's shared memory: one barrier of the cluster a step, and no access to L2.
+//
+// More of them take a patch on every multiprocessor (GRID).  Records and edge values then travel through L2 as 8-byte words that carry the number of the step
+// they are for, and the blocks wait for one another at a counter that orders nothing: when everybody has arrived, what was sent is there or about to be, and
+// a word is read again until its number is right.  That takes 0.85 us, a barrier that publishes the others' writes 1.3, behind 448 atomics and stores of a block 2.3.
+// (Words alone, one from every block, without the counter: 1.8, and with the edge values 8: many warps that read again and again hold up the words themselves.)
 //
 // Cells are numbered by bands: bands of 8 or more rows (a power of two), in a band column by column, in a column downwards.  A patch is a range of
 // that numbering, a place in it is a cell's index in shared memory, and the ranges are cut at the beginning of a launch so that cells and
@@ -22,24 +27,25 @@
 // the rest of the steps runs as in the gather engine, which no crowd can overrun.
 //
 // What bounds it: the chain of one step, thread by thread some 350 instructions at about 6 cycles each (look, commit, apply, edge values), the longest of them in the
-// block next to a goal, where most arrivals and restarts are.  Hence one environment a thread in straight code, a loop only for what is left over (with
-// everything in one loop 3.1 us where it is 2.7 now; 1,024 threads, whose 64 registers spill, 5.3 where 768 take 3.4), residents and arrivals in
-// different warps, an arrival looked at as soon as it is there, and remote atomics whose answer nobody waits for.  B200, us a step, gather engine's cluster / here: 600
-// environments on 32 x 150 cells 3.7 / 1.8, 1,500 on 80 x 80 3.9 / 2.1, 4,096 on 64 x 64 with an untrained table 4.0 / 2.4, after 6,000 steps 4.0 / 2.7,
-// 8,192 on 100 x 100 4.5 / 3.4 and on 250 x 250 4.9 / 3.0, 12,000 on 200 x 200 5.7 / 4.1.
-//
-// (The same with a patch on every multiprocessor, records and edge values as words in L2 that carry the number of their step: 65,536 on 256 x 256 5.7, the gather
-// engine 6.1; 150,001 on 1001 x 613 6.7 / 6.8; 1,048,576 on 1024 x 1024 21 / 22.  Not worth a second engine.)
+// block next to a goal, where most arrivals and restarts are (256 x 256 cells, 65,536 environments: 24 cells with 486 environments, 214 arrivals and 204 restarts a
+// step, half of all blocks have 35 and none).  Hence one environment a thread in straight code, a loop only for what is left over (4,096 on 64 x 64 with
+// everything in one loop 3.1 us, now 2.7; 1,024 threads, whose 64 registers spill, 8,192 on 100 x 100 5.3, 768 take 3.4), residents and arrivals in
+// different warps, an arrival looked at as soon as it is there, and atomics whose answer nobody waits for.  B200, us a step, gather engine / here, with trained
+// tables: in a cluster 600 environments on 32 x 150 cells 3.7 / 1.8, 1,500 on 80 x 80 3.9 / 2.1, 4,096 on 64 x 64 4.0 / 2.7, 8,192 on 100 x 100 4.5 / 3.4 and on 250 x 250
+// 4.9 / 3.0, 12,000 on 200 x 200 5.7 / 4.1; on the whole GPU 3,000 on 350 x 350 3.8 / 2.8, 16,000 on 300 x 300 6.0 / 3.1, 20,000 on 1000 x 900 5.5 / 3.2, 30,000 on
+// 150 x 150 6.3 / 5.4, 65,536 on 256 x 256 6.1 / 4.3, 100,000 on 300 x 290 7.1 / 5.3.
 //
 // Reference semantics: those of tile_engine.cu.
 #include "global_table.cuh"
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 namespace cudarl {
 
 constexpr unsigned AWAY = 0x80000000u;           // a destination on another patch: block << 16 | cell of that patch
 constexpr unsigned NO_CELL = 0xFFFFFFFFu, HOLE = 0xFFFFFFFFu;
+constexpr unsigned PT_AT_ONCE = 256u;            // GRID: arrivals of a step that are fetched before their number is known
 
 // An environment on a patch, 8 bytes: number (26 bits), cell (14), steps of the episode (24).
 __device__ __forceinline__ uint2 patch_rec(unsigned id, unsigned loc, unsigned t) { return make_uint2(id | loc << 26, t << 8 | loc >> 6); }
@@ -56,10 +62,30 @@ __device__ __forceinline__ void put_there(unsigned a, unsigned v) { asm volatile
 __device__ __forceinline__ void put_there(unsigned a, uint2 v) { asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" :: "r"(a), "l"((unsigned long long)v.y << 32 | v.x) : "memory"); }      // in one piece
 __device__ __forceinline__ unsigned add_there(unsigned a, unsigned v) { unsigned o; asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(o) : "r"(a), "r"(v) : "memory"); return o; }
 
+// Across the whole GPU: 32 bits under the number of the step they are for.
+typedef unsigned long long Word;
+__device__ __forceinline__ void send_word(Word* q, unsigned v, unsigned tag) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(q), "l"((Word)v << 32 | tag) : "memory");
+}
+__device__ __forceinline__ Word look_word(const Word* q) { Word v; asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(q) : "memory"); return v; }
+// The word when it has come; false after two seconds.
+__device__ __noinline__ bool wait_word(const Word* q, unsigned tag, unsigned& v) {
+    unsigned long long t0 = 0ull;
+    for (unsigned it = 1u;; ++it) {
+        const Word w = look_word(q);
+        if ((unsigned)w == tag) { v = (unsigned)(w >> 32); return true; }
+        if ((it & 1023u) == 0u) {
+            unsigned long long now; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (t0 == 0ull) t0 = now;
+            else if (now - t0 > GRID_WAIT_NS) return false;
+        }
+    }
+}
+
 // What the patches of a launch are cut from: records sorted by cell number / 8 into pp.dealt, cut[] = the first such bin of each block's patch,
 // s_first[] = the first record of it.  A counting sort, as in the gather engine.
-template <unsigned THREADS>
-__device__ void cut_patches(const Params& p, const StepLaunch& l, const PatchP& pp, ClusterSpace& space, unsigned* s_cut, unsigned* s_first) {
+template <unsigned THREADS, class Space>
+__device__ bool cut_patches(const Params& p, const StepLaunch& l, const PatchP& pp, Space& space, unsigned* s_cut, unsigned* s_first) {
     __shared__ unsigned s_warp[33], s_sum;
     const unsigned tid = threadIdx.x, lane = tid & 31u, G = gridDim.x, b = blockIdx.x;
     const unsigned share = (p.N + G - 1u) / G, first = min(b * share, p.N), last = min(first + share, p.N);
@@ -68,7 +94,7 @@ __device__ void cut_patches(const Params& p, const StepLaunch& l, const PatchP& 
         return (((((unsigned)r.y >> pp.shift) * (unsigned)p.W + (unsigned)r.x) << pp.shift) | ((unsigned)r.y & ((1u << pp.shift) - 1u))) >> 3;
     };
     for (unsigned i = first + tid; i < last; i += THREADS) pp.rank[i] = atomicAdd(pp.count + bin(l.in[i]), 1u);
-    space.arrive(); space.wait();
+    space.arrive(); if (!space.wait()) return false;
     unsigned sum = 0u;
     for (unsigned k = b0 + tid; k < b1; k += THREADS) sum += pp.count[k];
     if (tid == 0u) s_sum = 0u;
@@ -77,9 +103,10 @@ __device__ void cut_patches(const Params& p, const StepLaunch& l, const PatchP& 
     if (lane == 0u && sum) atomicAdd(&s_sum, sum);
     __syncthreads();
     if (tid == 0u) pp.part[b] = s_sum;
-    space.arrive(); space.wait();
+    space.arrive(); if (!space.wait()) return false;
     unsigned carry = 0u;
-    for (unsigned k = 0; k < b; ++k) carry += pp.part[k];
+    for (unsigned k = tid; k < b; k += THREADS) carry += pp.part[k];
+    block_scan_excl(carry, s_warp, &carry);
     // patch j starts behind the bin in which the weight of all before it passes j parts of G
     const unsigned long long weight = (unsigned long long)pp.w_env * p.N + (unsigned long long)PT_BIN_WEIGHT * pp.bins;
 #pragma unroll 1
@@ -101,11 +128,12 @@ __device__ void cut_patches(const Params& p, const StepLaunch& l, const PatchP& 
         carry += total;
     }
     if (b == 0u && tid == 0u) { pp.cut[0] = 0u; pp.cut[G] = pp.bins; }
-    space.arrive(); space.wait();
+    space.arrive(); if (!space.wait()) return false;
     for (unsigned i = first + tid; i < last; i += THREADS) { const int4 r = l.in[i]; pp.dealt[pp.count[bin(r)] + pp.rank[i]] = r; }
     for (unsigned j = tid; j <= G; j += THREADS) { const unsigned c = pp.cut[j]; s_cut[j] = c; s_first[j] = c < pp.bins ? pp.count[c] : p.N; }
-    space.arrive(); space.wait();
+    space.arrive(); if (!space.wait()) return false;
     for (unsigned k = b0 + tid; k < b1; k += THREADS) pp.count[k] = 0u;
+    return true;
 }
 
 // What an environment finds out before it is counted.
@@ -115,29 +143,33 @@ struct Look {
 };
 constexpr unsigned OVER = 0x100u;                // in mv: the episode ends
 
-template <unsigned THREADS, bool PLAIN>
+// GRID: a patch on every multiprocessor, else in a cluster.
+template <unsigned THREADS, bool PLAIN, bool GRID>
 __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constant__ Params p, const __grid_constant__ StepLaunch l, const __grid_constant__ PatchP pp) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ unsigned s_cut[PT_BLOCKS + 1u], s_first[PT_BLOCKS + 1u], s_sum[5], s_flag;
+    constexpr unsigned BLOCKS = GRID ? PT_MOST_BLOCKS : PT_BLOCKS;
+    __shared__ unsigned s_cut[BLOCKS + 1u], s_first[BLOCKS + 1u], s_sum[5], s_flag, s_in;
+    __shared__ Word s_word;                                        // GRID: the counter as everybody has arrived
     __shared__ unsigned s_mailed[3], s_stop[2], s_news[2][PT_BLOCKS];      // written by the other blocks: records sent here (by step modulo 3), whether a block stops, episodes each has ended (by parity)
     __shared__ unsigned s_taken, s_holes, s_full, s_over, s_edges;   // this step: slots given to arrivals, slots left, a record without room, episodes that ended here; edge values owed
     const bool may = may_start(p, &s_flag);                         // (the same for every block: nothing sets the error word while the cluster runs)
     const unsigned tid = threadIdx.x, b = blockIdx.x, G = gridDim.x, W = (unsigned)p.W;
     const unsigned LB = pp.shift, B = 1u << LB, BM = B - 1u, band = W << LB;
-    ClusterSpace space{p};
+    using Space = std::conditional_t<GRID, GridSpace, ClusterSpace>;
+    Space space = [&]() -> Space { if constexpr (GRID) return GridSpace(p, pp.barrier, 0u, &s_flag); else return ClusterSpace{p}; }();
     if (tid < 5u) s_sum[tid] = 0u;
     if (tid < 3u) s_mailed[tid] = 0u;
     if (tid < 2u) s_stop[tid] = 0u;
     if (tid < 2u * PT_BLOCKS) (&s_news[0][0])[tid] = 0u;
     if (tid == 0u) s_taken = s_holes = s_full = s_over = s_edges = 0u;
     if (!may) return;
-    cut_patches<THREADS>(p, l, pp, space, s_cut, s_first);
+    if (!cut_patches<THREADS>(p, l, pp, space, s_cut, s_first)) return;
 
     // ---- the patch into shared memory ----
     float4* const rows = reinterpret_cast<float4*>(smem);
     uint2* const counts = reinterpret_cast<uint2*>(rows + pp.cells);                 // four 16-bit counters a cell
     uint2* const mail = counts + pp.cells;                                           // three lists of arrivals, by step modulo 3; HOLE: not come yet
-    uint2* const rec = mail + 3u * THREADS;                                          // slots
+    uint2* const rec = mail + (GRID ? 0u : 3u * THREADS);                                          // slots
     uint2* const owned = rec + pp.slots;                                             // per slot and then per arrival: the (cell, action) it applies and the target
     unsigned* const from = reinterpret_cast<unsigned*>(owned + pp.slots + THREADS);  // per edge value: block << 16 | cell of that block, or NO_CELL
     float* const ghost = reinterpret_cast<float*>(from + pp.ghosts);                 // the edge values, twice, by parity of the step
@@ -180,7 +212,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
             return a == 0u ? 2u * B + u : a == 1u ? 2u * B + loc - cells : a == 2u ? gdown + u : loc;
         };
         for (unsigned k = tid; k < nghost; k += THREADS) from[k] = NO_CELL;
-        for (unsigned k = tid; k < 3u * THREADS; k += THREADS) mail[k] = make_uint2(0u, HOLE);
+        if (!GRID) for (unsigned k = tid; k < 3u * THREADS; k += THREADS) mail[k] = make_uint2(0u, HOLE);
 #pragma unroll 1
         for (unsigned c0 = tid & ~31u; c0 < pp.bits; c0 += THREADS) {
             const unsigned c = c0 + (tid & 31u), w = __ballot_sync(FULL, c < pp.bits && (cw_load(p.cw, c) & (CW_OBST | CW_GOAL)));
@@ -194,25 +226,37 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
             if (y >= (unsigned)p.H) { rows[k] = make_float4(0.f, 0.f, 0.f, 0.f); moves[k] = 0x0Fu; continue; }       // below the last band's last row
             const unsigned s = y * W + x;
             rows[k] = p.Q[s]; moves[k] = __ldg(p.gp.mv + s);
+            bool outside = false;
             for (unsigned a = 0; a < 4u; ++a) {
                 const bool there = a == 0u ? y > 0u : a == 1u ? x + 1u < W : a == 2u ? y + 1u < (unsigned)p.H : x > 0u;
                 const unsigned n = moved(k, a);
                 if (!there || n < cells) continue;
                 const unsigned g = ghost_of(k, a), f = place(k0 + n) & ~AWAY;
-                from[g] = f;                                       // and its block is told that the value is wanted here
-                put_there(at_block(edge + add_there(at_block(&s_edges, f >> 16), 1u), f >> 16), (f & 0x3FFFu) | b << 14 | g << 18);
+                from[g] = f;
+                outside = true;
+                if constexpr (!GRID) put_there(at_block(edge + add_there(at_block(&s_edges, f >> 16), 1u), f >> 16), (f & 0x3FFFu) | b << 14 | g << 18);     // its block is told that the value is wanted here
             }
+            if (GRID && outside) edge[atomicAdd(&s_edges, 1u)] = k;
         }
         unsigned hi = s_first[b + 1u] - s_first[b], head = 0u, free_slots = 0u;     // slots in use, the ring of holes among them
         for (unsigned j = tid; j < hi; j += THREADS) {
             const int4 r = pp.dealt[s_first[b] + j];
             rec[j] = patch_rec((unsigned)r.w, key_of((unsigned)r.x, (unsigned)r.y) - k0, (unsigned)r.z);
         }
-        space.arrive(); space.wait();
+        if constexpr (GRID) __syncthreads(); else { space.arrive(); space.wait(); }
         const unsigned edges = s_edges;
+        unsigned tag = l.epoch;                                    // GRID: the number of the step
+        auto ghost_word = [&](unsigned k) -> const Word* { const unsigned f = from[k]; return f == NO_CELL ? nullptr : pp.edge + (s_cut[f >> 16] << 3) + (f & 0xFFFFu); };
+        const Word* const my_ghost = GRID && tid < nghost ? ghost_word(tid) : nullptr;
         const unsigned my_edge = tid < edges ? edge[tid] : 0u;     // the first of them: where it goes does not change
-        const unsigned my_edge_at = tid < edges ? at_block(ghost + (my_edge >> 18), (my_edge >> 14) & 15u) : 0u;
+        const unsigned my_edge_at = !GRID && tid < edges ? at_block(ghost + (my_edge >> 18), (my_edge >> 14) & 15u) : 0u;
         auto edges_out = [&](unsigned par) {
+            if constexpr (GRID) {
+                Word* const m = pp.edge + (size_t)par * pp.keys + k0;
+#pragma unroll 1
+                for (unsigned k = tid; k < edges; k += THREADS) { const unsigned c = edge[k]; send_word(m + c, __float_as_uint(max4(rows[c])), tag); }
+                return;
+            }
             if (tid < edges) put_there(my_edge_at + par * pp.ghosts * 4u, __float_as_uint(max4(rows[my_edge & 0x3FFFu])));
 #pragma unroll 1
             for (unsigned k = tid + THREADS; k < edges; k += THREADS) {
@@ -220,18 +264,24 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
                 put_there(at_block(ghost + par * pp.ghosts + (e >> 18), (e >> 14) & 15u), __float_as_uint(max4(rows[e & 0x3FFFu])));
             }
         };
+        // GRID: the blocks wait for one another at a counter that orders nothing; what was sent is there then or about to be, and is read again until its number is right.
+        Word* const counter = reinterpret_cast<Word*>(pp.barrier) + 32u;      // two, by the parity of the step; arrivals, from bit 24 on the episodes that ended, from bit 56 on blocks that stop
+        auto arrive = [&](unsigned par, Word news) {
+            if constexpr (GRID) { if (tid == THREADS - 1u) asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" :: "l"(counter + 32u * par), "l"(1ull + news) : "memory"); }
+            else { __syncwarp(); space.arrive(); }
+        };
         edges_out(0u);
-        space.arrive();
+        arrive(0u, 0ull);
         const unsigned tmax = p.max_steps > 0 ? (unsigned)p.max_steps : 0x7FFFFFFFu;
         const bool early = PLAIN || l.eps_mode != 2;               // the epsilon of a step is known before the others have arrived
         unsigned long long g = p.step;
-        unsigned ended = 0u;                                       // episodes finished in this launch, by all
+        unsigned ended = 0u;                                       // episodes finished in this launch, by all (GRID: in the steps of the other parity)
         const unsigned i = THREADS - 1u - tid;                     // the arrival this thread takes: those that have least to do take the first
         auto leave = [&](unsigned j) { unsigned at = head + free_slots + atomicAdd(&s_holes, 1u); if (at >= pp.slots) at -= pp.slots; if (at >= pp.slots) at -= pp.slots; holes[at] = (unsigned short)j; };
         uint2 arr;                                                 // the arrival, as it came
 
         unsigned turn = 0u;                                        // the step modulo 3
-        for (bool over = false; !over; ++step, ++g, turn = turn == 2u ? 0u : turn + 1u) {
+        for (bool over = false; !over; ++step, ++g, ++tag, turn = turn == 2u ? 0u : turn + 1u) {
             const unsigned par = step & 1u, next = par ^ 1u;
             uint2* const here = mail + turn * THREADS;             // this step's arrivals
             const unsigned there = turn == 2u ? 0u : turn + 1u;    // the list of the next step's
@@ -257,7 +307,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
                     const unsigned s = sample_start_if(p, p.env_offset + id, g + 1ull, TAG_START, [&](unsigned c) { return pp.bits ? closed[c >> 5] >> (c & 31u) & 1u : cw_load(p.cw, c) & (CW_OBST | CW_GOAL); }), y = over_w(s);
                     o.dest = place(key_of(s - y * W, y)); o.t = 0u; o.mv |= OVER;
                 }
-                if (o.dest & AWAY) o.at = add_there(at_block(s_mailed + there, (o.dest >> 16) & 15u), 1u);      // (the answer is not waited for here)
+                if (o.dest & AWAY) {                               // (the answer is not waited for here)
+                    if constexpr (GRID) o.at = atomicAdd(pp.listed + there * G + (o.dest >> 16 & 0xFFu), 1u);
+                    else o.at = add_there(at_block(s_mailed + there, (o.dest >> 16) & 15u), 1u);
+                }
             };
             // Counts the environment; what it applies, and whether its slot j is free.
             auto commit = [&](const Look& o, bool arrival, unsigned j, bool& left) -> uint2 {
@@ -276,9 +329,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
                 const uint2 now = patch_rec(o.id, o.dest & 0xFFFFu, o.t);
                 left = false;
                 if (o.dest & AWAY) {
-                    const unsigned d = (o.dest >> 16) & 15u;
-                    if (o.at < THREADS) put_there(at_block(mail + there * THREADS + o.at, d), now);
-                    else {                                         // no room: everybody stops after this step, and this is where it stands then
+                    const unsigned d = (o.dest >> 16) & 0xFFu;
+                    if (o.at < THREADS) {
+                        if constexpr (GRID) {
+                            Word* const q = pp.list + (((size_t)there * G + d) * THREADS + o.at) * 2u;
+                            asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" :: "l"(q), "l"((Word)now.x << 32 | (tag + 1u)), "l"((Word)now.y << 32 | (tag + 1u)) : "memory");
+                        } else put_there(at_block(mail + there * THREADS + o.at, d), now);
+                    } else {                                         // no room: everybody stops after this step, and this is where it stands then
                         unsigned x, y; cell_of((s_cut[d] << 3) + rec_loc(now), x, y);
                         p.st[o.id] = make_int4((int)x, (int)y, (int)o.t, (int)o.id);
                         s_full = 1u;
@@ -309,26 +366,87 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
             // Looked at while the barrier is under way.  (Should everybody stop before this step, it is still where it was.)
             const bool resident = tid < hi;
             uint2 r = make_uint2(0u, HOLE);
+            const Word* const post = pp.list + (((size_t)turn * G + b) * THREADS + i) * 2u;       // GRID: this thread's place in the list
+            auto delivered = [&](uint2& q) -> bool {
+                Word u, v;
+                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(u), "=l"(v) : "l"(post) : "memory");
+                if ((unsigned)u != tag || (unsigned)v != tag) return false;
+                q = make_uint2((unsigned)(u >> 32), (unsigned)(v >> 32));
+                return true;
+            };
             if (early && !last) {
                 if (resident) r = rec[tid];
+                else if constexpr (GRID) { if (i < PT_AT_ONCE && !delivered(r)) r.y = HOLE; }
                 else { const unsigned long long v = *reinterpret_cast<volatile unsigned long long*>(here + i); r = make_uint2((unsigned)v, (unsigned)(v >> 32)); }
             }
             Look first;
             const bool act = r.y != HOLE;
             if (act) look(r, first);
-            __syncwarp();
-            space.wait();
-            if (tid == 0u) s_taken = s_holes = 0u;                 // (the last step's were read before the barrier; nobody adds before the next __syncthreads)
-            const unsigned arrived = min(s_mailed[turn], THREADS);
-            arr = i < arrived ? here[i] : make_uint2(0u, HOLE);
-            over = last || s_stop[par] != 0u;
+            unsigned arrived;
+            Word news = 0ull;
+            if constexpr (GRID) {
+                unsigned listed = 0u;
+                bool ok = true, have = false;
+                if (my_ghost) {                                    // perhaps it is here already
+                    const Word w = look_word(my_ghost + (size_t)par * pp.keys);
+                    have = (unsigned)w == tag;
+                    if (have) ghost[par * pp.ghosts + tid] = __uint_as_float((unsigned)(w >> 32));
+                }
+                if (i == 0u) {
+                    const unsigned target = (step / 2u + 1u) * G;
+                    unsigned long long t0 = 0ull;
+                    Word w;
+                    for (unsigned it = 1u;; ++it) {
+                        w = look_word(counter + 32u * par);
+                        if (((unsigned)w & 0xFFFFFFu) >= target) break;
+                        if ((it & 1023u) == 0u) {
+                            unsigned long long now; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+                            if (t0 == 0ull) t0 = now;
+                            else if (now - t0 > GRID_WAIT_NS) { atomicOr(&p.ctl->error, ERR_COPY_TIMEOUT); w = ~0ull; break; }
+                        }
+                    }
+                    s_word = w;
+                }
+                __syncthreads();
+                news = s_word;
+                if (news == ~0ull) return;
+                if (i == PT_AT_ONCE) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(listed) : "l"(pp.listed + turn * G + b) : "memory");
+                bool came = act && !resident;                      // this thread's arrival
+                if (came) arr = r;
+                else if (i < PT_AT_ONCE) came = delivered(arr);
+                for (unsigned k = tid; k < nghost; k += THREADS) {
+                    const Word* const q = k == tid ? my_ghost : ghost_word(k);
+                    unsigned v = 0u;
+                    if (!q || (k == tid && have)) continue;
+                    const Word w = look_word(q + (size_t)par * pp.keys);
+                    if ((unsigned)w == tag) v = (unsigned)(w >> 32); else ok = ok && wait_word(q + (size_t)par * pp.keys, tag, v);
+                    ghost[par * pp.ghosts + k] = __uint_as_float(v);
+                }
+                if (i == PT_AT_ONCE) { s_in = listed; }
+                if (tid == 0u) s_taken = s_holes = 0u;
+                __syncthreads();
+                if (i == PT_AT_ONCE && atomicExch(pp.listed + turn * G + b, 0u) == NOBODY) ok = false;      // (its answer is waited for: it is done before anybody adds for the step after the next but one)
+                arrived = min(s_in, THREADS);
+                if (i >= arrived) arr = make_uint2(0u, HOLE);
+                else if (!came) { unsigned u = 0u, v = HOLE; ok = ok && wait_word(post, tag, u) && wait_word(post + 1, tag, v); arr = make_uint2(u, v); }
+                if (!ok) { atomicOr(&p.ctl->error, ERR_COPY_TIMEOUT); s_full = 1u; }       // (what was to come never came: the launch ends for all)
+            } else {
+                __syncwarp();
+                space.wait();
+                if (tid == 0u) s_taken = s_holes = 0u;             // (the last step's were read before the barrier; nobody adds before the next __syncthreads)
+                arrived = min(s_mailed[turn], THREADS);
+                arr = i < arrived ? here[i] : make_uint2(0u, HOLE);
+            }
+            over = last || (GRID ? (news >> 56) != 0ull : s_stop[par] != 0u);
             if (!PLAIN && l.eps_mode == 2 && step) {
-                for (unsigned k = 0; k < G; ++k) ended += s_news[par][k];
-                eps_index.next(p, l, PLAIN, ended, true);
+                unsigned all;
+                if constexpr (GRID) { const unsigned sum = (unsigned)(news >> 24); all = sum + ended; ended = sum; }      // the sums of the steps of both parities
+                else { for (unsigned k = 0; k < G; ++k) ended += s_news[par][k]; all = ended; }
+                eps_index.next(p, l, PLAIN, all, true);
                 if (!over) { eps = __ldg(p.eps_tab + eps_index.at); thr = !(eps > 0.0f) ? 0u : eps >= 1.0f ? (1u << 24) : (unsigned)ceilf(eps * 16777216.0f); }
             }
             if (over) break;
-            __syncthreads();
+            if constexpr (!GRID) __syncthreads();
             uint2 duty = make_uint2(NOBODY, 0u);
             bool left = false;
             if (act) duty = commit(first, !resident, tid, left);
@@ -364,21 +482,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
             }
             if (mine.y != HOLE) rec[slot] = mine;
             if (left) leave(tid);
-            if (tid < G) {
+            if (!GRID && tid < G) {
                 if (s_full != 0u || new_hi > pp.limit) put_there(at_block(s_stop + next, tid), 1u);
                 if (!PLAIN && l.eps_mode == 2) put_there(at_block(&s_news[next][b], tid), s_over);
             }
             __syncthreads();
+            ++tag;
             edges_out(next);
+            --tag;
+            if constexpr (GRID) arrive(next, ((Word)s_over << 24) + (s_full != 0u || new_hi > pp.limit ? 1ull << 56 : 0ull));
             for (unsigned k = tid; k < cells / 2u; k += THREADS) reinterpret_cast<uint4*>(counts)[k] = make_uint4(0u, 0u, 0u, 0u);
-            if (tid == 0u) { s_mailed[turn] = 0u; s_over = 0u; }   // (the next to add to this list do so after the barrier)
-            if (i < arrived) here[i].y = HOLE;
+            if constexpr (!GRID) {
+                if (tid == 0u) { s_mailed[turn] = 0u; s_over = 0u; }       // (the next to add to this list do so after the barrier)
+                if (i < arrived) here[i].y = HOLE;
+            }
             const unsigned used = min(taken, free_slots);
             head += used; if (head >= pp.slots) head -= pp.slots;
             free_slots += s_holes - used;
             hi = new_hi;
-            __syncwarp();
-            space.arrive();
+            if constexpr (GRID) { __syncwarp(); if (i == 0u) s_over = 0u; } else arrive(0u, 0ull);
             if (l.eps_mode == 1) { ++eps_index.at; if (step + 1u < l.steps) eps = __ldg(p.eps_tab + eps_index.at); }
         }
         {                                                          // back to environment order
@@ -397,32 +519,35 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
         }
         add_tallies(p, l, tally, s_sum, true, eps);
     }
-    space.arrive(); space.wait();                                  // (nobody leaves while others may still write into its shared memory)
+    if constexpr (!GRID) { space.arrive(); space.wait(); }         // (nobody leaves while others may still write into its shared memory)
     if (step < l.steps) {                                          // the same for every block
         int4* const work = fits ? p.st : pp.dealt;
-        run_steps<Home::Registers, THREADS, PLAIN, true>(p, l, space, work, nullptr, step);
+        if constexpr (GRID) {
+            space.arrive(); if (!space.wait()) return;
+            if (tid < 3u) pp.listed[tid * G + b] = 0u;             // what was listed for the step that nobody took
+            if (l.chunk <= THREADS) run_steps<Home::Registers, THREADS, PLAIN, false>(p, l, space, work, nullptr, step);
+            else                    run_steps<Home::Shared, THREADS, PLAIN, false>(p, l, space, work, smem, step);
+        } else run_steps<Home::Registers, THREADS, PLAIN, true>(p, l, space, work, nullptr, step);
         if (!fits) {
             __syncthreads();
             const unsigned first = b * l.chunk, n = first < p.N ? min(l.chunk, p.N - first) : 0u;
-            if (tid < n) { const int4 r = work[first + tid]; p.st[r.w] = r; }
+            for (unsigned k = tid; k < n; k += THREADS) { const int4 r = work[first + k]; p.st[r.w] = r; }
         }
     }
+    if (GRID && last_to_finish<false>(p)) { pp.barrier[0] = 0u; pp.barrier[64] = pp.barrier[65] = pp.barrier[128] = pp.barrier[129] = 0u; }
 }
 
 // ------------------------------------------------------------------------------------------------
 constexpr size_t PT_SHARED = 218u * 1024u;       // dynamic shared memory of a block: 227 KB less the static words here and in step_loop.cuh
 static size_t patch_shared(const PatchP& pp) {
-    return 25 * (size_t)pp.cells + 18 * (size_t)pp.slots + 32 * (size_t)pp.threads + 16 * (size_t)pp.ghosts + (size_t)(pp.bits + 31u) / 32u * 4u + 16;
+    return 25 * (size_t)pp.cells + 18 * (size_t)pp.slots + (pp.grid ? 8u : 32u) * (size_t)pp.threads + 16 * (size_t)pp.ghosts + (size_t)(pp.bits + 31u) / 32u * 4u + 16;
 }
-// Whether the patches of a world fit the blocks' shared memory, and how it is shared out.  Not where episodes start on one cell, and everybody passes through one
-// patch: 12,000 on 200 x 190 cells 3.9 / 5.2 (us a step, gather engine's cluster / here).  Up to one environment a thread, and on crowded grids threads left for
-// the arrivals: 12,000 on 200 x 200 5.7 / 4.1, on 100 x 100 5.2 / 5.3, 10,000 there 5.2 / 4.6; 16,384 on 128 x 128 5.3 / 5.7.
-bool patch_plan(const Params& p, PatchP& pp) {
+// Whether the patches of a world fit the blocks' shared memory, and how it is shared out.
+static bool plan(const Params& p, PatchP& pp, bool grid) {
     pp = PatchP{};
     const size_t S = p.S, N = p.N;
-    if (N > PT_MOST_ENVS || (N > PT_DENSE_ENVS && S < 2 * N) || p.start_mode != 2) return false;
-    const unsigned G = (unsigned)std::min<size_t>(PT_BLOCKS, std::max<size_t>(1, (std::max(S, N) + 63) / 64));
-    pp.blocks = G;
+    const unsigned G = grid ? std::min(p.sms, PT_MOST_BLOCKS) : (unsigned)std::min<size_t>(PT_BLOCKS, std::max<size_t>(1, (std::max(S, N) + 63) / 64));
+    pp.grid = grid;
     unsigned sh = 3u;
     while (sh < 7u && ((size_t)2 << (2u * sh)) <= S / G) ++sh;       // bands about as high as a patch is wide
     while (sh > 3u && (((size_t)p.H + (1u << sh) - 1u) >> sh << sh) * 8u > (size_t)p.H * 9u) --sh;      // (and no more than an eighth of the last one empty)
@@ -430,11 +555,13 @@ bool patch_plan(const Params& p, PatchP& pp) {
     pp.w_rcp = p.W > 1 ? (unsigned)((1ull << 32) / (unsigned)p.W) : 0xFFFFFFFFu;
     const size_t keys = ((((size_t)p.H + (1u << sh) - 1u) >> sh) << sh) * (size_t)p.W;
     if (keys > (size_t)G * 16384u) return false;
-    pp.bins = (unsigned)keys / 8u;
+    pp.keys = (unsigned)keys; pp.bins = pp.keys / 8u;
     const size_t avg_n = (N + G - 1) / G;
     pp.threads = avg_n <= 128u ? 256u : avg_n <= 256u ? 512u : 768u;        // residents and arrivals in different warps
+    if (grid && pp.threads == 256u) pp.threads = 512u;
     pp.limit = (unsigned)(avg_n * 2u + 256u);
     pp.slots = pp.limit + pp.threads;
+    if (pp.slots > 32767u) return false;
     // an environment weighs as much as w_env / 16 cells: the more the better the blocks' work is balanced, and the larger the patches where nobody is
     for (unsigned w = 128u; w >= 8u; w -= (w + 3u) / 4u) {
         pp.w_env = w;
@@ -443,29 +570,45 @@ bool patch_plan(const Params& p, PatchP& pp) {
         pp.bits = (unsigned)S;                           // (without, a restart takes an access to L2 or two)
         if (patch_shared(pp) > PT_SHARED) pp.bits = 0u;
         pp.shared = (unsigned)patch_shared(pp);
-        if (pp.cells <= 16384u && pp.ghosts <= 16384u && pp.shared <= PT_SHARED) return true;
+        if (pp.cells <= 16384u && pp.ghosts <= 16384u && pp.shared <= PT_SHARED) { pp.blocks = G; return true; }
     }
     return false;
 }
-template <unsigned THREADS, bool PLAIN>
+// Not where episodes start on one cell, and everybody passes through one patch: 12,000 on 200 x 190 cells 3.9 / 5.2 (us a step, gather engine / a cluster here).
+// In a cluster up to one environment a thread, and on crowded grids threads left for the arrivals: 12,000 on 100 x 100 5.2 / 5.3, 10,000 there 5.2 / 4.6.  On the
+// whole GPU up to one a thread: 150,001 on 1001 x 613 5.75 / 5.84 (dealt by cell / here).
+bool patch_plan(const Params& p, PatchP& pp) {
+    const size_t S = p.S, N = p.N;
+    if (p.start_mode == 2) {
+        if ((N <= PT_DENSE_ENVS || (N <= PT_MOST_ENVS && S >= 2 * N)) && plan(p, pp, false)) return true;
+        if (N <= (size_t)PT_MOST_THREADS * p.sms && plan(p, pp, true)) return true;
+    }
+    pp = PatchP{};
+    return false;
+}
+template <unsigned THREADS, bool PLAIN, bool GRID>
 static cudaError_t launch(const Params& p, const StepLaunch& l, const PatchP& pp, cudaStream_t st) {
-    auto* const fn = k_patch_steps<THREADS, PLAIN>;
-    cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT_SHARED);
+    auto* const fn = k_patch_steps<THREADS, PLAIN, GRID>;
+    cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT_SHARED);
+    if (e == cudaSuccess && !GRID) e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(pp.blocks); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = pp.shared; cfg.stream = st;
+    cfg.gridDim = dim3(pp.blocks); cfg.blockDim = dim3(THREADS); cfg.stream = st;
+    cfg.dynamicSmemBytes = std::max<size_t>(pp.shared, l.chunk > THREADS ? (size_t)l.chunk * STATE_BYTES : 0u);
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = pp.blocks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    if (GRID) { at[0].id = cudaLaunchAttributeCooperative; at[0].val.cooperative = 1; }
+    else {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = pp.blocks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    }
     cfg.attrs = at; cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, fn, p, l, pp);
 }
-cudaError_t launch_patch_steps(const Params& p, const StepLaunch& l, const PatchP& pp, cudaStream_t st) {
-    const bool pl = plain(p, l);
-    if (pp.threads == 256u) return pl ? launch<256u, true>(p, l, pp, st) : launch<256u, false>(p, l, pp, st);
-    if (pp.threads == 768u) return pl ? launch<768u, true>(p, l, pp, st) : launch<768u, false>(p, l, pp, st);
-    return pl ? launch<512u, true>(p, l, pp, st) : launch<512u, false>(p, l, pp, st);
+template <bool PLAIN>
+static cudaError_t launch(const Params& p, const StepLaunch& l, const PatchP& pp, cudaStream_t st) {
+    if (pp.grid) return pp.threads == 512u ? launch<512u, PLAIN, true>(p, l, pp, st) : launch<768u, PLAIN, true>(p, l, pp, st);
+    return pp.threads == 256u ? launch<256u, PLAIN, false>(p, l, pp, st) : pp.threads == 512u ? launch<512u, PLAIN, false>(p, l, pp, st) : launch<768u, PLAIN, false>(p, l, pp, st);
 }
+cudaError_t launch_patch_steps(const Params& p, const StepLaunch& l, const PatchP& pp, cudaStream_t st) { return plain(p, l) ? launch<true>(p, l, pp, st) : launch<false>(p, l, pp, st); }
 
 }  // namespace cudarl

@@ -23,12 +23,15 @@ def same_stats(gpu, cpu):
     (160, 161, 12288), (160, 161, 12289),            # on crowded and on other grids, and one more
     (5000, 1, 33), (1, 5000, 1025), (7, 3000, 6000), (3000, 9, 6000),        # one cell wide, one high: most of a band is empty
     (3, 2, 5000), (2, 1, 1500),  # fewer bins of cells than blocks: patches without a cell
-    (340, 330, 1500), (420, 400, 1500),              # the map of start cells does not fit; nor the patches: the gather engine
+    (340, 330, 1500),            # the map of start cells does not fit
+    # on all multiprocessors: both sides of 512 threads, one and several environments a thread, the most; a large grid; one that does not fit
+    (420, 400, 1500), (9000, 3, 20000), (120, 97, 37888), (256, 256, 37889), (256, 256, 65536), (400, 300, 113664), (120, 97, 113664), (120, 97, 113665),
+    (1001, 613, 70001), (1300, 1100, 2000),
 ])
 def test_worlds_cut_into_patches(pkg, orc, w, h, n):
     cfg = world(pkg, w, h, n, num_goals=1 if w * h < 100 else 3, obstacle_p=0.0 if w * h < 100 else 0.15, max_steps=37, env_offset=3)
     gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
-    for k in (15, 16, 2, 90):        # one less than the fewest steps of such a launch, the fewest, a launch of the other engine between
+    for k in (15, 16, 2, 31, 32, 90):        # one less than the fewest steps of such a launch, the fewest, a launch of the other engine between
         gpu.set_trace(k != 90)                       # with and without the options
         gpu.train_steps(k); cpu.train_steps(k)
         assert_same(gpu, cpu, "+%d" % k)
@@ -36,7 +39,7 @@ def test_worlds_cut_into_patches(pkg, orc, w, h, n):
     same_stats(gpu, cpu)
 
 
-@pytest.mark.parametrize("w,h,n", [(91, 93, 3000), (201, 199, 8000)])
+@pytest.mark.parametrize("w,h,n", [(91, 93, 3000), (201, 199, 8000), (301, 299, 80000)])
 @pytest.mark.parametrize("kw", [{"eps_kind": 2, "eps0": 1.0, "eps_decay": 0.9}, {"eps_kind": 1, "eps0": 1.0, "eps_decay": 0.99},
                                 {"eps_kind": 3, "eps0": 1.0, "eps_end": 0.1, "eps_steps": 60, "legacy_clamp": 1}])
 def test_epsilons_traps_and_clamp(pkg, orc, w, h, n, kw):
@@ -56,7 +59,7 @@ def crowd_world(pkg, n, **kw):
     return world(pkg, 200, 190, n, num_goals=1, obstacle_p=0.0, obstacle_kind=pkg.OBST_NONE, goal_mode=pkg.GOAL_LIST, goals=[(199, 189)], **kw)
 
 
-@pytest.mark.parametrize("n", [3000, 12000])
+@pytest.mark.parametrize("n", [3000, 12000, 50000])
 @pytest.mark.parametrize("together", [False, True])
 def test_crowds_that_no_patch_holds(pkg, orc, n, together):
     """Everybody on one cell when a launch begins, or -- the rows lead all of them there -- by its middle; spread out again later."""
@@ -76,7 +79,7 @@ def test_crowds_that_no_patch_holds(pkg, orc, n, together):
         same_stats(gpu, cpu)
 
 
-@pytest.mark.parametrize("n", [2500, 10000])
+@pytest.mark.parametrize("n", [2500, 10000, 40000])
 def test_many_cross_at_once(pkg, orc, n):
     """All environments of a few cells walk abreast: more records in a step than their receiver has room for."""
     cfg = crowd_world(pkg, n, max_steps=0, eps0=0.0, lr=0.001)
@@ -92,16 +95,17 @@ def test_many_cross_at_once(pkg, orc, n):
     same_stats(gpu, cpu)
 
 
-def test_table_and_states_changed_between_launches(pkg, orc):
+@pytest.mark.parametrize("n", [9000, 30000])
+def test_table_and_states_changed_between_launches(pkg, orc, n):
     """Nothing of a launch is left in the next: the table set and updated, states set, cells changed in between."""
-    cfg = world(pkg, 150, 140, 9000, max_steps=60)
+    cfg = world(pkg, 150, 140, n, max_steps=60)
     gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
     rng = np.random.RandomState(5)
     for turn in range(4):
         gpu.train_steps(16); cpu.train_steps(16)
         assert_same(gpu, cpu, "turn %d" % turn)
         q = rng.uniform(0, 1, (140, 150, 4)).astype(np.float32)
-        x, y = rng.randint(0, 150, 9000).astype(np.int32), rng.randint(0, 140, 9000).astype(np.int32)
+        x, y = rng.randint(0, 150, n).astype(np.int32), rng.randint(0, 140, n).astype(np.int32)
         b = dict(sx=rng.randint(0, 150, 2000), sy=rng.randint(0, 140, 2000), a=rng.randint(0, 4, 2000), r=np.ones(2000, np.float32),
                  nx=rng.randint(0, 150, 2000), ny=rng.randint(0, 140, 2000), dn=np.zeros(2000, np.uint8))
         for m in (gpu, cpu):
@@ -111,9 +115,10 @@ def test_table_and_states_changed_between_launches(pkg, orc):
     same_stats(gpu, cpu)
 
 
-def test_a_failed_wait_ends_the_launch(pkg):
+@pytest.mark.parametrize("n", [5000, 30000])
+def test_a_failed_wait_ends_the_launch(pkg, n):
     """With the tests' poll bound a launch records the failure and leaves; every later launch does nothing."""
-    g = pkg.VecGridWorld(world(pkg, 120, 97, 5000))
+    g = pkg.VecGridWorld(world(pkg, 120, 97, n))
     g.train_steps(20); g.synchronize()
     g.debug_set_copy_wait_polls(1)
     g.train_steps(20)
