@@ -498,22 +498,24 @@ bool use_gather(const cudarl_ctx* c) {
     if (f.tile_edge != 0) return false;
     return c->p.S <= (1u << 21) || c->p.N <= (1u << 18);
 }
-int alloc_patch(cudarl_ctx* c) {
+// What the patch engine works with: made by the first launch of it, which a context that never trains does without (creating one for 65,536 environments on 256 x 256 cells
+// and stepping it once took 2.2 ms, with these 3.1 and more).  The records are sorted into the spare copy of the states.
+int ensure_patch(cudarl_ctx* c) {
+    if (c->dpatch) return 0;
     PatchP& pp = c->patch;
-    if (c->p.gp.arena || !c->p.N || !patch_plan(c->p, pp)) { pp = PatchP{}; return 0; }
     const size_t N = c->p.N, G = pp.blocks;
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t at = off; off += (bytes + 255) / 256 * 256; return at; };
     const size_t count = take(pp.bins * sizeof(unsigned)), barrier = take(pp.grid ? 1024 : 0), listed = take(pp.grid ? 3 * G * 4 : 0),
                  list = take(pp.grid ? 3 * G * pp.threads * 16 : 0), edge = take(pp.grid ? 2 * (size_t)pp.keys * 8 : 0);
     c->patch_zero = off;                                 // zero before the first launch: no step has the number 0
-    const size_t part = take(G * 4), cut = take((G + 1) * 4), rank = take(N * 4), dealt = take(N * sizeof(int4));
+    const size_t part = take(G * 4), cut = take((G + 1) * 4), rank = take(N * 4);
     CK(cudaMalloc(&c->dpatch, off));
     CK(cudaMemsetAsync(c->dpatch, 0, c->patch_zero, c->st));
     unsigned char* const m = (unsigned char*)c->dpatch;
     pp.count = (unsigned*)(m + count); pp.barrier = (unsigned*)(m + barrier); pp.listed = (unsigned*)(m + listed);
     pp.list = (unsigned long long*)(m + list); pp.edge = (unsigned long long*)(m + edge);
-    pp.part = (unsigned*)(m + part); pp.cut = (unsigned*)(m + cut); pp.rank = (unsigned*)(m + rank); pp.dealt = (int4*)(m + dealt);
+    pp.part = (unsigned*)(m + part); pp.cut = (unsigned*)(m + cut); pp.rank = (unsigned*)(m + rank); pp.dealt = c->p.st2;
     return 0;
 }
 int alloc_gather(cudarl_ctx* c) {
@@ -536,7 +538,8 @@ int alloc_gather(cudarl_ctx* c) {
         gp.bins = (unsigned*)c->dgbins; gp.part = gp.bins + gp.nbins; gp.rank = gp.part + gp.grid;
         for (auto& wk : c->dwork) CK(cudaMalloc(&wk, N * sizeof(int4)));
     }
-    return alloc_patch(c);
+    if (gp.arena || !p.N || !patch_plan(p, c->patch)) c->patch = PatchP{};
+    return 0;
 }
 
 // the move bytes of the engine in use, after a change of the grid
@@ -709,6 +712,7 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         l.in = c->dealt >= 0 ? (const int4*)c->dwork[c->dealt] : c->p.st;
         l.out = dealing ? (int4*)c->dwork[c->dealt == 0 ? 1 : 0] : const_cast<int4*>(l.in);
         if (patches) {                                       // from wherever the records are to the order of the environments
+            { int rc = ensure_patch(c); if (rc) return rc; }
             if (c->patch_epoch > 0xFFFFFFFFu - 4096u) {      // every number has been used
                 CK(cudaMemsetAsync(c->dpatch, 0, c->patch_zero, c->st));
                 c->patch_epoch = 1;
