@@ -1,61 +1,154 @@
-// arena_engine.cu -- the fused train step for the smallest worlds: the whole world in the shared memory of one block (k_arena_steps), up to 32
-// environments in one warp (k_solo_steps), one in a thread (k_one_steps), many steps per launch.
+// arena_engine.cu -- the fused train step for the smallest worlds, many steps per launch: the whole world in the shared memory of one block, one environment per
+// thread (k_arena_steps, up to 1,024), or a single one in one thread (k_one_steps).  Where shared memory holds no counters beside the rows, up to 32 environments run
+// in one warp without any (k_solo_steps).
 //
 // A small world is latency, nothing else: in the gather engine (gather_engine.cu) a step is two barriers between blocks and several
 // dependent accesses to L2.  Here the table, the counters and the move bytes lie in shared memory, the environments in registers, and
-// the barrier is the block's.  The step of k_arena_steps is step_loop.cuh; the other two, further down, have neither counters nor barriers.
+// the barrier is the block's (or, in one warp, none):
 //
-// What bounds k_arena_steps: one block's issue slots, about 300 instructions per warp and step.  B200, us per step, here / gather engine: 200
-// on 20 x 20 cells 1.1 / 4.7, 1,000 on 32 x 32 2.2 / 4.7; 4,096 on 64 x 64 16 / 4.7.  The same spread over
-// the distributed shared memory of a cluster was no faster than L2 (4,096 on 64 x 64: 4.4 with 16 blocks; scattered 16-byte accesses to
-// other blocks' shared memory are served one by one), nor with a copy of the table in every block (3.9: every update is then stored 8 times).
+//   count   every environment reads the row of its cell, chooses, counts itself in the (cell, action) counter, moves on, takes its TD target from Q_t;
+//   apply   the first on a (cell, action) applies its update as often as it was counted.
+//
+// The draws depend on nothing: up to 512 environments as many threads again make them some steps ahead.
+//
+// What bounds it: one thread's instructions, some 120 a step at 5 - 6 cycles each, with 1,024 environments the block's issue slots.  B200, us a step, as an instance of the
+// gather engine's loop (draws in the same thread, options tested where they are off) / here: 18 environments on 20 x 19 cells 0.87 / 0.59, 120 on 50 x 62 1.00 / 0.66,
+// 200 on 20 x 20 1.10 / 0.84, 500 on 60 x 60 1.71 / 1.22, 1,000 on 32 x 32 2.23 / 1.85; and, with 33 bytes a cell instead of 49, on grids that no block held: 300 on 80 x 80
+// 3.8 / 0.93, 1,000 on 70 x 70 3.9 / 1.7.  (4,096 on 64 x 64 took 16 in one block; spread over the distributed shared memory of a cluster 4.4: remote rows are
+// served one by one.  patch_engine.cu, where environments move between the blocks instead, takes 2.7.)
 #include "step_loop.cuh"
 
 namespace cudarl {
 
-constexpr size_t ARENA_MOST = 226u * 1024u;      // dynamic shared memory of a block (227 KB less the static words of step_loop.cuh)
 constexpr size_t SOLO_MOST = 216u * 1024u;       // 8.3 KB go to the draws
 constexpr unsigned ARENA_ENVS = 1024u;
-// rows (16 bytes a cell), two rows of counters by step parity (16 bytes each), a move byte
-inline size_t solo_bytes(unsigned S) { return (size_t)S * 16u + (S + 15u) / 16u * 16u; }      // without the counters
-inline size_t arena_bytes(unsigned S) { return (size_t)S * 48u + (S + 15u) / 16u * 16u; }
+inline size_t solo_bytes(unsigned S) { return (size_t)S * 16u + (S + 15u) / 16u * 16u; }      // rows and move bytes
 
-struct ArenaSpace {
-    static constexpr bool ALONE = true;
-    float4* rows; unsigned* counters; const unsigned char* mv; unsigned S;
-    __device__ __forceinline__ float4 row(unsigned s) const { return rows[s]; }
-    __device__ __forceinline__ unsigned moves(unsigned s) const { return mv[s]; }
-    __device__ __forceinline__ unsigned add(unsigned par, unsigned idx, unsigned n) const { return atomicAdd(counters + par * 4u * S + idx, n); }
-    __device__ __forceinline__ void count(unsigned par, unsigned idx, unsigned n) const { atomicAdd(counters + par * 4u * S + idx, n); }
-    __device__ __forceinline__ bool note(unsigned par, unsigned idx) const { return (atomicOr(counters + par * 4u * S + idx, NOTED) & NOTED) != 0u; }
-    __device__ __forceinline__ void clear(unsigned par, unsigned idx) const { counters[par * 4u * S + idx] = 0u; }
-    __device__ __forceinline__ uint4 counts(unsigned par, unsigned s) const { return reinterpret_cast<const uint4*>(counters)[par * S + s]; }
-    __device__ __forceinline__ void store(unsigned idx, float v) const { reinterpret_cast<float*>(rows)[idx] = v; }
-    __device__ __forceinline__ void arrive() const {}
-    __device__ __forceinline__ bool wait() const { __syncthreads(); return true; }
+// One environment per thread, WALK threads; with HELP as many again make the draws ahead, CHUNK steps of them.
+template <unsigned WALK, bool HELP> struct Arena {
+    static constexpr unsigned CHUNK = HELP ? (WALK <= 64u ? 32u : 2048u / WALK) : 1u, DRAWS = HELP ? 2u * CHUNK * WALK : 0u;
+    // rows (16 bytes a cell), two copies of four 16-bit counters by step parity, a bit per cell where no episode starts, move bytes, draws
+    static constexpr size_t MOST = 224u * 1024u;
+    static size_t bytes(unsigned S) { return (size_t)S * 32u + (S + 31u) / 32u * 4u + (S + 15u) / 16u * 16u + DRAWS * 4u; }
+    // the walkers' barrier: one warp needs none
+    static __device__ __forceinline__ void sync() {
+        if constexpr (WALK == 32u) __syncwarp();
+        else if constexpr (HELP) asm volatile("barrier.cta.sync 1, %0;" :: "n"(WALK) : "memory");
+        else __syncthreads();
+    }
 };
 
-template <unsigned AB, bool PLAIN>
-__global__ void __launch_bounds__(AB, 1) k_arena_steps(const __grid_constant__ Params p, const __grid_constant__ StepLaunch l) {
+// PLAIN: no traps, no clamp, no trace, epsilon by step.
+template <unsigned WALK, bool HELP, bool PLAIN>
+__global__ void __launch_bounds__(HELP ? 2u * WALK : WALK, 1) k_arena_steps(const __grid_constant__ Params p, const __grid_constant__ StepLaunch l) {
+    using A = Arena<WALK, HELP>;
+    constexpr unsigned CHUNK = A::CHUNK, ALL = HELP ? 2u * WALK : WALK;
     extern __shared__ __align__(16) unsigned char arena[];
-    __shared__ unsigned s_flag;
+    __shared__ unsigned s_flag, s_sum[5], s_ended, s_thr[2][CHUNK];
     if (!may_start(p, &s_flag)) return;
-    const unsigned S = p.S;
+    const unsigned tid = threadIdx.x, S = p.S, W = (unsigned)p.W;
     float4* const rows = reinterpret_cast<float4*>(arena);
-    uint4* const counters = reinterpret_cast<uint4*>(arena) + S;
-    unsigned char* const moves = arena + (size_t)S * 48u;
-    for (unsigned s = threadIdx.x; s < S; s += AB) {
-        rows[s] = p.Q[s]; moves[s] = __ldg(p.gp.mv + s);
-        counters[s] = make_uint4(0u, 0u, 0u, 0u); counters[S + s] = make_uint4(0u, 0u, 0u, 0u);
+    uint2* const counts = reinterpret_cast<uint2*>(rows + S);                        // [2][S]
+    unsigned* const draws = reinterpret_cast<unsigned*>(counts + 2u * S);            // [2][CHUNK][WALK]: the 24 bits compared with epsilon, above them the action to explore
+    unsigned* const closed = draws + A::DRAWS;
+    unsigned char* const moves = reinterpret_cast<unsigned char*>(closed + (S + 31u) / 32u);
+    if (tid < 5u) s_sum[tid] = 0u;
+    if (tid == 5u) s_ended = 0u;
+    for (unsigned s = tid; s < S; s += ALL) { rows[s] = p.Q[s]; moves[s] = __ldg(p.gp.mv + s); counts[s] = make_uint2(0u, 0u); counts[S + s] = make_uint2(0u, 0u); }
+#pragma unroll 1
+    for (unsigned c0 = tid & ~31u; c0 < S; c0 += ALL) {
+        const unsigned c = c0 + (tid & 31u), w = __ballot_sync(FULL, c < S && (cw_load(p.cw, c) & (CW_OBST | CW_GOAL)));
+        if ((tid & 31u) == 0u) closed[c0 >> 5] = w;
+    }
+    const unsigned slot = HELP && tid >= WALK ? tid - WALK : tid;
+    const bool walker = !HELP || tid < WALK, act = slot < p.N;
+    const unsigned tmax = p.max_steps > 0 ? (unsigned)p.max_steps : 0x7FFFFFFFu;
+    Tally tally{0u, 0u, 0u, 0u, 0u};
+    const int4 r0 = act ? l.out[slot] : make_int4(0, 0, 0, 0);
+    const unsigned id = (unsigned)r0.w;
+    unsigned s = (unsigned)r0.y * W + (unsigned)r0.x, t = (unsigned)r0.z, before = NOBODY;        // before: the (cell, action) applied in the last step
+    EpsilonIndex eps_index(p, l, PLAIN);
+    float eps = __ldg(p.eps_tab + eps_index.at);
+    auto threshold = [](float e) -> unsigned { return !(e > 0.0f) ? 0u : e >= 1.0f ? (1u << 24) : (unsigned)ceilf(e * 16777216.0f); };
+    unsigned thr = threshold(eps);
+    auto draw = [&](unsigned long long g) -> unsigned {
+        const U4 r = philox4x32_10(p.env_offset + id, 0u, (unsigned)g, (unsigned)(g >> 32), p.policy_keys);
+        return (r.x >> 8) | (r.y << 24);
+    };
+    auto make_draws = [&](unsigned first) {
+        const unsigned c = (first / CHUNK) & 1u, m = min(CHUNK, l.steps - first);
+#pragma unroll 1
+        for (unsigned k = 0; k < m; ++k) draws[(c * CHUNK + k) * WALK + slot] = draw(p.step + first + k);
+        if (l.eps_mode == 1 && slot < m) s_thr[c][slot] = threshold(__ldg(p.eps_tab + p.eps_idx + first + slot));
+    };
+    if (HELP && !walker) make_draws(0u);
+    __syncthreads();
+#pragma unroll 1
+    for (unsigned first = 0; first < l.steps; first += HELP ? CHUNK : l.steps) {
+        if (HELP && !walker) { if (first + CHUNK < l.steps) make_draws(first + CHUNK); }
+        else {
+            const unsigned c = HELP ? (first / CHUNK) & 1u : 0u, m = HELP ? min(CHUNK, l.steps - first) : l.steps;
+#pragma unroll 1
+            for (unsigned k = 0; k < m; ++k) {
+                const unsigned long long g = p.step + first + k;
+                const unsigned par = (first + k) & 1u;
+                if (l.eps_mode == 1) thr = HELP ? s_thr[c][k] : threshold(__ldg(p.eps_tab + p.eps_idx + k));
+                unsigned own = NOBODY; float target = 0.0f, value = 0.0f;
+                if (before != NOBODY) reinterpret_cast<unsigned short*>(counts + (par ^ 1u) * S)[before] = 0u;      // (everybody has read it; nobody uses that parity now)
+                before = NOBODY;
+                if (act) {
+                    const unsigned w = HELP ? draws[(c * CHUNK + k) * WALK + slot] : draw(g);
+                    const float4 row = rows[s];
+                    unsigned mv = moves[s];
+                    const unsigned a = (w & 0xFFFFFFu) < thr ? (w >> 24) & 3u : (unsigned)argmax4(row);
+                    mv >>= a;                             // bit 0: the move is blocked, bit 4: it ends on a goal
+                    own = s * 4u + a;
+                    const unsigned sh = (a & 1u) * 16u, old = atomicAdd(reinterpret_cast<unsigned*>(counts + par * S) + (own >> 1), 1u << sh);
+                    const unsigned d = (a & 1u) ? 1u : W, cell = s;
+                    const bool blocked = (mv & 1u) != 0u, done = (mv & 16u) != 0u;
+                    s = blocked ? s : a - 1u < 2u ? s + d : s - d;
+                    float m4 = max4(rows[s]);
+                    value = pick(row, (int)a);
+                    if (!PLAIN && p.legacy_clamp && m4 < 0.0f) m4 = 0.0f;
+                    float r = -0.01f;
+                    if (!PLAIN && p.ntraps && blocked) { const unsigned y = cell / W; r = blocked_step_reward(p, (int)(cell - y * W), (int)y, (int)a); }     // a trap charges its penalty
+                    target = done ? 1.0f : __fmaf_rn(p.gamma, m4, r);
+                    if (!PLAIN && l.trace && first + k + 1u == l.steps) { p.tr_a[id] = (int)a; p.tr_r[id] = done ? 1.0f : r; p.tr_d[id] = done ? 1 : 0; }
+                    t = min(t + 1u, STEP_SAT);
+                    if (done || t >= tmax) {
+                        s = sample_start_if(p, p.env_offset + id, g + 1ull, TAG_START, [&](unsigned cc) { return closed[cc >> 5] >> (cc & 31u) & 1u; }); t = 0u;
+                        if (done) ++tally.goals; else ++tally.timeouts;
+                        if (!PLAIN && l.eps_mode == 2) atomicAdd(&s_ended, 1u);
+                    }
+                    if ((old >> sh) & 0xFFFFu) own = NOBODY;      // the first on a (cell, action) applies its update
+                }
+                A::sync();
+                if (own != NOBODY) {
+                    const uint2 q = counts[par * S + (own >> 2)];
+                    const unsigned a = own & 3u, n = ((a & 2u) ? q.y : q.x) >> ((a & 1u) * 16u) & 0xFFFFu, both = q.x + q.y, tot = (both & 0xFFFFu) + (both >> 16);
+                    if (tot > 1u) tally.conf += n;
+                    if (tot > CROWDED_CELL) {                     // the lowest chosen action speaks for the cell
+                        const unsigned c0 = q.x & 0xFFFFu, c1 = q.x >> 16;
+                        if ((a == 0u ? 0u : a == 1u ? c0 : a == 2u ? c0 + c1 : c0 + c1 + (q.y & 0xFFFFu)) == 0u) { ++tally.crowded; tally.on_crowded += tot; }
+                    }
+                    reinterpret_cast<float*>(rows)[own] = apply_counted(value, target, p.lr, n);
+                    before = own;
+                }
+                if (!PLAIN && l.eps_mode == 2) {                  // (nobody adds to the ended episodes before the second barrier)
+                    if (first + k + 1u < l.steps) { eps_index.next(p, l, PLAIN, *reinterpret_cast<volatile unsigned*>(&s_ended), true); eps = __ldg(p.eps_tab + eps_index.at); thr = threshold(eps); }
+                }
+                A::sync();
+            }
+        }
+        if (HELP) __syncthreads();
     }
     __syncthreads();
-    ArenaSpace space{rows, reinterpret_cast<unsigned*>(counters), moves, S};
-    run_steps<Home::Registers, AB, PLAIN, true>(p, l, space, l.out, nullptr);
-    __syncthreads();
-    for (unsigned s = threadIdx.x; s < S; s += AB) p.Q[s] = rows[s];
+    for (unsigned k = tid; k < S; k += ALL) p.Q[k] = rows[k];
+    if (walker && act) { const unsigned y = s / W; l.out[slot] = make_int4((int)(s - y * W), (int)y, (int)t, (int)id); }
+    add_tallies(p, l, tally, s_sum, true, eps);
 }
 
-// 2 to 32 environments: one warp steps them, without counters or a barrier in the step -- who stands on the same (cell, action) is found
+// 2 to 32 environments on grids of more than 6,676 cells: one warp steps them, without counters or a barrier in the step -- who stands on the same (cell, action) is found
 // with a match across the warp, and the lowest of them applies the update for all.  A second warp makes the random draws, which depend
 // on nothing, a chunk of steps ahead.  SHARED: the world in shared memory; else in global memory, where the rows the warp walks over stay in
 // its first-level cache.
@@ -234,48 +327,42 @@ __global__ void __launch_bounds__(64, 1) k_one_steps(const __grid_constant__ Par
     add_tallies(p, l, tally, s_sum, true, eps);
 }
 
-template <unsigned AB>
-static bool allow() {
-    return cudaFuncSetAttribute((const void*)k_arena_steps<AB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ARENA_MOST) == cudaSuccess &&
-           cudaFuncSetAttribute((const void*)k_arena_steps<AB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ARENA_MOST) == cudaSuccess;
+template <unsigned WALK, bool HELP>
+static cudaError_t launch_one(const Params& p, const StepLaunch& l, cudaStream_t st) {
+    using A = Arena<WALK, HELP>;
+    auto* const fn = plain(p, l) ? k_arena_steps<WALK, HELP, true> : k_arena_steps<WALK, HELP, false>;
+    const cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A::MOST);
+    if (e != cudaSuccess) return e;
+    fn<<<1, HELP ? 2u * WALK : WALK, A::bytes(p.S), st>>>(p, l);
+    return cudaGetLastError();
 }
-// One block holds up to 1,024 environments at one per thread; twice that takes longer than the gather engine.
+// One block holds up to 1,024 environments at one per thread; twice that takes longer than the other engines.  Up to 512 half the threads make draws.
 bool arena_plan(Params& p) {
     GatherP& gp = p.gp;
     const unsigned n = p.N ? p.N : 1u;
-    if (n <= 32u) {
-        gp.threads = gp.chunk = 32u; gp.grid = 1u; gp.arena = 1u;
-        return cudaFuncSetAttribute((const void*)k_one_steps<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLO_MOST) == cudaSuccess &&
-               cudaFuncSetAttribute((const void*)k_one_steps<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLO_MOST) == cudaSuccess &&
-               cudaFuncSetAttribute((const void*)k_solo_steps<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLO_MOST) == cudaSuccess &&
-               cudaFuncSetAttribute((const void*)k_solo_steps<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLO_MOST) == cudaSuccess;
-    }
-    if (n > ARENA_ENVS || arena_bytes(p.S) > ARENA_MOST) return false;
-    gp.threads = n <= 256u ? 256u : 1024u;
+    gp.threads = n <= 32u ? 32u : n <= 64u ? 64u : n <= 128u ? 128u : n <= 256u ? 256u : n <= 512u ? 512u : 1024u;
     gp.chunk = gp.threads; gp.grid = 1u; gp.arena = 1u;
-    return allow<256u>() && allow<1024u>();
-}
-
-template <unsigned AB>
-static cudaError_t launch_one(const Params& p, const StepLaunch& l, cudaStream_t st) {
-    if (plain(p, l)) k_arena_steps<AB, true><<<1, AB, arena_bytes(p.S), st>>>(p, l);
-    else             k_arena_steps<AB, false><<<1, AB, arena_bytes(p.S), st>>>(p, l);
-    return cudaGetLastError();
+    if (n <= 32u) return true;
+    return n <= ARENA_ENVS && (n <= 512u ? Arena<512u, true>::bytes(p.S) : Arena<1024u, false>::bytes(p.S)) <= Arena<1024u, false>::MOST;
 }
 cudaError_t launch_arena_steps(const Params& p, const StepLaunch& l, cudaStream_t st) {
-    if (p.gp.threads == 32u) {
-        const bool fits = solo_bytes(p.S) <= SOLO_MOST, pl = plain(p, l);
-        if (p.N == 1u) {
-            const size_t bytes = fits ? solo_bytes(p.S) : 0u;
-            const bool options = p.ntraps || p.legacy_clamp || l.trace;
-            (fits ? options ? k_one_steps<true, true> : k_one_steps<true, false> : options ? k_one_steps<false, true> : k_one_steps<false, false>)<<<1, 64, bytes, st>>>(p, l);
-            return cudaGetLastError();
-        }
-        if (fits) { if (pl) k_solo_steps<true, true><<<1, 64, solo_bytes(p.S), st>>>(p, l); else k_solo_steps<true, false><<<1, 64, solo_bytes(p.S), st>>>(p, l); }
-        else { if (pl) k_solo_steps<false, true><<<1, 64, 0, st>>>(p, l); else k_solo_steps<false, false><<<1, 64, 0, st>>>(p, l); }
+    const bool pl = plain(p, l);
+    if (p.N == 1u || (p.N <= 32u && Arena<32u, true>::bytes(p.S) > Arena<32u, true>::MOST)) {
+        const bool fits = solo_bytes(p.S) <= SOLO_MOST, options = p.ntraps || p.legacy_clamp || l.trace;
+        auto* const fn = p.N == 1u ? fits ? options ? k_one_steps<true, true> : k_one_steps<true, false> : options ? k_one_steps<false, true> : k_one_steps<false, false>
+                                   : fits ? pl ? k_solo_steps<true, true> : k_solo_steps<true, false> : pl ? k_solo_steps<false, true> : k_solo_steps<false, false>;
+        if (fits) { const cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLO_MOST); if (e != cudaSuccess) return e; }
+        fn<<<1, 64, fits ? solo_bytes(p.S) : 0u, st>>>(p, l);
         return cudaGetLastError();
     }
-    return p.gp.threads == 256u ? launch_one<256u>(p, l, st) : launch_one<1024u>(p, l, st);
+    switch (p.gp.threads) {
+        case 32u: return launch_one<32u, true>(p, l, st);
+        case 64u: return launch_one<64u, true>(p, l, st);
+        case 128u: return launch_one<128u, true>(p, l, st);
+        case 256u: return launch_one<256u, true>(p, l, st);
+        case 512u: return launch_one<512u, true>(p, l, st);
+        default: return launch_one<1024u, false>(p, l, st);
+    }
 }
 
 }  // namespace cudarl

@@ -7,7 +7,6 @@ namespace cudarl {
 
 // The table and the counters in global memory.
 struct GlobalTable {
-    static constexpr bool ALONE = false;
     const Params& p;
     __device__ __forceinline__ float4 row(unsigned s) const { return p.Q[s]; }
     __device__ __forceinline__ unsigned moves(unsigned s) const { return __ldg(p.gp.mv + s); }

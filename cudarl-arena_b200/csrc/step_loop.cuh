@@ -1,6 +1,6 @@
-// step_loop.cuh -- the fused train step with one thread per environment, many steps per launch; shared by the engines that differ in
-// where the table and the counters live and in how the threads of a launch wait for one another (gather_engine.cu: L2 and a barrier
-// of the grid or of one cluster; arena_engine.cu: shared memory and the block's barrier).
+// step_loop.cuh -- the fused train step with one thread per environment, many steps per launch, as the gather engine takes it (gather_engine.cu; patch_engine.cu where
+// a patch overflows): table and counters in L2, a barrier of the grid or of one cluster.  And what all engines of many steps per launch share: the counted
+// updates, the epsilon by episodes, the sums.
 //
 //   count   every environment reads the row of its cell, chooses its action, counts itself in the (cell, action) counter with an
 //           atomic, moves on, and takes the TD target of its (cell, action) from Q_t;
@@ -15,7 +15,7 @@
 // crowded ones 4.7 -> 5.5).  Counters alternate by step parity; who counted clears its counter in the next step's count phase, when
 // everybody has read it and nobody uses that parity.
 //
-// A Space gives: ALONE (the launch is one block), row(s), moves(s), add(par, idx, n) -> old count, count(par, idx, n), note(par, idx) -> marked before, clear(par, idx),
+// A Space gives: row(s), moves(s), add(par, idx, n) -> old count, count(par, idx, n), note(par, idx) -> marked before, clear(par, idx),
 // counts(par, s) -> uint4, store(idx, v), arrive(), wait() -> false when the launch has to be given up.
 #pragma once
 #include "kernels.cuh"
@@ -68,7 +68,7 @@ struct EpsilonIndex {
         at = (unsigned)min(k - l.eps_base_k, (unsigned long long)(l.eps_len - 1u));
         ep_next = (k + 1ull) * p.N;
     }
-    // alone: `local` counts the episodes of this launch (one block), else the control block does
+    // alone: `local` is the number of episodes finished in this launch, else the control block has all
     __device__ __forceinline__ void next(const Params& p, const StepLaunch& l, bool plain, unsigned local, bool alone) {
         if (l.eps_mode == 1) ++at;
         else if (!plain && l.eps_mode == 2) {
@@ -148,7 +148,7 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
     EpsilonIndex eps_index(p, l, PLAIN);
     if (l.eps_mode == 1) eps_index.at += skip;
     float eps = __ldg(p.eps_tab + eps_index.at);
-    if (!PLAIN && l.eps_mode == 2 && !Space::ALONE) {       // every block has read the finished episodes before any adds those of the first step
+    if (!PLAIN && l.eps_mode == 2) {       // every block has read the finished episodes before any adds those of the first step
         space.arrive();
         if (!space.wait()) return;
     }
@@ -205,7 +205,7 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
                 if (applies) m_tv[j] = make_float2(target, value);
             }
         }
-        if (!PLAIN && l.eps_mode == 2 && !Space::ALONE) {              // finished episodes of this step, before anybody can pass the barrier
+        if (!PLAIN && l.eps_mode == 2) {              // finished episodes of this step, before anybody can pass the barrier
             __syncthreads();
             if (tid == 0u && s_ep) { atomicAdd(&ctl->episodes, (unsigned long long)s_ep); s_ep = 0u; }
         }
@@ -243,7 +243,7 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
             if (FIRST) __syncwarp();                  // the lanes' rounds side by side, however they got here
             if (applies) space.store(own, apply_counted(value, target, p.lr, n));
         }
-        eps_index.next(p, l, PLAIN, Space::ALONE ? *reinterpret_cast<volatile unsigned*>(&s_ep) : 0u, Space::ALONE);        // between the two barriers: nobody adds to the episodes before everybody has passed the second
+        eps_index.next(p, l, PLAIN, 0u, false);        // between the two barriers: nobody adds to the episodes before everybody has passed the second
         space.arrive();
         if (l.eps_mode && step + 1u < l.steps) eps = __ldg(p.eps_tab + eps_index.at);
         if (!space.wait()) return;
@@ -257,7 +257,7 @@ __device__ __forceinline__ void run_steps(const Params& p, const StepLaunch& l, 
         const unsigned y = s / W;
         work[first + j] = make_int4((int)(s - y * W), (int)y, (int)t, (int)id);
     }
-    add_tallies(p, l, tally, s_sum, l.eps_mode != 2 || Space::ALONE, eps);
+    add_tallies(p, l, tally, s_sum, l.eps_mode != 2, eps);
 }
 
 // Whether a launch needs none of the options PLAIN leaves out.
