@@ -539,6 +539,13 @@ int alloc_gather(cudarl_ctx* c) {
         for (auto& wk : c->dwork) CK(cudaMalloc(&wk, N * sizeof(int4)));
     }
     if (gp.arena || !p.N || !patch_plan(p, c->patch)) c->patch = PatchP{};
+    // On the whole GPU the block beside a goal is what a step waits for once all paths lead there: as many environments arrive in a step as N / sqrt(cells x goals), but for a factor.
+    // B200, us a step after 20,000 - 40,000 steps, gather engine / patches: 65,536 on 256 x 256 with one goal (256) 6.5 / 7.5, with eight (90) 6.15 / 5.65; 100,000 on 300 x 290 with three (196)
+    // 7.74 / 7.69; 30,000 on 150 x 150 with one (200) 5.7 / 4.3.
+    if (c->patch.grid) {
+        const size_t goals = std::max<size_t>(1, (size_t)std::count(c->cells.begin(), c->cells.end(), (uint8_t)2));
+        if ((double)N * (double)N > 40000.0 * (double)S * (double)goals) c->patch = PatchP{};
+    }
     return 0;
 }
 
