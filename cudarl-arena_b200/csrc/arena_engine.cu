@@ -55,11 +55,7 @@ __global__ void __launch_bounds__(HELP ? 2u * WALK : WALK, 1) k_arena_steps(cons
     if (tid < 5u) s_sum[tid] = 0u;
     if (tid == 5u) s_ended = 0u;
     for (unsigned s = tid; s < S; s += ALL) { rows[s] = p.Q[s]; moves[s] = __ldg(p.gp.mv + s); counts[s] = make_uint2(0u, 0u); counts[S + s] = make_uint2(0u, 0u); }
-#pragma unroll 1
-    for (unsigned c0 = tid & ~31u; c0 < S; c0 += ALL) {
-        const unsigned c = c0 + (tid & 31u), w = __ballot_sync(FULL, c < S && (cw_load(p.cw, c) & (CW_OBST | CW_GOAL)));
-        if ((tid & 31u) == 0u) closed[c0 >> 5] = w;
-    }
+    map_closed(p, closed, S, tid, ALL);
     const unsigned slot = HELP && tid >= WALK ? tid - WALK : tid;
     const bool walker = !HELP || tid < WALK, act = slot < p.N;
     const unsigned tmax = p.max_steps > 0 ? (unsigned)p.max_steps : 0x7FFFFFFFu;

@@ -213,19 +213,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
         };
         for (unsigned k = tid; k < nghost; k += THREADS) from[k] = NO_CELL;
         if (!GRID) for (unsigned k = tid; k < 3u * THREADS; k += THREADS) mail[k] = make_uint2(0u, HOLE);
-#pragma unroll 1
-        for (unsigned c0 = tid & ~31u; c0 < pp.bits; c0 += THREADS) {
-            const unsigned c = c0 + (tid & 31u), w = __ballot_sync(FULL, c < pp.bits && (cw_load(p.cw, c) & (CW_OBST | CW_GOAL)));
-            if ((tid & 31u) == 0u) closed[c0 >> 5] = w;
+        map_closed(p, closed, pp.bits, tid, THREADS);
+#pragma unroll 4
+        for (unsigned k = tid; k < cells; k += THREADS) {
+            unsigned x, y; cell_of(k0 + k, x, y);
+            const bool real = y < (unsigned)p.H;                   // not below the last band's last row
+            const unsigned s = real ? y * W + x : 0u;
+            const float4 row = p.Q[s]; const unsigned char mv = __ldg(p.gp.mv + s);
+            rows[k] = row; moves[k] = real ? mv : 0x0Fu;
+            counts[k] = make_uint2(0u, 0u);
         }
         __syncthreads();
 #pragma unroll 1
         for (unsigned k = tid; k < cells; k += THREADS) {
             unsigned x, y; cell_of(k0 + k, x, y);
-            counts[k] = make_uint2(0u, 0u);
-            if (y >= (unsigned)p.H) { rows[k] = make_float4(0.f, 0.f, 0.f, 0.f); moves[k] = 0x0Fu; continue; }       // below the last band's last row
-            const unsigned s = y * W + x;
-            rows[k] = p.Q[s]; moves[k] = __ldg(p.gp.mv + s);
+            if (y >= (unsigned)p.H) continue;
             bool outside = false;
             for (unsigned a = 0; a < 4u; ++a) {
                 const bool there = a == 0u ? y > 0u : a == 1u ? x + 1u < W : a == 2u ? y + 1u < (unsigned)p.H : x > 0u;
