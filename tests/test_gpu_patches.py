@@ -24,8 +24,8 @@ def same_stats(gpu, cpu):
     (5000, 1, 33), (1, 5000, 1025), (7, 3000, 6000), (3000, 9, 6000),        # one cell wide, one high: most of a band is empty
     (3, 2, 5000), (2, 1, 1500),  # fewer bins of cells than blocks: patches without a cell
     (340, 330, 1500),            # the map of start cells does not fit
-    # on all multiprocessors: both sides of 512 threads, one and several environments a thread, the most; a large grid; one that does not fit
-    (420, 400, 1500), (9000, 3, 20000), (130, 110, 37888), (256, 256, 37889), (256, 256, 65536), (400, 300, 113664), (400, 300, 113665), (256, 256, 88681),       # (.., and more than arrive at one goal in time)
+    # on all multiprocessors: both sides of 512 threads, the most environments, the most for three goals; a large grid; one that does not fit
+    (420, 400, 1500), (9000, 3, 20000), (130, 110, 37888), (256, 256, 37889), (256, 256, 65536), (400, 300, 113664), (400, 300, 113665), (256, 256, 88680), (256, 256, 88682),
     (1001, 613, 70001), (1300, 1100, 2000),
 ])
 def test_worlds_cut_into_patches(pkg, orc, w, h, n):
