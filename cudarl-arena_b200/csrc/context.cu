@@ -726,7 +726,6 @@ int run_gather(cudarl_ctx* c, int64_t n) {
                 c->patch_epoch = 1;
             }
             l.chunk = (c->p.N + c->patch.blocks - 1u) / c->patch.blocks; l.epoch = c->patch_epoch;
-            if (l.chunk > c->patch.threads) l.chunk = (l.chunk + 31u) / 32u * 32u;
             CK(launch_patch_steps(c->p, l, c->patch, c->st));
             c->patch_epoch += (uint32_t)m + 2u; c->dealt = -1;
         } else {

@@ -527,8 +527,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
         if constexpr (GRID) {
             space.arrive(); if (!space.wait()) return;
             if (tid < 3u) pp.listed[tid * G + b] = 0u;             // what was listed for the step that nobody took
-            if (l.chunk <= THREADS) run_steps<Home::Registers, THREADS, PLAIN, false>(p, l, space, work, nullptr, step);
-            else                    run_steps<Home::Shared, THREADS, PLAIN, false>(p, l, space, work, smem, step);
+            run_steps<Home::Registers, THREADS, PLAIN, false>(p, l, space, work, nullptr, step);
         } else run_steps<Home::Registers, THREADS, PLAIN, true>(p, l, space, work, nullptr, step);
         if (!fits) {
             __syncthreads();
@@ -561,6 +560,7 @@ static bool plan(const Params& p, PatchP& pp, bool grid) {
     const size_t avg_n = (N + G - 1) / G;
     pp.threads = avg_n <= 128u ? 256u : avg_n <= 256u ? 512u : 768u;        // residents and arrivals in different warps
     if (grid && pp.threads == 256u) pp.threads = 512u;
+    if (avg_n > pp.threads) return false;            // (what a launch gives up goes on with one environment a thread)
     pp.limit = (unsigned)(avg_n * 2u + 256u);
     pp.slots = pp.limit + pp.threads;
     if (pp.slots > 32767u) return false;
@@ -596,7 +596,7 @@ static cudaError_t launch(const Params& p, const StepLaunch& l, const PatchP& pp
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(pp.blocks); cfg.blockDim = dim3(THREADS); cfg.stream = st;
-    cfg.dynamicSmemBytes = std::max<size_t>(pp.shared, l.chunk > THREADS ? (size_t)l.chunk * STATE_BYTES : 0u);
+    cfg.dynamicSmemBytes = pp.shared;
     cudaLaunchAttribute at[1];
     if (GRID) { at[0].id = cudaLaunchAttributeCooperative; at[0].val.cooperative = 1; }
     else {
