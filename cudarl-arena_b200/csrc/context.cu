@@ -364,12 +364,12 @@ size_t stage_bytes(const Params& p) {
 inline size_t up64(size_t b) { return (b + 63) / 64 * 64; }
 
 // After the box has been posted: has any kernel recorded an internal failure (a copy that never landed, a full
-// scratch area, a record outside its tile)?  The word is sticky; the results of the context are not to be trusted.
+// scratch area, a record lost or outside its tile)?  The word is sticky; the results of the context are not to be trusted.
 int check_posted_error(cudarl_ctx* c) {
     const unsigned err = box32(c, 0);
     if (err) return fail(c, CUDARL_ERR_DEVICE + (int)err, "device error bits " + std::to_string(err) +
                          ((err & ERR_COPY_TIMEOUT) ? " (a wait of a kernel ran out)" : "") +
-                         ((err & ERR_SCRATCH_OVERFLOW) ? " (scratch area full)" : "") + ((err & ERR_BAD_STATE) ? " (a record outside its tile or the grid)" : ""));
+                         ((err & ERR_SCRATCH_OVERFLOW) ? " (scratch area full)" : "") + ((err & ERR_BAD_STATE) ? " (a record lost, or outside its tile or the grid)" : ""));
     if (c->comm && g_nccl.CommGetAsyncError) {               // a collective that failed after it was enqueued (a peer that went away)
         ncclResult_t ar = ncclSuccess;
         const ncclResult_t qr = g_nccl.CommGetAsyncError(c->comm, &ar);

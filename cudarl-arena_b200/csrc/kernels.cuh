@@ -98,7 +98,7 @@ struct PatchP {
     unsigned *count, *part, *rank, *cut;    // the counting sort: per bin (zero between launches), per block, per environment; first bin of every patch
     int4* dealt;               // the records sorted by bin
     // grid: words under the number of their step
-    unsigned* barrier;         // a barrier of the grid; from word 64 on, two counters 256 bytes apart; zero between launches
+    unsigned* barrier;         // a barrier of the grid; from word 64 on, two counters 256 bytes apart; word 192, the environments that have come back; zero between launches
     unsigned* listed;          // 3 x blocks: records in a block's list, by step modulo 3; zero before they are for
     unsigned long long *list, *edge;        // 3 x blocks x threads records of two words; 2 x keys: max_a Q of the cells along the patches' edges
 };

@@ -188,6 +188,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
     unsigned step = 0u;
     if (fits) {
         Tally tally{0u, 0u, 0u, 0u, 0u};
+        unsigned kept = 0u;                                        // GRID: records this thread has written back
         EpsilonIndex eps_index(p, l, PLAIN);
         float eps = __ldg(p.eps_tab + eps_index.at);
         auto find = [&](unsigned key) -> unsigned {                // the block a cell belongs to
@@ -267,6 +268,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
             }
         };
         // GRID: the blocks wait for one another at a counter that orders nothing; what was sent is there then or about to be, and is read again until its number is right.
+        // The lists' lengths have no number.  That they are complete rests on the atomics: whoever adds has the answer before its block arrives, so the addition is done, in the one
+        // place where it and the receiver's exchange can be done.  (A fence before the arrival, which would also say so to the memory model, takes 0.25 - 0.45 us a step, by a warp of
+        // its own 0.13 - 1.0.)  An addition that came late all the same would be found by the next to use the list, who would wait for a record in vain, or by the sum at the
+        // end of the launch: either way the error word is set.
         Word* const counter = reinterpret_cast<Word*>(pp.barrier) + 32u;      // two, by the parity of the step; arrivals, from bit 24 on the episodes that ended, from bit 56 on blocks that stop
         auto arrive = [&](unsigned par, Word news) {
             if constexpr (GRID) { if (tid == THREADS - 1u) asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" :: "l"(counter + 32u * par), "l"(1ull + news) : "memory"); }
@@ -340,7 +345,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
                     } else {                                         // no room: everybody stops after this step, and this is where it stands then
                         unsigned x, y; cell_of((s_cut[d] << 3) + rec_loc(now), x, y);
                         p.st[o.id] = make_int4((int)x, (int)y, (int)o.t, (int)o.id);
-                        s_full = 1u;
+                        s_full = 1u; ++kept;
                     }
                     if (!arrival) { rec[j].y = HOLE; left = true; }
                 } else if (!arrival) rec[j] = now;
@@ -399,7 +404,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
                     unsigned long long t0 = 0ull;
                     Word w;
                     for (unsigned it = 1u;; ++it) {
-                        w = look_word(counter + 32u * par);
+                        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(counter + 32u * par) : "memory");
                         if (((unsigned)w & 0xFFFFFFu) >= target) break;
                         if ((it & 1023u) == 0u) {
                             unsigned long long now; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
@@ -412,7 +417,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
                 __syncthreads();
                 news = s_word;
                 if (news == ~0ull) return;
-                if (i == PT_AT_ONCE) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(listed) : "l"(pp.listed + turn * G + b) : "memory");
+                if (i == PT_AT_ONCE) listed = atomicExch(pp.listed + turn * G + b, 0u);      // (nobody adds to it again before this block's next arrival)
                 bool came = act && !resident;                      // this thread's arrival
                 if (came) arr = r;
                 else if (i < PT_AT_ONCE) came = delivered(arr);
@@ -424,10 +429,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
                     if ((unsigned)w == tag) v = (unsigned)(w >> 32); else ok = ok && wait_word(q + (size_t)par * pp.keys, tag, v);
                     ghost[par * pp.ghosts + k] = __uint_as_float(v);
                 }
-                if (i == PT_AT_ONCE) { s_in = listed; }
+                if (i == PT_AT_ONCE) s_in = listed;
                 if (tid == 0u) s_taken = s_holes = 0u;
                 __syncthreads();
-                if (i == PT_AT_ONCE && atomicExch(pp.listed + turn * G + b, 0u) == NOBODY) ok = false;      // (its answer is waited for: it is done before anybody adds for the step after the next but one)
                 arrived = min(s_in, THREADS);
                 if (i >= arrived) arr = make_uint2(0u, HOLE);
                 else if (!came) { unsigned u = 0u, v = HOLE; ok = ok && wait_word(post, tag, u) && wait_word(post + 1, tag, v); arr = make_uint2(u, v); }
@@ -506,10 +510,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
             if (l.eps_mode == 1) { ++eps_index.at; if (step + 1u < l.steps) eps = __ldg(p.eps_tab + eps_index.at); }
         }
         {                                                          // back to environment order
-            auto put = [&](const uint2 r) { unsigned x, y; cell_of(k0 + rec_loc(r), x, y); p.st[rec_id(r)] = make_int4((int)x, (int)y, (int)rec_t(r), (int)rec_id(r)); };
+            auto put = [&](const uint2 r) { unsigned x, y; cell_of(k0 + rec_loc(r), x, y); p.st[rec_id(r)] = make_int4((int)x, (int)y, (int)rec_t(r), (int)rec_id(r)); ++kept; };
 #pragma unroll 1
             for (unsigned j = tid; j < hi; j += THREADS) if (rec[j].y != HOLE) put(rec[j]);
             if (arr.y != HOLE) put(arr);
+        }
+        if constexpr (GRID) {
+            kept = __reduce_add_sync(FULL, kept);
+            if ((tid & 31u) == 0u && kept) atomicAdd(pp.barrier + 192u, kept);
         }
         // the rows back into the table, along its rows
 #pragma unroll 1
@@ -537,7 +545,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
             for (unsigned k = tid; k < n; k += THREADS) { const int4 r = work[first + k]; p.st[r.w] = r; }
         }
     }
-    if (GRID && last_to_finish<false>(p)) { pp.barrier[0] = 0u; pp.barrier[64] = pp.barrier[65] = pp.barrier[128] = pp.barrier[129] = 0u; }
+    if (GRID && last_to_finish<false>(p)) {
+        if (fits && *reinterpret_cast<volatile unsigned*>(pp.barrier + 192u) != p.N) atomicOr(&p.ctl->error, ERR_BAD_STATE);      // not every environment has come back
+        pp.barrier[0] = 0u; pp.barrier[64] = pp.barrier[65] = pp.barrier[128] = pp.barrier[129] = 0u; pp.barrier[192] = 0u;
+    }
 }
 
 // ------------------------------------------------------------------------------------------------

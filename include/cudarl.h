@@ -55,7 +55,7 @@ enum { CUDARL_QINIT_ZERO = 0,           /* src/q_learning.cu:13 */
 /* Failures recorded by kernels (sticky bits, also in cudarl_stats.device_error). */
 #define CUDARL_ERR_DEVICE 3000
 enum { CUDARL_DEVERR_SCRATCH_OVERFLOW = 1, /* a work area was too small for the step */
-       CUDARL_DEVERR_BAD_STATE = 2,        /* a record outside its tile or outside the grid */
+       CUDARL_DEVERR_BAD_STATE = 2,        /* a record outside its tile or outside the grid, or lost */
        CUDARL_DEVERR_CHAIN_CYCLE = 8,      /* update_batch: a collision chain longer than the batch (no kernel follows chains that far any more) */
        CUDARL_DEVERR_COPY_TIMEOUT = 32 };  /* a wait inside a kernel (for a tile copy, for the other blocks of a launch) ran out */
 
