@@ -499,9 +499,10 @@ bool use_gather(const cudarl_ctx* c) {
     return c->p.S <= (1u << 21) || c->p.N <= (1u << 18);
 }
 // What the patch engine works with: made by the first launch of it, which a context that never trains does without (creating one for 65,536 environments on 256 x 256 cells
-// and stepping it once took 2.2 ms, with these 3.1 and more).  The records are sorted into the spare copy of the states.
-int ensure_patch(cudarl_ctx* c) {
-    if (c->dpatch) return 0;
+// and stepping it once took 2.2 ms, with these 3.1 and more).  The records are sorted into the spare copy of the states.  False where the memory cannot be had: the gather
+// engine, which has all it needs, then takes the steps, these and all others of the context.
+bool ensure_patch(cudarl_ctx* c) {
+    if (c->dpatch) return true;
     PatchP& pp = c->patch;
     const size_t N = c->p.N, G = pp.blocks;
     size_t off = 0;
@@ -510,13 +511,19 @@ int ensure_patch(cudarl_ctx* c) {
                  list = take(pp.grid ? 3 * G * pp.threads * 16 : 0), edge = take(pp.grid ? 2 * (size_t)pp.keys * 8 : 0);
     c->patch_zero = off;                                 // zero before the first launch: no step has the number 0
     const size_t part = take(G * 4), cut = take((G + 1) * 4), rank = take(N * 4);
-    CK(cudaMalloc(&c->dpatch, off));
-    CK(cudaMemsetAsync(c->dpatch, 0, c->patch_zero, c->st));
-    unsigned char* const m = (unsigned char*)c->dpatch;
+    void* block = nullptr;
+    if (cudaMalloc(&block, off) != cudaSuccess || cudaMemsetAsync(block, 0, c->patch_zero, c->st) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(block);
+        c->patch = PatchP{};
+        return false;
+    }
+    c->dpatch = block;
+    unsigned char* const m = (unsigned char*)block;
     pp.count = (unsigned*)(m + count); pp.barrier = (unsigned*)(m + barrier); pp.listed = (unsigned*)(m + listed);
     pp.list = (unsigned long long*)(m + list); pp.edge = (unsigned long long*)(m + edge);
     pp.part = (unsigned*)(m + part); pp.cut = (unsigned*)(m + cut); pp.rank = (unsigned*)(m + rank); pp.dealt = c->p.st2;
-    return 0;
+    return true;
 }
 int alloc_gather(cudarl_ctx* c) {
     Params& p = c->p; GatherP& gp = p.gp;
@@ -707,7 +714,7 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         int64_t m = std::min(n - k, most);
         if (c->cfg.sync_every > 0 && c->comm) m = std::min<int64_t>(m, c->cfg.sync_every - c->h_step % c->cfg.sync_every);
         const PatchSteps ps = patch_steps(c->p, c->patch);
-        const bool patches = c->patch.blocks && m >= ps.fewest;
+        const bool patches = c->patch.blocks && m >= ps.fewest && ensure_patch(c);
         if (patches) m = std::min(m, ps.most);
         const unsigned deal = patches ? 0u : c->p.gp.deal_every;
         const bool dealing = deal && (c->dealt < 0 || c->since_deal >= deal);
@@ -720,7 +727,6 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         l.in = c->dealt >= 0 ? (const int4*)c->dwork[c->dealt] : c->p.st;
         l.out = dealing ? (int4*)c->dwork[c->dealt == 0 ? 1 : 0] : const_cast<int4*>(l.in);
         if (patches) {                                       // from wherever the records are to the order of the environments
-            { int rc = ensure_patch(c); if (rc) return rc; }
             if (c->patch_epoch > 0xFFFFFFFFu - 4096u) {      // every number has been used
                 CK(cudaMemsetAsync(c->dpatch, 0, c->patch_zero, c->st));
                 c->patch_epoch = 1;

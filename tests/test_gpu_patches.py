@@ -1,5 +1,6 @@
 """The patch engine of the train step against the oracle: launches of many steps of worlds cut into patches of every shape, and the ways out of it in the
 middle of a launch -- a patch with more environments than slots, more records in a step than the receiver has room for."""
+import ctypes as C
 import os
 
 import numpy as np
@@ -127,3 +128,36 @@ def test_a_failed_wait_ends_the_launch(pkg, n):
     with pytest.raises(pkg.CudarlError) as ei:
         g.synchronize()
     assert ei.value.code == 3000 + 32
+
+
+def test_buffers_that_cannot_be_had(pkg, orc):
+    """The patches' buffers (here 20 MB) are made by the first launch of them: where there is no memory left, the steps run as they do without."""
+    gpu, cpu = pair(pkg, orc, world(pkg, 1000, 900, 20000, eps_kind=pkg.EPS_MULT_PER_STEP, eps0=1.0, eps_decay=0.99), threads=THREADS)
+    gpu.train_steps(20); cpu.train_steps(20)
+    assert_same(gpu, cpu, "before")
+    rt = next(lib for lib in map(_library, ("libcudart.so.12", "libcudart.so", "/usr/local/cuda/lib64/libcudart.so.12")) if lib)
+    held, size = [], 1 << 36
+    while size >= 1 << 23:
+        p = C.c_void_p()
+        if rt.cudaMalloc(C.byref(p), C.c_size_t(size)) == 0:
+            held.append(p)
+        else:
+            size //= 2
+    try:
+        gpu.train_steps(150)
+        gpu.synchronize()
+    finally:
+        rt.cudaGetLastError()
+        for p in held:
+            rt.cudaFree(p)
+    cpu.train_steps(150)
+    gpu.train_steps(150); cpu.train_steps(150)
+    assert_same(gpu, cpu, "after")
+    same_stats(gpu, cpu)
+
+
+def _library(name):
+    try:
+        return C.CDLL(name)
+    except OSError:
+        return None
