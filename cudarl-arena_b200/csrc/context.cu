@@ -108,6 +108,7 @@ struct cudarl_ctx {
     unsigned since_deal = 0;               // steps since then
     void* dwork[2] = {nullptr, nullptr};
     PatchP patch{};                        // patch engine: launches of many steps of those of the gather engine's worlds that it takes
+    bool patch_off = false;                // with the goals as they are, patches are slower
     void* dpatch = nullptr; size_t patch_zero = 0; uint32_t patch_epoch = 1;
     uint32_t barrier_base = 0;             // arrivals at the grid barrier by all launches so far
     bool tile_mode = false;               // true: the records live in tile regions (train steps), false: in environment order
@@ -546,19 +547,20 @@ int alloc_gather(cudarl_ctx* c) {
         for (auto& wk : c->dwork) CK(cudaMalloc(&wk, N * sizeof(int4)));
     }
     if (gp.arena || !p.N || !patch_plan(p, c->patch)) c->patch = PatchP{};
-    // On the whole GPU the block beside a goal is what a step waits for once all paths lead there: as many environments arrive in a step as N / sqrt(cells x goals), but for a factor.
-    // B200, us a step after 20,000 - 40,000 steps, gather engine / patches: 65,536 on 256 x 256 with one goal (256) 6.5 / 7.5, with eight (90) 6.15 / 5.65; 100,000 on 300 x 290 with three (196)
-    // 7.74 / 7.69; 30,000 on 150 x 150 with one (200) 5.7 / 4.3.
-    if (c->patch.grid) {
-        const size_t goals = std::max<size_t>(1, (size_t)std::count(c->cells.begin(), c->cells.end(), (uint8_t)2));
-        if ((double)N * (double)N > 40000.0 * (double)S * (double)goals) c->patch = PatchP{};
-    }
     return 0;
 }
 
-// the move bytes of the engine in use, after a change of the grid
+// On the whole GPU the block beside a goal is what a step waits for once all paths lead there: as many environments arrive in a step as N / sqrt(cells x goals), but for a factor.
+// B200, us a step after 20,000 - 40,000 steps, gather engine / patches: 65,536 on 256 x 256 with one goal (256) 6.5 / 7.5, with eight (90) 6.15 / 5.65; 100,000 on 300 x 290 with three (196)
+// 7.74 / 7.69; 30,000 on 150 x 150 with one (200) 5.7 / 4.3.
+bool too_many_arrivals(const cudarl_ctx* c) {
+    const size_t goals = std::max<size_t>(1, (size_t)std::count(c->cells.begin(), c->cells.end(), (uint8_t)2));
+    return (double)c->p.N * (double)c->p.N > 40000.0 * (double)c->p.S * (double)goals;
+}
+// the move bytes of the engine in use, and whether the world's goals are ones for patches, after a change of the grid
 void refresh_moves(cudarl_ctx* c) {
     if (!c->cls_dirty) return;
+    c->patch_off = c->patch.grid && too_many_arrivals(c);
     if (c->gather) launch_gather_moves(c->p, c->st); else launch_tile_classes(c->p, c->st);
     c->cls_dirty = false;
 }
@@ -714,7 +716,7 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         int64_t m = std::min(n - k, most);
         if (c->cfg.sync_every > 0 && c->comm) m = std::min<int64_t>(m, c->cfg.sync_every - c->h_step % c->cfg.sync_every);
         const PatchSteps ps = patch_steps(c->p, c->patch);
-        const bool patches = c->patch.blocks && m >= ps.fewest && ensure_patch(c);
+        const bool patches = c->patch.blocks && !c->patch_off && m >= ps.fewest && ensure_patch(c);
         if (patches) m = std::min(m, ps.most);
         const unsigned deal = patches ? 0u : c->p.gp.deal_every;
         const bool dealing = deal && (c->dealt < 0 || c->since_deal >= deal);

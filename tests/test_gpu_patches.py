@@ -135,7 +135,7 @@ def test_buffers_that_cannot_be_had(pkg, orc):
     gpu, cpu = pair(pkg, orc, world(pkg, 1000, 900, 20000, eps_kind=pkg.EPS_MULT_PER_STEP, eps0=1.0, eps_decay=0.99), threads=THREADS)
     gpu.train_steps(20); cpu.train_steps(20)
     assert_same(gpu, cpu, "before")
-    rt = next(lib for lib in map(_library, ("libcudart.so.12", "libcudart.so", "/usr/local/cuda/lib64/libcudart.so.12")) if lib)
+    rt = _runtime()
     held, size = [], 1 << 36
     while size >= 1 << 23:
         p = C.c_void_p()
@@ -154,6 +154,33 @@ def test_buffers_that_cannot_be_had(pkg, orc):
     gpu.train_steps(150); cpu.train_steps(150)
     assert_same(gpu, cpu, "after")
     same_stats(gpu, cpu)
+
+
+def makes_buffers(gpu, n):
+    """Whether training n steps makes the patches' buffers, as the first launch of patches does (on the whole GPU more than 4 MB)."""
+    free, total = C.c_size_t(), C.c_size_t()
+    left = []
+    for k in (20, n):
+        gpu.train_steps(k); gpu.synchronize()
+        assert _runtime().cudaMemGetInfo(C.byref(free), C.byref(total)) == 0
+        left.append(free.value)
+    return left[0] - left[1] >= 4 << 20
+
+
+def test_engine_follows_the_goals(pkg, orc):
+    """65,536 environments on 256 x 256 cells take patches with eight goals, not with one; set_goal leaves one."""
+    cfg = world(pkg, 256, 256, 65536, num_goals=8)
+    other = pkg.VecGridWorld(cfg)
+    assert makes_buffers(other, 100) and not makes_buffers(other, 100)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    gpu.set_goal(100, 100)
+    assert not makes_buffers(gpu, 600)
+    cpu.set_goal(100, 100); cpu.train_steps(620)
+    assert_same(gpu, cpu, "one goal")
+
+
+def _runtime():
+    return next(lib for lib in map(_library, ("libcudart.so.12", "libcudart.so", "/usr/local/cuda/lib64/libcudart.so.12")) if lib)
 
 
 def _library(name):
