@@ -702,11 +702,11 @@ int open_kernel_segment(cudarl_ctx* c) {
 }
 
 // A launch of patches takes longer to begin than one of the gather engine: 4,096 environments on 64 x 64 cells (a cluster), 16 steps a call 5.0 us a step without, 4.6 with, 32 a
-// call 4.5 / 3.6; 65,536 on 256 x 256 (the whole GPU), 16 a call 7.1 / 7.2.  The population drifts, so they are cut anew: 30,000 on 150 x 150 with one goal every 1,024 steps
+// call 4.5 / 3.6, but 8,192 on 91 x 91 16 a call 4.6 / 4.75; 65,536 on 256 x 256 (the whole GPU), 16 a call 7.1 / 7.2.  The population drifts, so they are cut anew: 30,000 on 150 x 150 with one goal every 1,024 steps
 // 5.7, every 256 5.0, but 65,536 on 256 x 256 4.30 / 4.39; in a cluster every 256 is 1 - 5 % slower.
 // (The table goes into shared memory and back: 50 environments on 1000 x 900 cells, 32 a call 3.5 / 4.4, 64 3.3 / 3.5, 512 3.1 / 2.7; 5,000 on 900 x 900, 32 a call 4.9 / 4.5.)
 struct PatchSteps { int64_t fewest, most; };
-inline PatchSteps patch_steps(const Params& p, const PatchP& pp) { return pp.grid ? PatchSteps{std::max<int64_t>(32, p.S / 8192u), 512} : PatchSteps{16, 1024}; }
+inline PatchSteps patch_steps(const Params& p, const PatchP& pp) { return pp.grid ? PatchSteps{std::max<int64_t>(32, p.S / 8192u), 512} : PatchSteps{p.N <= 6144u ? 16 : 32, 1024}; }
 // n steps in launches of many: up to the next averaging of the replicas, and not so many that a launch keeps the GPU for long or
 // that a block's 32-bit sums could overflow.
 int run_gather(cudarl_ctx* c, int64_t n) {

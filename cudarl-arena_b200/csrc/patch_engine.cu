@@ -11,7 +11,7 @@
 //   commit    every environment counts itself, and is put back or sent
 //   apply     the first on a (cell, action) applies its update as often as it was counted; edge values out
 //
-// Up to some 10,000 environments the blocks are one cluster and write into one another's shared memory: one barrier of the cluster a step, and no access to L2.
+// Up to 8,192 environments the blocks are one cluster and write into one another's shared memory: one barrier of the cluster a step, and no access to L2.
 //
 // More of them take a patch on every multiprocessor (GRID).  Records and edge values then travel through L2 as 8-byte words that carry the number of the step
 // they are for, and the blocks wait for one another at a counter that orders nothing: when everybody has arrived, what was sent is there or about to be, and
@@ -590,12 +590,16 @@ static bool plan(const Params& p, PatchP& pp, bool grid) {
     return false;
 }
 // Not where episodes start on one cell, and everybody passes through one patch: 12,000 on 200 x 190 cells 3.9 / 5.2 (us a step, gather engine / a cluster here).
-// In a cluster up to one environment a thread, and on crowded grids threads left for the arrivals: 12,000 on 100 x 100 5.2 / 5.3, 10,000 there 5.2 / 4.6.  On the
-// whole GPU up to one a thread: 150,001 on 1001 x 613 5.75 / 5.84 (dealt by cell / here).
+// Not on crowded grids: a patch is eight cells or more, and the one beside the goal has most of the population; how well that goes depends on where it lies.  Us a step, gather engine /
+// patches, 256 or 512 a call, one goal: in a cluster 1,100 on 17 x 17 3.1 / 2.4, on 12 x 12 2.8 / 3.5; 1,500 on 10 x 10 3.0 / 3.8; 4,096 on 32 x 32 3.8 / 2.8, on 16 x 16 4.0 / 4.6; 6,144 on 40 x 40
+// 4.0 / 4.05 (16 a call 4.3 / 5.0); 8,192 on 64 x 64 4.4 / 3.5, on 45 x 45 4.3 / 5.2; on the whole GPU 10,240 on 72 x 72 5.0 / 3.7, 12,288 on 78 x 78 4.8 / 5.2, 10,000 on 50 x 50 4.9 / 5.2.
+// In a cluster up to 512 a block: 10,240 on 101 x 101 5.0 / 5.1, and there on the whole GPU 3.7; 12,288 on 157 x 157 with five goals 5.2 / 5.3 / 3.7.
+// On the whole GPU up to one environment a thread: 150,001 on 1001 x 613 5.75 / 5.84 (dealt by cell / here).
 bool patch_plan(const Params& p, PatchP& pp) {
     const size_t S = p.S, N = p.N;
-    if (p.start_mode == 2) {
-        if ((N <= PT_DENSE_ENVS || (N <= PT_MOST_ENVS && S >= 2 * N)) && plan(p, pp, false)) return true;
+    const bool sparse = N <= (N <= 4096u ? 4u : 2u) * S;
+    if (p.start_mode == 2 && sparse) {
+        if (N <= PT_MOST_ENVS && plan(p, pp, false)) return true;
         if (N <= (size_t)PT_MOST_THREADS * p.sms && plan(p, pp, true)) return true;
     }
     pp = PatchP{};

@@ -40,6 +40,22 @@ def test_worlds_cut_into_patches(pkg, orc, w, h, n):
     same_stats(gpu, cpu)
 
 
+@pytest.mark.parametrize("w,h,n,patches", [
+    (32, 32, 4096, True), (32, 32, 4097, False), (16, 16, 1025, False), (64, 64, 8192, True), (64, 64, 8193, False), (97, 120, 8193, True), (70, 73, 10220, True), (70, 73, 10221, False)])
+def test_crowded_grids_are_not_cut(pkg, orc, w, h, n, patches):
+    """Both sides of the limits of environments a cell, and of the most in a cluster."""
+    gpu, cpu = pair(pkg, orc, world(pkg, w, h, n, max_steps=37), threads=THREADS)
+    if n > 8192:
+        assert makes_buffers(gpu, 40) == patches
+    else:
+        gpu.train_steps(20); gpu.train_steps(40)
+    cpu.train_steps(60)
+    for k in (15, 16, 31, 32, 90):
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert_same(gpu, cpu, "+%d" % k)
+    same_stats(gpu, cpu)
+
+
 @pytest.mark.parametrize("w,h,n", [(91, 93, 3000), (201, 199, 8000), (301, 299, 80000)])
 @pytest.mark.parametrize("kw", [{"eps_kind": 2, "eps0": 1.0, "eps_decay": 0.9}, {"eps_kind": 1, "eps0": 1.0, "eps_decay": 0.99},
                                 {"eps_kind": 3, "eps0": 1.0, "eps_end": 0.1, "eps_steps": 60, "legacy_clamp": 1}])
