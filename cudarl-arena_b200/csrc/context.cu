@@ -109,6 +109,7 @@ struct cudarl_ctx {
     void* dwork[2] = {nullptr, nullptr};
     PatchP patch{};                        // patch engine: launches of many steps of those of the gather engine's worlds that it takes
     bool patch_off = false;                // with the goals as they are, patches are slower
+    uint64_t gave_up = 0; int64_t rest = 0, rest_end = 0;      // PatchP::gave_up as last seen; for how many steps, and until which one, patches have not been tried since
     void* dpatch = nullptr; size_t patch_zero = 0; uint32_t patch_epoch = 1;
     uint32_t barrier_base = 0;             // arrivals at the grid barrier by all launches so far
     bool tile_mode = false;               // true: the records live in tile regions (train steps), false: in environment order
@@ -508,7 +509,7 @@ bool ensure_patch(cudarl_ctx* c) {
     const size_t N = c->p.N, G = pp.blocks;
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t at = off; off += (bytes + 255) / 256 * 256; return at; };
-    const size_t count = take(pp.bins * sizeof(unsigned)), barrier = take(pp.grid ? 1024 : 0), listed = take(pp.grid ? 3 * G * 4 : 0),
+    const size_t count = take(pp.bins * sizeof(unsigned)), broken = take(4), barrier = take(pp.grid ? 1024 : 0), listed = take(pp.grid ? 3 * G * 4 : 0),
                  list = take(pp.grid ? 3 * G * pp.threads * 16 : 0), edge = take(pp.grid ? 2 * (size_t)pp.keys * 8 : 0);
     c->patch_zero = off;                                 // zero before the first launch: no step has the number 0
     const size_t part = take(G * 4), cut = take((G + 1) * 4), rank = take(N * 4);
@@ -524,6 +525,7 @@ bool ensure_patch(cudarl_ctx* c) {
     pp.count = (unsigned*)(m + count); pp.barrier = (unsigned*)(m + barrier); pp.listed = (unsigned*)(m + listed);
     pp.list = (unsigned long long*)(m + list); pp.edge = (unsigned long long*)(m + edge);
     pp.part = (unsigned*)(m + part); pp.cut = (unsigned*)(m + cut); pp.rank = (unsigned*)(m + rank); pp.dealt = c->p.st2;
+    pp.broken = (unsigned*)(m + broken); pp.gave_up = &((HostBox*)c->stage.dev)->gave_up;
     return true;
 }
 int alloc_gather(cudarl_ctx* c) {
@@ -707,6 +709,18 @@ int open_kernel_segment(cudarl_ctx* c) {
 // (The table goes into shared memory and back: 50 environments on 1000 x 900 cells, 32 a call 3.5 / 4.4, 64 3.3 / 3.5, 512 3.1 / 2.7; 5,000 on 900 x 900, 32 a call 4.9 / 4.5.)
 struct PatchSteps { int64_t fewest, most; };
 inline PatchSteps patch_steps(const Params& p, const PatchP& pp) { return pp.grid ? PatchSteps{std::max<int64_t>(32, p.S / 8192u), 512} : PatchSteps{p.N <= 6144u ? 16 : 32, 1024}; }
+// Whether patches are to be left alone for now: since they gave up two launches, for 1,024 steps, and for twice as many (up to 8,192) where they do so again soon after.  The sort and the
+// table cost a short launch a tenth and more: 32 steps a call, all environments drawn to one cell of 200 x 190, gather engine / tried in every launch / now, us a
+// step: 8,000 at lr 0.1 6.6 / 9.0 / 6.6, 3,000 at 1e-5 3.96 / 4.35 / 3.97, 38,000 at 0.1 11.0 / 11.3 / 11.0; 256 steps a call 6.1 / 7.6 / 6.1, 3.5 / 3.6 / 3.5, 10.5 / 10.6 / 10.5.
+// The word is only looked at: a program that does not wait for its steps finds it when the launch has ended.
+bool patches_rest(cudarl_ctx* c) {
+    const uint64_t g = *const_cast<const volatile unsigned long long*>(&c->box->gave_up);
+    if (g != c->gave_up) {
+        c->rest = c->rest && (int64_t)g - 1 < c->rest_end + 1024 ? std::min<int64_t>(2 * c->rest, 8192) : 1024;
+        c->gave_up = g; c->rest_end = c->h_step + c->rest;
+    }
+    return c->h_step < c->rest_end;
+}
 // n steps in launches of many: up to the next averaging of the replicas, and not so many that a launch keeps the GPU for long or
 // that a block's 32-bit sums could overflow.
 int run_gather(cudarl_ctx* c, int64_t n) {
@@ -716,7 +730,7 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         int64_t m = std::min(n - k, most);
         if (c->cfg.sync_every > 0 && c->comm) m = std::min<int64_t>(m, c->cfg.sync_every - c->h_step % c->cfg.sync_every);
         const PatchSteps ps = patch_steps(c->p, c->patch);
-        const bool patches = c->patch.blocks && !c->patch_off && m >= ps.fewest && ensure_patch(c);
+        const bool patches = c->patch.blocks && !c->patch_off && m >= ps.fewest && !patches_rest(c) && ensure_patch(c);
         if (patches) m = std::min(m, ps.most);
         const unsigned deal = patches ? 0u : c->p.gp.deal_every;
         const bool dealing = deal && (c->dealt < 0 || c->since_deal >= deal);
@@ -856,6 +870,7 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
             hostio_retain(); c->retained = true;
             CK(stage_take(&c->stage, stage_bytes(p)));
             c->box = (HostBox*)c->stage.host;
+            c->box->gave_up = 0;
             int r2;
             r2 = alloc_table(c); if (r2) return r2;
             c->gather = use_gather(c);

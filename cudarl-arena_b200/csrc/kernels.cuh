@@ -38,7 +38,7 @@ enum : unsigned { ERR_SCRATCH_OVERFLOW = 1u, ERR_BAD_STATE = 2u, ERR_COPY_TIMEOU
 // the call it belongs to: the host waits for each word it needs by its number, so the words need no order among themselves and no
 // fence (launch to seen result 7.3 us on a B200 machine, 9.3 with values, fence and flag, 9 - 10 for a copy or a synchronisation of
 // the stream).  Word 0 carries Ctl::error and is also the flag behind arrays in the stage, which do take a fence.
-struct HostBox { unsigned long long w[32]; };
+struct HostBox { unsigned long long w[31], gave_up; };           // (gave_up: see PatchP)
 struct Handover { HostBox* box; unsigned ticket; };              // box == nullptr: nothing to hand over
 
 // ---- tile engine (tile_engine.cu): the layout the train step runs on ---------------------------
@@ -97,6 +97,8 @@ struct PatchP {
     unsigned bits, w_rcp;      // cells in the map of start cells (all or none); floor(2^32 / W): umulhi(n, w_rcp) is n / W or one less, for every n < 2^32
     unsigned *count, *part, *rank, *cut;    // the counting sort: per bin (zero between launches), per block, per environment; first bin of every patch
     int4* dealt;               // the records sorted by bin
+    unsigned* broken;          // the number (epoch) of the launch after the last that patches have not seen through its first half
+    volatile unsigned long long* gave_up;   // a word of the box: one more than the first step of the last such launch that came behind another
     // grid: words under the number of their step
     unsigned* barrier;         // a barrier of the grid; from word 64 on, two counters 256 bytes apart; word 192, the environments that have come back; zero between launches
     unsigned* listed;          // 3 x blocks: records in a block's list, by step modulo 3; zero before they are for

@@ -24,7 +24,8 @@
 //
 // What does not fit -- more environments on a patch than its block has slots for, more records in a step than the receiver has room for -- ends
 // the launch's patches with that step, for all blocks at the same one: the records go back to environment order, the rows into the table, and
-// the rest of the steps runs as in the gather engine, which no crowd can overrun.
+// the rest of the steps runs as in the gather engine, which no crowd can overrun.  Two launches in a row that end so in their first half, and the host hears of it and leaves the next
+// steps to the gather engine.
 //
 // What bounds it: the chain of one step, thread by thread some 350 instructions at about 6 cycles each (look, commit, apply, edge values), the longest of them in the
 // block next to a goal, where most arrivals and restarts are (256 x 256 cells, 65,536 environments: 24 cells with 486 environments, 214 arrivals and 204 restarts a
@@ -531,6 +532,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_patch_steps(const __grid_constan
     }
     if constexpr (!GRID) { space.arrive(); space.wait(); }         // (nobody leaves while others may still write into its shared memory)
     if (step < l.steps) {                                          // the same for every block
+        if (b == 0u && tid == 0u && 2u * step < l.steps) {
+            if (*pp.broken == l.epoch) *pp.gave_up = p.step + 1ull;
+            *pp.broken = l.epoch + l.steps + 2u;
+        }
         int4* const work = fits ? p.st : pp.dealt;
         if constexpr (GRID) {
             space.arrive(); if (!space.wait()) return;

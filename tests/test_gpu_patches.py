@@ -96,6 +96,28 @@ def test_crowds_that_no_patch_holds(pkg, orc, n, together):
         same_stats(gpu, cpu)
 
 
+@pytest.mark.parametrize("w,h,n", [(200, 190, 3000), (200, 190, 38000), (400, 390, 90000)])
+@pytest.mark.parametrize("kw", [{}, {"eps_kind": 2, "eps0": 0.2, "eps_decay": 0.9}])
+def test_patches_given_up_are_tried_again_later(pkg, orc, w, h, n, kw):
+    """A crowd that no patch holds for hundreds of steps, in short calls with others of the gather engine between (it deals 90,000 environments by cell); then everybody begins anew."""
+    cfg = world(pkg, w, h, n, num_goals=2, obstacle_p=0.0, obstacle_kind=pkg.OBST_NONE, goal_mode=pkg.GOAL_LIST, goals=[(w - 1, h - 1), (0, h - 1)], **dict(dict(max_steps=150, eps0=0.02, lr=0.05), **kw))
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    rng = np.random.RandomState(n)
+    crowd = np.where(rng.rand(n) < 0.97, 20, rng.randint(0, w, n)).astype(np.int32)
+    for turn in range(3):
+        for m in (gpu, cpu):
+            m.set_state(crowd, np.full(n, 30, np.int32), None)
+        for k in (33, 64, 5, 40):
+            gpu.train_steps(k); cpu.train_steps(k)
+            assert_same(gpu, cpu, "turn %d, +%d" % (turn, k))
+        for m in (gpu, cpu):
+            m.reset_all()
+        for k in (200, 7, 300):
+            gpu.train_steps(k); cpu.train_steps(k)
+            assert_same(gpu, cpu, "turn %d, again, +%d" % (turn, k))
+            same_stats(gpu, cpu)
+
+
 @pytest.mark.parametrize("n", [2500, 10000, 38000])
 def test_many_cross_at_once(pkg, orc, n):
     """All environments of a few cells walk abreast: more records in a step than their receiver has room for."""
