@@ -704,14 +704,15 @@ int open_kernel_segment(cudarl_ctx* c) {
 }
 
 // A launch of patches takes longer to begin than one of the gather engine: 4,096 environments on 64 x 64 cells (a cluster), 16 steps a call 5.0 us a step without, 4.6 with, 32 a
-// call 4.5 / 3.6, but 8,192 on 91 x 91 16 a call 4.6 / 4.75; 65,536 on 256 x 256 (the whole GPU), 16 a call 7.1 / 7.2.  The population drifts, so they are cut anew: 30,000 on 150 x 150 with one goal every 1,024 steps
-// 5.7, every 256 5.0, but 65,536 on 256 x 256 4.30 / 4.39; in a cluster every 256 is 1 - 5 % slower.
+// call 4.5 / 3.6, but 8,192 on 91 x 91 16 a call 4.6 / 4.75; on the whole GPU 30,000 on 150 x 150 32 a call 6.0 / 5.1, 10,240 on 202 x 202
+// 5.7 / 3.9, but 65,536 on 256 x 256 with eight goals, once the population has formed, 32 a call 6.1 / 6.8, 64 6.05 / 6.4, 128 6.0 / 6.2, 512 6.0 / 6.25 (while epsilon is high 6.1 / 4.3 - 5.7).
+// The population drifts, so they are cut anew: 30,000 on 150 x 150 with one goal every 1,024 steps 5.7, every 256 5.0, but 65,536 on 256 x 256 4.30 / 4.39; in a cluster every 256 is 1 - 5 % slower.
 // (The table goes into shared memory and back: 50 environments on 1000 x 900 cells, 32 a call 3.5 / 4.4, 64 3.3 / 3.5, 512 3.1 / 2.7; 5,000 on 900 x 900, 32 a call 4.9 / 4.5.)
 struct PatchSteps { int64_t fewest, most; };
-inline PatchSteps patch_steps(const Params& p, const PatchP& pp) { return pp.grid ? PatchSteps{std::max<int64_t>(32, p.S / 8192u), 512} : PatchSteps{p.N <= 6144u ? 16 : 32, 1024}; }
+inline PatchSteps patch_steps(const Params& p, const PatchP& pp) { return pp.grid ? PatchSteps{std::max<int64_t>(pp.threads > 512u ? 128 : 32, p.S / 8192u), 512} : PatchSteps{p.N <= 6144u ? 16 : 32, 1024}; }
 // Whether patches are to be left alone for now: since they gave up two launches, for 1,024 steps, and for twice as many (up to 8,192) where they do so again soon after.  The sort and the
 // table cost a short launch a tenth and more: 32 steps a call, all environments drawn to one cell of 200 x 190, gather engine / tried in every launch / now, us a
-// step: 8,000 at lr 0.1 6.6 / 9.0 / 6.6, 3,000 at 1e-5 3.96 / 4.35 / 3.97, 38,000 at 0.1 11.0 / 11.3 / 11.0; 256 steps a call 6.1 / 7.6 / 6.1, 3.5 / 3.6 / 3.5, 10.5 / 10.6 / 10.5.
+// step: 8,000 at lr 0.1 6.6 / 9.0 / 6.6, 3,000 at 1e-5 3.96 / 4.35 / 3.97; 256 steps a call 6.1 / 7.6 / 6.1, 3.5 / 3.6 / 3.5.
 // The word is only looked at: a program that does not wait for its steps finds it when the launch has ended.
 bool patches_rest(cudarl_ctx* c) {
     const uint64_t g = *const_cast<const volatile unsigned long long*>(&c->box->gave_up);

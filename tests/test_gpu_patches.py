@@ -32,7 +32,7 @@ def same_stats(gpu, cpu):
 def test_worlds_cut_into_patches(pkg, orc, w, h, n):
     cfg = world(pkg, w, h, n, num_goals=1 if w * h < 100 else 3, obstacle_p=0.0 if w * h < 100 else 0.15, max_steps=37, env_offset=3)
     gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
-    for k in (15, 16, 2, 31, 32, 90):        # one less than the fewest steps of such a launch, the fewest, a launch of the other engine between
+    for k in (15, 16, 2, 31, 32, 90) + ((127, 128) if n > 37888 else ()):        # one less than the fewest steps of such a launch, the fewest, a launch of the other engine between
         gpu.set_trace(k != 90)                       # with and without the options
         gpu.train_steps(k); cpu.train_steps(k)
         assert_same(gpu, cpu, "+%d" % k)
@@ -66,7 +66,7 @@ def test_epsilons_traps_and_clamp(pkg, orc, w, h, n, kw):
     cells = gpu.get_cells()
     for k in np.flatnonzero(cells == 1)[:60]:
         gpu.add_trap(int(k % w), int(k // w), -0.3); cpu.add_trap(int(k % w), int(k // w), -0.3)
-    for k in (16, 1, 33, 47):
+    for k in (16, 1, 33, 47) + ((129, 131) if n > 37888 else ()):
         gpu.train_steps(k); cpu.train_steps(k)
         assert_same(gpu, cpu, "+%d" % k)
         same_stats(gpu, cpu)
@@ -209,7 +209,7 @@ def test_engine_follows_the_goals(pkg, orc):
     """65,536 environments on 256 x 256 cells take patches with eight goals, not with one; set_goal leaves one."""
     cfg = world(pkg, 256, 256, 65536, num_goals=8)
     other = pkg.VecGridWorld(cfg)
-    assert makes_buffers(other, 100) and not makes_buffers(other, 100)
+    assert not makes_buffers(other, 107) and makes_buffers(other, 128) and not makes_buffers(other, 128)
     gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
     gpu.set_goal(100, 100)
     assert not makes_buffers(gpu, 600)
