@@ -18,6 +18,7 @@
 #include <string>
 #include <vector>
 #include <map>
+#include <mutex>
 #include <new>
 
 using namespace cudarl;
@@ -25,6 +26,12 @@ using namespace cudarl;
 namespace {
 
 thread_local std::string g_err;
+
+// What a context's train steps hold of its GPU while they are under way: the multiprocessors of its last launch of them.
+struct Steps { int device = -1; cudaStream_t st = nullptr; std::atomic<unsigned> sms{0}; };
+// Those of all contexts of this process.  (Never destroyed: contexts may be let go after the statics of this file.)
+struct StepsList { std::mutex lock; std::vector<Steps*> all; };
+StepsList& steps_list() { static StepsList* const l = new StepsList; return *l; }
 
 // ---- host Philox4x32-10 for the one-time grid construction ---------------------------------------
 struct HW { uint32_t w[4]; };
@@ -81,6 +88,7 @@ __global__ void k_ctl_eps(Ctl* c, unsigned mode, unsigned len, unsigned long lon
 }  // namespace
 
 struct cudarl_ctx {
+    Steps steps;
     cudarl_config cfg{};
     Params p{};
     cudaStream_t st = nullptr;
@@ -722,6 +730,29 @@ bool patches_rest(cudarl_ctx* c) {
     }
     return c->h_step < c->rest_end;
 }
+// Multiprocessors that train steps of other contexts hold on this one's GPU, or `enough` of them.
+unsigned held_by_others(cudarl_ctx* c, unsigned enough) {
+    StepsList& l = steps_list();
+    std::lock_guard<std::mutex> guard(l.lock);                   // (no context goes while its stream is asked)
+    unsigned held = 0;
+    for (Steps* o : l.all) {
+        unsigned n = o->sms.load(std::memory_order_relaxed);
+        if (!n || o == &c->steps || o->device != c->cfg.device) continue;
+        if (cudaStreamQuery(o->st) == cudaErrorNotReady) { held += n; if (held >= enough) break; }
+        else o->sms.compare_exchange_strong(n, 0u, std::memory_order_relaxed);
+    }
+    return held;
+}
+// Whether there is room for patches beside the train steps of other contexts: a block of patches has a multiprocessor to itself, blocks of the gather engine's clusters share one, and a launch
+// on the whole GPU waits until all others are done.  B200, train_steps(256) of all worlds in turn, us for a step of all, gather engine / patches: 8 / 9 / 16 / 32 worlds of 5,000 on 80 x 80
+// 4.6 / 4.1, 4.6 / 4.9, 5.5 / 7.8, 7.0 / 15; 1, 2, 8, 32 of 3,000 on 350 x 350 (whole GPU) 3.8 / 2.8, 3.8 / 5.5, 4.5 / 22, 7.1 / 89; 1, 2, 4 of 65,536 on 256 x 256 6.4 / 6.0, 7.2 / 11.5, 14.7 / 23.4.
+// (As it is now: 16 and 32 of 5,000 5.5 and 7.1, 2, 8, 32 of 3,000 4.15, 4.7, 7.3, 2 of 65,536 8.1.)  Where the gather engine's blocks, too, get in one another's way, patches stay: 9 / 16 / 32 worlds of
+// 8,192 on 250 x 250 5.5 / 3.8, 7.1 / 6.6, 14.3 / 13.2, on 181 x 181 5.5 / 4.05, 6.8 / 7.1, 13.2 / 14.0, with half of them in each engine 5.6, 9, 22; but on 128 x 128 5.2 / 5.0, 6.4 / 8.1, 12.4 / 16.1.
+bool patches_have_room(cudarl_ctx* c) {
+    if (!c->patch.grid && c->p.N > 6144u && c->p.S >= 3u * c->p.N) return true;
+    const unsigned room = c->patch.grid ? 1u : PT_CLUSTERS * PT_BLOCKS + 1u - c->patch.blocks;
+    return held_by_others(c, room) < room;
+}
 // n steps in launches of many: up to the next averaging of the replicas, and not so many that a launch keeps the GPU for long or
 // that a block's 32-bit sums could overflow.
 int run_gather(cudarl_ctx* c, int64_t n) {
@@ -731,7 +762,7 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         int64_t m = std::min(n - k, most);
         if (c->cfg.sync_every > 0 && c->comm) m = std::min<int64_t>(m, c->cfg.sync_every - c->h_step % c->cfg.sync_every);
         const PatchSteps ps = patch_steps(c->p, c->patch);
-        const bool patches = c->patch.blocks && !c->patch_off && m >= ps.fewest && !patches_rest(c) && ensure_patch(c);
+        const bool patches = c->patch.blocks && !c->patch_off && m >= ps.fewest && !patches_rest(c) && patches_have_room(c) && ensure_patch(c);
         if (patches) m = std::min(m, ps.most);
         const unsigned deal = patches ? 0u : c->p.gp.deal_every;
         const bool dealing = deal && (c->dealt < 0 || c->since_deal >= deal);
@@ -755,6 +786,7 @@ int run_gather(cudarl_ctx* c, int64_t n) {
             CK(c->p.gp.arena ? launch_arena_steps(c->p, l, c->st) : launch_gather_steps(c->p, l, c->st));
             c->barrier_base += c->p.gp.grid * gather_barriers(l);
         }
+        c->steps.sms.store(patches ? c->patch.blocks : std::min(c->p.gp.grid, c->p.sms), std::memory_order_relaxed);
         if (dealing) { c->dealt = c->dealt == 0 ? 1 : 0; c->since_deal = 0; }
         c->since_deal += (unsigned)m;
         c->h_step += m; c->kseg_count += m; k += m;
@@ -766,6 +798,7 @@ int run_gather(cudarl_ctx* c, int64_t n) {
 
 int run_steps(cudarl_ctx* c, int64_t n) {
     if (c->gather) return run_gather(c, n);
+    c->steps.sms.store(c->p.sms, std::memory_order_relaxed);
     { int re = enter_tiles(c); if (re) return re; }
     for (int64_t k = 0; k < n; ++k) {
         if (c->bucket_every > 0 && c->since_bucket >= c->bucket_every) { int rs = rebucket_tiles(c); if (rs) return rs; }
@@ -789,6 +822,11 @@ int run_steps(cudarl_ctx* c, int64_t n) {
 }
 
 void free_all(cudarl_ctx* c) {
+    {
+        StepsList& l = steps_list();
+        std::lock_guard<std::mutex> guard(l.lock);
+        l.all.erase(std::remove(l.all.begin(), l.all.end(), &c->steps), l.all.end());
+    }
     if (c->st) cudaStreamSynchronize(c->st);
     for (size_t r = 0; r < c->peer_tables.size(); ++r) if ((int)r != c->rank && c->peer_tables[r]) cudaIpcCloseMemHandle(c->peer_tables[r]);
     if (c->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->comm);
@@ -858,6 +896,8 @@ int cudarl_create(const cudarl_config* f, cudarl_ctx** out) {
         p.start_cell = sc; p.fallback_start = fb;
         auto body = [&]() -> int {
             CK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
+            c->steps.device = f->device; c->steps.st = c->st;
+            { StepsList& l = steps_list(); std::lock_guard<std::mutex> guard(l.lock); l.all.push_back(&c->steps); }
             CK(cudaEventCreateWithFlags(&c->ev_eps, cudaEventDisableTiming));
             CK(cudaEventCreate(&c->ev0)); CK(cudaEventCreate(&c->ev1));
             { int sms = 0; CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device)); p.sms = (unsigned)std::max(sms, 1); }

@@ -87,7 +87,7 @@ struct GatherP {
     unsigned cluster, arena;                // all blocks in one cluster; the world in the shared memory of one block
 };
 // ---- patch engine (patch_engine.cu): the world in the shared memory of several blocks, for launches of many steps ----
-constexpr unsigned PT_MOST_THREADS = 768u, PT_BLOCKS = 16u, PT_MOST_BLOCKS = 256u, PT_MOST_ENVS = 8192u, PT_BIN_WEIGHT = 128u;      // 16 for each of a bin's cells
+constexpr unsigned PT_MOST_THREADS = 768u, PT_BLOCKS = 16u, PT_MOST_BLOCKS = 256u, PT_MOST_ENVS = 8192u, PT_CLUSTERS = 8u, PT_BIN_WEIGHT = 128u;      // 16 for each of a bin's cells
 struct PatchP {
     unsigned blocks, threads;  // 0 blocks: the world does not fit
     bool grid;                 // on all multiprocessors instead of in a cluster

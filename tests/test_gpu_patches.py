@@ -2,6 +2,7 @@
 middle of a launch -- a patch with more environments than slots, more records in a step than the receiver has room for."""
 import ctypes as C
 import os
+import threading
 
 import numpy as np
 import pytest
@@ -215,6 +216,45 @@ def test_engine_follows_the_goals(pkg, orc):
     assert not makes_buffers(gpu, 600)
     cpu.set_goal(100, 100); cpu.train_steps(620)
     assert_same(gpu, cpu, "one goal")
+
+
+def test_room_beside_other_worlds(pkg, orc):
+    """A launch on the whole GPU would wait for the steps of another context, and its steps for the launch: while they are under way, the gather engine takes them."""
+    other = pkg.VecGridWorld(world(pkg, 120, 97, 5000))
+    other.train_steps(64); other.synchronize()
+    gpu, cpu = pair(pkg, orc, world(pkg, 350, 350, 3000), threads=THREADS)
+    other.train_steps(150000)                            # some 0.4 s
+    assert not makes_buffers(gpu, 200)
+    other.synchronize()
+    assert makes_buffers(gpu, 200)
+    cpu.train_steps(440)
+    assert_same(gpu, cpu, "beside another")
+    same_stats(gpu, cpu)
+
+
+def test_many_worlds_at_once(pkg, orc):
+    """More worlds than there is room for as clusters, each trained by a thread of its own, some on the whole GPU, some let go while others train."""
+    sizes = [(50, 50, 1500), (64, 64, 4096), (350, 350, 3000), (20, 20, 200)] * 3
+    wrong = []
+
+    def one(k, w, h, n):
+        try:
+            for again in range(2):
+                cfg = world(pkg, w, h, n, seed=k + 100 * again)
+                gpu, cpu = pair(pkg, orc, cfg)
+                for m in (64, 33, 200, 16):
+                    gpu.train_steps(m); cpu.train_steps(m)
+                gpu.train_steps(40); cpu.train_steps(40)
+                assert_same(gpu, cpu, "world %d" % k)
+                gpu.close()
+        except Exception as e:
+            wrong.append(e)
+    threads = [threading.Thread(target=one, args=(k,) + s) for k, s in enumerate(sizes)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
 
 
 def _runtime():
