@@ -21,19 +21,19 @@ def same_stats(gpu, cpu):
 
 @pytest.mark.parametrize("w,h,n", [
     (40, 30, 1100), (64, 64, 4096), (120, 97, 1025),
-    (97, 120, 2048), (97, 120, 2049), (97, 120, 4097), (97, 120, 10240), (97, 120, 10241),       # both sides of 256 and 512 threads; the most environments
-    (160, 161, 12288), (160, 161, 12289),            # on crowded and on other grids, and one more
+    (97, 120, 2048), (97, 120, 2049), (97, 120, 4096), (97, 120, 4097), (97, 120, 8192), (97, 120, 8193), (97, 120, 10240), (97, 120, 10241),       # both sides of 256 and 512 threads; the most environments
+    (160, 161, 12288), (160, 161, 12289),
     (5000, 1, 33), (1, 5000, 1025), (7, 3000, 6000), (3000, 9, 6000),        # one cell wide, one high: most of a band is empty
     (3, 2, 5000), (2, 1, 1500),  # fewer bins of cells than blocks: patches without a cell
     (340, 330, 1500),            # the map of start cells does not fit
     # on all multiprocessors: both sides of 512 threads, the most environments, the most for three goals; a large grid; one that does not fit
     (420, 400, 1500), (9000, 3, 20000), (130, 110, 37888), (256, 256, 37889), (256, 256, 65536), (400, 300, 113664), (400, 300, 113665), (256, 256, 88680), (256, 256, 88682),
-    (1001, 613, 70001), (1300, 1100, 2000),
+    (1001, 613, 70001), (1300, 1100, 2000), (1000, 900, 20000), (1180, 1050, 3000),      # the last but two does not fit, the last nearly fills the shared memory
 ])
 def test_worlds_cut_into_patches(pkg, orc, w, h, n):
     cfg = world(pkg, w, h, n, num_goals=1 if w * h < 100 else 3, obstacle_p=0.0 if w * h < 100 else 0.15, max_steps=37, env_offset=3)
     gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
-    for k in (15, 16, 2, 31, 32, 90) + ((127, 128) if n > 37888 else ()):        # one less than the fewest steps of such a launch, the fewest, a launch of the other engine between
+    for k in (15, 16, 2, 31, 32, 90) + ((127, 128) if n > 37888 else ()) + ((w * h // 8192 + 1,) if w * h > 1 << 18 else ()):        # one less than the fewest steps of such a launch, the fewest, a launch of the other engine between
         gpu.set_trace(k != 90)                       # with and without the options
         gpu.train_steps(k); cpu.train_steps(k)
         assert_same(gpu, cpu, "+%d" % k)
@@ -133,6 +133,103 @@ def test_many_cross_at_once(pkg, orc, n):
         gpu.train_steps(k); cpu.train_steps(k)
         assert_same(gpu, cpu, "+%d" % k)
     same_stats(gpu, cpu)
+
+
+@pytest.mark.parametrize("w,h,n,rows,each", [(400, 400, 16000, 32, 400), (200, 190, 2500, 64, 250)])
+def test_a_column_walks_abreast(pkg, orc, w, h, n, rows, each):
+    """`each` environments on every eight cells of a column, few enough for the patches there, all of which step into the wide patch beside them at once: more than its list
+    of arrivals holds -- on the whole GPU, and in a cluster."""
+    cfg = world(pkg, w, h, n, num_goals=1, obstacle_p=0.0, obstacle_kind=pkg.OBST_NONE, goal_mode=pkg.GOAL_LIST, goals=[(w - 1, h - 1)], max_steps=0, eps0=0.0, lr=0.001)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    rng = np.random.RandomState(n)
+    q = np.zeros((h, w, 4), np.float32); q[..., 1] = 1000.0
+    m = each * rows // 8
+    for at in (5, 40):
+        x, y = rng.randint(at + 1, w, n).astype(np.int32), rng.randint(0, h, n).astype(np.int32)
+        x[:m] = at; y[:m] = np.arange(m) % rows
+        for k in (gpu, cpu):
+            k.set_q(q); k.set_state(x, y, np.zeros(n, np.int32))
+        for k in (64, 100):
+            gpu.train_steps(k); cpu.train_steps(k)
+            assert_same(gpu, cpu, "+%d" % k)
+    same_stats(gpu, cpu)
+
+
+def counted_crowds(cpu, w, steps):
+    """Trains the oracle; (cell, step) pairs with more than 24 environments, and the environments on them."""
+    cells = chained = 0
+    for _ in range(steps):
+        x, y, _t = cpu.get_state()
+        c = np.bincount(y * w + x)
+        cells += int((c > 24).sum()); chained += int(c[c > 24].sum())
+        cpu.train_steps(1)
+    return cells, chained
+
+
+@pytest.mark.parametrize("w,h,n,k", [(60, 60, 1500, 40), (60, 60, 3000, 40), (80, 80, 8000, 40), (120, 120, 20000, 64), (300, 290, 40000, 140)])
+@pytest.mark.parametrize("together", [False, True])
+def test_crowded_cells_of_patches(pkg, orc, w, h, n, k, together):
+    """Cells with more than 24 environments, in patches to the end and in patches that are given up when the rows have led everybody to one place."""
+    cfg = world(pkg, w, h, n, num_goals=2, obstacle_p=0.0, obstacle_kind=pkg.OBST_NONE, goal_mode=pkg.GOAL_LIST, goals=[(w - 1, h - 1), (0, h - 1)], max_steps=200, eps0=0.05)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    rng = np.random.RandomState(n)
+    x, y = rng.randint(0, w, n).astype(np.int32), rng.randint(0, h, n).astype(np.int32)
+    crowd = rng.randint(0, 2 * n, n)                     # eight cells with a fortieth of the population each, or some 375
+    m = (crowd < 100 * min(n // 100, 150)) & (crowd % 100 < 40)
+    x[m], y[m] = (crowd[m] % 4) * (w // 4), (crowd[m] // 4 % 2) * (h // 2)
+    if together:
+        my, mx = np.mgrid[0:h, 0:w]
+        q = np.zeros((h, w, 4), np.float32); cx, cy = w // 2, h // 2
+        q[..., 1] = mx < cx; q[..., 3] = mx > cx; q[..., 2] = (mx == cx) & (my < cy); q[..., 0] = (mx == cx) & (my >= cy)
+        gpu.set_q(q); cpu.set_q(q)
+    for v in (gpu, cpu):
+        v.set_state(x, y, None)
+    cells = chained = 0
+    for steps in (k, 2 * k):
+        more = counted_crowds(cpu, w, steps)
+        gpu.train_steps(steps)
+        cells += more[0]; chained += more[1]
+        s = gpu.get_stats()
+        assert (s.long_chains, s.chained) == (cells, chained)
+        assert_same(gpu, cpu, "+%d" % steps)
+    assert cells > 0
+    same_stats(gpu, cpu)
+
+
+@pytest.mark.parametrize("n", [3000, 8000, 20000, 38000])
+@pytest.mark.parametrize("kw", [{"eps_kind": 1, "eps0": 0.3, "eps_decay": 0.98}, {"eps_kind": 2, "eps0": 0.3, "eps_decay": 0.9}, {"eps_kind": 3, "eps0": 0.3, "eps_end": 0.02, "eps_steps": 150, "legacy_clamp": 1}])
+def test_patches_given_up_with_options(pkg, orc, n, kw):
+    """Patches that a crowd ends in the middle of a launch: the epsilon goes on where it was, by step and by the episodes of all blocks, with traps, a trace and the clamp."""
+    w, h = 200, 190
+    cfg = world(pkg, w, h, n, num_goals=2, obstacle_p=0.02, goal_mode=pkg.GOAL_LIST, goals=[(100, 94), (199, 189)], max_steps=70, lr=0.05, **kw)
+    gpu, cpu = pair(pkg, orc, cfg, threads=THREADS)
+    for c in np.flatnonzero(gpu.get_cells() == 1)[:200]:
+        gpu.add_trap(int(c % w), int(c // w), -0.3); cpu.add_trap(int(c % w), int(c // w), -0.3)
+    y, x = np.mgrid[0:h, 0:w]
+    q = np.zeros((h, w, 4), np.float32)
+    q[..., 1] = x < 100; q[..., 3] = x > 100; q[..., 2] = (x == 100) & (y < 94); q[..., 0] = (x == 100) & (y > 94)
+    gpu.set_q(q); cpu.set_q(q)
+    gpu.set_trace(True)
+    for k in (130, 33, 200):
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert_same(gpu, cpu, "+%d" % k)
+        assert all(np.array_equal(a, b) for a, b in zip(gpu.get_trace(), cpu.get_trace()))
+        same_stats(gpu, cpu)
+
+
+@pytest.mark.parametrize("w,h,n", [(9, 8, 20), (20, 19, 300), (32, 32, 1000), (64, 64, 1500), (64, 64, 4096), (90, 93, 8000), (120, 120, 20000), (300, 290, 40000)])
+@pytest.mark.parametrize("seed", range(2))
+def test_rows_with_ties_infinities_and_no_numbers(pkg, orc, w, h, n, seed):
+    """In worlds of one block, in clusters and on the whole GPU: rows, edge values and counted updates."""
+    rng = np.random.RandomState(seed)
+    gpu, cpu = pair(pkg, orc, world(pkg, w, h, n, num_goals=1 if n < 38000 else 8, obstacle_p=0.1, max_steps=13, eps0=0.2, lr=0.5, legacy_clamp=seed), threads=THREADS)
+    q = rng.choice(np.array([0.0, -0.0, 1.0, -1.0, np.inf, -np.inf, np.nan, np.nan, -3.4e38, 1e-42], np.float32), (h, w, 4))
+    gpu.set_q(q); cpu.set_q(q)
+    for k in (1, 40, 130):
+        gpu.train_steps(k); cpu.train_steps(k)
+        assert all(np.array_equal(a, b) for a, b in zip(gpu.get_state(), cpu.get_state())), "+%d" % k
+        assert np.array_equal(gpu.get_q(), cpu.get_q(), equal_nan=True), "+%d" % k
+        same_stats(gpu, cpu)
 
 
 @pytest.mark.parametrize("n", [9000, 30000])
