@@ -763,7 +763,7 @@ int run_gather(cudarl_ctx* c, int64_t n) {
         if (c->cfg.sync_every > 0 && c->comm) m = std::min<int64_t>(m, c->cfg.sync_every - c->h_step % c->cfg.sync_every);
         const PatchSteps ps = patch_steps(c->p, c->patch);
         const bool patches = c->patch.blocks && !c->patch_off && m >= ps.fewest && !patches_rest(c) && patches_have_room(c) && ensure_patch(c);
-        if (patches) m = std::min(m, ps.most);
+        if (patches) { const int64_t parts = (m + ps.most - 1) / ps.most; m = (m + parts - 1) / parts; }        // of one size: 600 steps as 512 + 88 would leave 88 to the gather engine
         const unsigned deal = patches ? 0u : c->p.gp.deal_every;
         const bool dealing = deal && (c->dealt < 0 || c->since_deal >= deal);
         if (deal) m = std::min<int64_t>(m, dealing ? deal : deal - c->since_deal);
