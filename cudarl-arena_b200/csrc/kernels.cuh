@@ -97,7 +97,7 @@ struct PatchP {
     unsigned bits, w_rcp;      // cells in the map of start cells (all or none); floor(2^32 / W): umulhi(n, w_rcp) is n / W or one less, for every n < 2^32
     unsigned *count, *part, *rank, *cut;    // the counting sort: per bin (zero between launches), per block, per environment; first bin of every patch
     int4* dealt;               // the records sorted by bin
-    unsigned* broken;          // the number (epoch) of the launch after the last that patches have not seen through its first half
+    unsigned* broken;          // the number (epoch) of the launch after the last that patches have not seen through its first eighth
     volatile unsigned long long* gave_up;   // a word of the box: one more than the first step of the last such launch that came behind another
     // grid: words under the number of their step
     unsigned* barrier;         // a barrier of the grid; from word 64 on, two counters 256 bytes apart; word 192, the environments that have come back; zero between launches
