@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(HELP ? 2u * WALK : WALK, 1) k_arena_steps(cons
     add_tallies(p, l, tally, s_sum, true, eps);
 }
 
-// 2 to 32 environments on grids of more than 6,676 cells: one warp steps them, without counters or a barrier in the step -- who stands on the same (cell, action) is found
+// 2 to 32 environments on grids of more than 6,676 cells, and on others in launches of few steps: one warp steps them, without counters or a barrier in the step -- who stands on the same (cell, action) is found
 // with a match across the warp, and the lowest of them applies the update for all.  A second warp makes the random draws, which depend
 // on nothing, a chunk of steps ahead.  SHARED: the world in shared memory; else in global memory, where the rows the warp walks over stay in
 // its first-level cache.
@@ -343,8 +343,11 @@ bool arena_plan(Params& p) {
 }
 cudaError_t launch_arena_steps(const Params& p, const StepLaunch& l, cudaStream_t st) {
     const bool pl = plain(p, l);
-    if (p.N == 1u || (p.N <= 32u && Arena<32u, true>::bytes(p.S) > Arena<32u, true>::MOST)) {
-        const bool fits = solo_bytes(p.S) <= SOLO_MOST, options = p.ntraps || p.legacy_clamp || l.trace;
+    // Up to 32 environments walk over few cells in few steps: not worth fetching the world into shared memory.  Us a step, 1 / 2 / 4 / 8 / 16 steps a call, fetched / not: 32 environments on 40 x 40
+    // 7.0 / 6.2, 4.1 / 3.65, 2.1 / 2.6 ..; 60 x 60 10.3 / 6.2, 5.1 / 3.6, 2.6 / 2.6, 1.6 / 1.9 ..; 80 x 83 13.6 / 6.2, 7.2 / 3.5, 3.65 / 2.6, 2.1 / 1.9, 1.3 / 1.65; 110 x 110 (in one warp) 14.6 / 6.2 .. 1.8 / 1.65.
+    const bool few = p.N > 1u && p.N <= 32u && l.steps * 800ull <= p.S;
+    if (p.N == 1u || few || (p.N <= 32u && Arena<32u, true>::bytes(p.S) > Arena<32u, true>::MOST)) {
+        const bool fits = !few && solo_bytes(p.S) <= SOLO_MOST, options = p.ntraps || p.legacy_clamp || l.trace;
         auto* const fn = p.N == 1u ? fits ? options ? k_one_steps<true, true> : k_one_steps<true, false> : options ? k_one_steps<false, true> : k_one_steps<false, false>
                                    : fits ? pl ? k_solo_steps<true, true> : k_solo_steps<true, false> : pl ? k_solo_steps<false, true> : k_solo_steps<false, false>;
         if (fits) { const cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLO_MOST); if (e != cudaSuccess) return e; }

@@ -116,6 +116,7 @@ struct cudarl_ctx {
     unsigned since_deal = 0;               // steps since then
     void* dwork[2] = {nullptr, nullptr};
     PatchP patch{};                        // patch engine: launches of many steps of those of the gather engine's worlds that it takes
+    GatherP single{};                      // one block's worlds whose launches of one step a cluster takes; grid 0: none
     bool patch_off = false;                // with the goals as they are, patches are slower
     uint64_t gave_up = 0; int64_t rest = 0, rest_end = 0;      // PatchP::gave_up as last seen; for how many steps, and until which one, patches have not been tried since
     void* dpatch = nullptr; size_t patch_zero = 0; uint32_t patch_epoch = 1;
@@ -541,11 +542,18 @@ int alloc_gather(cudarl_ctx* c) {
     const size_t S = p.S, N = p.N ? p.N : 1;
     CK(cudaMalloc(&c->dgbar, 256)); CK(cudaMemsetAsync(c->dgbar, 0, 256, c->st));
     CK(cudaMalloc(&c->dgmv, S));
-    if (!arena_plan(p)) {
-        gp = GatherP{}; gather_plan(p);
+    const bool arena = arena_plan(p);
+    // One block fetches a world of 5,000 to 7,000 cells longer than a step takes: calls of one step go to a cluster (40 environments on 80 x 80 cells 10.3 us fetched, 7.5 there, 1,000 on 83 x 83
+    // 10.3 / 8.2, on 67 x 67 8.2 / 8.2; two steps a call 5.1 / 5.2 and 5.9 / 6.2 a step).
+    const bool single = arena && N > 32 && S > 4722;
+    if (!arena || single) {
+        Params q = p;
+        q.gp = GatherP{}; gather_plan(q);
         // 32 bytes a cell, twice the table: only for the launches that count in global memory, not for one block's worlds (or none)
         CK(cudaMalloc(&c->dgcnt, 8 * S * sizeof(unsigned))); CK(cudaMemsetAsync(c->dgcnt, 0, 8 * S * sizeof(unsigned), c->st));
-        gp.cnt[0] = (unsigned*)c->dgcnt; gp.cnt[1] = gp.cnt[0] + 4 * S;
+        q.gp.cnt[0] = (unsigned*)c->dgcnt; q.gp.cnt[1] = q.gp.cnt[0] + 4 * S;
+        q.gp.barrier = (unsigned*)c->dgbar; q.gp.mv = (unsigned char*)c->dgmv;
+        (single ? c->single : gp) = q.gp;
     }
     gp.barrier = (unsigned*)c->dgbar;
     gp.mv = (unsigned char*)c->dgmv;
@@ -782,6 +790,10 @@ int run_gather(cudarl_ctx* c, int64_t n) {
             l.chunk = (c->p.N + c->patch.blocks - 1u) / c->patch.blocks; l.epoch = c->patch_epoch;
             CK(launch_patch_steps(c->p, l, c->patch, c->st));
             c->patch_epoch += (uint32_t)m + 2u; c->dealt = -1;
+        } else if (m == 1 && c->single.grid) {
+            Params q = c->p;
+            q.gp = c->single; l.chunk = q.gp.chunk;
+            CK(launch_gather_steps(q, l, c->st));
         } else {
             CK(c->p.gp.arena ? launch_arena_steps(c->p, l, c->st) : launch_gather_steps(c->p, l, c->st));
             c->barrier_base += c->p.gp.grid * gather_barriers(l);
