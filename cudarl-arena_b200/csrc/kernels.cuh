@@ -7,7 +7,7 @@
 
 namespace cudarl {
 
-// ---- per-cell word (16 bits per grid cell, array padded to 16 bytes): the cell's class ------------
+// ---- per-cell word (16 bits per grid cell, array padded to 256 bytes): the cell's class ------------
 enum : unsigned {
     CW_OBST = 1u,      // cell blocks movement                     (src/kernels.cu:29-36 of the reference)
     CW_GOAL = 2u,      // cell ends the episode, reward 1          (src/environment.cu:43-46)
@@ -126,7 +126,7 @@ struct World {
     float lr, gamma;
     int legacy_clamp;
     float4* Q;             // the table: S float4, row s = the 4 action values of cell s; every kernel updates it in place
-    unsigned short* cw;    // S cell words (padded to 16 bytes)
+    unsigned short* cw;    // S cell words (padded to 256 bytes: map_closed of step_loop.cuh reads 64 at a time)
     const uint2* traps;    // sparse trap table, ascending by cell: {cell, penalty as float bits}
     unsigned ntraps;
     // environment state outside train steps: one int4 {x, y, t, id} per environment (all int32, one

@@ -32,9 +32,9 @@
 // step, half of all blocks have 35 and none).  Hence one environment a thread in straight code, a loop only for what is left over (4,096 on 64 x 64 with
 // everything in one loop 3.1 us, now 2.7; 1,024 threads, whose 64 registers spill, 8,192 on 100 x 100 5.3, 768 take 3.4), residents and arrivals in
 // different warps, an arrival looked at as soon as it is there, and atomics whose answer nobody waits for.  B200, us a step, gather engine / here, with trained
-// tables: in a cluster 600 environments on 32 x 150 cells 3.7 / 1.8, 1,500 on 80 x 80 3.9 / 2.1, 4,096 on 64 x 64 4.0 / 2.7, 8,192 on 100 x 100 4.5 / 3.4 and on 250 x 250
-// 4.9 / 3.0, 12,000 on 200 x 200 5.7 / 4.1; on the whole GPU 3,000 on 350 x 350 3.8 / 2.8, 16,000 on 300 x 300 6.0 / 3.1, 20,000 on 1000 x 900 5.5 / 3.2, 30,000 on
-// 150 x 150 6.3 / 5.4, 65,536 on 256 x 256 6.1 / 4.3, 100,000 on 300 x 290 7.1 / 5.3.
+// tables: in a cluster 1,500 environments on 80 x 80 cells 3.9 / 2.1, 4,096 on 64 x 64 4.0 / 2.7, 8,192 on 91 x 91 4.3 / 3.4 and on 250 x 250 4.6 / 2.9; on the whole GPU 3,000 on
+// 350 x 350 3.8 / 2.6, 10,240 on 202 x 202 5.4 / 3.3, 16,000 on 300 x 300 6.1 / 3.1, 30,000 on 150 x 150 5.9 / 4.3, 100,000 on 300 x 290 7.6 / 7.0, 65,536 on 256 x 256 with eight goals 6.1 / 4.3 after
+// 12,000 steps of a falling epsilon and 5.1 after 40,000, but 6.0 / 6.2 with epsilon 0.1 from the beginning, when all paths lead to the goals.
 //
 // Reference semantics: those of tile_engine.cu.
 #include "global_table.cuh"
@@ -599,7 +599,7 @@ static bool plan(const Params& p, PatchP& pp, bool grid) {
 // patches, 256 or 512 a call, one goal: in a cluster 1,100 on 17 x 17 3.1 / 2.4, on 12 x 12 2.8 / 3.5; 1,500 on 10 x 10 3.0 / 3.8; 4,096 on 32 x 32 3.8 / 2.8, on 16 x 16 4.0 / 4.6; 6,144 on 40 x 40
 // 4.0 / 4.05 (16 a call 4.3 / 5.0); 8,192 on 64 x 64 4.4 / 3.5, on 45 x 45 4.3 / 5.2; on the whole GPU 10,240 on 72 x 72 5.0 / 3.7, 12,288 on 78 x 78 4.8 / 5.2, 10,000 on 50 x 50 4.9 / 5.2.
 // In a cluster up to 512 a block: 10,240 on 101 x 101 5.0 / 5.1, and there on the whole GPU 3.7; 12,288 on 157 x 157 with five goals 5.2 / 5.3 / 3.7.
-// On the whole GPU up to one environment a thread: 150,001 on 1001 x 613 5.75 / 5.84 (dealt by cell / here).
+// On the whole GPU up to one environment a thread.
 bool patch_plan(const Params& p, PatchP& pp) {
     const size_t S = p.S, N = p.N;
     const bool sparse = N <= (N <= 4096u ? 4u : 2u) * S;

@@ -1,5 +1,6 @@
-"""The patch engine of the train step against the oracle: launches of many steps of worlds cut into patches of every shape, and the ways out of it in the
-middle of a launch -- a patch with more environments than slots, more records in a step than the receiver has room for."""
+"""The patch engine of the train step against the oracle: launches of many steps of worlds cut into patches of every shape, the ways out of it in the
+middle of a launch -- a patch with more environments than slots, more records in a step than the receiver has room for -- and when it is not taken: crowded grids, few
+goals, other contexts' steps under way, no memory."""
 import ctypes as C
 import os
 import threading
